@@ -158,9 +158,63 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
     return d;
 }
 
+// One 32 x 32 chunk of f32 output out of a warp's swizzled slice into C, VEC elements per access: 32 / VEC lanes
+// cover a row's 128 bytes, so an instruction touches VEC whole row segments.  With one lane per row (each lane
+// walking its own row) the alpha/beta form cost 32 sectors per 4-byte access: 1000 x 3001 x 1111 took 98.8 us, 22.5 so.
+// For alpha/beta the old values of a whole batch of rows are fetched before the first is used.
+template <int VEC>
+__device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, const uint8_t *slice,
+                                            uint32_t lane, const GemmParams &p) {
+    constexpr uint32_t kLanes = 32 / VEC;        // lanes per row
+    constexpr uint32_t kBatch = VEC == 4 ? 8 : 16;
+    const uint32_t sub = lane / kLanes, c = (lane % kLanes) * VEC;
+    const bool update = p.epilogue == EPI_ALPHA_BETA;
+#pragma unroll 1
+    for (uint32_t b = 0; b < 32; b += kBatch * VEC) {
+        float old[kBatch][VEC];
+        if (update) {
+#pragma unroll
+            for (uint32_t i = 0; i < kBatch; ++i) {
+                const uint32_t rr = b + i * VEC + sub;
+                const float *src = chunk + (uint64_t)rr * ldc + c;
+                if (rr < rows && c < cols) {
+                    if constexpr (VEC == 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(src);
+                        old[i][0] = v.x; old[i][1] = v.y; old[i][2] = v.z; old[i][3] = v.w;
+                    } else {
+                        old[i][0] = *src;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i) {
+            const uint32_t rr = b + i * VEC + sub;
+            if (rr < rows && c < cols) {
+                const uint8_t *at = slice + rr * 128 + (((c >> 2) ^ (rr & 7)) * 16) + (c & 3) * 4;
+                float v[VEC];
+                if constexpr (VEC == 4) {
+                    const float4 x = *reinterpret_cast<const float4 *>(at);
+                    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+                } else {
+                    v[0] = *reinterpret_cast<const float *>(at);
+                }
+                if (update) {
+#pragma unroll
+                    for (int q = 0; q < VEC; ++q) v[q] = __fadd_rn(__fmul_rn(p.alpha, v[q]), __fmul_rn(p.beta, old[i][q]));
+                }
+                float *dst = chunk + (uint64_t)rr * ldc + c;
+                if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+                else *dst = v[0];
+            }
+        }
+    }
+}
+
 // REGS = 168 is what the block's 320 threads can have; REGS = 128 (still no spills) is for the GEMM that runs
 // beside the expert-parallel dispatch kernel: registers are handed out to four warps at a time, so the ten
-// warps count as twelve, and 12 x 32 x 128 leaves room for one block of that kernel on the same SM.
+// warps count as twelve, and 12 x 32 x 128 leaves room for one block of that kernel on the same SM.  It and the
+// build with loader warps (a gathered A) run the first GEMM of an expert FFN only, so REGS = 128 has no f32 output.
 template <int BN, int REGS>
 __global__ void __maxnreg__(REGS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -522,8 +576,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-            } else {
-                // ---- f32 output: one chunk (32 columns) per 128-byte group
+            } else if constexpr (REGS > 128) {
+                // ---- f32 output: one chunk (32 columns) per 128-byte group (the 128-register build has bf16 output only)
 #pragma unroll 1
                 for (int g = 0; g < kChunks; ++g) {
                     uint32_t r[32];
@@ -581,23 +635,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             tma_store_commit();
                         }
                         store_pending = true;
-                    } else if (row_ok) {
-                        float *dst = reinterpret_cast<float *>(p.c) + (uint64_t)row * p.ldc + col;
-                        const bool vec = col + 32 <= p.N && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
-                        if (p.epilogue == EPI_ALPHA_BETA) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col + j < p.N)
-                                    dst[j] = __fadd_rn(__fmul_rn(p.alpha, __uint_as_float(r[j])), __fmul_rn(p.beta, dst[j]));
-                        } else if (vec) {
-#pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                reinterpret_cast<uint4 *>(dst)[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col + j < p.N) dst[j] = __uint_as_float(r[j]);
+                    } else {
+                        // Rows the copy engine cannot take (a ragged group's last rows, C it cannot address, the
+                        // alpha/beta form): the chunk goes through the warp's slice of shared memory so that every
+                        // access to C is a run of whole row segments.
+                        if (store_pending) {
+                            if (lane == 0) tma_store_wait_read();
+                            store_pending = false;
                         }
+                        __syncwarp();   // the previous chunk has been read out of the slice
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
+                                make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+                        __syncwarp();
+                        const uint32_t rows_here = min(32u, t.m_end > row0 ? t.m_end - row0 : 0u);
+                        float *chunk = reinterpret_cast<float *>(p.c) + (uint64_t)row0 * p.ldc + col;
+                        if (col + 32 <= p.N && p.ldc % 4u == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15u) == 0)
+                            write_chunk<4>(chunk, p.ldc, rows_here, 32, slice, lane, p);
+                        else
+                            write_chunk<1>(chunk, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p);
                     }
                 }
             }

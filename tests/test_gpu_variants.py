@@ -27,3 +27,26 @@ def test_scalar_gemm_tile_edges_bit_exact(gpu, orc, m, n, k):
     run(fe, ctx, stream, "scalar_gemm_v1", a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k)
     assert (bits(Cb.read()) == bits(orc.gemm_f32(m, n, k, a, b))).all()
     A.unchanged(); B.unchanged()
+
+
+# ---- tensor-core GEMM: outputs that the copy engine does not write (alpha/beta form, C at any alignment)
+@pytest.mark.parametrize("m,n,k,ldc,offset", [(129, 40, 64, 40, 0), (128, 256, 64, 257, 0), (200, 136, 96, 140, 1), (257, 300, 72, 304, 0),
+                                              (16, 1000, 128, 1001, 3)])
+def test_gemm_tcgen05_direct_output_exact(gpu, orc, m, n, k, ldc, offset):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    lda, ldb = (k + 7) // 8 * 8, (n + 7) // 8 * 8
+    a = synth.gemm_inputs_v1((m - 1) * lda + k, 1, 1, 5)[0]   # dyadic alphabet: every summation order is exact
+    b = synth.gemm_inputs_v1(1, (k - 1) * ldb + n, 1, 6)[1]
+    size = (m - 1) * ldc + n
+    c = synth.uniform_f32(0, 9, size)
+    A, B = Guarded(fe, stream, a), Guarded(fe, stream, b)
+    for alpha, beta in ((2.0, -1.0), (1.0, 0.0)):
+        Cb = Guarded(fe, stream, np.concatenate([np.zeros(offset, np.float32), c]))
+        run(fe, ctx, stream, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_TCGEN05, a=A.slice, b=B.slice,
+            c=Cb.buf.view(GUARD + offset, size), m=m, n=n, k=k, lda=lda, ldb=ldb, ldc=ldc, alpha=alpha, beta=beta)
+        want = orc.gemm_bf16(m, n, k, a, b, lda=lda, ldb=ldb, ldc=ldc, alpha=alpha, beta=beta, c=c)
+        got = Cb.read()[offset:]
+        for r in range(m):
+            assert (bits(got[r * ldc:r * ldc + n]) == bits(want[r * n:(r + 1) * n])).all(), r
+            assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
