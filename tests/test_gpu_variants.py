@@ -50,3 +50,44 @@ def test_gemm_tcgen05_direct_output_exact(gpu, orc, m, n, k, ldc, offset):
         for r in range(m):
             assert (bits(got[r * ldc:r * ldc + n]) == bits(want[r * n:(r + 1) * n])).all(), r
             assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
+
+
+# ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
+@pytest.mark.parametrize("cols", [3, 29, 32, 33, 61, 64, 65, 125, 129, 256, 513, 1021, 1024, 1025, 2045, 2048, 2050, 3001, 4093, 4094, 4095, 4096])
+def test_row_softmax_widths(gpu, orc, cols):
+    from fe2o3_b200 import synth
+    rows = 37
+    x = synth.normal_f32(2, cols, rows * cols, 2.0).reshape(rows, cols)
+    softmax_case(gpu, orc, x)
+    mask = (synth.u32_below(2, 5000 + cols, rows * cols, 4) != 0).reshape(rows, cols)
+    mask[:, cols // 2] = True
+    got = softmax_case(gpu, orc, x, mask)
+    assert (bits(got[~mask]) == 0).all()
+
+
+@pytest.mark.parametrize("cols", [20, 64, 1000, 1023, 4095])
+@pytest.mark.parametrize("in_at,out_at", [(1, 1), (2, 3)])   # the same phase in a vector, and different ones
+def test_row_softmax_views_and_bad_rows(gpu, orc, cols, in_at, out_at):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    rows = 11
+    x = synth.normal_f32(2, 9000 + cols, rows * cols, 2.0).reshape(rows, cols)
+    mask = np.ones((rows, cols), np.uint8)
+    x[3, cols - 1] = np.inf      # refused although it is masked: the physical input counts
+    mask[3, cols - 1] = 0
+    mask[7] = 0                  # no active element
+    n = rows * cols
+    i = Guarded(fe, stream, np.concatenate([np.zeros(in_at, np.float32), x.ravel()]))
+    o = Guarded(fe, stream, np.full(out_at + n, -1, np.float32))
+    m = Guarded(fe, stream, np.concatenate([np.zeros(in_at, np.uint8), mask.ravel()]))
+    p = fe.prepare(ctx, "row_softmax_v1", input=i.buf.view(GUARD + in_at, n), output=o.buf.view(GUARD + out_at, n),
+                   mask=m.buf.view(GUARD + in_at, n), rows=rows, cols=cols)
+    with pytest.raises(fe.Fe2o3Error):
+        p.launch_and_wait(stream)
+    assert p.kernel_status == 2
+    got = o.read()[out_at:].reshape(rows, cols)
+    good = [r for r in range(rows) if r not in (3, 7)]
+    _, want = orc.row_softmax(x[good], mask[good] != 0)
+    assert (np.abs(got[good] - want) <= 1e-5 * np.abs(want)).all()
+    assert (got[[3, 7]] == -1).all()
+    i.unchanged(); m.unchanged()
