@@ -52,6 +52,13 @@ int32_t attention_tc_launch(const AttnTcPlan *, cudaStream_t);
 void attention_tc_geometry(const AttnTcPlan *, fe2o3_geometry *);
 void attention_tc_free(AttnTcPlan *);
 int32_t attention_tc_init_device();
+struct AttnSplitPlan;
+bool attention_split_supported(const fe2o3_flash_attention_v1_args *);
+int32_t attention_split_plan(fe2o3_ctx *, const fe2o3_flash_attention_v1_args *, AttnSplitPlan **);
+int32_t attention_split_launch(const AttnSplitPlan *, cudaStream_t);
+void attention_split_geometry(const AttnSplitPlan *, fe2o3_geometry *);
+void attention_split_free(AttnSplitPlan *);
+int32_t attention_split_init_device();
 int32_t device_scan_init_device();
 
 // ---- error bookkeeping ---------------------------------------------------------
@@ -132,7 +139,8 @@ struct fe2o3_prepared {
     alignas(8) uint8_t kernarg[320];
     uint32_t schedule;   // GEMM: resolved schedule
     GemmTcPlan gemm[2];  // tcgen05 plans (FFN uses both)
-    AttnTcPlan *attn;
+    AttnTcPlan *attn;    // head size 64
+    AttnSplitPlan *attn_split;   // the other head sizes the tensor cores take
     void *scratch[2];    // device workspace owned by the prepared object (split bf16 operands of the f32 GEMM)
     fe2o3_geometry geo;
 };
@@ -689,6 +697,7 @@ int32_t prepare_common(fe2o3_ctx *ctx, uint32_t op, const void *args, fe2o3_prep
     p->ctx = ctx;
     p->op = op;
     p->attn = nullptr;
+    p->attn_split = nullptr;
     p->scratch[0] = p->scratch[1] = nullptr;
     p->schedule = 0;
     memset(p->kernarg, 0, sizeof p->kernarg);
@@ -727,6 +736,7 @@ int32_t launch_prepared(fe2o3_prepared *p, cudaStream_t s) {
         }
         case OP_FLASH_ATTENTION: {
             if (p->attn) return attention_tc_launch(p->attn, s);
+            if (p->attn_split) return attention_split_launch(p->attn_split, s);
             return launch_attention_simt(ctx, s, reinterpret_cast<const fe2o3_flash_attention_v1_args *>(p->kernarg),
                                          nullptr, false);
         }
@@ -836,6 +846,7 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
     // opt-in shared memory sizes are a per-device function attribute: set them for this device
     int32_t init = gemm_tc_init_device();
     if (init == FE2O3_OK) init = attention_tc_init_device();
+    if (init == FE2O3_OK) init = attention_split_init_device();
     if (init == FE2O3_OK) init = device_scan_init_device();
     if (init != FE2O3_OK) return init;
     fe2o3_ctx *ctx = new (std::nothrow) fe2o3_ctx();
@@ -1395,6 +1406,12 @@ int32_t fe2o3_flash_attention_v1_prepare(fe2o3_ctx *ctx, const fe2o3_flash_atten
         attention_tc_geometry((*out)->attn, &(*out)->geo);
         return FE2O3_OK;
     }
+    if (attention_split_supported(a)) {
+        st = attention_split_plan(ctx, a, &(*out)->attn_split);
+        if (st != FE2O3_OK) return fail_prepare(out, st);
+        attention_split_geometry((*out)->attn_split, &(*out)->geo);
+        return FE2O3_OK;
+    }
     return launch_attention_simt(ctx, nullptr, a, &(*out)->geo, true);
 }
 int32_t fe2o3_moe_expert_ffn_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_expert_ffn_v1_args *a, fe2o3_prepared **out) {
@@ -1589,6 +1606,7 @@ const char *fe2o3_prepared_symbol(const fe2o3_prepared *p) { return p ? kOps[p->
 int32_t fe2o3_prepared_destroy(fe2o3_prepared *p) {
     if (!p) return FE2O3_OK;
     if (p->attn) attention_tc_free(p->attn);
+    if (p->attn_split) attention_split_free(p->attn_split);
     // the workspace may still be read by a launch in flight: freeing synchronises with the device (cudaFree does)
     for (void *w : p->scratch)
         if (w) cudaFree(w);

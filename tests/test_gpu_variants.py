@@ -91,3 +91,47 @@ def test_row_softmax_views_and_bad_rows(gpu, orc, cols, in_at, out_at):
     assert (np.abs(got[good] - want) <= 1e-5 * np.abs(want)).all()
     assert (got[[3, 7]] == -1).all()
     i.unchanged(); m.unchanged()
+
+
+# ---- attention with f32-precision probabilities (head sizes other than 64): 128-row tiles, 64-key blocks
+@pytest.mark.parametrize("B,H,S,D,causal", [(1, 1, 1, 128, False), (1, 3, 63, 128, True), (2, 1, 65, 96, True), (1, 2, 129, 72, False),
+                                            (1, 1, 257, 32, True), (1, 5, 300, 128, True), (1, 1, 600, 8, False), (2, 13, 500, 56, True),
+                                            # more two-tile units than SMs: several rounds, dealt in both directions
+                                            (4, 50, 200, 128, False), (4, 45, 400, 40, True)])
+def test_attention_split_probabilities(gpu, orc, B, H, S, D, causal):
+    from fe2o3_b200 import synth
+    from test_gpu_parity import attn_run
+    fe = gpu[0]
+    n = B * H * S * D
+    q, k, v = (synth.normal_bf16(3, d, n, 1.0).reshape(B, H, S, D) for d in (1, 2, 3))
+    got, _ = attn_run(gpu, q, k, v, 1.0 / np.sqrt(D), causal, fe.DTYPE_BF16)
+    v32 = synth.bf16_to_f32(v)
+    _, want = orc.flash_attention(synth.bf16_to_f32(q), synth.bf16_to_f32(k), v32, 1.0 / np.sqrt(D), causal)
+    # probabilities are exact sums of three bf16 terms.  What rounds: the score (8 accumulations of at most
+    # 128 products, below 1e-5 absolute after scaling), its exponential (1e-6 relative) and 3 * S / 16 <= 113
+    # accumulations of p * v at 2^-23 each: together below 2.5e-5 of the largest |v|
+    assert np.isfinite(got).all()
+    assert np.abs(got - want).max() <= 2.5e-5 * np.abs(v32).max()
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_split_leaves_bad_rows_unwritten(gpu, orc, causal):
+    from fe2o3_b200 import synth
+    fe, ctx, stream = gpu
+    B, H, S, D = 1, 3, 150, 128
+    q, k, v = (synth.normal_bf16(3, d, B * H * S * D, 1.0).reshape(B, H, S, D) for d in (1, 2, 3))
+    k[0, 1, 70, 17] = 0x7f80   # +inf: scores of both signs of infinity, so some probabilities are 0 and the sums finite
+    Q, K, V = Guarded(fe, stream, q), Guarded(fe, stream, k), Guarded(fe, stream, v)
+    O = Guarded(fe, stream, np.full(q.size, -7, np.float32))
+    p = fe.prepare(ctx, "flash_attention_v1", q=Q.slice, k=K.slice, v=V.slice, output=O.slice, batch=B, heads=H, seq=S, dim=D,
+                   scale=1.0 / np.sqrt(D), causal=int(causal), input_dtype=fe.DTYPE_BF16)
+    with pytest.raises(fe.Fe2o3Error):
+        p.launch_and_wait(stream)
+    assert p.kernel_status == 2
+    got = O.read().reshape(B, H, S, D)
+    bad = np.zeros((B, H, S), bool)
+    bad[0, 1, 70 if causal else 0:] = True
+    k[0, 1, 70, 17] = 0
+    _, want = orc.flash_attention(*(synth.bf16_to_f32(x) for x in (q, k, v)), 1.0 / np.sqrt(D), causal)
+    assert (got[bad] == -7).all()
+    assert np.abs(got - want)[~bad].max() <= 2.5e-5 * 6
