@@ -13,6 +13,10 @@
 // A CTA owns a 128 x BN output tile; one K block is 64 bf16 = 128 bytes.
 //   A stage: one TMA box {64 k, 128 rows}  -> 128 rows x 128 B, 8-row groups 1 KiB apart
 //   B stage: BN/64 TMA boxes {64 n, 64 k}   -> per box 64 k-rows x 128 B (8 KiB)
+// What bounds the large products is power (at 1000 W the clock falls to 1.1 GHz, and the tensor pipe is 90 % busy
+// at it) and, before that, the 48 KiB of operands that a 128 x 256 tile stages per k block: a pair of CTAs on two
+// SMs (CG = 2) owns a 256 x 256 tile, each staging its rows of A and half of B, one issuer driving both tensor
+// pipes (cta_group::2).  8192^3: 907 us with single CTAs, 832 so.
 // Persistent CTAs (one per SM) walk a static tile list; ten warps:
 //   warp 0  TMA producer (one lane)        warp 1  MMA issuer (one lane) + TMEM owner
 //   warps 2-9  epilogue: TMEM -> registers -> shared memory -> bulk tensor store,
@@ -29,20 +33,19 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 64;          // bf16 elements per K block (128 bytes)
 constexpr int UMMA_K = 16;
-constexpr int kStages = 4;
 constexpr int kEpilogueWarps = 8;
 constexpr int kThreads = 32 * (2 + kEpilogueWarps);
-constexpr int kGatherThreads = 128;  // four more warps when A is gathered row by row: fourteen warps count as sixteen in
-                                     // the register file (registers go out to four warps at a time), which the
-                                     // 128-register build of the kernel fills exactly; with two loader warps on the
-                                     // 168-register build the gathered GEMM was 6 % slower than the one fed by TMA
-                                     // and gained 11-18 us per MoE pass against the compaction pass, with four 40 us
+constexpr int kGatherThreads = 128;  // four more warps when A is gathered row by row (copy-engine gathers, so that the bytes
+                                     // are counted like every other load's), on the 128-register build
 constexpr int kGroupM = 16;     // m-tiles per rasterisation band (keeps a wave's A and B panels in L2)
 
-template <int BN>
+// CG = blocks per tile.  CG = 2: a pair of blocks on two neighbouring SMs owns a 256 x BN tile; each block stages its
+// own 128 rows of A and its half of B's columns, so a k block costs 32 KiB of staging per SM instead of 48.
+template <int BN, int CG>
 struct SmemLayout {
+    static constexpr int kStages = CG == 2 ? 6 : 4;
     static constexpr uint32_t kABytes = BM * BK * 2;
-    static constexpr uint32_t kBBytes = BN * BK * 2;
+    static constexpr uint32_t kBBytes = BN / CG * BK * 2;
     static constexpr uint32_t kStageBytes = kABytes + kBBytes;
     static constexpr uint32_t kStagingOffset = kStages * kStageBytes;          // 4 KiB output slice per epilogue warp
     static constexpr uint32_t kBarOffset = kStagingOffset + kEpilogueWarps * 4096;
@@ -60,6 +63,8 @@ struct TileCoord {
 // the expert-parallel FFN): by the source rank of the tile's first row, this rank's own rows first
 // (they never cross NVLink), then ranks +1, +2, ... which is the order in which the other ranks send
 // to this one; inside a source by local expert, then m, n fastest.
+// TM: rows of a tile (128, or 256 for a pair of blocks).
+template <int TM>
 __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &p, uint32_t n_tiles,
                                                  const uint32_t *s_off, const uint32_t *s_pair) {
     TileCoord t;
@@ -67,19 +72,20 @@ __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &
     t.expert = 0;
     t.m0 = t.n0 = t.m_end = t.mt_index = 0;
     if (p.experts == 0) {
-        const uint32_t m_tiles = (p.M + BM - 1) / BM;
+        constexpr uint32_t kBand = kGroupM * BM / TM;
+        const uint32_t m_tiles = (p.M + TM - 1) / TM;
         if (id >= m_tiles * n_tiles) return t;
-        const uint32_t band = id / (kGroupM * n_tiles);
-        const uint32_t first_m = band * kGroupM;
-        const uint32_t band_m = min((uint32_t)kGroupM, m_tiles - first_m);
-        const uint32_t local = id - band * kGroupM * n_tiles;
-        t.m0 = (first_m + local % band_m) * BM;
+        const uint32_t band = id / (kBand * n_tiles);
+        const uint32_t first_m = band * kBand;
+        const uint32_t band_m = min(kBand, m_tiles - first_m);
+        const uint32_t local = id - band * kBand * n_tiles;
+        t.m0 = (first_m + local % band_m) * TM;
         t.n0 = (local / band_m);
         t.m_end = p.M;
         t.valid = true;
         return t;
     }
-    if (p.ep.rows_flags || p.ep.progress_mode) {
+    if (TM == BM && (p.ep.rows_flags || p.ep.progress_mode)) {
         // groups = (run j, local expert le): the tiles whose first row belongs to source (rank + j) mod W; inside
         // an expert's segment the runs lie in exactly that order (the owner's own rows first)
         const uint32_t W = p.ep.world;
@@ -108,11 +114,11 @@ __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &
         uint32_t base = 0;
         for (uint32_t e = 0; e < p.experts; ++e) {
             const uint32_t rows = s_off[e + 1] - s_off[e];
-            const uint32_t mt = (rows + BM - 1) / BM;
+            const uint32_t mt = (rows + TM - 1) / TM;
             const uint32_t cnt = mt * n_tiles;
             if (id < base + cnt) {
                 const uint32_t local = id - base;
-                t.m0 = s_off[e] + (local % mt) * BM;
+                t.m0 = s_off[e] + (local % mt) * TM;
                 t.n0 = local / mt;
                 t.m_end = s_off[e + 1];
                 t.expert = p.expert_mod ? e % p.expert_mod : e;   // index of the B matrix
@@ -133,6 +139,11 @@ __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &
     t.mt_index = __shfl_sync(0xffffffffu, t.mt_index, 0);
     t.valid = __shfl_sync(0xffffffffu, (uint32_t)t.valid, 0) != 0;
     return t;
+}
+
+// Four-row pieces of a 128-row tile at m0 that hold rows of its group.
+__device__ __forceinline__ uint32_t gathered_quads(uint32_t m0, uint32_t m_end) {
+    return m_end > m0 ? (min(m_end - m0, (uint32_t)BM) + 3) / 4 : 0u;
 }
 
 // erf by Abramowitz & Stegun 7.1.26 (absolute error below 1.5e-7, far under the bf16 step of the
@@ -215,11 +226,12 @@ __device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t
 // beside the expert-parallel dispatch kernel: registers are handed out to four warps at a time, so the ten
 // warps count as twelve, and 12 x 32 x 128 leaves room for one block of that kernel on the same SM.  It and the
 // build with loader warps (a gathered A) run the first GEMM of an expert FFN only, so REGS = 128 has no f32 output.
-template <int BN, int REGS>
+template <int BN, int REGS, int CG>
 __global__ void __maxnreg__(REGS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, GemmParams p) {
-    using L = SmemLayout<BN>;
+    using L = SmemLayout<BN, CG>;
+    constexpr int kStages = L::kStages;
     extern __shared__ uint8_t smem_raw[];
     // 128-byte swizzle atoms are 1 KiB: align the tile region.
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -236,6 +248,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n_tiles = (p.N + BN - 1) / BN;
     const uint32_t num_kb = (p.K + BK - 1) / BK;
+    // this block's place in its pair, and the tiles it walks (both blocks of a pair walk the same ones)
+    const uint32_t crank = CG == 2 ? cluster_rank() : 0u;
+    const uint32_t first_tile = blockIdx.x / CG, tile_step = gridDim.x / CG;
     // the second GEMM of the expert FFN may take over each SM as this kernel's CTA leaves it
     if (p.ep.progress_mode == 1) launch_dependents();
 
@@ -245,12 +260,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // They find the status word set and do nothing but their arrival counting.
         s_abort = (p.ep.pair_offsets && p.status && __ldcg(p.status) != 0u) ? 1 : 0;
         for (int i = 0; i < kStages; ++i) {
-            mbar_init(&full[i], p.gather_perm ? 1 + kGatherThreads : 1);   // the producer's expect-tx arrival + every loader thread
+            mbar_init(&full[i], 1);   // the producer's expect-tx arrival; in a pair rank 0's barrier counts both blocks' bytes
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&tmem_full[i], 1);
-            mbar_init(&tmem_empty[i], kEpilogueWarps);
+            mbar_init(&tmem_empty[i], kEpilogueWarps * CG);
         }
         mbar_fence_init();
     }
@@ -300,13 +315,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         ep_trace(p.ep.trace_flags, p.ep.rows_flags ? FE2O3_EP_T_FFN1_BEGIN : FE2O3_EP_T_FFN2_BEGIN);
 #endif
     if (warp == 1) {
-        tmem_alloc(tmem_slot, 2 * BN);
-        tmem_relinquish();
+        if constexpr (CG == 2) {
+            tmem_alloc_pair(tmem_slot, 2 * BN);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(tmem_slot, 2 * BN);
+            tmem_relinquish();
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (CG == 2) cluster_sync();   // the other block's barriers are initialised
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // A role that gives up ends the other roles' waits too, in both blocks of a pair.
+    auto give_up = [&] {
+        kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
+        atomicExch(&s_abort, 1);
+        if constexpr (CG == 2) st_shared_cluster(cluster_addr(&s_abort, crank ^ 1u), 1u);
+    };
     const bool dead = s_abort != 0 || (p.experts && s_table_bad);   // uniform over the CTA: read after the barrier, before any role can set it
 
     if (warp == 0) {
@@ -319,9 +346,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t stage = 0, phase = 0, loaded = 0;
         uint32_t seen = 0;   // sources whose "rows complete" flag this CTA has already acquired
         bool ok = !dead;
-        for (uint32_t id = blockIdx.x; ok; id += gridDim.x) {
-            TileCoord t = decode_tile(id, p, n_tiles, s_off, s_pair);
+        for (uint32_t id = first_tile; ok; id += tile_step) {
+            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
+            if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             if (p.ep.rows_flags) {
                 // Sources with rows in this tile.  Their rows were written by the source ranks' SMs
                 // (generic proxy, then a system-scope release of the flag); this warp acquires the flag
@@ -342,7 +370,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 fence_proxy_async_global();
 #ifdef FE2O3_EP_TRACE
                 if (blockIdx.x == 0 && lane == 0 && p.ep.trace_flags) {
-                    if (id == blockIdx.x) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_FIRST_WAIT_DONE);
+                    if (id == first_tile) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_FIRST_WAIT_DONE);
                     if (seen == (1u << p.ep.world) - 1u) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_LAST_WAIT_DONE);
                 }
 #endif
@@ -358,53 +386,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 fence_proxy_async_global();
             }
+            // bytes of a k block that rank 0's (or the only) barrier counts; of a gathered A only rows of the group are fetched
+            uint32_t bytes = CG * L::kStageBytes;
+            if (p.gather_perm) {
+                bytes = CG * L::kBBytes + gathered_quads(t.m0, t.m_end) * 512u;
+                if (CG == 2) bytes += gathered_quads(t.m0 + BM, t.m_end) * 512u;   // (rank 1's rows; only rank 0 uses this)
+            }
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++loaded) {
                 if (!mbar_wait_warp(&empty[stage], phase ^ 1, &s_abort)) { ok = false; break; }
                 if (elect_one()) {
                     uint8_t *sa = smem + stage * L::kStageBytes;
                     uint8_t *sb = sa + L::kABytes;
-                    mbar_arrive_expect_tx(&full[stage], p.gather_perm ? L::kBBytes : L::kStageBytes);
-                    if (!p.gather_perm) tma_load_2d(sa, &tmA, &full[stage], (int32_t)(kb * BK), (int32_t)t.m0);
+                    if constexpr (CG == 2) {
+                        // both blocks' bytes are counted by rank 0's barrier; rank 1's may arrive before the
+                        // expectation is set, which the barrier's pending arrival makes harmless
+                        const uint32_t bar = cluster_addr(&full[stage], 0);
+                        if (crank == 0) mbar_arrive_expect_tx(&full[stage], bytes);
+                        if (!p.gather_perm) tma_load_2d_pair(sa, &tmA, bar, (int32_t)(kb * BK), (int32_t)t.m0);
 #pragma unroll
-                    for (int j = 0; j < BN / 64; ++j) {
-                        if (p.experts)
-                            tma_load_3d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK),
-                                        (int32_t)t.expert);
-                        else
-                            tma_load_2d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK));
+                        for (int j = 0; j < BN / CG / 64; ++j) {
+                            const int32_t col = (int32_t)(t.n0 * BN + crank * (BN / CG) + j * 64);
+                            if (p.experts) tma_load_3d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK), (int32_t)t.expert);
+                            else tma_load_2d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK));
+                        }
+                    } else {
+                        mbar_arrive_expect_tx(&full[stage], bytes);
+                        if (!p.gather_perm) tma_load_2d(sa, &tmA, &full[stage], (int32_t)(kb * BK), (int32_t)t.m0);
+#pragma unroll
+                        for (int j = 0; j < BN / 64; ++j) {
+                            if (p.experts)
+                                tma_load_3d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK),
+                                            (int32_t)t.expert);
+                            else
+                                tma_load_2d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK));
+                        }
                     }
                 }
                 __syncwarp();
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }
-        if (!ok && lane == 0) {
-            kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
-            atomicExch(&s_abort, 1);
-        }
+        if (!ok && lane == 0) give_up();
         // Drain: every copy issued must have landed before the CTA exits (the newest phase of each ring slot).
-        for (uint32_t b = 0; b < kStages && b < loaded; ++b) {
+        // Rank 1's copies are counted by rank 0's barriers, and no block of a pair leaves before the other.
+        for (uint32_t b = 0; crank == 0 && b < kStages && b < loaded; ++b) {
             const uint32_t last = loaded - 1 - b;
             mbar_wait_warp(&full[last % kStages], (last / kStages) & 1);
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer (warp converged, one elected lane issues)
-        constexpr uint32_t idesc = umma_idesc(1u, BM, BN, 0u, 1u);
+        // ------------------------------------------------ MMA issuer (warp converged, one elected lane issues; rank 0 of a pair)
+        constexpr uint32_t idesc = umma_idesc(1u, BM * CG, BN, 0u, 1u);
         uint32_t stage = 0, phase = 0, it = 0;
-        bool ok = !dead;
+        bool ok = !dead && crank == 0;
         const uint64_t desc_a0 = umma_smem_desc(smem_u32(smem), 16, 1024);
         const uint64_t desc_b0 = umma_smem_desc(smem_u32(smem) + L::kABytes, 8192, 1024);
-        for (uint32_t id = blockIdx.x; ok; id += gridDim.x, ++it) {
-            TileCoord t = decode_tile(id, p, n_tiles, s_off, s_pair);
+        for (uint32_t id = first_tile; ok; id += tile_step, ++it) {
+            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
+            if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
             if (!mbar_wait_warp(&tmem_empty[buf], acc_phase ^ 1, &s_abort)) { ok = false; break; }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + buf * BN;
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_warp(&full[stage], phase, &s_abort)) { ok = false; break; }
-                // gathered A rows were written by cp.async (generic proxy): order them before the tensor core's reads
-                if (p.gather_perm) fence_proxy_async_smem();
                 tc_fence_after();
                 if (elect_one()) {
                     // only the 16-byte-unit start address field of the descriptors moves
@@ -412,63 +457,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const uint64_t bdesc = desc_b0 + ((stage * L::kStageBytes) >> 4);
                     // A: K-major, advance 16 elements = 32 bytes inside the 128-byte row
                     // B: MN-major, advance 16 k-rows = 2 KiB; 64-column groups are 8 KiB apart
-                    umma_f16(d_tmem, adesc, bdesc, idesc, kb != 0u);
+                    if constexpr (CG == 2) {
 #pragma unroll
-                    for (int k = 1; k < BK / UMMA_K; ++k)
-                        umma_f16(d_tmem, adesc + ((k * UMMA_K * 2) >> 4), bdesc + ((k * UMMA_K * 128) >> 4), idesc, 1u);
-                    umma_commit(&empty[stage]);
-                    if (kb + 1 == num_kb) umma_commit(&tmem_full[buf]);
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            umma_f16_pair(d_tmem, adesc + ((k * UMMA_K * 2) >> 4), bdesc + ((k * UMMA_K * 128) >> 4), idesc,
+                                          (uint32_t)(k != 0) | (uint32_t)(kb != 0u));
+                        umma_commit_pair(&empty[stage]);
+                        if (kb + 1 == num_kb) umma_commit_pair(&tmem_full[buf]);
+                    } else {
+                        umma_f16(d_tmem, adesc, bdesc, idesc, kb != 0u);
+#pragma unroll
+                        for (int k = 1; k < BK / UMMA_K; ++k)
+                            umma_f16(d_tmem, adesc + ((k * UMMA_K * 2) >> 4), bdesc + ((k * UMMA_K * 128) >> 4), idesc, 1u);
+                        umma_commit(&empty[stage]);
+                        if (kb + 1 == num_kb) umma_commit(&tmem_full[buf]);
+                    }
                 }
                 __syncwarp();
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }
-        if (!ok && lane == 0) {
-            kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
-            atomicExch(&s_abort, 1);
-        }
+        if (!ok && crank == 0 && lane == 0) give_up();
     } else if (warp >= 2 + kEpilogueWarps) {
-        // ------------------------------------------------ gather loaders (blocks launched with them only)
-        // 128 threads fetch the tile's 128 rows of A for every K block: thread = (row mod 16, 16-byte chunk of
-        // the row's 128 bytes), eight rows each, so that eight neighbouring lanes read one whole line.  The
-        // rows go straight into the 128-byte-swizzled stage the tensor core reads; a row that is not a route
-        // (past the group's end, or a dropped slot) is filled with zeros.  Completion is signalled to the
-        // stage's barrier by the copies themselves.
-        const uint32_t lt = threadIdx.x - 32 * (2 + kEpilogueWarps);
-        const uint32_t chunk = lt & 7, r0 = lt >> 3;   // r0 in 0..15
-        const uint8_t *src_base = reinterpret_cast<const uint8_t *>(p.gather_src);
+        // ------------------------------------------------ gather issuers (blocks launched with them only)
+        // Four warps fetch 32 rows of the tile each, four rows an instruction, by the copy engine: the rows' token
+        // numbers sit in registers for the whole tile.  A slot without a route names the row after the last token,
+        // which the copy engine fills with zeros; whole quads past the group's end are not fetched (what they leave in
+        // the stage only reaches rows of the accumulator that nobody stores).
+        const uint32_t r0 = (warp - (2 + kEpilogueWarps)) * 32;
         uint32_t stage = 0, phase = 0;
         bool ok = !dead;
-        for (uint32_t id = blockIdx.x; ok; id += gridDim.x) {
-            TileCoord t = decode_tile(id, p, n_tiles, s_off, s_pair);
+        for (uint32_t id = first_tile; ok; id += tile_step) {
+            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
-            constexpr int kRowsPerThread = 128 * 8 / kGatherThreads;
-            uint32_t tok[kRowsPerThread];
+            if constexpr (CG == 2) t.m0 += crank * BM;
+            const uint32_t quads = gathered_quads(t.m0 + r0, t.m_end);   // of this warp's 32 rows: 8 or fewer count
+            const uint32_t row = t.m0 + r0 + lane;
+            const uint32_t route = row < t.m_end ? __ldg(p.gather_perm + row) : 0xffffffffu;
+            const uint32_t mine = route == 0xffffffffu ? p.gather_tokens : min(route >> 1, p.gather_tokens);
+            int32_t tok[32];
 #pragma unroll
-            for (int i = 0; i < kRowsPerThread; ++i) {
-                const uint32_t row = t.m0 + r0 + (kGatherThreads / 8) * i;
-                const uint32_t route = row < t.m_end ? __ldg(p.gather_perm + row) : 0xffffffffu;
-                tok[i] = (route == 0xffffffffu || (route >> 1) >= p.gather_tokens) ? 0xffffffffu : (route >> 1);
-            }
+            for (int i = 0; i < 32; ++i) tok[i] = (int32_t)__shfl_sync(0xffffffffu, mine, i);
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_warp(&empty[stage], phase ^ 1, &s_abort)) { ok = false; break; }
-                const uint32_t sa = smem_u32(smem + stage * L::kStageBytes) + r0 * 128 + ((chunk ^ (r0 & 7)) << 4);
-                const uint64_t col = (uint64_t)kb * (BK * 2) + chunk * 16;
+                if (elect_one()) {
+                    uint8_t *sa = smem + stage * L::kStageBytes + r0 * 128;
+                    const uint32_t bar = CG == 2 ? cluster_addr(&full[stage], 0) : smem_u32(&full[stage]);
+                    auto fetch = [&](int i) {
+                        tma_gather4<CG == 2>(sa + i * 512, &tmA, bar, (int32_t)(kb * BK), tok[4 * i], tok[4 * i + 1], tok[4 * i + 2],
+                                             tok[4 * i + 3]);
+                    };
+                    if (quads >= 8) {
 #pragma unroll
-                for (int i = 0; i < kRowsPerThread; ++i) {
-                    const bool live = tok[i] != 0xffffffffu;
-                    const uint8_t *src = live ? src_base + (uint64_t)tok[i] * p.K * 2 + col : src_base;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa + i * (kGatherThreads / 8) * 128), "l"(src), "r"(live ? 16 : 0) : "memory");
+                        for (int i = 0; i < 8; ++i) fetch(i);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 7; ++i)
+                            if (i < (int)quads) fetch(i);
+                    }
                 }
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[stage])) : "memory");
+                __syncwarp();
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");   // no copy may be in flight when the block exits
-        if (!ok && lane == 0) {
-            kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
-            atomicExch(&s_abort, 1);
-        }
+        if (!ok && lane == 0) give_up();
     } else {
         // ------------------------------------------------ epilogue warps
         // Eight warps: two per TMEM lane quadrant, each taking half of the tile's columns.  A warp
@@ -485,14 +537,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t it = 0;
         bool ok = !dead;
         bool store_pending = false;
+        auto release_accumulator = [&](uint32_t buf) {   // the issuer of a pair is rank 0
+            if constexpr (CG == 2) mbar_arrive_cluster(cluster_addr(&tmem_empty[buf], 0));
+            else mbar_arrive(&tmem_empty[buf]);
+        };
         if (p.zero_ptr && !dead) {
             const uint64_t stride = (uint64_t)gridDim.x * (kEpilogueWarps * 32);
             for (uint64_t i = (uint64_t)blockIdx.x * (kEpilogueWarps * 32) + ew * 32 + lane; i < p.zero_vecs; i += stride)
                 p.zero_ptr[i] = make_uint4(0u, 0u, 0u, 0u);
         }
-        for (uint32_t id = blockIdx.x; ok; id += gridDim.x, ++it) {
-            TileCoord t = decode_tile(id, p, n_tiles, s_off, s_pair);
+        for (uint32_t id = first_tile; ok; id += tile_step, ++it) {
+            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
+            if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
             if (!mbar_wait_warp(&tmem_full[buf], acc_phase, &s_abort)) { ok = false; break; }
             tc_fence_after();
@@ -539,7 +596,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (g == kChunks / 2 - 1 && c2 == 1) {   // the accumulator has been read completely
                             tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+                            if (lane == 0) release_accumulator(buf);
                         }
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -586,7 +643,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (g == kChunks - 1) {   // the accumulator has been read completely
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+                        if (lane == 0) release_accumulator(buf);
                     }
                     const uint32_t col = col_base + g * 32;
                     if (col >= p.N) continue;
@@ -675,16 +732,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (store_pending && lane == 0) tma_store_wait_read();
         // rows stored into other ranks' memory must be visible there before "outputs ready" is raised
         if (p.epilogue == EPI_SCATTER_PEER) __threadfence_system();
-        if (!ok && lane == 0) {
-            kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
-            atomicExch(&s_abort, 1);
-        }
+        if (!ok && lane == 0) give_up();
     }
     tc_fence_before();
     __syncthreads();
+    // no block of a pair leaves while the other may still signal its barriers or read its shared memory
+    if constexpr (CG == 2) cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 2 * BN);
+        if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, 2 * BN);
+        else tmem_dealloc(tmem_base, 2 * BN);
     }
 #ifdef FE2O3_EP_TRACE
     if (p.ep.trace_flags && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
@@ -814,21 +871,41 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
     const uint64_t m_tiles = (uint64_t)(M + BM - 1) / BM + experts;  // grouped: each expert may add a ragged tile
     uint64_t tiles = m_tiles * n_tiles;
     plan->grid = (uint32_t)(tiles < (uint64_t)ctx->sm_count ? (tiles ? tiles : 1) : (uint64_t)ctx->sm_count);
-    plan->smem = plan->bn == 256 ? SmemLayout<256>::kTotal : SmemLayout<128>::kTotal;
+    plan->smem = plan->bn == 256 ? SmemLayout<256, 1>::kTotal : SmemLayout<128, 1>::kTotal;
+    // 256-row tiles on pairs of SMs stage a third less per multiply-add, which shortens a round of tiles by about a
+    // tenth where the k loop sets its length: 8192^3 907 against 832 us, 2048x2048x4096 36.9 against 34.8 (both
+    // orders in one call).  A pair's two epilogues run in step, so where the output does (K = 128 of 8192x8192: 54
+    // against 61 us, K = 1024: 13.9 against 14.3) the single blocks stay; and they stay where the coarser tiles make
+    // more rounds (512 rows an expert, d 2048: 194 against 209 us a layer pass).  Groups end in a partly filled tile,
+    // half of one on average.
+    plan->pair = 0;
+    if (plan->bn == 256 && K > 1024 && !ep && ctx->sm_count >= 2) {
+        auto rounds = [&](uint64_t rows_per_tile, uint64_t slots) {
+            const uint64_t m_tiles = experts ? (2 * (uint64_t)M + experts * rows_per_tile) / (2 * rows_per_tile)
+                                             : (M + rows_per_tile - 1) / rows_per_tile;
+            return (m_tiles * n_tiles + slots - 1) / slots;
+        };
+        const uint64_t pairs = ctx->sm_count / 2;
+        if (9 * rounds(2 * BM, pairs) < 10 * rounds(BM, ctx->sm_count)) {
+            plan->pair = 1;
+            tiles = ((uint64_t)(M + 2 * BM - 1) / (2 * BM) + experts) * n_tiles;
+            plan->grid = 2 * (uint32_t)(tiles < pairs ? (tiles ? tiles : 1) : pairs);
+            plan->smem = SmemLayout<256, 2>::kTotal;
+        }
+    }
     plan->overlap_previous = 0;
     return FE2O3_OK;
 }
 
 // Function attributes are per device: called by fe2o3_ctx_create with the context's device current.
 int32_t gemm_tc_init_device() {
-    FE2O3_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<256, 168>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SmemLayout<256>::kTotal));
-    FE2O3_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<128, 168>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SmemLayout<128>::kTotal));
-    FE2O3_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<256, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SmemLayout<256>::kTotal));
-    FE2O3_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SmemLayout<128>::kTotal));
+    auto set = [](auto kernel, uint32_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+    FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 1>, SmemLayout<256, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<128, 168, 1>, SmemLayout<128, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 1>, SmemLayout<256, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<128, 128, 1>, SmemLayout<128, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 2>, SmemLayout<256, 2>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 2>, SmemLayout<256, 2>::kTotal));
     return FE2O3_OK;
 }
 
@@ -840,7 +917,12 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
     cfg.dynamicSmemBytes = plan->smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    if (plan->overlap_previous) {
+    if (plan->pair) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim = {2, 1, 1};
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    } else if (plan->overlap_previous) {
         // programmatic dependent launch: the kernel may start while the kernel before it in the stream (the
         // expert-parallel dispatch, which says when) is still running; the two synchronise through flags
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -851,12 +933,13 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
     cudaError_t e;
     // the 128-register build: for a block that shares its SM with the small blocks of the kernel before it, and for
     // one that carries the loader warps of a gathered A
+    auto launch = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, plan->tmA, plan->tmB, plan->tmC, plan->p); };
     if (plan->overlap_previous == 1 || plan->p.gather_perm)
-        e = plan->bn == 256 ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<256, 128>, plan->tmA, plan->tmB, plan->tmC, plan->p)
-                            : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<128, 128>, plan->tmA, plan->tmB, plan->tmC, plan->p);
+        e = plan->pair ? launch(gemm_tc_kernel<256, 128, 2>)
+                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 128, 1>) : launch(gemm_tc_kernel<128, 128, 1>);
     else
-        e = plan->bn == 256 ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<256, 168>, plan->tmA, plan->tmB, plan->tmC, plan->p)
-                            : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<128, 168>, plan->tmA, plan->tmB, plan->tmC, plan->p);
+        e = plan->pair ? launch(gemm_tc_kernel<256, 168, 2>)
+                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 168, 1>) : launch(gemm_tc_kernel<128, 168, 1>);
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "gemm_tc");
 }
@@ -864,6 +947,11 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
 // Makes the plan's A operand a gather: row r of A = row (perm[r] >> 1) of src.  Needs whole 64-column K blocks.
 bool gemm_tc_set_gather(GemmTcPlan *plan, const uint32_t *perm, const void *src, uint32_t tokens) {
     if (plan->p.K % BK != 0 || (reinterpret_cast<uintptr_t>(src) & 15u) != 0) return false;
+    if (tokens) {   // the copy engine's gather form wants a box one row high
+        const uint64_t dims[2] = {plan->p.K, tokens}, stride[1] = {(uint64_t)plan->p.K * 2};
+        const uint32_t box[2] = {BK, 1};
+        if (fe2o3_make_tmap_bf16(&plan->tmA, reinterpret_cast<uint64_t>(src), 2, dims, stride, box) != FE2O3_OK) return false;
+    }
     plan->p.gather_perm = perm;
     plan->p.gather_src = src;
     plan->p.gather_tokens = tokens;
@@ -883,9 +971,9 @@ void gemm_tc_geometry(const GemmTcPlan *plan, fe2o3_geometry *geo) {
 }
 
 // kernel symbols of the runtime adapter carried by this source (the schedule a large launch resolves to)
-static Fe2o3KernelRegistration reg_tiled("tiled_gemm_lds_slice1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168>));
-static Fe2o3KernelRegistration reg_general("tiled_gemm_general_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168>));
-static Fe2o3KernelRegistration reg_ffn("moe_expert_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168>));
-static Fe2o3KernelRegistration reg_gffn("moe_grouped_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168>));
-static Fe2o3KernelRegistration reg_ffnc("moe_expert_ffn_combine_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128>));
-static Fe2o3KernelRegistration reg_epffn("moe_ep_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168>));
+static Fe2o3KernelRegistration reg_tiled("tiled_gemm_lds_slice1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
+static Fe2o3KernelRegistration reg_general("tiled_gemm_general_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
+static Fe2o3KernelRegistration reg_ffn("moe_expert_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
+static Fe2o3KernelRegistration reg_gffn("moe_grouped_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
+static Fe2o3KernelRegistration reg_ffnc("moe_expert_ffn_combine_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1>));
+static Fe2o3KernelRegistration reg_epffn("moe_ep_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));

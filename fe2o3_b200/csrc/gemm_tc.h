@@ -50,7 +50,7 @@ struct GemmParams {
     GemmEp ep;
     // Gathered A (first GEMM of the single-GPU expert FFN): row r of A is row (gather_perm[r] >> 1) of
     // gather_src ([gather_tokens][K] bf16), or zero when gather_perm[r] names no route; the block is then
-    // launched with four loader warps more, which fetch the rows straight into the swizzled A stage.
+    // launched with four warps more, which have the copy engine gather the rows into the swizzled A stage.
     const uint32_t *gather_perm;
     const void *gather_src;
     uint32_t gather_tokens;
@@ -72,6 +72,7 @@ struct GemmTcPlan {
     CUtensorMap tmA, tmB, tmC;
     GemmParams p;
     uint32_t bn;
+    uint32_t pair;               // 256-row tiles, each owned by a cluster of two blocks
     uint32_t grid;
     uint32_t smem;
     uint32_t overlap_previous;   // launch with programmatic stream serialization: 1 = may run beside the (small) blocks of the

@@ -52,6 +52,34 @@ def test_gemm_tcgen05_direct_output_exact(gpu, orc, m, n, k, ldc, offset):
             assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
 
 
+# ---- tensor-core GEMM on pairs of SMs (k above 1024): second half of a pair without rows or columns, ragged ends
+@pytest.mark.parametrize("m,n,k,ldc,beta", [(128, 264, 1032, 264, 0.0), (129, 384, 1088, 384, 0.0), (256, 512, 1056, 512, -1.0),
+                                            (257, 392, 1100, 395, 0.5), (1, 130, 1025, 131, -1.0), (700, 2600, 1040, 2600, 0.0)])
+def test_gemm_pair_tiles_exact(gpu, orc, m, n, k, ldc, beta):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    lda, ldb = (k + 7) // 8 * 8, (n + 7) // 8 * 8
+    a = synth.gemm_inputs_v1((m - 1) * lda + k, 1, 1, 5)[0]   # dyadic alphabet: every summation order is exact
+    b = synth.gemm_inputs_v1(1, (k - 1) * ldb + n, 1, 6)[1]
+    c = synth.uniform_f32(0, 9, (m - 1) * ldc + n)
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, c)
+    run(fe, ctx, stream, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_TCGEN05, a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k,
+            lda=lda, ldb=ldb, ldc=ldc, alpha=1.0, beta=beta)
+    want = orc.gemm_bf16(m, n, k, a, b, lda=lda, ldb=ldb, ldc=ldc, alpha=1.0, beta=beta, c=c)
+    got = Cb.read()
+    for r in range(m):
+        assert (bits(got[r * ldc:r * ldc + n]) == bits(want[r * n:(r + 1) * n])).all(), r
+        assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
+
+
+@pytest.mark.parametrize("T,d,f,E,cap", [(300, 1088, 1152, 4, 600), (900, 1152, 1088, 4, 250)])
+def test_moe_pair_tiles(gpu, orc, T, d, f, E, cap):
+    from test_gpu_parity import assert_close, moe_pipeline
+    compact, want_compact, out, want_out, accepted = moe_pipeline(gpu, orc, T, d, f, E, cap)
+    assert_close(out, want_out, 2e-2, 2e-3, "combined output")
+    assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
+
+
 # ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
 @pytest.mark.parametrize("cols", [3, 29, 32, 33, 61, 64, 65, 125, 129, 256, 513, 1021, 1024, 1025, 2045, 2048, 2050, 3001, 4093, 4094, 4095, 4096])
 def test_row_softmax_widths(gpu, orc, cols):
