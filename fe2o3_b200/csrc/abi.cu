@@ -1435,6 +1435,7 @@ int32_t fe2o3_moe_expert_ffn_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_expert_f
                                       reinterpret_cast<const void *>(a->x.ptr), a->tokens);
     gemm_tc_geometry(&p->gemm[0], &p->geo);
     p->geo.launches = gathered ? 2 : 3;
+    gemm_tc_set_early_weights(&p->gemm[1]);
     return FE2O3_OK;
 }
 
@@ -1464,6 +1465,7 @@ int32_t fe2o3_moe_expert_ffn_combine_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_
     // the second GEMM adds into the output, which starts from +0: cleared by the first GEMM's idle epilogue warps
     p->gemm[0].p.zero_ptr = reinterpret_cast<uint4 *>(a->combined_output.ptr);
     p->gemm[0].p.zero_vecs = (uint64_t)a->tokens * a->d_model / 4;
+    gemm_tc_set_early_weights(&p->gemm[1]);
     gemm_tc_geometry(&p->gemm[0], &p->geo);
     p->geo.launches = 2;
     return FE2O3_OK;
@@ -1493,6 +1495,7 @@ int32_t fe2o3_moe_grouped_ffn_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_grouped
                           a->d_ff, a->d_model, a->d_model, 1.f, 0.f, 0u, off, a->groups, a->experts_cycle,
                           a->experts_cycle);
     if (st != FE2O3_OK) return fail_prepare(out, st);
+    gemm_tc_set_early_weights(&p->gemm[1]);
     gemm_tc_geometry(&p->gemm[0], &p->geo);
     p->geo.launches = 2;
     return FE2O3_OK;

@@ -150,6 +150,8 @@ __device__ __forceinline__ void ep_trace(uint32_t *, uint32_t) {}
 // stream serialization, start once every block of this grid has executed this (or exited).  That kernel
 // sees none of this grid's memory effects unless it synchronises by other means (flags, here).
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The other half: returns once every kernel that this launch depends on has completed and its writes are visible.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Orders this thread's earlier generic-proxy observations (a flag it acquired) before its later
 // asynchronous-proxy reads of global memory (bulk tensor loads of the rows that flag covers).
 __device__ __forceinline__ void fence_proxy_async_global() {

@@ -37,13 +37,14 @@ constexpr int kEpilogueWarps = 8;
 constexpr int kThreads = 32 * (2 + kEpilogueWarps);
 constexpr int kGatherThreads = 128;  // four more warps when A is gathered row by row (copy-engine gathers, so that the bytes
                                      // are counted like every other load's), on the 128-register build
+constexpr uint32_t kEarlyWeights = 2;   // GemmParams::after_previous
 constexpr int kGroupM = 16;     // m-tiles per rasterisation band (keeps a wave's A and B panels in L2)
 
 // CG = blocks per tile.  CG = 2: a pair of blocks on two neighbouring SMs owns a 256 x BN tile; each block stages its
 // own 128 rows of A and its half of B's columns, so a k block costs 32 KiB of staging per SM instead of 48.
 template <int BN, int CG>
 struct SmemLayout {
-    static constexpr int kStages = CG == 2 ? 6 : 4;
+    static constexpr int kStages = BN == 64 ? 8 : BN == 128 || CG == 2 ? 6 : 4;   // 192 KiB in flight whatever the tile
     static constexpr uint32_t kABytes = BM * BK * 2;
     static constexpr uint32_t kBBytes = BN / CG * BK * 2;
     static constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -139,6 +140,28 @@ __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &
     t.mt_index = __shfl_sync(0xffffffffu, t.mt_index, 0);
     t.valid = __shfl_sync(0xffffffffu, (uint32_t)t.valid, 0) != 0;
     return t;
+}
+
+// Reads a table of n + 1 <= 33 row offsets as a running maximum cut off at `limit`; true when that changed an entry.
+// One lane per entry: read one after the other they cost nine trips to L2 at the start of every grouped GEMM.
+__device__ __forceinline__ bool load_table(uint32_t *dst, const uint32_t *src, uint32_t stride, uint32_t n, uint32_t limit,
+                                           uint32_t lane) {
+    const uint32_t raw = lane <= n ? __ldcg(src + lane * stride) : 0u;
+    const uint32_t last = n == 32 ? __ldcg(src + 32u * stride) : 0u;   // the 33rd entry, in every lane
+    uint32_t v = min(raw, limit);
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, v, off);
+        if ((int)lane >= off) v = max(v, o);
+    }
+    if (lane <= n) dst[lane] = v;
+    bool changed = lane <= n && v != raw;
+    if (n == 32) {
+        const uint32_t top = max(min(last, limit), __shfl_sync(0xffffffffu, v, 31));
+        if (lane == 31) dst[32] = top;
+        changed = changed || top != last;
+    }
+    return __any_sync(0xffffffffu, changed) != 0;
 }
 
 // Four-row pieces of a 128-row tile at m0 that hold rows of its group.
@@ -273,40 +296,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t ep_epoch = p.ep.epoch_counter ? __ldcg(p.ep.epoch_counter) + 1u : p.ep.epoch;
     // hand-over counters: two sets used by alternate passes; this pass's set was cleared during the previous one
     uint32_t *const progress = p.ep.progress ? p.ep.progress + (ep_epoch & 1u) * p.ep.progress_len : nullptr;
-    if (p.experts && threadIdx.x == 64) {
+    // A launch that starts early (programmatic stream serialization) touches nothing of the kernels before it until
+    // they have completed; only then may the next one start early, so that what lies two launches back is complete.
+    // The second GEMM of a pair launched together (kEarlyWeights) does read its weights and the segment table ahead:
+    // the GEMM just before it writes neither, and everything before that one is complete.
+    const bool early = p.after_previous == kEarlyWeights;
+    if (p.experts && warp == 2) {
         // The dispatch kernel that writes the table may still be running beside this kernel: wait for its
         // "table written" flag before reading (bounded like every wait).
-        s_table_bad = 0;
-        if (p.ep.table_flag && !flag_wait(p.ep.table_flag, ep_epoch, p.ep.spin_limit)) {
-            s_table_bad = 1;
-            kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
-        }
+        if (p.after_previous && !early) grid_dependency_wait();
+        const bool here = !p.ep.table_flag || flag_wait(p.ep.table_flag, ep_epoch, p.ep.spin_limit);
+        if (!__all_sync(0xffffffffu, here) && lane == 0) kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
+        if (lane == 0) s_table_bad = !here;
 #ifdef FE2O3_EP_TRACE
-        if (p.ep.trace_flags && p.ep.table_flag && p.ep.progress_mode != 2 && blockIdx.x == 0) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_TABLE_HERE);
+        if (lane == 0 && p.ep.trace_flags && p.ep.table_flag && p.ep.progress_mode != 2 && blockIdx.x == 0) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_TABLE_HERE);
 #endif
         // The segment table is device data (in the expert-parallel layer it derives from other ranks'
         // counts): it is made monotone and cut off at M here, so that no row index derived from it can
         // leave A or C, and the fault is reported instead.
-        const uint32_t stride = p.ep.pair_offsets ? p.ep.world : 1u;
-        uint32_t prev = 0;
-        bool bad = false;
-        for (uint32_t i = 0; i <= p.experts; ++i) {
-            uint32_t v = __ldcg(p.expert_offsets + i * stride);
-            if (v < prev || v > p.M) { bad = true; v = v < prev ? prev : p.M; }
-            s_off[i] = v;
-            prev = v;
-        }
-        if (bad) kstatus_set(p.status, FE2O3_KSTATUS_SLOT_RANGE);
-    }
-    if (p.ep.pair_offsets && threadIdx.x == 64) {   // the thread that has waited for the table
-        const uint32_t pairs = p.experts * p.ep.world;   // at most 32
-        uint32_t prev = 0;
-        for (uint32_t i = 0; i <= pairs; ++i) {   // monotone and inside A, like the segment table
-            uint32_t v = __ldcg(p.ep.pair_offsets + i);
-            v = v < prev ? prev : (v > p.M ? p.M : v);
-            s_pair[i] = v;
-            prev = v;
-        }
+        if (load_table(s_off, p.expert_offsets, p.ep.pair_offsets ? p.ep.world : 1u, p.experts, p.M, lane) && lane == 0)
+            kstatus_set(p.status, FE2O3_KSTATUS_SLOT_RANGE);
+        if (p.ep.pair_offsets) load_table(s_pair, p.ep.pair_offsets, 1u, p.experts * p.ep.world, p.M, lane);   // at most 32 pairs
     }
     if (p.ep.peer_ret)
         for (uint32_t i = threadIdx.x; i < p.ep.world; i += blockDim.x) s_peer[i] = p.ep.peer_ret[i];
@@ -327,6 +337,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncthreads();
     if constexpr (CG == 2) cluster_sync();   // the other block's barriers are initialised
     tc_fence_after();
+    if (p.after_previous && !(early && warp == 0)) {
+        grid_dependency_wait();
+        launch_dependents();
+    }
     const uint32_t tmem_base = *tmem_slot;
     // A role that gives up ends the other roles' waits too, in both blocks of a pair.
     auto give_up = [&] {
@@ -344,6 +358,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         __syncwarp();
         uint32_t stage = 0, phase = 0, loaded = 0;
+        uint32_t primed = 0; // k blocks of the first tile whose weights were fetched ahead of the wait
         uint32_t seen = 0;   // sources whose "rows complete" flag this CTA has already acquired
         bool ok = !dead;
         for (uint32_t id = first_tile; ok; id += tile_step) {
@@ -386,47 +401,67 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 fence_proxy_async_global();
             }
-            // bytes of a k block that rank 0's (or the only) barrier counts; of a gathered A only rows of the group are fetched
+            // bytes of a k block that rank 0's (or the only) barrier counts: of A only what holds rows of the group
             uint32_t bytes = CG * L::kStageBytes;
             if (p.gather_perm) {
                 bytes = CG * L::kBBytes + gathered_quads(t.m0, t.m_end) * 512u;
                 if (CG == 2) bytes += gathered_quads(t.m0 + BM, t.m_end) * 512u;   // (rank 1's rows; only rank 0 uses this)
+            } else if (CG == 1 && p.a_box_rows < (uint32_t)BM) {
+                bytes = L::kBBytes + (gathered_quads(t.m0, t.m_end) * 4 + p.a_box_rows - 1) / p.a_box_rows * p.a_box_rows * 128u;
+            }
+            auto load_a = [&](uint32_t kb, uint32_t st) {   // one lane
+                uint8_t *sa = smem + st * L::kStageBytes;
+                const int32_t x = (int32_t)(kb * BK);
+                if constexpr (CG == 2) {
+                    tma_load_2d_pair(sa, &tmA, cluster_addr(&full[st], 0), x, (int32_t)t.m0);
+                } else {
+                    tma_load_2d(sa, &tmA, &full[st], x, (int32_t)t.m0);
+                    for (uint32_t r = p.a_box_rows; r < (uint32_t)BM && t.m0 + r < t.m_end; r += p.a_box_rows)
+                        tma_load_2d(sa + r * 128, &tmA, &full[st], x, (int32_t)(t.m0 + r));
+                }
+            };
+            auto load_b = [&](uint32_t kb, uint32_t st) {   // one lane; sets the expectation first
+                uint8_t *sb = smem + st * L::kStageBytes + L::kABytes;
+                if constexpr (CG == 2) {
+                    // both blocks' bytes are counted by rank 0's barrier; rank 1's may arrive before the
+                    // expectation is set, which the barrier's pending arrival makes harmless
+                    const uint32_t bar = cluster_addr(&full[st], 0);
+                    if (crank == 0) mbar_arrive_expect_tx(&full[st], bytes);
+#pragma unroll
+                    for (int j = 0; j < BN / CG / 64; ++j) {
+                        const int32_t col = (int32_t)(t.n0 * BN + crank * (BN / CG) + j * 64);
+                        if (p.experts) tma_load_3d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK), (int32_t)t.expert);
+                        else tma_load_2d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK));
+                    }
+                } else {
+                    mbar_arrive_expect_tx(&full[st], bytes);
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) {
+                        const int32_t col = (int32_t)(t.n0 * BN + j * 64);
+                        if (p.experts) tma_load_3d(sb + j * 8192, &tmB, &full[st], col, (int32_t)(kb * BK), (int32_t)t.expert);
+                        else tma_load_2d(sb + j * 8192, &tmB, &full[st], col, (int32_t)(kb * BK));
+                    }
+                }
+            };
+            if (early && id == first_tile) {   // the whole ring is free: its weights first, then the rows once they are there
+                primed = min((uint32_t)kStages, num_kb);
+                if (elect_one())
+                    for (uint32_t kb = 0; kb < primed; ++kb) load_b(kb, kb);
+                __syncwarp();
+                grid_dependency_wait();
             }
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++loaded) {
                 if (!mbar_wait_warp(&empty[stage], phase ^ 1, &s_abort)) { ok = false; break; }
                 if (elect_one()) {
-                    uint8_t *sa = smem + stage * L::kStageBytes;
-                    uint8_t *sb = sa + L::kABytes;
-                    if constexpr (CG == 2) {
-                        // both blocks' bytes are counted by rank 0's barrier; rank 1's may arrive before the
-                        // expectation is set, which the barrier's pending arrival makes harmless
-                        const uint32_t bar = cluster_addr(&full[stage], 0);
-                        if (crank == 0) mbar_arrive_expect_tx(&full[stage], bytes);
-                        if (!p.gather_perm) tma_load_2d_pair(sa, &tmA, bar, (int32_t)(kb * BK), (int32_t)t.m0);
-#pragma unroll
-                        for (int j = 0; j < BN / CG / 64; ++j) {
-                            const int32_t col = (int32_t)(t.n0 * BN + crank * (BN / CG) + j * 64);
-                            if (p.experts) tma_load_3d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK), (int32_t)t.expert);
-                            else tma_load_2d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK));
-                        }
-                    } else {
-                        mbar_arrive_expect_tx(&full[stage], bytes);
-                        if (!p.gather_perm) tma_load_2d(sa, &tmA, &full[stage], (int32_t)(kb * BK), (int32_t)t.m0);
-#pragma unroll
-                        for (int j = 0; j < BN / 64; ++j) {
-                            if (p.experts)
-                                tma_load_3d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK),
-                                            (int32_t)t.expert);
-                            else
-                                tma_load_2d(sb + j * 8192, &tmB, &full[stage], (int32_t)(t.n0 * BN + j * 64), (int32_t)(kb * BK));
-                        }
-                    }
+                    if (loaded >= primed) load_b(kb, stage);
+                    if (!p.gather_perm) load_a(kb, stage);
                 }
                 __syncwarp();
                 if (++stage == kStages) { stage = 0; phase ^= 1; }
             }
         }
         if (!ok && lane == 0) give_up();
+        if (early && primed == 0) grid_dependency_wait();
         // Drain: every copy issued must have landed before the CTA exits (the newest phase of each ring slot).
         // Rank 1's copies are counted by rank 0's barriers, and no block of a pair leaves before the other.
         for (uint32_t b = 0; crank == 0 && b < kStages && b < loaded; ++b) {
@@ -833,14 +868,44 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
                      uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta, uint32_t epilogue,
                      const uint32_t *expert_offsets, uint32_t experts, uint32_t expert_mod, uint32_t b_matrices,
                      const GemmEp *ep, uint32_t expected_rows) {
-    // 256-wide tiles whenever N allows.  Half-width tiles would fill the last round of SMs better when a rank
-    // has few row tiles (512 tiles on 148 SMs are 4 rounds, 1024 half tiles 7 half rounds), but they re-read A
-    // twice as often and were measured slower, not faster, on 4096 and 8192 rows (passes of 530 against 481 us
-    // and 686 against 590 us).
-    plan->bn = (N > 128) ? 256 : 128;
+    // Tile shape.  A launch costs its rounds of tiles times what a round takes, which beyond the fixed ~4 us of a
+    // launch goes as 0.55 : 0.68 : 1 for 64, 128 and 256 columns (measured, us: 1024^3 8.3 : 9.4 : 11.3 in one round
+    // each, 2048x2048x512 14.4 : 11.1 : 9.3 in four, two and one), so a small result takes the narrowest tile that
+    // still needs one round: 512^3 8.4 -> 6.1, 1536^3 14.1 -> 11.8.
+    // 256-row tiles on pairs of SMs stage a third less per multiply-add, which shortens a round by about a tenth
+    // where the k loop sets its length: 8192^3 907 against 832 us, 2048x2048x4096 36.9 against 34.8.  A pair's two
+    // epilogues run in step, so where the output does (K = 128 of 8192x8192: 54 against 61 us, K = 1024: 13.9
+    // against 14.3) single blocks stay, as they do where coarser tiles make more rounds (512 rows an expert, d 2048:
+    // 194 against 209 us a layer pass).  Groups end in a partly filled tile, half of one on average.
+    // The expert-parallel GEMMs count finished 256-wide tiles and keep them: half-width ones re-read A twice as
+    // often and were slower there on 4096 and 8192 rows (530 against 481 us and 686 against 590 us a pass).
     (void)expected_rows;
+    plan->bn = N > 128 ? 256 : 128;
+    plan->pair = 0;
+    uint32_t a_box = BM;
+    if (!ep) {
+        const uint64_t sms = ctx->sm_count;
+        auto rounds = [&](uint64_t tile_rows, uint64_t tile_cols, uint64_t slots) {
+            uint64_t m_tiles = (M + tile_rows - 1) / tile_rows;
+            if (experts) m_tiles = M <= experts * tile_rows / 2 ? experts : (2 * (uint64_t)M + experts * tile_rows) / (2 * tile_rows);
+            return (m_tiles * ((N + tile_cols - 1) / tile_cols) + slots - 1) / slots;
+        };
+        uint64_t best = 100 * rounds(BM, 256, sms);
+        plan->bn = 256;
+        auto consider = [&](uint32_t bn, uint32_t pair, uint64_t cost) {
+            if (cost < best) { best = cost; plan->bn = bn; plan->pair = pair; }
+        };
+        if (K > 1024 && N > 128 && sms >= 2) consider(256, 1, 90 * rounds(2 * BM, 256, sms / 2));
+        consider(128, 0, 68 * rounds(BM, 128, sms));
+        // (bf16 output leaves in pieces of 64 columns a warp, half a tile's columns)
+        if (epilogue != EPI_GELU_BF16) consider(64, 0, 55 * rounds(BM, 64, sms));
+        // A group's tile takes only the copies of A that hold its rows: of 32 rows up to 24 rows a group on average
+        // (16 rows, d 2048: 96.5 -> 93.6 us a layer pass), of 64 up to 48; with more, one copy of the whole tile is
+        // cheaper than several (64 rows a group: 98.2 against 96.3 us)
+        if (experts && !plan->pair) a_box = M <= 24 * experts ? 32 : M <= 48 * experts ? 64 : BM;
+    }
     uint64_t dA[2] = {K, M}, sA[1] = {(uint64_t)lda * 2};
-    uint32_t bA[2] = {BK, BM};
+    uint32_t bA[2] = {BK, a_box};
     int32_t st = fe2o3_make_tmap_bf16(&plan->tmA, a, 2, dA, sA, bA);
     if (st != FE2O3_OK) return st;
     if (experts) {
@@ -866,33 +931,15 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
         bulk = 1;
     }
     plan->p = GemmParams{reinterpret_cast<void *>(c), M, N, K, ldc, alpha, beta, epilogue, expert_offsets, experts,
-                         expert_mod, bulk, ctx->status_word, ep ? *ep : GemmEp{}, nullptr, nullptr, 0u, nullptr, nullptr, 0u, nullptr, 0ull};
+                         expert_mod, bulk, ctx->status_word, ep ? *ep : GemmEp{}, nullptr, nullptr, 0u, nullptr, nullptr, 0u, nullptr, 0ull, a_box, 0u};
+    plan->p.after_previous = ep ? 0u : 1u;
     const uint32_t n_tiles = (N + plan->bn - 1) / plan->bn;
-    const uint64_t m_tiles = (uint64_t)(M + BM - 1) / BM + experts;  // grouped: each expert may add a ragged tile
-    uint64_t tiles = m_tiles * n_tiles;
-    plan->grid = (uint32_t)(tiles < (uint64_t)ctx->sm_count ? (tiles ? tiles : 1) : (uint64_t)ctx->sm_count);
-    plan->smem = plan->bn == 256 ? SmemLayout<256, 1>::kTotal : SmemLayout<128, 1>::kTotal;
-    // 256-row tiles on pairs of SMs stage a third less per multiply-add, which shortens a round of tiles by about a
-    // tenth where the k loop sets its length: 8192^3 907 against 832 us, 2048x2048x4096 36.9 against 34.8 (both
-    // orders in one call).  A pair's two epilogues run in step, so where the output does (K = 128 of 8192x8192: 54
-    // against 61 us, K = 1024: 13.9 against 14.3) the single blocks stay; and they stay where the coarser tiles make
-    // more rounds (512 rows an expert, d 2048: 194 against 209 us a layer pass).  Groups end in a partly filled tile,
-    // half of one on average.
-    plan->pair = 0;
-    if (plan->bn == 256 && K > 1024 && !ep && ctx->sm_count >= 2) {
-        auto rounds = [&](uint64_t rows_per_tile, uint64_t slots) {
-            const uint64_t m_tiles = experts ? (2 * (uint64_t)M + experts * rows_per_tile) / (2 * rows_per_tile)
-                                             : (M + rows_per_tile - 1) / rows_per_tile;
-            return (m_tiles * n_tiles + slots - 1) / slots;
-        };
-        const uint64_t pairs = ctx->sm_count / 2;
-        if (9 * rounds(2 * BM, pairs) < 10 * rounds(BM, ctx->sm_count)) {
-            plan->pair = 1;
-            tiles = ((uint64_t)(M + 2 * BM - 1) / (2 * BM) + experts) * n_tiles;
-            plan->grid = 2 * (uint32_t)(tiles < pairs ? (tiles ? tiles : 1) : pairs);
-            plan->smem = SmemLayout<256, 2>::kTotal;
-        }
-    }
+    const uint64_t tile_rows = plan->pair ? 2 * BM : BM;
+    const uint64_t m_tiles = (M + tile_rows - 1) / tile_rows + experts;  // grouped: each expert may add a ragged tile
+    const uint32_t group = plan->pair ? 2 : 1;   // blocks per tile
+    const uint64_t tiles = m_tiles * n_tiles, slots = ctx->sm_count / group;
+    plan->grid = group * (uint32_t)(tiles < slots ? (tiles ? tiles : 1) : slots);
+    plan->smem = plan->pair ? SmemLayout<256, 2>::kTotal : plan->bn == 256 ? SmemLayout<256, 1>::kTotal : plan->bn == 128 ? SmemLayout<128, 1>::kTotal : SmemLayout<64, 1>::kTotal;
     plan->overlap_previous = 0;
     return FE2O3_OK;
 }
@@ -902,6 +949,7 @@ int32_t gemm_tc_init_device() {
     auto set = [](auto kernel, uint32_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
     FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 1>, SmemLayout<256, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<128, 168, 1>, SmemLayout<128, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<64, 168, 1>, SmemLayout<64, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 1>, SmemLayout<256, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<128, 128, 1>, SmemLayout<128, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 2>, SmemLayout<256, 2>::kTotal));
@@ -916,19 +964,18 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
     cfg.blockDim = dim3(kThreads + (plan->p.gather_perm ? kGatherThreads : 0), 1, 1);
     cfg.dynamicSmemBytes = plan->smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (plan->pair) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim = {2, 1, 1};
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    } else if (plan->overlap_previous) {
-        // programmatic dependent launch: the kernel may start while the kernel before it in the stream (the
-        // expert-parallel dispatch, which says when) is still running; the two synchronise through flags
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs++].val.clusterDim = {2, 1, 1};
+    }
+    if (plan->overlap_previous || plan->p.after_previous) {
+        // programmatic dependent launch: the kernel may start while the kernel before it in the stream is still
+        // running.  The expert-parallel GEMMs and the kernels before them (which say when) synchronise through
+        // flags; the others wait inside for that kernel to complete, with their set-up behind them.
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     cudaError_t e;
     // the 128-register build: for a block that shares its SM with the small blocks of the kernel before it, and for
@@ -939,7 +986,8 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
                        : plan->bn == 256 ? launch(gemm_tc_kernel<256, 128, 1>) : launch(gemm_tc_kernel<128, 128, 1>);
     else
         e = plan->pair ? launch(gemm_tc_kernel<256, 168, 2>)
-                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 168, 1>) : launch(gemm_tc_kernel<128, 168, 1>);
+                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 168, 1>)
+                       : plan->bn == 128 ? launch(gemm_tc_kernel<128, 168, 1>) : launch(gemm_tc_kernel<64, 168, 1>);
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "gemm_tc");
 }
@@ -964,6 +1012,12 @@ void gemm_tc_set_combine(GemmTcPlan *plan, const uint32_t *perm, const float *we
     plan->p.combine_perm = perm;
     plan->p.combine_weights = weights;
     plan->p.combine_tokens = tokens;
+}
+
+// The launch just before this one on the stream is the GEMM whose output is this one's A, and writes nothing else that
+// this one reads: its weights may be fetched while that one still runs.
+void gemm_tc_set_early_weights(GemmTcPlan *plan) {
+    if (plan->p.after_previous) plan->p.after_previous = kEarlyWeights;
 }
 
 void gemm_tc_geometry(const GemmTcPlan *plan, fe2o3_geometry *geo) {

@@ -66,6 +66,9 @@ struct GemmParams {
     // expert FFN clears the output that the second one accumulates into.
     uint4 *zero_ptr;
     uint64_t zero_vecs;
+    uint32_t a_box_rows;     // rows of one A copy (a tile of a group with few rows takes only the copies that hold some)
+    uint32_t after_previous; // launched early (programmatic stream serialization): 1 = waits for the kernels before it before
+                             // it touches memory, 2 = fetches its first weights and the segment table ahead of that wait
 };
 
 struct GemmTcPlan {
@@ -76,7 +79,8 @@ struct GemmTcPlan {
     uint32_t grid;
     uint32_t smem;
     uint32_t overlap_previous;   // launch with programmatic stream serialization: 1 = may run beside the (small) blocks of the
-                                 // kernel before it on the same SMs, 2 = takes over SMs as blocks of the kernel before it exit
+                                 // kernel before it on the same SMs, 2 = takes over SMs as blocks of the kernel before it exit (these two
+                                 // synchronise through flags); 0 = started early too, but waits for that kernel to complete
 };
 
 int32_t fe2o3_make_tmap_bf16(CUtensorMap *out, uint64_t base, uint32_t rank, const uint64_t *dims,
@@ -92,4 +96,5 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s);
 int32_t gemm_tc_init_device();
 bool gemm_tc_set_gather(GemmTcPlan *plan, const uint32_t *perm, const void *src, uint32_t tokens);
 void gemm_tc_set_combine(GemmTcPlan *plan, const uint32_t *perm, const float *weights, uint32_t tokens);
+void gemm_tc_set_early_weights(GemmTcPlan *plan);
 void gemm_tc_geometry(const GemmTcPlan *plan, fe2o3_geometry *geo);

@@ -52,10 +52,12 @@ def test_gemm_tcgen05_direct_output_exact(gpu, orc, m, n, k, ldc, offset):
             assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
 
 
-# ---- tensor-core GEMM on pairs of SMs (k above 1024): second half of a pair without rows or columns, ragged ends
-@pytest.mark.parametrize("m,n,k,ldc,beta", [(128, 264, 1032, 264, 0.0), (129, 384, 1088, 384, 0.0), (256, 512, 1056, 512, -1.0),
-                                            (257, 392, 1100, 395, 0.5), (1, 130, 1025, 131, -1.0), (700, 2600, 1040, 2600, 0.0)])
-def test_gemm_pair_tiles_exact(gpu, orc, m, n, k, ldc, beta):
+# ---- tensor-core GEMM tile shapes: 64, 128 and 256 columns, and pairs of SMs (k above 1024) whose second half has
+# no rows or no columns
+@pytest.mark.parametrize("m,n,k,ldc,beta", [(1, 130, 1025, 131, -1.0), (129, 72, 520, 72, 0.0), (1000, 1000, 96, 1003, 0.5),
+                                            (1100, 2050, 64, 2052, 0.0), (1281, 1912, 1032, 1912, 0.0), (1281, 2000, 1100, 2003, -1.0),
+                                            (700, 3400, 1040, 3400, 0.0), (700, 3400, 72, 3400, 0.0)])
+def test_gemm_tile_shapes_exact(gpu, orc, m, n, k, ldc, beta):
     fe, ctx, stream = gpu
     from fe2o3_b200 import synth
     lda, ldb = (k + 7) // 8 * 8, (n + 7) // 8 * 8
@@ -72,8 +74,10 @@ def test_gemm_pair_tiles_exact(gpu, orc, m, n, k, ldc, beta):
         assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
 
 
-@pytest.mark.parametrize("T,d,f,E,cap", [(300, 1088, 1152, 4, 600), (900, 1152, 1088, 4, 250)])
-def test_moe_pair_tiles(gpu, orc, T, d, f, E, cap):
+@pytest.mark.parametrize("T,d,f,E,cap", [(1000, 1088, 1152, 4, 2000), (1040, 1152, 1088, 4, 500),
+                                         # few rows a group: copies of 32 and 64 rows, groups without rows
+                                         (1, 128, 256, 8, 2), (40, 128, 256, 4, 3), (90, 192, 320, 4, 180)])
+def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     from test_gpu_parity import assert_close, moe_pipeline
     compact, want_compact, out, want_out, accepted = moe_pipeline(gpu, orc, T, d, f, E, cap)
     assert_close(out, want_out, 2e-2, 2e-3, "combined output")
