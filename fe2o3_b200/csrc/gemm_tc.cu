@@ -169,6 +169,9 @@ __device__ __forceinline__ uint32_t gathered_quads(uint32_t m0, uint32_t m_end) 
     return m_end > m0 ? (min(m_end - m0, (uint32_t)BM) + 3) / 4 : 0u;
 }
 
+// ... and those that its four gather warps, which take them in turn, fetch: one each at least.
+__device__ __forceinline__ uint32_t fetched_quads(uint32_t m0, uint32_t m_end) { return max(gathered_quads(m0, m_end), 4u); }
+
 // erf by Abramowitz & Stegun 7.1.26 (absolute error below 1.5e-7, far under the bf16 step of the
 // hidden activations this feeds): one reciprocal, one exp2 and a degree-5 polynomial, no branches.
 __device__ __forceinline__ float gelu_erf(float x) {
@@ -404,8 +407,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // bytes of a k block that rank 0's (or the only) barrier counts: of A only what holds rows of the group
             uint32_t bytes = CG * L::kStageBytes;
             if (p.gather_perm) {
-                bytes = CG * L::kBBytes + gathered_quads(t.m0, t.m_end) * 512u;
-                if (CG == 2) bytes += gathered_quads(t.m0 + BM, t.m_end) * 512u;   // (rank 1's rows; only rank 0 uses this)
+                bytes = CG * L::kBBytes + fetched_quads(t.m0, t.m_end) * 512u;
+                if (CG == 2) bytes += fetched_quads(t.m0 + BM, t.m_end) * 512u;   // (rank 1's rows; only rank 0 uses this)
             } else if (CG == 1 && p.a_box_rows < (uint32_t)BM) {
                 bytes = L::kBBytes + (gathered_quads(t.m0, t.m_end) * 4 + p.a_box_rows - 1) / p.a_box_rows * p.a_box_rows * 128u;
             }
@@ -515,19 +518,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (!ok && crank == 0 && lane == 0) give_up();
     } else if (warp >= 2 + kEpilogueWarps) {
         // ------------------------------------------------ gather issuers (blocks launched with them only)
-        // Four warps fetch 32 rows of the tile each, four rows an instruction, by the copy engine: the rows' token
+        // Four warps fetch the tile's rows in turn, four rows an instruction, by the copy engine: the rows' token
         // numbers sit in registers for the whole tile.  A slot without a route names the row after the last token,
         // which the copy engine fills with zeros; whole quads past the group's end are not fetched (what they leave in
-        // the stage only reaches rows of the accumulator that nobody stores).
-        const uint32_t r0 = (warp - (2 + kEpilogueWarps)) * 32;
+        // the stage only reaches rows of the accumulator that nobody stores).  Every warp fetches one quad of each k block
+        // at least: if nothing of a stage waited for it, the ring could run on while it still waits for an earlier
+        // phase, whose parity would then have come and gone.
+        const uint32_t gw = warp - (2 + kEpilogueWarps);   // quads gw, gw + 4, ...
         uint32_t stage = 0, phase = 0;
         bool ok = !dead;
         for (uint32_t id = first_tile; ok; id += tile_step) {
             TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;
-            const uint32_t quads = gathered_quads(t.m0 + r0, t.m_end);   // of this warp's 32 rows: 8 or fewer count
-            const uint32_t row = t.m0 + r0 + lane;
+            const uint32_t quads = (fetched_quads(t.m0, t.m_end) + 3 - gw) / 4;   // this warp's: 1 to 8
+            const uint32_t row = t.m0 + ((lane >> 2) * 4 + gw) * 4 + (lane & 3);
             const uint32_t route = row < t.m_end ? __ldg(p.gather_perm + row) : 0xffffffffu;
             const uint32_t mine = route == 0xffffffffu ? p.gather_tokens : min(route >> 1, p.gather_tokens);
             int32_t tok[32];
@@ -536,10 +541,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_warp(&empty[stage], phase ^ 1, &s_abort)) { ok = false; break; }
                 if (elect_one()) {
-                    uint8_t *sa = smem + stage * L::kStageBytes + r0 * 128;
+                    uint8_t *sa = smem + stage * L::kStageBytes + gw * 512;
                     const uint32_t bar = CG == 2 ? cluster_addr(&full[stage], 0) : smem_u32(&full[stage]);
                     auto fetch = [&](int i) {
-                        tma_gather4<CG == 2>(sa + i * 512, &tmA, bar, (int32_t)(kb * BK), tok[4 * i], tok[4 * i + 1], tok[4 * i + 2],
+                        tma_gather4<CG == 2>(sa + i * 2048, &tmA, bar, (int32_t)(kb * BK), tok[4 * i], tok[4 * i + 1], tok[4 * i + 2],
                                              tok[4 * i + 3]);
                     };
                     if (quads >= 8) {
@@ -548,7 +553,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     } else {
 #pragma unroll
                         for (int i = 0; i < 7; ++i)
-                            if (i < (int)quads) fetch(i);
+                            if (i == 0 || i < (int)quads) fetch(i);
                     }
                 }
                 __syncwarp();

@@ -84,6 +84,26 @@ def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
 
 
+def test_moe_layer_of_few_tokens_many_passes(gpu):
+    """Groups of a few rows: gather warps without rows must stay in step with the ring.  No wait may run out and every
+    pass gives the same bits."""
+    fe, ctx, stream = gpu
+    import torch
+    from fe2o3_b200.moe import MoeTop2Layer
+    layers = [MoeTop2Layer(ctx, stream, T, 1024, 2048, 8) for T in (16, 33)]
+    for layer in layers:
+        for t in (layer.x, layer.wg, layer.w1, layer.w2):
+            t.normal_(0, 0.1)
+    want = [layer.forward().clone() for layer in layers]
+    for _ in range(1500):
+        for layer in layers:
+            layer.forward()
+    torch.cuda.synchronize()
+    assert ctx.take_kernel_status(stream) == 0
+    for layer, w in zip(layers, want):
+        assert (layer.out.view(torch.int32) == w.view(torch.int32)).all()
+
+
 # ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
 @pytest.mark.parametrize("cols", [3, 29, 32, 33, 61, 64, 65, 125, 129, 256, 513, 1021, 1024, 1025, 2045, 2048, 2050, 3001, 4093, 4094, 4095, 4096])
 def test_row_softmax_widths(gpu, orc, cols):
