@@ -51,6 +51,27 @@ int32_t fe2o3_cuda_status(cudaError_t e, const char *what);
         if (e__ != cudaSuccess) return fe2o3_cuda_status(e__, #call); \
     } while (0)
 
+// Launches a kernel that may start while the kernel before it in the stream drains (programmatic stream
+// serialization): it must call grid_dependency_wait before it touches global memory.  `cluster` blocks per cluster.
+template <typename... P, typename... A>
+static inline cudaError_t fe2o3_launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                             uint32_t cluster, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs++].val.clusterDim = {cluster, 1, 1};
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 static inline uint32_t ceil_div_u32(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 // Flag block of one rank of the expert-parallel layer, in u32 words (world = W):
@@ -152,6 +173,11 @@ __device__ __forceinline__ void ep_trace(uint32_t *, uint32_t) {}
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The other half: returns once every kernel that this launch depends on has completed and its writes are visible.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// First statement of a kernel launched early that has no set-up to overlap.
+__device__ __forceinline__ void begin_after_previous() {
+    grid_dependency_wait();
+    launch_dependents();
+}
 // Orders this thread's earlier generic-proxy observations (a flag it acquired) before its later
 // asynchronous-proxy reads of global memory (bulk tensor loads of the rows that flag covers).
 __device__ __forceinline__ void fence_proxy_async_global() {
@@ -314,6 +340,13 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t ld_shared_cluster(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -405,10 +405,8 @@ moe_gate_warp_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict_
 //     shares its counter).  The warp synchronises with itself only; there is no block barrier in
 //     the loop.  Rows are padded by 16 bytes so that the 16-byte reads of eight tokens do not
 //     collide on banks.
-//   The EPL logits of a lane advance as EPL / 2 packed f32x2 products and sums per k (each half
-//     rounded exactly like the scalar instruction).  EPL = 2 spreads a token over E / 2 lanes, so a
-//     rank's 2048 tokens of an expert-parallel layer still make 256 warps, each running at the pace
-//     of the dependent additions; EPL = 4 halves the instructions per multiply-add for large batches.
+//   The logits of a lane advance as packed f32x2 products and sums, two per instruction (each half
+//     rounded exactly like the scalar instruction).
 // Needs E in {4, 8, 16}, d_model a multiple of 64 with E * d_model * 4 bytes of shared memory
 // available, 16-byte aligned x and Wg.
 constexpr int kGateKC2 = 64;                       // k values per stage
@@ -436,6 +434,7 @@ moe_gate_lanes_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict
     uint8_t *ring = gate_lanes_smem + (size_t)d_model * E * 4 + (size_t)warp * STAGES * kStageBytes;
     const uint32_t tok0 = (blockIdx.x * WARPS + warp) * TPW;
     const uint32_t nchunks = d_model / kGateKC2;
+    begin_after_previous();
     auto copy_chunk = [&](uint32_t chunk) {
         if (chunk < nchunks) {
             uint8_t *stage = ring + (chunk % STAGES) * kStageBytes;
@@ -455,6 +454,7 @@ moe_gate_lanes_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict
     // the first chunks are on their way while the block widens Wg
 #pragma unroll
     for (int c = 0; c < STAGES - 1; ++c) copy_chunk(c);
+#pragma unroll 8
     for (uint32_t v = tid; v < d_model * E / 8; v += 32 * WARPS) {
         const uint4 w = __ldg(reinterpret_cast<const uint4 *>(wg) + v);
         float4 *dst = reinterpret_cast<float4 *>(gate_w + v * 8);
@@ -483,18 +483,13 @@ moe_gate_lanes_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float xf = __uint_as_float(h ? (words[i] & 0xffff0000u) : (words[i] << 16));
-                    const uint64_t xx = pack_f32x2(xf, xf);
                     const float *w = wk + (v * 8 + 2 * i + h) * E;
-                    if constexpr (EPL == 2) {
-                        const float2 a = *reinterpret_cast<const float2 *>(w);
-                        acc[0] = add_f32x2(acc[0], mul_f32x2(xx, pack_f32x2(a.x, a.y)));
-                    } else {
+                    const uint64_t xx = pack_f32x2(xf, xf);
 #pragma unroll
-                        for (int q = 0; q < EPL / 4; ++q) {
-                            const float4 a = *reinterpret_cast<const float4 *>(w + 4 * q);
-                            acc[2 * q] = add_f32x2(acc[2 * q], mul_f32x2(xx, pack_f32x2(a.x, a.y)));
-                            acc[2 * q + 1] = add_f32x2(acc[2 * q + 1], mul_f32x2(xx, pack_f32x2(a.z, a.w)));
-                        }
+                    for (int q = 0; q < EPL / 4; ++q) {
+                        const float4 a = *reinterpret_cast<const float4 *>(w + 4 * q);
+                        acc[2 * q] = add_f32x2(acc[2 * q], mul_f32x2(xx, pack_f32x2(a.x, a.y)));
+                        acc[2 * q + 1] = add_f32x2(acc[2 * q + 1], mul_f32x2(xx, pack_f32x2(a.z, a.w)));
                     }
                 }
             }
@@ -521,8 +516,103 @@ static cudaError_t launch_gate_lanes(cudaStream_t s, const uint16_t *x, const ui
     // the attribute is per device and cheap to set: set it on every launch for the current device
     cudaError_t e = cudaFuncSetAttribute(moe_gate_lanes_kernel<E, EPL, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    moe_gate_lanes_kernel<E, EPL, WARPS, STAGES><<<grid, 32 * WARPS, smem, s>>>(x, wg, lg, tokens, d_model);
-    return cudaSuccess;
+    return fe2o3_launch_early(moe_gate_lanes_kernel<E, EPL, WARPS, STAGES>, grid, 32 * WARPS, smem, s, 1, x, wg, lg, tokens, d_model);
+}
+
+// ---- gate logits of a moderate batch: one chain per lane, one warp per block ----------------
+// The same arithmetic and order.  The floor is the chain of d_model dependent additions (4 cycles each: 4.3 us at
+// d_model 2048), so everything else has to fit beside it: an addition's lane issues a product and 1.3 shared-memory
+// reads per k, of operands that are already f32.  Each warp streams 64 k of its 32 / E tokens and of Wg into a ring
+// with asynchronous copies, reads a landed chunk raw into registers before it adds up the chunk ahead of it, and
+// writes it back widened after that.  Nothing is shared between warps and there is no set-up pass over Wg, so 64
+// tokens of 8 experts are 16 blocks on 16 SMs: 19.4 us a launch with Wg widened once per block and two chains a lane, 12.0 so.
+template <int E>
+__global__ void __launch_bounds__(32)
+moe_gate_chain_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ wg, float *__restrict__ logits,
+                      uint32_t tokens, uint32_t d_model) {
+    constexpr int KC = 64, STAGES = 8, TPW = 32 / E;
+    constexpr int kXG = TPW * KC / 8, kWG = KC * E / 8;   // 16-byte pieces of a chunk of x and of Wg
+    constexpr int kXR = (kXG + 31) / 32, kWR = kWG / 32;
+    __shared__ __align__(16) uint4 ring[STAGES][kXG + kWG];
+    __shared__ __align__(16) float xs[2][TPW][KC + 4];
+    __shared__ __align__(16) float ws[2][KC * E];
+    const uint32_t lane = threadIdx.x, tt = lane / E, e = lane % E, tok0 = blockIdx.x * TPW, nchunks = d_model / KC;
+    begin_after_previous();
+    auto copy = [&](uint32_t c) {
+        if (c < nchunks) {
+            uint4 *stage = ring[c % STAGES];
+#pragma unroll
+            for (int i = 0; i < kXR; ++i) {
+                const uint32_t g = i * 32 + lane;
+                if (kXG % 32 == 0 || g < (uint32_t)kXG)   // rows beyond the batch re-read the last row
+                    cp_async_16(stage + g, x + (uint64_t)min(tok0 + (g >> 3), tokens - 1) * d_model + c * KC + (g & 7) * 8);
+            }
+#pragma unroll
+            for (int i = 0; i < kWR; ++i) cp_async_16(stage + kXG + i * 32 + lane, wg + (uint64_t)c * KC * E + (i * 32 + lane) * 8);
+        }
+        cp_async_commit();   // an empty group keeps the group count uniform at the tail
+    };
+    uint4 xr[kXR], wr[kWR];
+    auto read_raw = [&](uint32_t c) {
+        const uint4 *stage = ring[c % STAGES];
+#pragma unroll
+        for (int i = 0; i < kXR; ++i)
+            if (kXG % 32 == 0 || i * 32 + lane < (uint32_t)kXG) xr[i] = stage[i * 32 + lane];
+#pragma unroll
+        for (int i = 0; i < kWR; ++i) wr[i] = stage[kXG + i * 32 + lane];
+    };
+    auto widen_to = [](float *dst, uint4 v) {
+        reinterpret_cast<float4 *>(dst)[0] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u),
+                                                         __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+        reinterpret_cast<float4 *>(dst)[1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u),
+                                                         __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+    };
+    auto write_wide = [&](uint32_t buf) {
+#pragma unroll
+        for (int i = 0; i < kXR; ++i) {
+            const uint32_t g = i * 32 + lane;
+            if (kXG % 32 == 0 || g < (uint32_t)kXG) widen_to(&xs[buf][g >> 3][(g & 7) * 8], xr[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kWR; ++i) widen_to(&ws[buf][(i * 32 + lane) * 8], wr[i]);
+    };
+#pragma unroll
+    for (int c = 0; c < STAGES - 1; ++c) copy(c);
+    cp_async_wait<STAGES - 2>();
+    __syncwarp();
+    read_raw(0);
+    write_wide(0);
+    float acc = 0.0f;
+    for (uint32_t c = 0; c < nchunks; ++c) {
+        const uint32_t buf = c & 1;
+        copy(c + STAGES - 1);           // into the stage of chunk c - 1, which every lane has read
+        cp_async_wait<STAGES - 2>();    // this lane's pieces of chunk c + 1 have landed
+        __syncwarp();                   // everybody's have, and the widened chunk c is written
+        if (c + 1 < nchunks) read_raw(c + 1);
+        const float *xk = xs[buf][tt], *wk = ws[buf] + e;
+        float4 xn[2];
+        float wn[8];
+        auto operands = [&](int k) {
+            xn[0] = *reinterpret_cast<const float4 *>(xk + k);
+            xn[1] = *reinterpret_cast<const float4 *>(xk + k + 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) wn[i] = wk[(k + i) * E];
+        };
+        operands(0);
+#pragma unroll
+        for (int k = 0; k < KC; k += 8) {
+            const float xv[8] = {xn[0].x, xn[0].y, xn[0].z, xn[0].w, xn[1].x, xn[1].y, xn[1].z, xn[1].w};
+            float p[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) p[i] = __fmul_rn(xv[i], wn[i]);
+            if (k + 8 < KC) operands(k + 8);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc = __fadd_rn(acc, p[i]);
+        }
+        if (c + 1 < nchunks) write_wide(buf ^ 1);   // (chunk c - 1, which it held, is added up: the barrier above)
+    }
+    cp_async_wait<0>();
+    if (tok0 + tt < tokens) logits[(uint64_t)(tok0 + tt) * E + e] = acc;
 }
 
 // ---- top-2 routing over many blocks --------------------------------------------
@@ -707,11 +797,170 @@ moe_route_place_kernel(fe2o3_moe_top2_v1_args a, const uint32_t *scratch) {
     if (sb != kDrop) perm[sb] = 2u * t + 1u;
 }
 
+// ---- top-2 routing in one launch --------------------------------------------------
+// The same result again for batches that one cluster covers (eight blocks of 1024 threads, two tokens a thread).
+// What the two launches above take is almost all latency (6.7 + 5.8 us whatever the batch), so here every token is
+// read once: its selection stays in registers, the per-expert counts of warps and blocks are scanned in shared
+// memory and the blocks' totals are read from one another's shared memory between two cluster barriers.  Order of
+// the routes: block, pass, warp, lane = token order, rank 0 before rank 1 inside a token (a token's two routes go
+// to different experts).
+constexpr uint32_t kClusterRouteThreads = 1024, kClusterRoutePasses = 2, kClusterRouteBlocks = 8;
+
+template <int EE>
+__device__ __forceinline__ void top2_of_aligned_row(const float *row, uint32_t &best, uint32_t &second, bool &finite) {
+    float v[EE];
+#pragma unroll
+    for (int i = 0; i < EE; i += 4) {
+        const float4 q = __ldcg(reinterpret_cast<const float4 *>(row + i));
+        v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+    }
+    best = 0; second = kDrop;
+    float bs = v[0], ss = 0.f;
+    finite = isfinite(v[0]);
+#pragma unroll
+    for (uint32_t e = 1; e < EE; ++e) {
+        finite = finite && isfinite(v[e]);
+        if (precedes(v[e], e, bs, best)) {
+            second = best; ss = bs;
+            best = e; bs = v[e];
+        } else if (second == kDrop || precedes(v[e], e, ss, second)) {
+            second = e; ss = v[e];
+        }
+    }
+}
+
+template <int EE>   // experts, or 0: taken from the arguments
+__global__ void __launch_bounds__(kClusterRouteThreads)
+moe_route_cluster_kernel(fe2o3_moe_top2_v1_args a, uint32_t passes, uint32_t *status) {
+    __shared__ uint32_t s_cnt[kClusterRoutePasses * 32][33];   // [pass, warp][expert]: routes, then routes before
+    __shared__ uint32_t s_total[32], s_off[33], s_base[32];
+    __shared__ uint32_t s_bad, s_any_bad;
+    const uint32_t T = a.tokens, E = EE ? EE : a.experts, cap = a.capacity;
+    const uint64_t R = 2ull * T;
+    begin_after_previous();
+    if (a.logits.len != (uint64_t)T * E || a.top2_experts.len != R || a.requested_counts.len != E ||
+        a.admitted_counts.len != E || a.expert_offsets.len != E + 1 || a.route_slots.len != R ||
+        a.permutation.len != R || a.inverse.len != R || E < 2 || E > 32) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) kstatus_set(status, FE2O3_KSTATUS_LENGTH);
+        return;
+    }
+    const float *logits = reinterpret_cast<const float *>(a.logits.ptr);
+    uint32_t *top2 = reinterpret_cast<uint32_t *>(a.top2_experts.ptr);
+    uint32_t *slots = reinterpret_cast<uint32_t *>(a.route_slots.ptr);
+    uint32_t *perm = reinterpret_cast<uint32_t *>(a.permutation.ptr);
+    uint32_t *inverse = reinterpret_cast<uint32_t *>(a.inverse.ptr);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t best[kClusterRoutePasses], second[kClusterRoutePasses], pa[kClusterRoutePasses], pb[kClusterRoutePasses];
+    bool bad = false;
+#pragma unroll
+    for (uint32_t it = 0; it < kClusterRoutePasses; ++it) {
+        best[it] = second[it] = pa[it] = pb[it] = 0;
+        if (it >= passes) continue;
+        const uint32_t t = (blockIdx.x * passes + it) * blockDim.x + tid;
+        const bool active = t < T;
+        bool finite = true;
+        if (active) {
+            const float *row = logits + (uint64_t)t * E;
+            if constexpr (EE != 0) top2_of_aligned_row<EE>(row, best[it], second[it], finite);
+            else top2_of_row(row, E, best[it], second[it], finite);
+        }
+        bad = bad || !finite;
+        uint32_t mine = 0;   // lane e: this warp's routes to expert e
+        for (uint32_t e = 0; e < E; ++e) {
+            const uint32_t mb = __ballot_sync(0xffffffffu, active && best[it] == e);
+            const uint32_t ms = __ballot_sync(0xffffffffu, active && second[it] == e);
+            const uint32_t before = __popc(mb & lt) + __popc(ms & lt);
+            if (best[it] == e) pa[it] = before;
+            if (second[it] == e) pb[it] = before;
+            if (lane == e) mine = __popc(mb) + __popc(ms);
+        }
+        if (lane < E) s_cnt[it * warps + warp][lane] = mine;
+    }
+    const bool block_bad = __syncthreads_or(bad) != 0;
+    if (tid == 0) s_bad = block_bad;
+    for (uint32_t e = warp; e < E; e += warps) {
+        uint32_t running = 0;
+        for (uint32_t r0 = 0; r0 < passes * warps; r0 += 32) {
+            const uint32_t r = r0 + lane;
+            const uint32_t v = r < passes * warps ? s_cnt[r][e] : 0u;
+            uint32_t inc = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t n = __shfl_up_sync(0xffffffffu, inc, off);
+                if ((int)lane >= off) inc += n;
+            }
+            if (r < passes * warps) s_cnt[r][e] = running + inc - v;
+            running += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) s_total[e] = running;
+    }
+    cluster_sync();   // every block's totals are there
+    if (warp == 0) {
+        uint32_t base = 0, total = 0, any = 0;
+        for (uint32_t b = 0; b < gridDim.x; ++b) {   // the grid is one cluster
+            const uint32_t v = lane < E ? ld_shared_cluster(cluster_addr(&s_total[lane], b)) : 0u;
+            any |= ld_shared_cluster(cluster_addr(&s_bad, b));
+            if (b < blockIdx.x) base += v;
+            total += v;
+        }
+        const uint32_t adm = min(total, cap);
+        uint32_t inc = adm;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, inc, off);
+            if ((int)lane >= off) inc += n;
+        }
+        if (lane < E) {
+            s_base[lane] = base;
+            s_off[lane + 1] = inc;
+        }
+        if (lane == 0) {
+            s_off[0] = 0;
+            s_any_bad = any;
+        }
+        if (blockIdx.x == 0 && any == 0) {
+            uint32_t *offsets = reinterpret_cast<uint32_t *>(a.expert_offsets.ptr);
+            if (lane < E) {
+                reinterpret_cast<uint32_t *>(a.requested_counts.ptr)[lane] = total;
+                reinterpret_cast<uint32_t *>(a.admitted_counts.ptr)[lane] = adm;
+                offsets[lane + 1] = inc;
+            }
+            if (lane == 0) offsets[0] = 0;
+        }
+    }
+    __syncthreads();
+    cluster_arrive();   // this block has read what it needs of the others
+    if (s_any_bad) {    // failure preserves every output
+        if (blockIdx.x == 0 && tid == 0) kstatus_set(status, FE2O3_KSTATUS_NONFINITE);
+    } else {
+        for (uint64_t s = (uint64_t)s_off[E] + blockIdx.x * blockDim.x + tid; s < R; s += (uint64_t)gridDim.x * blockDim.x)
+            perm[s] = kDrop;   // unused tail of the permutation
+#pragma unroll
+        for (uint32_t it = 0; it < kClusterRoutePasses; ++it) {
+            const uint32_t t = (blockIdx.x * passes + it) * blockDim.x + tid;
+            if (it >= passes || t >= T) continue;
+            const uint32_t ea = best[it], eb = second[it], r = it * warps + warp;
+            const uint32_t ga = s_base[ea] + s_cnt[r][ea] + pa[it], gb = s_base[eb] + s_cnt[r][eb] + pb[it];
+            const uint32_t sa = ga < cap ? s_off[ea] + ga : kDrop, sb = gb < cap ? s_off[eb] + gb : kDrop;
+            const uint64_t at = 2ull * t;
+            top2[at] = ea; top2[at + 1] = eb;
+            slots[at] = sa; slots[at + 1] = sb;
+            inverse[at] = sa; inverse[at + 1] = sb;
+            if (sa != kDrop) perm[sa] = 2u * t;
+            if (sb != kDrop) perm[sb] = 2u * t + 1u;
+        }
+    }
+    __syncwarp();
+    cluster_wait();     // nobody leaves while another block may still read its totals
+}
+
 // ---- route weights ------------------------------------------------------------
 // One thread per token; the arithmetic is route_weight_pair (common.cuh).
 __global__ void moe_route_weights_kernel(const float *__restrict__ logits, const uint32_t *__restrict__ top2,
                                          float *__restrict__ weights, uint32_t tokens, uint32_t experts) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    begin_after_previous();
     if (t >= tokens) return;
     const float l0 = logits[(uint64_t)t * experts + top2[2ull * t]];
     const float l1 = logits[(uint64_t)t * experts + top2[2ull * t + 1]];
@@ -792,7 +1041,7 @@ moe_combine_kernel(const float *__restrict__ compact, const uint32_t *__restrict
 
 }  // namespace
 
-int32_t launch_moe_gate(fe2o3_ctx *, cudaStream_t s, const void *args, fe2o3_geometry *geo, bool plan_only) {
+int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_geometry *geo, bool plan_only) {
     const fe2o3_moe_gate_v1_args *a = static_cast<const fe2o3_moe_gate_v1_args *>(args);
     const uint32_t E = a->experts;
     const uint32_t tpb = E >= 256 ? 1 : 256 / E;
@@ -808,16 +1057,26 @@ int32_t launch_moe_gate(fe2o3_ctx *, cudaStream_t s, const void *args, fe2o3_geo
         const uint16_t *x = reinterpret_cast<const uint16_t *>(a->x.ptr), *wg = reinterpret_cast<const uint16_t *>(a->wg.ptr);
         float *lg = reinterpret_cast<float *>(a->logits.ptr);
         if (lanes_ok) {
-            // few tokens: two experts per lane (most warps, pace of the dependent sums); many: four per lane
-            const bool wide = a->tokens > 4096u;
-#define FE2O3_GATE_LANES(EE, g)                                                                                            \
-    (wide ? launch_gate_lanes<EE, 4, 8, 6>(s, x, wg, lg, a->tokens, a->d_model, g)                                         \
-          : launch_gate_lanes<EE, 2, 4, 8>(s, x, wg, lg, a->tokens, a->d_model, g))
-            fe2o3_geometry g{};
-            cudaError_t e = E == 4 ? FE2O3_GATE_LANES(4, &g) : E == 8 ? FE2O3_GATE_LANES(8, &g) : FE2O3_GATE_LANES(16, &g);
+            // One chain per lane while the pace is that of the dependent sums, four when a scheduler holds so many warps
+            // that instructions are (a layer pass, four against one chain, us: 64 tokens of 8 experts, d 2048: 92.0
+            // against 78.5; 4096 tokens: 314 against 309; 16384: 1052 against 1082; 5000 of 16 experts: 142.9 against 143.7)
+            const bool wide = (uint64_t)a->tokens * E > 65536u;
+            auto one_chain = E == 4 ? moe_gate_chain_kernel<4> : E == 8 ? moe_gate_chain_kernel<8> : moe_gate_chain_kernel<16>;
+            const uint32_t chain_grid = ceil_div_u32(a->tokens, 32 / E);
+#define FE2O3_GATE_LANES(EE, g) launch_gate_lanes<EE, 4, 8, 6>(s, x, wg, lg, a->tokens, a->d_model, g)
+            // Launched early, the blocks would pile up on the first SMs that the kernel before leaves (twelve to an SM:
+            // 107 against 94 us a pass of 512 tokens): they ask for so much shared memory that they spread evenly.
+            const uint32_t per_sm = ceil_div_u32(chain_grid, (uint32_t)ctx->sm_count);
+            const uint32_t own = E == 16 ? 29u : 20u;   // KiB of its own, with what each block reserves
+            const uint32_t spread = 220u / per_sm > own ? (220u / per_sm - own) * 1024u : 0u;
+            fe2o3_geometry g{{chain_grid, 1, 1}, {32, 1, 1}, wide ? 0u : spread, 1};
+            cudaError_t e = cudaSuccess;
+            if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, &g) : E == 8 ? FE2O3_GATE_LANES(8, &g) : FE2O3_GATE_LANES(16, &g);
             if (geo) *geo = g;
             if (plan_only) return FE2O3_OK;
-            e = E == 4 ? FE2O3_GATE_LANES(4, nullptr) : E == 8 ? FE2O3_GATE_LANES(8, nullptr) : FE2O3_GATE_LANES(16, nullptr);
+            if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, nullptr) : E == 8 ? FE2O3_GATE_LANES(8, nullptr) : FE2O3_GATE_LANES(16, nullptr);
+            else if (spread <= 48u * 1024u || (e = cudaFuncSetAttribute(one_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread)) == cudaSuccess)
+                e = fe2o3_launch_early(one_chain, chain_grid, 32, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
 #undef FE2O3_GATE_LANES
             if (e != cudaSuccess) return fe2o3_cuda_status(e, "moe_gate_v1");
             fe2o3_count_launch(1);
@@ -861,6 +1120,23 @@ int32_t launch_moe_top2(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_
     const uint32_t blocks = ceil_div_u32(a->tokens ? a->tokens : 1, kRouteBlock);
     // FE2O3_ROUTE_SINGLE_BLOCK=1 selects the one-block kernel (otherwise used beyond 4M tokens)
     static const bool force_single = getenv("FE2O3_ROUTE_SINGLE_BLOCK") != nullptr;
+    constexpr uint32_t kPerPass = kClusterRouteThreads * kClusterRouteBlocks;
+    if (a->tokens > 0 && a->tokens <= kPerPass * kClusterRoutePasses && !force_single) {
+        // small blocks: a block of 1024 threads takes 7.5 us where one of 64 takes 4.6
+        uint32_t cluster = 1;
+        while (cluster < kClusterRouteBlocks && cluster * 128u < a->tokens) cluster *= 2;
+        const uint32_t passes = ceil_div_u32(a->tokens, kPerPass);
+        const uint32_t threads = (ceil_div_u32(a->tokens, cluster * passes) + 31) / 32 * 32;
+        if (geo) *geo = fe2o3_geometry{{cluster, 1, 1}, {threads, 1, 1}, 0, 1};
+        if (plan_only) return FE2O3_OK;
+        const bool aligned = (a->logits.ptr & 15u) == 0;
+        auto kernel = aligned && a->experts == 8    ? moe_route_cluster_kernel<8>
+                      : aligned && a->experts == 16 ? moe_route_cluster_kernel<16>
+                                                    : moe_route_cluster_kernel<0>;
+        const cudaError_t e = fe2o3_launch_early(kernel, cluster, threads, 0, s, cluster, *a, passes, ctx->status_word);
+        fe2o3_count_launch(1);
+        return fe2o3_cuda_status(e, "moe_top2_v1");
+    }
     if (blocks <= FE2O3_ROUTE_MAX_BLOCKS && !force_single) {
         if (geo) *geo = fe2o3_geometry{{blocks, 1, 1}, {kRouteBlock, 1, 1}, 0, 2};
         if (plan_only) return FE2O3_OK;
@@ -884,12 +1160,11 @@ int32_t launch_moe_route_weights(fe2o3_ctx *, cudaStream_t s, const void *args, 
     const uint32_t grid = ceil_div_u32(a->tokens, 256);
     if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {256, 1, 1}, 0, 1};
     if (plan_only || a->tokens == 0) return FE2O3_OK;
-    moe_route_weights_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const float *>(a->logits.ptr),
-                                                  reinterpret_cast<const uint32_t *>(a->top2_experts.ptr),
-                                                  reinterpret_cast<float *>(a->route_weights.ptr), a->tokens,
-                                                  a->experts);
+    const cudaError_t e = fe2o3_launch_early(moe_route_weights_kernel, grid, 256, 0, s, 1, reinterpret_cast<const float *>(a->logits.ptr),
+                                             reinterpret_cast<const uint32_t *>(a->top2_experts.ptr),
+                                             reinterpret_cast<float *>(a->route_weights.ptr), a->tokens, a->experts);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "moe_route_weights_v1");
+    return fe2o3_cuda_status(e, "moe_route_weights_v1");
 }
 
 int32_t launch_moe_compact(cudaStream_t s, uint64_t x, uint64_t perm, uint64_t compact_x, uint32_t rows,

@@ -76,12 +76,40 @@ def test_gemm_tile_shapes_exact(gpu, orc, m, n, k, ldc, beta):
 
 @pytest.mark.parametrize("T,d,f,E,cap", [(1000, 1088, 1152, 4, 2000), (1040, 1152, 1088, 4, 500),
                                          # few rows a group: copies of 32 and 64 rows, groups without rows
-                                         (1, 128, 256, 8, 2), (40, 128, 256, 4, 3), (90, 192, 320, 4, 180)])
+                                         (1, 128, 256, 8, 2), (40, 128, 256, 4, 3), (90, 192, 320, 4, 180),
+                                         (64, 128, 128, 32, 128)])
 def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     from test_gpu_parity import assert_close, moe_pipeline
     compact, want_compact, out, want_out, accepted = moe_pipeline(gpu, orc, T, d, f, E, cap)
     assert_close(out, want_out, 2e-2, 2e-3, "combined output")
     assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
+
+
+# ---- routing in one launch: one warp to eight blocks of two passes, and the sizes around each step
+@pytest.mark.parametrize("T,E,cap,bad", [(1, 2, 1, 0), (33, 8, 100, 0), (1000, 5, 300, 0), (1024, 16, 2048, 0), (1025, 8, 200, 0),
+                                         (2049, 32, 4098, 0), (4097, 8, 900, 0), (8192, 8, 2100, 0), (8193, 16, 16386, 0),
+                                         (16384, 8, 4000, 0), (16385, 8, 4000, 0), (5000, 8, 10000, 1)])
+def test_moe_routing_one_launch_bit_exact(gpu, orc, T, E, cap, bad):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    logits = (np.round(synth.normal_f32(5, T + E, T * E, 1.0) * 8) / 8).astype(np.float32)   # ties between experts
+    if bad:
+        logits[T * E - 1] = np.inf
+    L = Guarded(fe, stream, logits)
+    R = 2 * T
+    outs = {k: Guarded(fe, stream, np.full(n, 0x12345678, np.uint32)) for k, n in
+            [("top2_experts", R), ("requested_counts", E), ("admitted_counts", E), ("expert_offsets", E + 1),
+             ("route_slots", R), ("permutation", R), ("inverse", R)]}
+    p = fe.prepare(ctx, "moe_top2_v1", logits=L.slice, tokens=T, experts=E, capacity=cap, **{k: g.slice for k, g in outs.items()})
+    if bad:   # refused, with every block's outputs as they were
+        with pytest.raises(fe.Fe2o3Error):
+            p.launch_and_wait(stream)
+        assert p.kernel_status == 2 and all((g.read() == 0x12345678).all() for g in outs.values())
+        return
+    p.launch_and_wait(stream)
+    _, want = orc.moe_top2_route(logits, T, E, cap)
+    for k, g in outs.items():
+        assert (g.read() == want[k]).all(), k
 
 
 def test_moe_layer_of_few_tokens_many_passes(gpu):
