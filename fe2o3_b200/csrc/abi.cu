@@ -882,6 +882,7 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
         delete ctx;
         return fe2o3_cuda_status(e, "cudaMalloc(scan scratch)");
     }
+    cudaMemset(ctx->scan_scratch, 0, FE2O3_SCAN_SCRATCH_BYTES);
     *out = ctx;
     return FE2O3_OK;
 }

@@ -36,13 +36,15 @@
 // separately: whichever block computes a tile's prefix performs the same chain of additions, and
 // repeated runs give identical bits.  The lane prefix inside a warp scan comes from a shuffle
 // instead of a subtraction.
-// A descriptor is one 64-bit word {state, value}; it carries everything its reader
-// needs, so relaxed device-scope accesses are enough.  The launch clears the ticket
-// and the descriptors first.  Every wait is bounded and records
+// A descriptor is one 64-bit word {launch number, value}; it carries everything its reader
+// needs, so relaxed device-scope accesses are enough.  The number is the count of launches
+// so far, kept on the device, so nothing has to be cleared between launches (a memset in
+// front of each cost 2 us): words of earlier launches never match.  The last block to
+// finish advances the count and resets the ticket.  Every wait is bounded and records
 // FE2O3_KSTATUS_WAIT_EXPIRED.
+// Arrays of up to kWaveMaxTiles tiles take device_scan_wave_kernel below instead.
 #include "common.cuh"
 
-#include <mutex>
 
 namespace {
 
@@ -57,8 +59,10 @@ constexpr int kLaneVecs = 2;                                        // consecuti
 constexpr int kPasses = kPartVecs / kLaneVecs;                      // warp scans per finish warp and tile
 constexpr int kScanThreads = 32 * (1 + kAggWarps + 1 + kFinishWarps);   // 448
 constexpr int kWindow = 6;                                          // descriptors per lane and step of the prefix warp: 192, a little over one tile per SM
-constexpr uint32_t kStateAggregate = 1;   // state 0: not yet published (the launch clears the descriptors)
 constexpr uint32_t kDescSpin = 1u << 22;
+// Up to here one tile per block in registers (2^20 + 3 elements: 12.5 -> 7.5 us, 4 M: 16.7 in the ring, 13.9 so; 6 M:
+// 19.6 against 21.7); beyond, the ring's bytes in flight win.
+constexpr uint32_t kWaveMaxTiles = 592;
 constexpr uint32_t kNoTile = 0xffffffffu;
 
 struct __align__(16) ScanShared {
@@ -70,8 +74,8 @@ struct __align__(16) ScanShared {
 };
 constexpr uint32_t kSmemBytes = kStages * kTileBytes + sizeof(ScanShared) + 1024;
 
-__device__ __forceinline__ void desc_store(uint64_t *p, uint32_t state, uint32_t value) {
-    const uint64_t v = ((uint64_t)state << 32) | value;
+__device__ __forceinline__ void desc_store(uint64_t *p, uint32_t epoch, uint32_t value) {
+    const uint64_t v = ((uint64_t)epoch << 32) | value;
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ uint64_t desc_load(const uint64_t *p) {
@@ -103,9 +107,125 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
     }
 }
 
+// Counters at the start of the scratch.
+struct ScanControl {
+    uint32_t ticket, launches, done;
+};
+// Last act of a block (one thread, when nobody in the block still reads descriptors).
+__device__ __forceinline__ void block_done(ScanControl *ctl, uint32_t epoch) {
+    if (atomicAdd(&ctl->done, 1u) == gridDim.x - 1) {
+        ctl->done = 0u;
+        ctl->ticket = 0u;
+        ctl->launches = epoch;
+    }
+}
+
+// ---- arrays of a few tiles per SM -------------------------------------------------------------
+// What bounds these is latency: one round trip for the data, one for the aggregates of the tiles before, one for
+// the stores (the ring above adds its own hand-overs: 2^20 elements took 12.4 us with it).  A block keeps one tile
+// of 8192 elements in registers, 16 a thread, publishes its sum and adds up the sums of all tiles before, one or
+// a few per thread in an order fixed by the tile's number.  Blocks start in the order of their numbers and wait
+// for lower ones only.
+constexpr int kWaveThreads = 512, kWaveWarps = kWaveThreads / 32, kWaveRows = kTileElems / (kWaveThreads * 4);
+
+template <bool kFloat>
+__global__ void __launch_bounds__(kWaveThreads)
+device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, ScanControl *ctl, uint64_t *desc,
+                        uint32_t *status) {
+    __shared__ uint32_t s_warp[kWaveWarps], s_before[kWaveWarps];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+    const uint64_t first = (uint64_t)tile * kTileElems, base = first + warp * (kTileElems / kWaveWarps) + lane * 4;
+    const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 && first + kTileElems <= n;
+    begin_after_previous();
+    const uint32_t epoch = __ldcg(&ctl->launches) + 1u;
+    uint4 x[kWaveRows];   // row j: 128 consecutive elements of the warp's part
+#pragma unroll
+    for (int j = 0; j < kWaveRows; ++j) {
+        const uint64_t e = base + j * 128;
+        if (vec) {
+            x[j] = __ldcs(reinterpret_cast<const uint4 *>(in + e));
+        } else {
+            x[j].x = e < n ? in[e] : 0u;
+            x[j].y = e + 1 < n ? in[e + 1] : 0u;
+            x[j].z = e + 2 < n ? in[e + 2] : 0u;
+            x[j].w = e + 3 < n ? in[e + 3] : 0u;
+        }
+    }
+    uint32_t own[kWaveRows], t[kWaveRows];   // each lane's total per row; the same scanned over the warp
+#pragma unroll
+    for (int j = 0; j < kWaveRows; ++j) own[j] = t[j] = sum4<kFloat>(x[j]);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int j = 0; j < kWaveRows; ++j) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, t[j], o);
+            if (lane >= (uint32_t)o) t[j] = add<kFloat>(up, t[j]);
+        }
+    }
+    uint32_t total[kWaveRows], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kWaveRows; ++j) {
+        total[j] = __shfl_sync(0xffffffffu, t[j], 31);
+        sum = add<kFloat>(sum, total[j]);
+    }
+    if (lane == 0) s_warp[warp] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        uint32_t aggregate = 0;
+#pragma unroll
+        for (int q = 0; q < kWaveWarps; ++q) aggregate = add<kFloat>(aggregate, s_warp[q]);
+        desc_store(desc + tile, epoch, aggregate);
+    }
+    uint32_t before = 0;
+    bool ok = true;
+    for (uint32_t i = tid; i < tile; i += kWaveThreads) {
+        uint64_t d = desc_load(desc + i);
+        for (uint32_t spins = 0; (uint32_t)(d >> 32) != epoch; d = desc_load(desc + i)) {
+            if (++spins > kDescSpin) { ok = false; break; }
+            __nanosleep(20);
+        }
+        before = add<kFloat>(before, (uint32_t)d);
+    }
+    if (!ok) kstatus_set(status, FE2O3_KSTATUS_WAIT_EXPIRED);
+    before = warp_sum<kFloat>(before);
+    if (lane == 0) s_before[warp] = before;
+    __syncthreads();
+    if (tid == 0) block_done(ctl, epoch);
+    uint32_t carry = 0;   // everything before this warp's first element
+#pragma unroll
+    for (int q = 0; q < kWaveWarps; ++q) carry = add<kFloat>(carry, s_before[q]);
+    for (uint32_t q = 0; q < warp; ++q) carry = add<kFloat>(carry, s_warp[q]);
+#pragma unroll
+    for (int j = 0; j < kWaveRows; ++j) {
+        uint32_t run;   // everything before this lane's first element of the row
+        if constexpr (kFloat) {
+            const uint32_t below = __shfl_up_sync(0xffffffffu, t[j], 1);
+            run = lane == 0 ? carry : add<true>(carry, below);
+        } else {
+            run = carry + t[j] - own[j];
+        }
+        carry = add<kFloat>(carry, total[j]);
+        uint32_t inc[4];
+        inc[0] = add<kFloat>(run, x[j].x);
+        inc[1] = add<kFloat>(inc[0], x[j].y);
+        inc[2] = add<kFloat>(inc[1], x[j].z);
+        inc[3] = add<kFloat>(inc[2], x[j].w);
+        const uint4 r = exclusive ? make_uint4(run, inc[0], inc[1], inc[2]) : make_uint4(inc[0], inc[1], inc[2], inc[3]);
+        const uint64_t e = base + j * 128;
+        if (vec) {
+            __stcs(reinterpret_cast<uint4 *>(out + e), r);
+        } else {
+            if (e < n) out[e] = r.x;
+            if (e + 1 < n) out[e + 1] = r.y;
+            if (e + 2 < n) out[e + 2] = r.z;
+            if (e + 3 < n) out[e + 3] = r.w;
+        }
+    }
+}
+
 template <bool kFloat>
 __global__ void __launch_bounds__(kScanThreads, 1)
-device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, uint32_t *ticket,
+device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, ScanControl *ctl,
                    uint64_t *desc, uint32_t *status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -125,6 +245,8 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
         mbar_fence_init();
     }
     __syncthreads();
+    begin_after_previous();
+    const uint32_t epoch = __ldcg(&ctl->launches) + 1u;
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -133,7 +255,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
             const uint32_t st = k % kStages, ph = (k / kStages) & 1;
             if (!mbar_wait_warp(&sh.empty[st], ph ^ 1)) { ok = false; break; }
             uint32_t t = 0;
-            if (lane == 0) t = atomicAdd(ticket, 1u);
+            if (lane == 0) t = atomicAdd(&ctl->ticket, 1u);
             t = __shfl_sync(0xffffffffu, t, 0);
             const uint64_t base = (uint64_t)t * kTileElems;
             if (base >= n) {
@@ -152,8 +274,30 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
                     mbar_arrive_expect_tx(&sh.full[st], kTileBytes);
                     bulk_load_1d(dst, in + base, kTileBytes, &sh.full[st]);
                 }
-            } else {   // the last tile, or input the copy engine cannot address: plain loads, zero beyond the end
-                for (uint32_t i = lane; i < kTileElems; i += 32) dst[i] = base + i < n ? in[base + i] : 0u;
+            } else if (aligned) {
+                // the last tile: whole 16-byte pieces by the copy engine, the rest by the lanes, zero beyond the end (one
+                // element after the other it took up to 50 us and set the time of every length that is not whole tiles)
+                const uint32_t have = (uint32_t)(n - base), whole = have & ~3u;
+                if (lane < 4 && whole < kTileElems) dst[whole + lane] = whole + lane < have ? in[base + whole + lane] : 0u;
+                for (uint32_t i = whole / 4 + 1 + lane; i < kTileElems / 4; i += 32) reinterpret_cast<uint4 *>(dst)[i] = make_uint4(0, 0, 0, 0);
+                __syncwarp();
+                if (lane == 0) {
+                    sh.tile[st] = t;
+                    if (whole) {
+                        mbar_arrive_expect_tx(&sh.full[st], whole * 4);
+                        bulk_load_1d(dst, in + base, whole * 4, &sh.full[st]);
+                    } else {
+                        mbar_arrive(&sh.full[st]);
+                    }
+                }
+            } else {   // input the copy engine cannot address: plain loads, sixteen in flight a lane
+                for (uint32_t i0 = lane; i0 < kTileElems; i0 += 32 * 16) {
+                    uint32_t v[16];
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) v[q] = base + i0 + 32 * q < n ? in[base + i0 + 32 * q] : 0u;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) dst[i0 + 32 * q] = v[q];
+                }
                 __syncwarp();
                 if (lane == 0) {
                     sh.tile[st] = t;
@@ -199,7 +343,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
                 uint32_t aggregate = 0;
                 for (int q = 0; q < kFinishWarps; ++q) aggregate = add<kFloat>(aggregate, sh.part[st][q]);
                 sh.arrivals[st] = 0;
-                desc_store(desc + tile, kStateAggregate, aggregate);
+                desc_store(desc + tile, epoch, aggregate);
                 mbar_arrive(&sh.agg_ready[st]);
             }
         }
@@ -224,13 +368,13 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
 #pragma unroll
                     for (int q = 0; q < kWindow; ++q) {   // all loads of the step in flight together
                         const uint32_t mine = b + 32 * q + lane;
-                        d[q] = mine < hi ? desc_load(desc + mine) : ((uint64_t)kStateAggregate << 32);
+                        d[q] = mine < hi ? desc_load(desc + mine) : ((uint64_t)epoch << 32);
                     }
 #pragma unroll
                     for (int q = 0; q < kWindow; ++q) {
                         const uint32_t mine = b + 32 * q + lane;
                         uint32_t spins = 0;
-                        while ((d[q] >> 32) == 0) {
+                        while ((uint32_t)(d[q] >> 32) != epoch) {
                             if (++spins > kDescSpin) { ok = false; break; }
                             __nanosleep(100);
                             d[q] = desc_load(desc + mine);
@@ -261,7 +405,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
 #pragma unroll
                         for (int q = 0; q < kWindow; ++q) {
                             const uint32_t mine = (h ? mid : covered) + 32 * q + lane;
-                            d[h][q] = mine < (h ? tile : mid) ? desc_load(desc + mine) : ((uint64_t)kStateAggregate << 32);
+                            d[h][q] = mine < (h ? tile : mid) ? desc_load(desc + mine) : ((uint64_t)epoch << 32);
                         }
                     uint32_t acc[2] = {0, 0};
 #pragma unroll
@@ -270,7 +414,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
                         for (int q = 0; q < kWindow; ++q) {
                             const uint32_t mine = (h ? mid : covered) + 32 * q + lane;
                             uint32_t spins = 0;
-                            while ((d[h][q] >> 32) == 0) {
+                            while ((uint32_t)(d[h][q] >> 32) != epoch) {
                                 if (++spins > kDescSpin) { ok = false; break; }
                                 __nanosleep(100);
                                 d[h][q] = desc_load(desc + mine);
@@ -388,6 +532,8 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
             }
         }
     }
+    __syncthreads();
+    if (tid == 0) block_done(ctl, epoch);
 }
 
 }  // namespace
@@ -398,18 +544,21 @@ int32_t launch_device_scan(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2
     const uint64_t n = a->values.len;
     const uint32_t tiles = (uint32_t)((n + kTileElems - 1) / kTileElems);
     const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
-    const uint32_t grid = tiles < sms ? (tiles ? tiles : 1u) : sms;
-    if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kScanThreads, 1, 1}, kSmemBytes, 1};
+    const bool wave = tiles <= kWaveMaxTiles;
+    const uint32_t grid = wave || tiles < sms ? (tiles ? tiles : 1u) : sms;
+    if (geo) *geo = wave ? fe2o3_geometry{{grid, 1, 1}, {kWaveThreads, 1, 1}, 0, 1} : fe2o3_geometry{{grid, 1, 1}, {kScanThreads, 1, 1}, kSmemBytes, 1};
     if (plan_only || n == 0) return FE2O3_OK;
-    // ticket at word 0, descriptors from byte 64
-    uint32_t *ticket = ctx->scan_scratch;
+    // counters at word 0, descriptors from byte 64
+    ScanControl *ctl = reinterpret_cast<ScanControl *>(ctx->scan_scratch);
     uint64_t *desc = reinterpret_cast<uint64_t *>(ctx->scan_scratch + 16);
-    FE2O3_CUDA(cudaMemsetAsync(ctx->scan_scratch, 0, 64 + (size_t)tiles * 8, s));
-    device_scan_kernel<kFloat><<<grid, kScanThreads, kSmemBytes, s>>>(reinterpret_cast<const uint32_t *>(a->values.ptr),
-                                                                      reinterpret_cast<uint32_t *>(a->output.ptr), n,
-                                                                      a->exclusive, ticket, desc, ctx->status_word);
+    const uint32_t *in = reinterpret_cast<const uint32_t *>(a->values.ptr);
+    uint32_t *out = reinterpret_cast<uint32_t *>(a->output.ptr);
+    const cudaError_t e = wave ? fe2o3_launch_early(device_scan_wave_kernel<kFloat>, grid, kWaveThreads, 0, s, 1, in, out, n,
+                                                    a->exclusive, ctl, desc, ctx->status_word)
+                               : fe2o3_launch_early(device_scan_kernel<kFloat>, grid, kScanThreads, kSmemBytes, s, 1, in, out, n,
+                                                    a->exclusive, ctl, desc, ctx->status_word);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), kFloat ? "device_scan_sum_f32" : "device_scan_sum_u32");
+    return fe2o3_cuda_status(e, kFloat ? "device_scan_sum_f32" : "device_scan_sum_u32");
 }
 
 // Function attributes are per device: called by fe2o3_ctx_create with the context's device current.

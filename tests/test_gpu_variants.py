@@ -132,6 +132,27 @@ def test_moe_layer_of_few_tokens_many_passes(gpu):
         assert (layer.out.view(torch.int32) == w.view(torch.int32)).all()
 
 
+# ---- prefix sum: one tile a block up to 592 tiles, the ring beyond; last tiles of every kind, aligned and not
+@pytest.mark.parametrize("n,offset", [(8191, 0), (8193, 1), (592 * 8192, 0), (592 * 8192 + 1, 0), (593 * 8192 + 8190, 0), (594 * 8192, 0),
+                                      (593 * 8192 + 4, 1)])
+def test_device_scan_tile_edges(gpu, orc, n, offset):
+    fe, ctx, stream = gpu
+    rng = np.random.default_rng(n)
+    v = rng.integers(0, 2**32, n + offset, dtype=np.uint64).astype(np.uint32)
+    V = fe.DeviceBuffer.from_host(stream, v)
+    O = Guarded(fe, stream, np.full(n + offset, 0xdeadbeef, np.uint32))
+    for exclusive in (0, 1):
+        run(fe, ctx, stream, "device_scan_u32", values=V.view(offset, n), output=O.buf.view(GUARD + offset, n), exclusive=exclusive)
+        assert (O.read()[offset:] == orc.scan_sum_u32(v[offset:], bool(exclusive))).all()
+    f = (v % 7).astype(np.float32) / 8   # sums of at most 2^26 eighths: within the bound the header states
+    F = fe.DeviceBuffer.from_host(stream, f)
+    G = Guarded(fe, stream, np.full(n + offset, np.nan, np.float32))
+    want, mag = orc.scan_sum_f32(f[offset:], False)
+    for _ in range(2):
+        run(fe, ctx, stream, "device_scan_f32", values=F.view(offset, n), output=G.buf.view(GUARD + offset, n), exclusive=0)
+        assert (np.abs(G.read()[offset:].astype(np.float64) - want) <= (128 + n / 8192 / 192) * 2.0 ** -24 * mag + 1e-30).all()
+
+
 # ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
 @pytest.mark.parametrize("cols", [3, 29, 32, 33, 61, 64, 65, 125, 129, 256, 513, 1021, 1024, 1025, 2045, 2048, 2050, 3001, 4093, 4094, 4095, 4096])
 def test_row_softmax_widths(gpu, orc, cols):
