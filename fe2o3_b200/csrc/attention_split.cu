@@ -164,6 +164,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    begin_after_previous();   // launched early: everything above ran beside the kernel before
     if (warp < 4) {
     regs_release<kRegsControl>();
     if (warp == 0) {
@@ -549,12 +550,13 @@ int32_t attention_split_init_device() {
 }
 
 int32_t attention_split_launch(const AttnSplitPlan *plan, cudaStream_t s) {
-    if (plan->groups == 1)
-        attention_split_kernel<1><<<plan->grid, kThreads, Layout<1>::kTotal, s>>>(plan->tmQ, plan->tmK, plan->tmV, plan->tmO, plan->p);
-    else
-        attention_split_kernel<2><<<plan->grid, kThreads, Layout<2>::kTotal, s>>>(plan->tmQ, plan->tmK, plan->tmV, plan->tmO, plan->p);
+    const cudaError_t e =
+        plan->groups == 1 ? fe2o3_launch_early(attention_split_kernel<1>, plan->grid, kThreads, Layout<1>::kTotal, s, 1, plan->tmQ,
+                                               plan->tmK, plan->tmV, plan->tmO, plan->p)
+                          : fe2o3_launch_early(attention_split_kernel<2>, plan->grid, kThreads, Layout<2>::kTotal, s, 1, plan->tmQ,
+                                               plan->tmK, plan->tmV, plan->tmO, plan->p);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "flash_attention_v1(tcgen05, split)");
+    return fe2o3_cuda_status(e, "flash_attention_v1(tcgen05, split)");
 }
 
 void attention_split_geometry(const AttnSplitPlan *plan, fe2o3_geometry *geo) {

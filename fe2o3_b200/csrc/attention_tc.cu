@@ -195,6 +195,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    begin_after_previous();   // launched early: everything above ran beside the kernel before
     // Each branch below opens with its own register re-balance, so that the code of a role is compiled
     // against that role's register count (a re-balance ahead of the branches would hold every role to
     // the smaller count).
@@ -623,9 +624,10 @@ int32_t attention_tc_init_device() {
 
 int32_t attention_tc_launch(const AttnTcPlan *plan, cudaStream_t s) {
     if (plan->grid == 0) return FE2O3_OK;
-    attention_tc_kernel<<<plan->grid, kThreads, kSmemTotal, s>>>(plan->tmQ, plan->tmK, plan->tmV, plan->tmO, plan->p);
+    const cudaError_t e = fe2o3_launch_early(attention_tc_kernel, plan->grid, kThreads, kSmemTotal, s, 1, plan->tmQ, plan->tmK, plan->tmV,
+                                             plan->tmO, plan->p);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "flash_attention_v1(tcgen05)");
+    return fe2o3_cuda_status(e, "flash_attention_v1(tcgen05)");
 }
 
 void attention_tc_geometry(const AttnTcPlan *plan, fe2o3_geometry *geo) {

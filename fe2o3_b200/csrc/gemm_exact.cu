@@ -104,6 +104,7 @@ gemm_exact_kernel(const T *__restrict__ A, const T *__restrict__ B, float *C, ui
         }
     };
 
+    begin_after_previous();
     if (K > 0) {
         fetch(0);
         stage(0);
@@ -161,17 +162,16 @@ int32_t launch_gemm_exact(cudaStream_t s, uint32_t dtype, bool epilogue, uint64_
     if (geo) *geo = fe2o3_geometry{{grid.x, grid.y, 1}, {kThreads, 1, 1}, 0, 1};
     if (plan_only || M == 0 || N == 0) return FE2O3_OK;
     float *C = reinterpret_cast<float *>(c);
+    cudaError_t e;
     if (dtype == FE2O3_DTYPE_F32) {
         const float *A = reinterpret_cast<const float *>(a), *B = reinterpret_cast<const float *>(b);
-        if (epilogue) gemm_exact_kernel<float, true><<<grid, kThreads, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
-        else gemm_exact_kernel<float, false><<<grid, kThreads, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
+        e = fe2o3_launch_early(epilogue ? gemm_exact_kernel<float, true> : gemm_exact_kernel<float, false>, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
     } else {
         const uint16_t *A = reinterpret_cast<const uint16_t *>(a), *B = reinterpret_cast<const uint16_t *>(b);
-        if (epilogue) gemm_exact_kernel<uint16_t, true><<<grid, kThreads, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
-        else gemm_exact_kernel<uint16_t, false><<<grid, kThreads, 0, s>>>(A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
+        e = fe2o3_launch_early(epilogue ? gemm_exact_kernel<uint16_t, true> : gemm_exact_kernel<uint16_t, false>, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
     }
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "gemm_exact");
+    return fe2o3_cuda_status(e, "gemm_exact");
 }
 
 static Fe2o3KernelRegistration reg_scalar("scalar_gemm_v1", reinterpret_cast<const void *>(gemm_exact_kernel<float, false>));

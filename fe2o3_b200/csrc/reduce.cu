@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 masked_reduce_u32_kernel(fe2o3_masked_reduce_u32_args args, uint32_t *partials, uint32_t *counter,
                          uint32_t *status) {
     __shared__ uint32_t smem[32];
+    begin_after_previous();
     if (args.values.len != args.active.len || args.output.len != 1) {
         if (blockIdx.x == 0 && threadIdx.x == 0) kstatus_set(status, FE2O3_KSTATUS_LENGTH);
         return;
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 masked_reduce_u32_packed_kernel(fe2o3_masked_reduce_u32_packed_args args, uint32_t *partials,
                                 uint32_t *counter, uint32_t *status) {
     __shared__ uint32_t smem[32];
+    begin_after_previous();
     const uint64_t n = args.values.len;
     if (args.mask.len != (n + 63) / 64 || args.output.len != 1) {
         if (blockIdx.x == 0 && threadIdx.x == 0) kstatus_set(status, FE2O3_KSTATUS_LENGTH);
@@ -278,11 +280,10 @@ int32_t launch_masked_reduce_u32(fe2o3_ctx *ctx, cudaStream_t s, const void *arg
     uint32_t grid = reduce_grid(ctx, a->values.len);
     if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kReduceThreads, 1, 1}, 0, 1};
     if (plan_only) return FE2O3_OK;
-    masked_reduce_u32_kernel<<<grid, kReduceThreads, 0, s>>>(*a, ctx->reduce_scratch,
-                                                              ctx->reduce_scratch + FE2O3_REDUCE_MAX_BLOCKS,
-                                                              ctx->status_word);
+    const cudaError_t e = fe2o3_launch_early(masked_reduce_u32_kernel, grid, kReduceThreads, 0, s, 1, *a, ctx->reduce_scratch,
+                                             ctx->reduce_scratch + FE2O3_REDUCE_MAX_BLOCKS, ctx->status_word);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "masked_reduce_u32");
+    return fe2o3_cuda_status(e, "masked_reduce_u32");
 }
 
 int32_t launch_masked_reduce_u32_packed(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_geometry *geo,
@@ -291,11 +292,10 @@ int32_t launch_masked_reduce_u32_packed(fe2o3_ctx *ctx, cudaStream_t s, const vo
     uint32_t grid = reduce_grid(ctx, a->values.len);
     if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kReduceThreads, 1, 1}, 0, 1};
     if (plan_only) return FE2O3_OK;
-    masked_reduce_u32_packed_kernel<<<grid, kReduceThreads, 0, s>>>(*a, ctx->reduce_scratch,
-                                                                     ctx->reduce_scratch + FE2O3_REDUCE_MAX_BLOCKS,
-                                                                     ctx->status_word);
+    const cudaError_t e = fe2o3_launch_early(masked_reduce_u32_packed_kernel, grid, kReduceThreads, 0, s, 1, *a, ctx->reduce_scratch,
+                                             ctx->reduce_scratch + FE2O3_REDUCE_MAX_BLOCKS, ctx->status_word);
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "masked_reduce_u32_packed");
+    return fe2o3_cuda_status(e, "masked_reduce_u32_packed");
 }
 
 int32_t launch_wave_lds_v1(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_geometry *geo, bool plan_only) {

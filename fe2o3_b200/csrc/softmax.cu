@@ -62,6 +62,7 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
     constexpr int kRowsPerBlock = kThreads / LANES;
     __shared__ float s_red[LANES > 32 ? 2 : 1][kThreads / 32];   // one set per exchange: no barrier before the next one
     const uint32_t local = threadIdx.x / LANES, lane = threadIdx.x % LANES;
+    begin_after_previous();
     uint32_t row = blockIdx.x * kRowsPerBlock + local;
     // a warp may hold several rows, all of which take part in its shuffles: those past the end redo the last row
     const bool beyond = row >= rows;
@@ -190,6 +191,7 @@ row_softmax_block_kernel(const float *__restrict__ in, float *__restrict__ out, 
     __shared__ float red[kThreads / 32];
     __shared__ int flags[2];
     const uint32_t row = blockIdx.x;
+    begin_after_previous();
     if (row >= rows) return;
     const float *src = in + (uint64_t)row * cols;
     const uint8_t *msk = mask ? mask + (uint64_t)row * cols : nullptr;
@@ -245,17 +247,13 @@ row_softmax_block_kernel(const float *__restrict__ in, float *__restrict__ out, 
 }
 
 template <int LANES, int NV>
-void launch_row(const fe2o3_row_softmax_v1_args *a, bool shifted, cudaStream_t s, uint32_t grid, uint32_t *status) {
+cudaError_t launch_row(const fe2o3_row_softmax_v1_args *a, bool shifted, cudaStream_t s, uint32_t grid, uint32_t *status) {
     const float *in = reinterpret_cast<const float *>(a->input.ptr);
     float *out = reinterpret_cast<float *>(a->output.ptr);
     const uint8_t *mask = reinterpret_cast<const uint8_t *>(a->mask.ptr);
-    if (shifted) {
-        if (mask) row_softmax_kernel<LANES, NV, true, true><<<grid, kThreads, 0, s>>>(in, out, mask, a->rows, a->cols, status);
-        else row_softmax_kernel<LANES, NV, false, true><<<grid, kThreads, 0, s>>>(in, out, mask, a->rows, a->cols, status);
-    } else {
-        if (mask) row_softmax_kernel<LANES, NV, true, false><<<grid, kThreads, 0, s>>>(in, out, mask, a->rows, a->cols, status);
-        else row_softmax_kernel<LANES, NV, false, false><<<grid, kThreads, 0, s>>>(in, out, mask, a->rows, a->cols, status);
-    }
+    auto kernel = shifted ? (mask ? row_softmax_kernel<LANES, NV, true, true> : row_softmax_kernel<LANES, NV, false, true>)
+                          : (mask ? row_softmax_kernel<LANES, NV, true, false> : row_softmax_kernel<LANES, NV, false, false>);
+    return fe2o3_launch_early(kernel, grid, kThreads, 0, s, 1, in, out, mask, a->rows, a->cols, status);
 }
 
 }  // namespace
@@ -273,29 +271,30 @@ int32_t launch_row_softmax(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2
     const uint32_t grid = vec ? ceil_div_u32(a->rows, kThreads / lanes) : a->rows;
     if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kThreads, 1, 1}, 0, 1};
     if (plan_only || a->rows == 0) return FE2O3_OK;
+    cudaError_t e;
     if (vec) {
         uint32_t *st = ctx->status_word;
         switch ((vectors + lanes - 1) / lanes) {
             case 1:
-                if (lanes == 8) launch_row<8, 1>(a, shifted, s, grid, st);
-                else if (lanes == 16) launch_row<16, 1>(a, shifted, s, grid, st);
-                else launch_row<32, 1>(a, shifted, s, grid, st);
+                if (lanes == 8) e = launch_row<8, 1>(a, shifted, s, grid, st);
+                else if (lanes == 16) e = launch_row<16, 1>(a, shifted, s, grid, st);
+                else e = launch_row<32, 1>(a, shifted, s, grid, st);
                 break;
-            case 2: launch_row<32, 2>(a, shifted, s, grid, st); break;
-            case 3: case 4: launch_row<32, 4>(a, shifted, s, grid, st); break;
-            case 9: launch_row<128, 9>(a, shifted, s, grid, st); break;   // up to 1025 vectors: 4095 columns at phase 3
+            case 2: e = launch_row<32, 2>(a, shifted, s, grid, st); break;
+            case 3: case 4: e = launch_row<32, 4>(a, shifted, s, grid, st); break;
+            case 9: e = launch_row<128, 9>(a, shifted, s, grid, st); break;   // up to 1025 vectors: 4095 columns at phase 3
             default:
-                if (lanes == 32) launch_row<32, 8>(a, shifted, s, grid, st);
-                else if (lanes == 64) launch_row<64, 8>(a, shifted, s, grid, st);
-                else launch_row<128, 8>(a, shifted, s, grid, st);
+                if (lanes == 32) e = launch_row<32, 8>(a, shifted, s, grid, st);
+                else if (lanes == 64) e = launch_row<64, 8>(a, shifted, s, grid, st);
+                else e = launch_row<128, 8>(a, shifted, s, grid, st);
         }
     } else {
-        row_softmax_block_kernel<<<grid, kThreads, 0, s>>>(
+        e = fe2o3_launch_early(row_softmax_block_kernel, grid, kThreads, 0, s, 1,
             reinterpret_cast<const float *>(a->input.ptr), reinterpret_cast<float *>(a->output.ptr),
             reinterpret_cast<const uint8_t *>(a->mask.ptr), a->rows, a->cols, ctx->status_word);
     }
     fe2o3_count_launch(1);
-    return fe2o3_cuda_status(cudaGetLastError(), "row_softmax_v1");
+    return fe2o3_cuda_status(e, "row_softmax_v1");
 }
 
 static Fe2o3KernelRegistration reg_softmax("row_softmax_v1", reinterpret_cast<const void *>(row_softmax_kernel<32, 8, false, false>));
