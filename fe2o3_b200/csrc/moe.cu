@@ -1068,14 +1068,16 @@ int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_
             // 107 against 94 us a pass of 512 tokens): they ask for so much shared memory that they spread evenly.
             const uint32_t per_sm = ceil_div_u32(chain_grid, (uint32_t)ctx->sm_count);
             const uint32_t own = E == 16 ? 29u : 20u;   // KiB of its own, with what each block reserves
-            const uint32_t spread = 220u / per_sm > own ? (220u / per_sm - own) * 1024u : 0u;
+            constexpr uint32_t kSpreadMax = 192u * 1024u;
+            const uint32_t spread = 220u / per_sm > own ? min((220u / per_sm - own) * 1024u, kSpreadMax) : 0u;
             fe2o3_geometry g{{chain_grid, 1, 1}, {32, 1, 1}, wide ? 0u : spread, 1};
             cudaError_t e = cudaSuccess;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, &g) : E == 8 ? FE2O3_GATE_LANES(8, &g) : FE2O3_GATE_LANES(16, &g);
             if (geo) *geo = g;
             if (plan_only) return FE2O3_OK;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, nullptr) : E == 8 ? FE2O3_GATE_LANES(8, nullptr) : FE2O3_GATE_LANES(16, nullptr);
-            else if (spread <= 48u * 1024u || (e = cudaFuncSetAttribute(one_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread)) == cudaSuccess)
+            else if (spread <= 48u * 1024u ||   // (one value for all launches: threads do not disturb one another)
+                     (e = cudaFuncSetAttribute(one_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpreadMax)) == cudaSuccess)
                 e = fe2o3_launch_early(one_chain, chain_grid, 32, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
 #undef FE2O3_GATE_LANES
             if (e != cudaSuccess) return fe2o3_cuda_status(e, "moe_gate_v1");
