@@ -59,6 +59,7 @@ int32_t attention_split_launch(const AttnSplitPlan *, cudaStream_t);
 void attention_split_geometry(const AttnSplitPlan *, fe2o3_geometry *);
 void attention_split_free(AttnSplitPlan *);
 int32_t attention_split_init_device();
+int32_t moe_gate_init_device();
 int32_t device_scan_init_device();
 
 // ---- error bookkeeping ---------------------------------------------------------
@@ -847,6 +848,7 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
     int32_t init = gemm_tc_init_device();
     if (init == FE2O3_OK) init = attention_tc_init_device();
     if (init == FE2O3_OK) init = attention_split_init_device();
+    if (init == FE2O3_OK) init = moe_gate_init_device();
     if (init == FE2O3_OK) init = device_scan_init_device();
     if (init != FE2O3_OK) return init;
     fe2o3_ctx *ctx = new (std::nothrow) fe2o3_ctx();

@@ -615,6 +615,10 @@ moe_gate_chain_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict
     if (tok0 + tt < tokens) logits[(uint64_t)(tok0 + tt) * E + e] = acc;
 }
 
+// Shared memory that a launch of the chain kernel may ask for beside its own (see launch_moe_gate).  The limit without
+// opt-in, 48 KiB, is for both together, so the opt-in is made for every size: 35 KiB beside 18 of its own are refused too.
+constexpr uint32_t kGateSpreadMax = 192u * 1024u;
+
 // ---- top-2 routing over many blocks --------------------------------------------
 // Same result as moe_top2_kernel.  Block b owns tokens [256 b, 256 b + 256).
 // Pass 1 counts, per block and expert, the routes the block requests and checks
@@ -1041,6 +1045,14 @@ moe_combine_kernel(const float *__restrict__ compact, const uint32_t *__restrict
 
 }  // namespace
 
+// Function attributes are per device: called by fe2o3_ctx_create with the context's device current.
+int32_t moe_gate_init_device() {
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    return FE2O3_OK;
+}
+
 int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_geometry *geo, bool plan_only) {
     const fe2o3_moe_gate_v1_args *a = static_cast<const fe2o3_moe_gate_v1_args *>(args);
     const uint32_t E = a->experts;
@@ -1068,17 +1080,14 @@ int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_
             // 107 against 94 us a pass of 512 tokens): they ask for so much shared memory that they spread evenly.
             const uint32_t per_sm = ceil_div_u32(chain_grid, (uint32_t)ctx->sm_count);
             const uint32_t own = E == 16 ? 29u : 20u;   // KiB of its own, with what each block reserves
-            constexpr uint32_t kSpreadMax = 192u * 1024u;
-            const uint32_t spread = 220u / per_sm > own ? min((220u / per_sm - own) * 1024u, kSpreadMax) : 0u;
+            const uint32_t spread = 220u / per_sm > own ? min((220u / per_sm - own) * 1024u, kGateSpreadMax) : 0u;
             fe2o3_geometry g{{chain_grid, 1, 1}, {32, 1, 1}, wide ? 0u : spread, 1};
             cudaError_t e = cudaSuccess;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, &g) : E == 8 ? FE2O3_GATE_LANES(8, &g) : FE2O3_GATE_LANES(16, &g);
             if (geo) *geo = g;
             if (plan_only) return FE2O3_OK;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, nullptr) : E == 8 ? FE2O3_GATE_LANES(8, nullptr) : FE2O3_GATE_LANES(16, nullptr);
-            else if (spread <= 48u * 1024u ||   // (one value for all launches: threads do not disturb one another)
-                     (e = cudaFuncSetAttribute(one_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpreadMax)) == cudaSuccess)
-                e = fe2o3_launch_early(one_chain, chain_grid, 32, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
+            else e = fe2o3_launch_early(one_chain, chain_grid, 32, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
 #undef FE2O3_GATE_LANES
             if (e != cudaSuccess) return fe2o3_cuda_status(e, "moe_gate_v1");
             fe2o3_count_launch(1);

@@ -85,6 +85,30 @@ def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
 
 
+# ---- gate, first launch of a process: sizes at which its blocks ask for shared memory that only together with the
+# kernel's own passes the limit without opt-in, so that an earlier launch of another size would hide a missing one
+@pytest.mark.parametrize("T,E", [(2048, 8), (1000, 16), (4000, 4)])
+def test_moe_gate_first_launch_of_a_process(T, E):
+    import os
+    import subprocess
+    import sys
+    code = """
+import sys
+sys.path.insert(0, %r)
+import numpy as np, fe2o3_b200 as fe, oracle
+from fe2o3_b200 import synth
+T, E, d = %d, %d, 128
+ctx = fe.GpuContext(0); s = ctx.default_stream()
+x, wg = synth.normal_bf16(1, 1, T * d, 1.0), synth.normal_bf16(1, 2, d * E, 0.1)
+X, W, L = fe.DeviceBuffer.from_host(s, x), fe.DeviceBuffer.from_host(s, wg), fe.DeviceBuffer.zeroed(s, T * E, np.float32)
+fe.prepare(ctx, "moe_gate_v1", x=X, wg=W, logits=L, tokens=T, d_model=d, experts=E).launch_and_wait(s)
+assert (L.to_host_vec(s).view(np.uint32) == oracle.moe_gate_logits(x, wg, T, d, E).view(np.uint32)).all()
+print("ok")
+""" % (os.path.dirname(os.path.dirname(os.path.abspath(__file__))), T, E)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
 # ---- routing in one launch: one warp to eight blocks of two passes, and the sizes around each step
 @pytest.mark.parametrize("T,E,cap,bad", [(1, 2, 1, 0), (33, 8, 100, 0), (1000, 5, 300, 0), (1024, 16, 2048, 0), (1025, 8, 200, 0),
                                          (2049, 32, 4098, 0), (4097, 8, 900, 0), (8192, 8, 2100, 0), (8193, 16, 16386, 0),
