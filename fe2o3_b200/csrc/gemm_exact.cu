@@ -59,7 +59,8 @@ gemm_exact_kernel(const T *__restrict__ A, const T *__restrict__ B, float *C, ui
     __shared__ __align__(16) float As[2][TK][TM + 4];   // k-major, so that a thread's four rows are one 16-byte read
     __shared__ __align__(16) float Bs[2][TK][TN];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const uint32_t row0 = blockIdx.x * TM, col0 = blockIdx.y * TN;
+    const uint32_t row_tiles = (M - 1) / TM + 1;
+    const uint32_t row0 = blockIdx.x % row_tiles * TM, col0 = blockIdx.x / row_tiles * TN;
     const bool vec_a = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
     const bool vec_b = ldb % 4 == 0 && reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0;
 
@@ -158,8 +159,12 @@ gemm_exact_kernel(const T *__restrict__ A, const T *__restrict__ B, float *C, ui
 int32_t launch_gemm_exact(cudaStream_t s, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c,
                           uint32_t M, uint32_t N, uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha,
                           float beta, fe2o3_geometry *geo, bool plan_only) {
-    dim3 grid(ceil_div_u32(M, TM), ceil_div_u32(N, TN), 1);   // rows in x: up to 2^31 blocks
-    if (geo) *geo = fe2o3_geometry{{grid.x, grid.y, 1}, {kThreads, 1, 1}, 0, 1};
+    // one flat index, rows first: the second and third grid dimensions end at 65535 tiles, which either a tall or a
+    // wide result can have
+    const uint64_t tiles = (uint64_t)ceil_div_u32(M, TM) * ceil_div_u32(N, TN);
+    if (tiles > 0x7fffffffull) { fe2o3_set_error("UnsupportedShape: too many output tiles"); return FE2O3_ERR_UNSUPPORTED_SHAPE; }
+    const uint32_t grid = (uint32_t)tiles;
+    if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kThreads, 1, 1}, 0, 1};
     if (plan_only || M == 0 || N == 0) return FE2O3_OK;
     float *C = reinterpret_cast<float *>(c);
     cudaError_t e;

@@ -29,6 +29,19 @@ def test_scalar_gemm_tile_edges_bit_exact(gpu, orc, m, n, k):
     A.unchanged(); B.unchanged()
 
 
+# more tiles in one direction than a second grid dimension holds (65535)
+@pytest.mark.parametrize("m,n", [(1, 5_000_000), (5_000_000, 1), (2, 65535 * 64 + 1)])
+def test_scalar_gemm_long_results_bit_exact(gpu, m, n):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    a, b = synth.uniform_f32(0, 1, m), synth.uniform_f32(0, 2, n)
+    A, B = Guarded(fe, stream, a), Guarded(fe, stream, b)
+    Cb = Guarded(fe, stream, np.full(m * n, np.nan, np.float32))
+    run(fe, ctx, stream, "scalar_gemm_v1", a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=1)
+    want = np.float32(0) + a[:, None] * b[None, :]   # one product, added to +0
+    assert (bits(Cb.read()) == bits(want).ravel()).all()
+
+
 # ---- tensor-core GEMM: outputs that the copy engine does not write (alpha/beta form, C at any alignment)
 @pytest.mark.parametrize("m,n,k,ldc,offset", [(129, 40, 64, 40, 0), (128, 256, 64, 257, 0), (200, 136, 96, 140, 1), (257, 300, 72, 304, 0),
                                               (16, 1000, 128, 1001, 3)])
