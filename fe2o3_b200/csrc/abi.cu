@@ -862,7 +862,6 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
     uint32_t *dev = nullptr;
     e = cudaMalloc(&dev, (ctx->reduce_scratch_elems + 1) * sizeof(uint32_t));
     if (e != cudaSuccess) { delete ctx; return fe2o3_cuda_status(e, "cudaMalloc(context scratch)"); }
-    cudaMemset(dev, 0, (ctx->reduce_scratch_elems + 1) * sizeof(uint32_t));
     ctx->reduce_scratch = dev;
     ctx->status_word = dev + ctx->reduce_scratch_elems;
     e = cudaMallocHost(&ctx->host_status, 64);
@@ -874,7 +873,6 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
         delete ctx;
         return fe2o3_cuda_status(e, "cudaMalloc(routing scratch)");
     }
-    cudaMemset(ctx->route_scratch, 0, FE2O3_ROUTE_SCRATCH_ELEMS * sizeof(uint32_t));
     e = cudaMalloc(&ctx->scan_scratch, FE2O3_SCAN_SCRATCH_BYTES);
     if (e != cudaSuccess) {
         cudaFree(dev);
@@ -884,7 +882,20 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
         delete ctx;
         return fe2o3_cuda_status(e, "cudaMalloc(scan scratch)");
     }
-    cudaMemset(ctx->scan_scratch, 0, FE2O3_SCAN_SCRATCH_BYTES);
+    // counters and the status word start at zero, and are there before any launch: the library's streams are
+    // non-blocking, so nothing but the host orders them behind these clears
+    e = cudaMemset(dev, 0, (ctx->reduce_scratch_elems + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(ctx->route_scratch, 0, FE2O3_ROUTE_SCRATCH_ELEMS * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(ctx->scan_scratch, 0, FE2O3_SCAN_SCRATCH_BYTES);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) {
+        cudaFree(dev);
+        cudaFree(ctx->route_scratch);
+        cudaFree(ctx->scan_scratch);
+        cudaFreeHost(ctx->host_status);
+        delete ctx;
+        return fe2o3_cuda_status(e, "cudaMemset(context scratch)");
+    }
     *out = ctx;
     return FE2O3_OK;
 }

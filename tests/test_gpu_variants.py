@@ -190,6 +190,22 @@ def test_device_scan_tile_edges(gpu, orc, n, offset):
         assert (np.abs(G.read()[offset:].astype(np.float64) - want) <= (128 + n / 8192 / 192) * 2.0 ** -24 * mag + 1e-30).all()
 
 
+def test_first_scan_of_a_context_on_its_own_stream(gpu, orc):
+    """The counters a scan starts from are zero before a context is handed out: nothing orders a non-blocking stream
+    behind clears that are still under way."""
+    fe, _, stream = gpu
+    v = np.arange(1, 700 * 8192 + 1, dtype=np.uint32)
+    V = fe.DeviceBuffer.from_host(stream, v)
+    want = orc.scan_sum_u32(v, False)
+    for _ in range(10):
+        O = fe.DeviceBuffer.from_host(stream, np.zeros(v.size, np.uint32))
+        ctx = fe.GpuContext(0)
+        own = ctx.create_stream()
+        p = fe.prepare(ctx, "device_scan_u32", values=V, output=O, exclusive=0)
+        p.launch_and_wait(own)
+        assert (O.to_host_vec(own) == want).all()
+
+
 # ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
 @pytest.mark.parametrize("cols", [3, 29, 32, 33, 61, 64, 65, 125, 129, 256, 513, 1021, 1024, 1025, 2045, 2048, 2050, 3001, 4093, 4094, 4095, 4096])
 def test_row_softmax_widths(gpu, orc, cols):
