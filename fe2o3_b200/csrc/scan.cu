@@ -42,7 +42,7 @@
 // front of each cost 2 us): words of earlier launches never match.  The last block to
 // finish advances the count and resets the ticket.  Every wait is bounded and records
 // FE2O3_KSTATUS_WAIT_EXPIRED.
-// Arrays of up to kWaveMaxTiles tiles take device_scan_wave_kernel below instead.
+// Arrays of up to kWaveTilesPerSm tiles an SM take device_scan_wave_kernel below instead.
 #include "common.cuh"
 
 
@@ -62,7 +62,7 @@ constexpr int kWindow = 6;                                          // descripto
 constexpr uint32_t kDescSpin = 1u << 22;
 // Up to here one tile per block in registers (2^20 + 3 elements: 12.5 -> 7.5 us, 4 M: 16.7 in the ring, 13.9 so; 6 M:
 // 19.6 against 21.7); beyond, the ring's bytes in flight win.
-constexpr uint32_t kWaveMaxTiles = 592;
+constexpr uint32_t kWaveTilesPerSm = 4;
 constexpr uint32_t kNoTile = 0xffffffffu;
 
 struct __align__(16) ScanShared {
@@ -124,19 +124,22 @@ __device__ __forceinline__ void block_done(ScanControl *ctl, uint32_t epoch) {
 // What bounds these is latency: one round trip for the data, one for the aggregates of the tiles before, one for
 // the stores (the ring above adds its own hand-overs: 2^20 elements took 12.4 us with it).  A block keeps one tile
 // of 8192 elements in registers, 16 a thread, publishes its sum and adds up the sums of all tiles before, one or
-// a few per thread in an order fixed by the tile's number.  Blocks start in the order of their numbers and wait
-// for lower ones only.
+// a few per thread in an order fixed by the tile's number.  The tile is a ticket here too: a block only waits for
+// blocks that have started, in whatever order they do, whether or not all are resident at once.
 constexpr int kWaveThreads = 512, kWaveWarps = kWaveThreads / 32, kWaveRows = kTileElems / (kWaveThreads * 4);
 
 template <bool kFloat>
 __global__ void __launch_bounds__(kWaveThreads)
 device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, ScanControl *ctl, uint64_t *desc,
                         uint32_t *status) {
-    __shared__ uint32_t s_warp[kWaveWarps], s_before[kWaveWarps];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+    __shared__ uint32_t s_warp[kWaveWarps], s_before[kWaveWarps], s_tile;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    begin_after_previous();
+    if (tid == 0) s_tile = atomicAdd(&ctl->ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
     const uint64_t first = (uint64_t)tile * kTileElems, base = first + warp * (kTileElems / kWaveWarps) + lane * 4;
     const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 && first + kTileElems <= n;
-    begin_after_previous();
     const uint32_t epoch = __ldcg(&ctl->launches) + 1u;
     uint4 x[kWaveRows];   // row j: 128 consecutive elements of the warp's part
 #pragma unroll
@@ -544,7 +547,7 @@ int32_t launch_device_scan(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2
     const uint64_t n = a->values.len;
     const uint32_t tiles = (uint32_t)((n + kTileElems - 1) / kTileElems);
     const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
-    const bool wave = tiles <= kWaveMaxTiles;
+    const bool wave = tiles <= kWaveTilesPerSm * sms;
     const uint32_t grid = wave || tiles < sms ? (tiles ? tiles : 1u) : sms;
     if (geo) *geo = wave ? fe2o3_geometry{{grid, 1, 1}, {kWaveThreads, 1, 1}, 0, 1} : fe2o3_geometry{{grid, 1, 1}, {kScanThreads, 1, 1}, kSmemBytes, 1};
     if (plan_only || n == 0) return FE2O3_OK;

@@ -169,7 +169,7 @@ def test_moe_layer_of_few_tokens_many_passes(gpu):
         assert (layer.out.view(torch.int32) == w.view(torch.int32)).all()
 
 
-# ---- prefix sum: one tile a block up to 592 tiles, the ring beyond; last tiles of every kind, aligned and not
+# ---- prefix sum: one tile a block up to four tiles an SM (592 on 148), the ring beyond; last tiles of every kind, aligned and not
 @pytest.mark.parametrize("n,offset", [(8191, 0), (8193, 1), (592 * 8192, 0), (592 * 8192 + 1, 0), (593 * 8192 + 8190, 0), (594 * 8192, 0),
                                       (593 * 8192 + 4, 1)])
 def test_device_scan_tile_edges(gpu, orc, n, offset):
@@ -203,7 +203,30 @@ def test_first_scan_of_a_context_on_its_own_stream(gpu, orc):
         own = ctx.create_stream()
         p = fe.prepare(ctx, "device_scan_u32", values=V, output=O, exclusive=0)
         p.launch_and_wait(own)
-        assert (O.to_host_vec(own) == want).all()
+        assert (O.to_host_vec(stream) == want).all()
+
+
+def test_scan_beside_other_kernels(gpu, orc):
+    """More register tiles than are resident at once, while another stream's kernels hold the SMs: a block only waits for
+    tiles that have started."""
+    fe, ctx, stream = gpu
+    side = ctx.create_stream()
+    n = 592 * 8192 - 5
+    v = np.arange(7, n + 7, dtype=np.uint32)
+    V, O = fe.DeviceBuffer.from_host(stream, v), fe.DeviceBuffer.from_host(stream, np.zeros(n, np.uint32))
+    m = 2048
+    A, B = (fe.DeviceBuffer.from_host(stream, np.zeros(m * m, np.uint16)) for _ in range(2))
+    C = fe.DeviceBuffer.zeroed(stream, m * m, np.float32)
+    gemm = fe.prepare(ctx, "tiled_gemm_v1", a=A, b=B, c=C, m=m, n=m, k=m)
+    scan = fe.prepare(ctx, "device_scan_u32", values=V, output=O, exclusive=0)
+    for _ in range(20):
+        for _ in range(3):
+            gemm.launch(side)
+        scan.launch(stream)
+    stream.synchronize()
+    side.synchronize()
+    assert ctx.take_kernel_status(stream) == 0
+    assert (O.to_host_vec(stream) == orc.scan_sum_u32(v, False)).all()
 
 
 # ---- row softmax: lanes per row 8 to 128, one to nine vectors per lane, rows at every phase of a 16-byte vector
