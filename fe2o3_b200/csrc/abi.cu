@@ -814,6 +814,8 @@ int32_t take_status(fe2o3_ctx *ctx, cudaStream_t s, uint32_t *status) {
     const uint32_t v = *ctx->host_status;
     if (status) *status = v;
     if (v != 0) FE2O3_CUDA(cudaMemsetAsync(ctx->status_word, 0, 4, s));
+    // (scan_state.h: until this every scan of the context only reports)
+    if (v == FE2O3_KSTATUS_SCAN_STATE) FE2O3_CUDA(cudaMemsetAsync(ctx->scan_scratch, 0, FE2O3_SCAN_SCRATCH_BYTES, s));
     return FE2O3_OK;
 }
 

@@ -36,15 +36,14 @@
 // separately: whichever block computes a tile's prefix performs the same chain of additions, and
 // repeated runs give identical bits.  The lane prefix inside a warp scan comes from a shuffle
 // instead of a subtraction.
-// A descriptor is one 64-bit word {launch number, value}; it carries everything its reader
-// needs, so relaxed device-scope accesses are enough.  The number is the count of launches
+// A descriptor is one 64-bit word {launch tag, value}; it carries everything its reader
+// needs, so relaxed device-scope accesses are enough.  The tag follows the count of launches
 // so far, kept on the device, so nothing has to be cleared between launches (a memset in
-// front of each cost 2 us): words of earlier launches never match.  The last block to
-// finish advances the count and resets the ticket.  Every wait is bounded and records
-// FE2O3_KSTATUS_WAIT_EXPIRED.
+// front of each cost 2 us): words of earlier launches never match.  scan_state.h has the rules.
+// Every wait is bounded and records FE2O3_KSTATUS_WAIT_EXPIRED.
 // Arrays of up to kWaveTilesPerSm tiles an SM take device_scan_wave_kernel below instead.
 #include "common.cuh"
-
+#include "scan_state.h"
 
 namespace {
 
@@ -74,8 +73,8 @@ struct __align__(16) ScanShared {
 };
 constexpr uint32_t kSmemBytes = kStages * kTileBytes + sizeof(ScanShared) + 1024;
 
-__device__ __forceinline__ void desc_store(uint64_t *p, uint32_t epoch, uint32_t value) {
-    const uint64_t v = ((uint64_t)epoch << 32) | value;
+__device__ __forceinline__ void desc_store(uint64_t *p, uint32_t tag, uint32_t value) {
+    const uint64_t v = ((uint64_t)tag << 32) | value;
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ uint64_t desc_load(const uint64_t *p) {
@@ -107,17 +106,20 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
     }
 }
 
-// Counters at the start of the scratch.
-struct ScanControl {
-    uint32_t ticket, launches, done;
+// What outlives a launch, as scan_state.h wants it.
+struct DeviceWords {
+    static __device__ __forceinline__ scan_word add(scan_word *p, scan_word v) { return atomicAdd(p, v); }
+    static __device__ __forceinline__ void fetch_or(scan_word *p, scan_word v) { atomicOr(p, v); }
+    static __device__ __forceinline__ void store(scan_word *p, scan_word v) { *p = v; }
 };
+constexpr uint32_t kMaxTiles = (uint32_t)(FE2O3_SCAN_MAX_ELEMENTS / kTileElems);
+constexpr uint32_t kMaxBlocks = 1024;
+static_assert(kMaxTiles + kMaxBlocks < 1u << kScanTicketBits && kMaxBlocks < 1u << kScanBlockBits, "counts of one launch fit their fields");
+
 // Last act of a block (one thread, when nobody in the block still reads descriptors).
-__device__ __forceinline__ void block_done(ScanControl *ctl, uint32_t epoch) {
-    if (atomicAdd(&ctl->done, 1u) == gridDim.x - 1) {
-        ctl->done = 0u;
-        ctl->ticket = 0u;
-        ctl->launches = epoch;
-    }
+__device__ __forceinline__ void block_done(scan_word *state, uint64_t *desc, uint32_t tag, uint32_t tickets, uint32_t *status) {
+    if (!scan_finish<DeviceWords>(state, reinterpret_cast<scan_word *>(desc), kMaxTiles, tag, gridDim.x, tickets))
+        kstatus_set(status, FE2O3_KSTATUS_SCAN_STATE);
 }
 
 // ---- arrays of a few tiles per SM -------------------------------------------------------------
@@ -129,18 +131,25 @@ __device__ __forceinline__ void block_done(ScanControl *ctl, uint32_t epoch) {
 constexpr int kWaveThreads = 512, kWaveWarps = kWaveThreads / 32, kWaveRows = kTileElems / (kWaveThreads * 4);
 
 template <bool kFloat>
-__global__ void __launch_bounds__(kWaveThreads)
-device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, ScanControl *ctl, uint64_t *desc,
+__global__ void __launch_bounds__(kWaveThreads, 3)   // three blocks an SM: 40 registers
+device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, scan_word *state, uint64_t *desc,
                         uint32_t *status) {
-    __shared__ uint32_t s_warp[kWaveWarps], s_before[kWaveWarps], s_tile;
+    __shared__ uint32_t s_warp[kWaveWarps], s_before[kWaveWarps];
+    __shared__ uint32_t s_tile, s_tag;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     begin_after_previous();
-    if (tid == 0) s_tile = atomicAdd(&ctl->ticket, 1u);
+    if (tid == 0) {
+        scan_word drawn;
+        s_tile = kNoTile;
+        if (scan_take<DeviceWords>(state, gridDim.x, drawn)) s_tile = scan_tickets(drawn);
+        else kstatus_set(status, FE2O3_KSTATUS_SCAN_STATE);
+        s_tag = scan_tag(drawn);
+    }
     __syncthreads();
-    const uint32_t tile = s_tile;
+    const uint32_t tile = s_tile, tag = s_tag;
+    if (tile == kNoTile) return;
     const uint64_t first = (uint64_t)tile * kTileElems, base = first + warp * (kTileElems / kWaveWarps) + lane * 4;
     const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0 && first + kTileElems <= n;
-    const uint32_t epoch = __ldcg(&ctl->launches) + 1u;
     uint4 x[kWaveRows];   // row j: 128 consecutive elements of the warp's part
 #pragma unroll
     for (int j = 0; j < kWaveRows; ++j) {
@@ -177,13 +186,13 @@ device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t 
         uint32_t aggregate = 0;
 #pragma unroll
         for (int q = 0; q < kWaveWarps; ++q) aggregate = add<kFloat>(aggregate, s_warp[q]);
-        desc_store(desc + tile, epoch, aggregate);
+        desc_store(desc + tile, tag, aggregate);
     }
     uint32_t before = 0;
     bool ok = true;
     for (uint32_t i = tid; i < tile; i += kWaveThreads) {
         uint64_t d = desc_load(desc + i);
-        for (uint32_t spins = 0; (uint32_t)(d >> 32) != epoch; d = desc_load(desc + i)) {
+        for (uint32_t spins = 0; (uint32_t)(d >> 32) != tag; d = desc_load(desc + i)) {
             if (++spins > kDescSpin) { ok = false; break; }
             __nanosleep(20);
         }
@@ -193,7 +202,7 @@ device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t 
     before = warp_sum<kFloat>(before);
     if (lane == 0) s_before[warp] = before;
     __syncthreads();
-    if (tid == 0) block_done(ctl, epoch);
+    if (tid == 0) block_done(state, desc, tag, gridDim.x, status);
     uint32_t carry = 0;   // everything before this warp's first element
 #pragma unroll
     for (int q = 0; q < kWaveWarps; ++q) carry = add<kFloat>(carry, s_before[q]);
@@ -228,7 +237,7 @@ device_scan_wave_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t 
 
 template <bool kFloat>
 __global__ void __launch_bounds__(kScanThreads, 1)
-device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, ScanControl *ctl,
+device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclusive, scan_word *state,
                    uint64_t *desc, uint32_t *status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -249,7 +258,8 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
     }
     __syncthreads();
     begin_after_previous();
-    const uint32_t epoch = __ldcg(&ctl->launches) + 1u;
+    const uint32_t tag = scan_tag(__ldcg(state));
+    const uint32_t tickets = (uint32_t)((n + kTileElems - 1) / kTileElems) + gridDim.x;   // every block draws one past the last tile
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
@@ -258,7 +268,12 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
             const uint32_t st = k % kStages, ph = (k / kStages) & 1;
             if (!mbar_wait_warp(&sh.empty[st], ph ^ 1)) { ok = false; break; }
             uint32_t t = 0;
-            if (lane == 0) t = atomicAdd(&ctl->ticket, 1u);
+            if (lane == 0) {
+                scan_word drawn;
+                t = kNoTile;
+                if (scan_take<DeviceWords>(state, tickets, drawn)) t = scan_tickets(drawn);
+                else kstatus_set(status, FE2O3_KSTATUS_SCAN_STATE);
+            }
             t = __shfl_sync(0xffffffffu, t, 0);
             const uint64_t base = (uint64_t)t * kTileElems;
             if (base >= n) {
@@ -346,7 +361,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
                 uint32_t aggregate = 0;
                 for (int q = 0; q < kFinishWarps; ++q) aggregate = add<kFloat>(aggregate, sh.part[st][q]);
                 sh.arrivals[st] = 0;
-                desc_store(desc + tile, epoch, aggregate);
+                desc_store(desc + tile, tag, aggregate);
                 mbar_arrive(&sh.agg_ready[st]);
             }
         }
@@ -371,13 +386,13 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
 #pragma unroll
                     for (int q = 0; q < kWindow; ++q) {   // all loads of the step in flight together
                         const uint32_t mine = b + 32 * q + lane;
-                        d[q] = mine < hi ? desc_load(desc + mine) : ((uint64_t)epoch << 32);
+                        d[q] = mine < hi ? desc_load(desc + mine) : ((uint64_t)tag << 32);
                     }
 #pragma unroll
                     for (int q = 0; q < kWindow; ++q) {
                         const uint32_t mine = b + 32 * q + lane;
                         uint32_t spins = 0;
-                        while ((uint32_t)(d[q] >> 32) != epoch) {
+                        while ((uint32_t)(d[q] >> 32) != tag) {
                             if (++spins > kDescSpin) { ok = false; break; }
                             __nanosleep(100);
                             d[q] = desc_load(desc + mine);
@@ -408,7 +423,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
 #pragma unroll
                         for (int q = 0; q < kWindow; ++q) {
                             const uint32_t mine = (h ? mid : covered) + 32 * q + lane;
-                            d[h][q] = mine < (h ? tile : mid) ? desc_load(desc + mine) : ((uint64_t)epoch << 32);
+                            d[h][q] = mine < (h ? tile : mid) ? desc_load(desc + mine) : ((uint64_t)tag << 32);
                         }
                     uint32_t acc[2] = {0, 0};
 #pragma unroll
@@ -417,7 +432,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
                         for (int q = 0; q < kWindow; ++q) {
                             const uint32_t mine = (h ? mid : covered) + 32 * q + lane;
                             uint32_t spins = 0;
-                            while ((uint32_t)(d[h][q] >> 32) != epoch) {
+                            while ((uint32_t)(d[h][q] >> 32) != tag) {
                                 if (++spins > kDescSpin) { ok = false; break; }
                                 __nanosleep(100);
                                 d[h][q] = desc_load(desc + mine);
@@ -536,7 +551,7 @@ device_scan_kernel(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t exclu
         }
     }
     __syncthreads();
-    if (tid == 0) block_done(ctl, epoch);
+    if (tid == 0) block_done(state, desc, tag, tickets, status);
 }
 
 }  // namespace
@@ -546,20 +561,20 @@ int32_t launch_device_scan(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2
     const fe2o3_device_scan_u32_args *a = static_cast<const fe2o3_device_scan_u32_args *>(args);
     const uint64_t n = a->values.len;
     const uint32_t tiles = (uint32_t)((n + kTileElems - 1) / kTileElems);
-    const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
+    const uint32_t sms = min(ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u, kMaxBlocks / kWaveTilesPerSm);
     const bool wave = tiles <= kWaveTilesPerSm * sms;
     const uint32_t grid = wave || tiles < sms ? (tiles ? tiles : 1u) : sms;
     if (geo) *geo = wave ? fe2o3_geometry{{grid, 1, 1}, {kWaveThreads, 1, 1}, 0, 1} : fe2o3_geometry{{grid, 1, 1}, {kScanThreads, 1, 1}, kSmemBytes, 1};
     if (plan_only || n == 0) return FE2O3_OK;
-    // counters at word 0, descriptors from byte 64
-    ScanControl *ctl = reinterpret_cast<ScanControl *>(ctx->scan_scratch);
+    // the state at byte 0, descriptors from byte 64
+    scan_word *state = reinterpret_cast<scan_word *>(ctx->scan_scratch);
     uint64_t *desc = reinterpret_cast<uint64_t *>(ctx->scan_scratch + 16);
     const uint32_t *in = reinterpret_cast<const uint32_t *>(a->values.ptr);
     uint32_t *out = reinterpret_cast<uint32_t *>(a->output.ptr);
     const cudaError_t e = wave ? fe2o3_launch_early(device_scan_wave_kernel<kFloat>, grid, kWaveThreads, 0, s, 1, in, out, n,
-                                                    a->exclusive, ctl, desc, ctx->status_word)
+                                                    a->exclusive, state, desc, ctx->status_word)
                                : fe2o3_launch_early(device_scan_kernel<kFloat>, grid, kScanThreads, kSmemBytes, s, 1, in, out, n,
-                                                    a->exclusive, ctl, desc, ctx->status_word);
+                                                    a->exclusive, state, desc, ctx->status_word);
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, kFloat ? "device_scan_sum_f32" : "device_scan_sum_u32");
 }

@@ -56,6 +56,7 @@ extern "C" {
 #define FE2O3_KSTATUS_WEIGHTS 3u
 #define FE2O3_KSTATUS_WAIT_EXPIRED 4u
 #define FE2O3_KSTATUS_SLOT_RANGE 5u
+#define FE2O3_KSTATUS_SCAN_STATE 6u
 
 typedef struct fe2o3_ctx fe2o3_ctx;
 typedef struct fe2o3_stream fe2o3_stream;
@@ -446,7 +447,10 @@ typedef struct fe2o3_masked_reduce_u32_packed_args {
  * crates/fe2o3-device/src/collective.rs:413-460 and :503-571 extended to a whole
  * array (output[i] = values[0] + ... + values[i]; the exclusive form is shifted
  * by one and starts at zero).  values.len == output.len <= 2^31; the output
- * may not overlap the input; one scan at a time per context. */
+ * may not overlap the input; one scan at a time per context.  Two that overlap
+ * spoil each other's outputs and leave the context's scan state in disorder:
+ * later scans then write nothing and report FE2O3_KSTATUS_SCAN_STATE until that
+ * status has been taken, which puts the state right. */
 #define FE2O3_SCAN_MAX_ELEMENTS (1ull << 31)
 typedef struct fe2o3_device_scan_u32_args {
     fe2o3_slice values, output;

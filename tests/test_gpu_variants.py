@@ -206,6 +206,29 @@ def test_first_scan_of_a_context_on_its_own_stream(gpu, orc):
         assert (O.to_host_vec(stream) == want).all()
 
 
+@pytest.mark.parametrize("n,tickets", [(3 * 8192, 5), (3 * 8192, 1 << 31), (700 * 8192, 1 << 31)])
+def test_scan_reports_and_recovers_from_disordered_counters(gpu, orc, n, tickets):
+    """Counters that are not those between two launches (here: tickets that nobody should have drawn) are reported by the
+    next scan, which writes nothing, and put right when that status is taken."""
+    import ctypes as C
+    fe, _, stream = gpu
+    ctx = fe.GpuContext(0)   # its own counters
+    own = ctx.create_stream()
+    state = C.c_uint64.from_address(ctx._h.value + 64).value   # fe2o3_ctx::scan_scratch; the low half of its first word counts tickets
+    v = np.arange(1, n + 1, dtype=np.uint32)
+    V, one = fe.DeviceBuffer.from_host(stream, v), fe.DeviceBuffer.from_host(stream, np.ones(1, np.uint32))
+    O = fe.DeviceBuffer.from_host(stream, np.full(n, 0xdeadbeef, np.uint32))
+    p = fe.prepare(ctx, "device_scan_u32", values=V, output=O, exclusive=0)
+    planted = fe.DeviceBuffer.from_host(stream, np.array([tickets], np.uint32))
+    fe.prepare(ctx, "masked_reduce_u32", values=planted, active=one, output=(state, 1)).launch_and_wait(own)
+    with pytest.raises(fe.Fe2o3Error):
+        p.launch_and_wait(own)
+    assert p.kernel_status == 6 and (O.to_host_vec(stream) == 0xdeadbeef).all()
+    for _ in range(2):
+        p.launch_and_wait(own)
+        assert (O.to_host_vec(stream) == orc.scan_sum_u32(v, False)).all()
+
+
 def test_scan_beside_other_kernels(gpu, orc):
     """More register tiles than are resident at once, while another stream's kernels hold the SMs: a block only waits for
     tiles that have started."""
