@@ -1446,7 +1446,7 @@ int32_t fe2o3_moe_expert_ffn_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_expert_f
     // saves the compaction pass (compact_x is then left untouched); FE2O3_FFN_GATHER=0 keeps the compaction.
     const char *gather_env = getenv("FE2O3_FFN_GATHER");
     bool gathered = false;
-    if (!(gather_env && gather_env[0] == '0'))
+    if (!(gather_env && gather_env[0] == '0') && a->tokens > 0)
         gathered = gemm_tc_set_gather(&p->gemm[0], reinterpret_cast<const uint32_t *>(a->permutation.ptr),
                                       reinterpret_cast<const void *>(a->x.ptr), a->tokens);
     gemm_tc_geometry(&p->gemm[0], &p->geo);
@@ -1473,6 +1473,11 @@ int32_t fe2o3_moe_expert_ffn_combine_v1_prepare(fe2o3_ctx *ctx, const fe2o3_moe_
         st = gemm_tc_plan(ctx, &p->gemm[1], a->hidden.ptr, a->w2.ptr, a->combined_output.ptr, rows, a->d_model, a->d_ff,
                           a->d_ff, a->d_model, a->d_model, 1.f, 0.f, EPI_COMBINE_ADD, off, a->experts);
     if (st != FE2O3_OK) return fail_prepare(out, st);
+    p->geo.launches = 2;
+    if (a->tokens == 0 && (a->x.ptr & 15u) == 0) {   // an empty output: nothing is launched, whatever the table says
+        p->gemm[0].p.M = p->gemm[1].p.M = 0;
+        return FE2O3_OK;
+    }
     if (!gemm_tc_set_gather(&p->gemm[0], perm, reinterpret_cast<const void *>(a->x.ptr), a->tokens)) {
         fe2o3_set_error("Unsupported{x must be 16-byte aligned with whole 64-column blocks}");
         return fail_prepare(out, FE2O3_ERR_UNSUPPORTED_SHAPE);

@@ -997,14 +997,13 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
     return fe2o3_cuda_status(e, "gemm_tc");
 }
 
-// Makes the plan's A operand a gather: row r of A = row (perm[r] >> 1) of src.  Needs whole 64-column K blocks.
+// Makes the plan's A operand a gather: row r of A = row (perm[r] >> 1) of src.  Needs whole 64-column K blocks and at
+// least one token: the copy engine's gather form wants a map whose box is one row high, and src without rows has none.
 bool gemm_tc_set_gather(GemmTcPlan *plan, const uint32_t *perm, const void *src, uint32_t tokens) {
-    if (plan->p.K % BK != 0 || (reinterpret_cast<uintptr_t>(src) & 15u) != 0) return false;
-    if (tokens) {   // the copy engine's gather form wants a box one row high
-        const uint64_t dims[2] = {plan->p.K, tokens}, stride[1] = {(uint64_t)plan->p.K * 2};
-        const uint32_t box[2] = {BK, 1};
-        if (fe2o3_make_tmap_bf16(&plan->tmA, reinterpret_cast<uint64_t>(src), 2, dims, stride, box) != FE2O3_OK) return false;
-    }
+    if (plan->p.K % BK != 0 || (reinterpret_cast<uintptr_t>(src) & 15u) != 0 || tokens == 0) return false;
+    const uint64_t dims[2] = {plan->p.K, tokens}, stride[1] = {(uint64_t)plan->p.K * 2};
+    const uint32_t box[2] = {BK, 1};
+    if (fe2o3_make_tmap_bf16(&plan->tmA, reinterpret_cast<uint64_t>(src), 2, dims, stride, box) != FE2O3_OK) return false;
     plan->p.gather_perm = perm;
     plan->p.gather_src = src;
     plan->p.gather_tokens = tokens;

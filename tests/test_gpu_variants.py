@@ -98,6 +98,23 @@ def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
 
 
+def test_expert_ffn_without_tokens(gpu):
+    """No token to gather, and a table that claims rows all the same: rows of zeros, and no launch for an empty output."""
+    fe, ctx, stream = gpu
+    d, f, rows = 128, 64, 200
+    B = lambda a: fe.DeviceBuffer.from_host(stream, a)
+    X, W1, W2 = B(np.ones(64, np.uint16)), B(np.ones(d * f, np.uint16)), B(np.ones(f * d, np.uint16))
+    PERM, OFF = B(np.arange(rows, dtype=np.uint32)), B(np.array([0, rows], np.uint32))
+    CX, HID = B(np.ones(rows * d, np.uint16)), B(np.ones(rows * f, np.uint16))
+    CO = Guarded(fe, stream, np.ones(rows * d, np.float32))
+    common = dict(w1=W1, w2=W2, permutation=PERM, expert_offsets=OFF, hidden=HID, tokens=0, d_model=d, d_ff=f, experts=1)
+    run(fe, ctx, stream, "moe_expert_ffn_v1", x=X.view(0, 0), compact_x=CX, compact_output=CO.slice, **common)
+    assert (CO.read() == 0).all()
+    run(fe, ctx, stream, "moe_expert_ffn_combine_v1", x=X.view(0, 0), route_weights=CO.buf.view(GUARD, 0),
+        combined_output=CO.buf.view(GUARD, 0), **common)
+    assert (CO.read() == 0).all()
+
+
 # ---- gate, first launch of a process: sizes at which its blocks ask for shared memory that only together with the
 # kernel's own passes the limit without opt-in, so that an earlier launch of another size would hide a missing one
 @pytest.mark.parametrize("T,E", [(2048, 8), (1000, 16), (4000, 4)])
