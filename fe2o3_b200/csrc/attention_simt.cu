@@ -1,22 +1,12 @@
-// CUDA-core attention: the reference kernel's per-key online recurrence
-// (examples/flash_attention_v1/src/kernel.rs:56-113: m' = max(m, s),
-// p = exp(m - m'), c = exp(s - m'), l = l*p + c, acc = acc*p + v*c, out = acc/l,
-// first key initialises m = s, l = 1, acc = v) for any [B][H][S][D] shape, f32
+// CUDA-core attention: the recurrence of attention_row.cuh for any [B][H][S][D] shape, f32
 // or bf16 inputs, causal or not.  One warp owns one query row; lanes split the
 // head dimension.  It serves the fixed f32 B1/H1/N8/D16 profile and every shape
-// the tensor-core kernel does not admit.
-#include "common.cuh"
+// the tensor-core kernels do not admit.
+#include "attention_row.cuh"
 
 namespace {
 
 constexpr int kMaxPerLane = 8;  // head_dim <= 256
-
-template <typename T>
-__device__ __forceinline__ float ld(const T *p, uint64_t i);
-template <>
-__device__ __forceinline__ float ld<float>(const float *p, uint64_t i) { return p[i]; }
-template <>
-__device__ __forceinline__ float ld<uint16_t>(const uint16_t *p, uint64_t i) { return bf16_bits_to_f32(p[i]); }
 
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -27,60 +17,10 @@ attention_simt_kernel(const T *__restrict__ q, const T *__restrict__ k, const T 
     const uint64_t row = (uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (row >= (uint64_t)bh * seq) return;
     const uint32_t head = (uint32_t)(row / seq), qr = (uint32_t)(row % seq);
-    const uint64_t base = (uint64_t)head * seq * dim;
-    float qv[kMaxPerLane], acc[kMaxPerLane];
-    bool finite = true;
-#pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
-        const uint32_t f = lane + 32 * i;
-        qv[i] = f < dim ? ld<T>(q, base + (uint64_t)qr * dim + f) : 0.0f;
-        acc[i] = 0.0f;
-        finite = finite && isfinite(qv[i]);
-    }
-    float m = 0.0f, l = 0.0f;
-    const uint32_t keys = causal ? qr + 1 : seq;
-    for (uint32_t kr = 0; kr < keys; ++kr) {
-        float part = 0.0f;
-        float vv[kMaxPerLane];
-#pragma unroll
-        for (int i = 0; i < kMaxPerLane; ++i) {
-            const uint32_t f = lane + 32 * i;
-            float kv = 0.0f;
-            vv[i] = 0.0f;
-            if (f < dim) {
-                kv = ld<T>(k, base + (uint64_t)kr * dim + f);
-                vv[i] = ld<T>(v, base + (uint64_t)kr * dim + f);
-            }
-            finite = finite && isfinite(kv) && isfinite(vv[i]);
-            part = fmaf(qv[i], kv, part);
-        }
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-        const float s = part * scale;
-        if (kr == 0) {
-            m = s;
-            l = 1.0f;
-#pragma unroll
-            for (int i = 0; i < kMaxPerLane; ++i) acc[i] = vv[i];
-            continue;
-        }
-        const float nm = fmaxf(m, s);
-        const float pw = expf(m - nm), cw = expf(s - nm);
-        l = l * pw + cw;
-#pragma unroll
-        for (int i = 0; i < kMaxPerLane; ++i) acc[i] = acc[i] * pw + vv[i] * cw;
-        m = nm;
-    }
-    finite = __all_sync(0xffffffffu, finite && isfinite(l) && l > 0.0f);
-    if (!finite) {  // finite-input policy: leave the row unwritten, record a status word
-        if (lane == 0) kstatus_set(status, FE2O3_KSTATUS_NONFINITE);
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
-        const uint32_t f = lane + 32 * i;
-        if (f < dim) out[base + (uint64_t)qr * dim + f] = acc[i] / l;
-    }
+    // finite-input policy: a row that reads a non-finite value is left unwritten, and a status word recorded
+    if (!attention_row<T, kMaxPerLane, false>(q, k, v, out, (uint64_t)head * seq * dim, qr, causal ? qr + 1 : seq, dim, scale, lane) &&
+        lane == 0)
+        kstatus_set(status, FE2O3_KSTATUS_NONFINITE);
 }
 
 }  // namespace

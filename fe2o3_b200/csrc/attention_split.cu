@@ -24,14 +24,18 @@
 //   direction (round 0 forwards, round 1 backwards); a tile stops at its own last block.
 //   Head sizes below 64 or between 64 and 128 are zero-filled by the copy engine on the
 //   way in and clipped on the way out; Q*K^T takes only the k steps in use.
-//   A row that met a non-finite score or value is left unwritten and reported, as the
-//   CUDA-core kernel does.
+//   A row that met a non-finite score or value is settled one by one by the CUDA-core
+//   recurrence (attention_row.cuh), which reads the row's own keys only: the tensor core
+//   also multiplies the values of keys that a causal row does not admit, by probabilities
+//   of 0, and 0 x Inf is NaN.  What that finds non-finite too is left unwritten and reported.
+//   The other warps may wait long meanwhile, so waits that run out start over as long as
+//   rows are being settled (Waits).
 // B2 H12 S1900 D128 causal: 8017 us on the CUDA cores, 65 us here (340 TFLOP/s of the
 // 22.2 GFLOP the function needs; longest unit 30 of an average 19.5 block pairs).
 // The rule in front (attention_split_supported) is what the copy engine can address:
 // rows of whole 16 bytes and 16-byte aligned bases; the rest, f32 inputs and head sizes
 // above 128 stay on the CUDA cores.  All waits are bounded.
-#include "common.cuh"
+#include "attention_row.cuh"
 #include "gemm_tc.h"
 
 #include <new>
@@ -63,9 +67,10 @@ struct Layout {
 constexpr uint32_t kTmemCols = 512, kColO = 128, kColP = 384;
 
 struct SplitParams {
+    const uint16_t *q, *k, *v;   // for rows that are settled one by one
     float *out;
     uint32_t bh, seq, dim;
-    float scale_log2;   // scale * log2(e)
+    float scale, scale_log2;   // scale_log2 = scale * log2(e)
     uint32_t causal;
     uint32_t q_blocks;  // 256-row blocks per head
     uint32_t units;     // work units; `half`: of one tile each, two per block
@@ -118,6 +123,20 @@ __device__ __forceinline__ uint32_t cut_bf16x2(uint64_t v, uint64_t &rest) {
     return __byte_perm(l, h, 0x7632);
 }
 
+// Waits on another role of the block.  `settled` counts rows settled one by one.
+struct Waits {
+    const volatile uint32_t *settled;
+    __device__ __forceinline__ bool operator()(uint64_t *bar, uint32_t parity) const {
+        uint32_t seen = 0;
+        while (!mbar_wait_warp(bar, parity)) {
+            const uint32_t now = __shfl_sync(0xffffffffu, *settled, 0);
+            if (now == seen) return false;
+            seen = now;
+        }
+        return true;
+    }
+};
+
 template <int NG>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -137,6 +156,8 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     uint64_t *p_ready = s_empty + QT;
     uint64_t *pv_done = p_ready + QT;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pv_done + QT);
+    uint32_t *settled = tmem_slot + 1;
+    const Waits wait{settled};
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -154,6 +175,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             mbar_init(&p_ready[t], 4);
             mbar_init(&pv_done[t], 1);
         }
+        *settled = 0;
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -182,7 +204,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         Unit u;
         for (uint32_t i = 0; ok && unit_at(p, i, u); ++i) {
             if (u.nkv == 0) continue;   // every role skips a unit whose rows all lie beyond seq
-            if (!mbar_wait_warp(q_empty, (n_units & 1) ^ 1)) { ok = false; break; }
+            if (!wait(q_empty, (n_units & 1) ^ 1)) { ok = false; break; }
             ++n_units;
             if (elect_one()) {
                 mbar_arrive_expect_tx(q_full, ((u.n[0] ? 1u : 0u) + (u.n[1] ? 1u : 0u)) * L::kQTile);
@@ -196,7 +218,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             __syncwarp();
             for (uint32_t j = 0; j < u.nkv; ++j, ++g) {
                 const uint32_t st = g % KV_STAGES, ph = (g / KV_STAGES) & 1;
-                if (!mbar_wait_warp(&k_empty[st], ph ^ 1)) { ok = false; break; }
+                if (!wait(&k_empty[st], ph ^ 1)) { ok = false; break; }
                 if (elect_one()) {
                     mbar_arrive_expect_tx(&k_full[st], L::kKvTile);
 #pragma unroll
@@ -205,7 +227,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                                     (int32_t)u.head);
                 }
                 __syncwarp();
-                if (!mbar_wait_warp(&v_empty[st], ph ^ 1)) {
+                if (!wait(&v_empty[st], ph ^ 1)) {
                     ok = false;
                     mbar_wait_warp(&k_full[st], ph);   // the K copy just issued must land before the CTA exits
                     break;
@@ -249,7 +271,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         uint32_t pv_st = 0, pv_ph = 0, pv_gt = 0, pv_acc = 0;
         auto issue_pv = [&]() {
             pending = false;
-            if (!mbar_wait_warp(&p_ready[t], pv_gt & 1) || !mbar_wait_warp(&v_full[pv_st], pv_ph)) { ok = false; return; }
+            if (!wait(&p_ready[t], pv_gt & 1) || !wait(&v_full[pv_st], pv_ph)) { ok = false; return; }
             tc_fence_after();
             if (elect_one()) {
                 const uint64_t dVs = dV + ((pv_st * L::kKvTile) >> 4);
@@ -271,19 +293,19 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             if (u.nkv == 0) continue;
             const uint32_t qph = n & 1, mine = t == 0 ? u.n[0] : u.n[1];
             ++n;
-            if (!mbar_wait_warp(q_full, qph)) { ok = false; break; }
+            if (!wait(q_full, qph)) { ok = false; break; }
             if (mine == 0 && lane == 0) mbar_arrive(q_empty);   // no such tile here: nothing of Q is read
             for (uint32_t j = 0; ok && j < u.nkv; ++j, ++g) {
                 const uint32_t st = g % KV_STAGES, ph = (g / KV_STAGES) & 1;
                 if (j >= mine) {   // past this tile's last block: only hand the other tile's K/V blocks on
                     if (pending) issue_pv();
-                    if (!ok || !mbar_wait_warp(&k_full[st], ph)) { ok = false; break; }
+                    if (!ok || !wait(&k_full[st], ph)) { ok = false; break; }
                     if (lane == 0) mbar_arrive(&k_empty[st]);
-                    if (!mbar_wait_warp(&v_full[st], ph)) { ok = false; break; }
+                    if (!wait(&v_full[st], ph)) { ok = false; break; }
                     if (lane == 0) mbar_arrive(&v_empty[st]);
                     continue;
                 }
-                if (!mbar_wait_warp(&s_empty[t], (gt & 1) ^ 1) || !mbar_wait_warp(&k_full[st], ph)) { ok = false; break; }
+                if (!wait(&s_empty[t], (gt & 1) ^ 1) || !wait(&k_full[st], ph)) { ok = false; break; }
                 tc_fence_after();
                 if (elect_one()) {
                     const uint64_t dKs = dK + ((st * L::kKvTile) >> 4);
@@ -331,7 +353,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             bool bad = false;          // a non-finite score of an admitted key
 
             for (uint32_t j = 0; j < mine; ++j, ++gt) {
-                if (!mbar_wait_warp(&s_full[t], gt & 1)) { ok = false; break; }
+                if (!wait(&s_full[t], gt & 1)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t s[2][32];
                 tmem_ld_32x32b_x32(tS, s[0]);
@@ -408,7 +430,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
                 // P of the previous block must have been consumed and O must be quiescent
                 if (j > 0) {
-                    if (!mbar_wait_warp(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
+                    if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
                     tc_fence_after();
                     if (__any_sync(0xffffffffu, move)) {
 #pragma unroll 1
@@ -436,7 +458,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 if (lane == 0) mbar_arrive(&p_ready[t]);
             }
             if (!ok) break;
-            if (!mbar_wait_warp(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
+            if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
             tc_fence_after();
             const float inv = 1.0f / l;
             bool good = !bad && isfinite(l) && l > 0.0f;
@@ -453,8 +475,8 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     o[h][q] = __float_as_uint(v);
                 }
             }
-            if (qrow < p.seq && !good) kstatus_set(p.status, FE2O3_KSTATUS_NONFINITE);
-            if (__all_sync(0xffffffffu, good || qrow >= p.seq)) {
+            const uint32_t unsettled = __ballot_sync(0xffffffffu, !good && qrow < p.seq);
+            if (unsettled == 0) {
                 // through shared memory and the copy engine: full-line writes that do not hold the warp
 #pragma unroll
                 for (int h = 0; h < NG * 2; ++h) {
@@ -483,6 +505,14 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     for (int q = 0; q < 32; ++q)
                         if (h * 32 + q < p.dim) dst[h * 32 + q] = __uint_as_float(o[h][q]);
             }
+            for (uint32_t rows = unsettled; rows != 0; rows &= rows - 1) {
+                const uint32_t row = row0 + __ffs(rows) - 1;
+                if (!attention_row<uint16_t, NG * 2, true>(p.q, p.k, p.v, p.out, (uint64_t)u.head * p.seq * p.dim, row,
+                                                           p.causal ? row + 1 : p.seq, p.dim, p.scale, lane) && lane == 0)
+                    kstatus_set(p.status, FE2O3_KSTATUS_NONFINITE);
+                if (lane == 0) atomicAdd(settled, 1u);
+            }
+            __syncwarp();
             // the next unit's first P*V overwrites O: order this thread's reads of O before its p_ready arrival
             tc_fence_before();
             __syncwarp();
@@ -534,7 +564,9 @@ int32_t attention_split_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args
     const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
     if (units > 0x7fffffffull) { delete plan; fe2o3_set_error("UnsupportedShape: too many rows"); return FE2O3_ERR_UNSUPPORTED_SHAPE; }
     const bool half = 2 * units <= sms;
-    plan->p = SplitParams{reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->dim, a->scale * 1.4426950408889634f, a->causal,
+    plan->p = SplitParams{reinterpret_cast<const uint16_t *>(a->q.ptr), reinterpret_cast<const uint16_t *>(a->k.ptr),
+                          reinterpret_cast<const uint16_t *>(a->v.ptr), reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->dim,
+                          a->scale, a->scale * 1.4426950408889634f, a->causal,
                           q_blocks, (uint32_t)(half ? 2 * units : units), half ? 1u : 0u, ctx->status_word};
     plan->grid = plan->p.units < sms ? plan->p.units : sms;
     plan->groups = a->dim <= 64 ? 1 : 2;

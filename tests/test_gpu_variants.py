@@ -352,3 +352,28 @@ def test_attention_split_leaves_bad_rows_unwritten(gpu, orc, causal):
     _, want = orc.flash_attention(*(synth.bf16_to_f32(x) for x in (q, k, v)), 1.0 / np.sqrt(D), causal)
     assert (got[bad] == -7).all()
     assert np.abs(got - want)[~bad].max() <= 2.5e-5 * 6
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S,D,key,bad", [(150, 128, 70, 0x7f80), (700, 72, 383, 0x7fc0), (260, 32, 256, 0xff80), (65, 8, 1, 0x7f80)])
+def test_attention_split_bad_value_spares_rows_that_do_not_admit_it(gpu, orc, S, D, key, bad, causal):
+    """The tensor core multiplies the values of masked keys too, by probabilities of 0: rows before a non-finite value
+    are written all the same, as the CUDA-core kernel writes them."""
+    from fe2o3_b200 import synth
+    fe, ctx, stream = gpu
+    B, H = 1, 3
+    q, k, v = (synth.normal_bf16(3, d, B * H * S * D, 1.0).reshape(B, H, S, D) for d in (1, 2, 3))
+    _, want = orc.flash_attention(*(synth.bf16_to_f32(x) for x in (q, k, v)), 1.0 / np.sqrt(D), causal)
+    v[0, 1, key, D - 1] = bad
+    Q, K, V = Guarded(fe, stream, q), Guarded(fe, stream, k), Guarded(fe, stream, v)
+    O = Guarded(fe, stream, np.full(q.size, -7, np.float32))
+    p = fe.prepare(ctx, "flash_attention_v1", q=Q.slice, k=K.slice, v=V.slice, output=O.slice, batch=B, heads=H, seq=S, dim=D,
+                   scale=1.0 / np.sqrt(D), causal=int(causal), input_dtype=fe.DTYPE_BF16)
+    with pytest.raises(fe.Fe2o3Error):
+        p.launch_and_wait(stream)
+    assert p.kernel_status == 2
+    got = O.read().reshape(B, H, S, D)
+    lost = np.zeros((B, H, S), bool)
+    lost[0, 1, key if causal else 0:] = True
+    assert (got[lost] == -7).all()
+    assert np.abs(got - want)[~lost].max() <= 2.5e-5 * 6   # as above: largest |v| below 6
