@@ -872,7 +872,7 @@ bool gemm_tc_supported(uint64_t a, uint64_t b, uint32_t lda, uint32_t ldb, uint3
 int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, uint64_t c, uint32_t M, uint32_t N,
                      uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta, uint32_t epilogue,
                      const uint32_t *expert_offsets, uint32_t experts, uint32_t expert_mod, uint32_t b_matrices,
-                     const GemmEp *ep, uint32_t expected_rows) {
+                     const GemmEp *ep) {
     // Tile shape.  A launch costs its rounds of tiles times what a round takes, which beyond the fixed ~4 us of a
     // launch goes as 0.55 : 0.68 : 1 for 64, 128 and 256 columns (measured, us: 1024^3 8.3 : 9.4 : 11.3 in one round
     // each, 2048x2048x512 14.4 : 11.1 : 9.3 in four, two and one), so a small result takes the narrowest tile that
@@ -884,7 +884,6 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
     // 194 against 209 us a layer pass).  Groups end in a partly filled tile, half of one on average.
     // The expert-parallel GEMMs count finished 256-wide tiles and keep them: half-width ones re-read A twice as
     // often and were slower there on 4096 and 8192 rows (530 against 481 us and 686 against 590 us a pass).
-    (void)expected_rows;
     plan->bn = N > 128 ? 256 : 128;
     plan->pair = 0;
     uint32_t a_box = BM;
@@ -936,7 +935,7 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
         bulk = 1;
     }
     plan->p = GemmParams{reinterpret_cast<void *>(c), M, N, K, ldc, alpha, beta, epilogue, expert_offsets, experts,
-                         expert_mod, bulk, ctx->status_word, ep ? *ep : GemmEp{}, nullptr, nullptr, 0u, nullptr, nullptr, 0u, nullptr, 0ull, a_box, 0u};
+                         expert_mod, bulk, ctx->status_word, ep ? *ep : GemmEp{}, nullptr, 0u, nullptr, nullptr, 0u, nullptr, 0ull, a_box, 0u};
     plan->p.after_previous = ep ? 0u : 1u;
     const uint32_t n_tiles = (N + plan->bn - 1) / plan->bn;
     const uint64_t tile_rows = plan->pair ? 2 * BM : BM;
@@ -1005,7 +1004,6 @@ bool gemm_tc_set_gather(GemmTcPlan *plan, const uint32_t *perm, const void *src,
     const uint32_t box[2] = {BK, 1};
     if (fe2o3_make_tmap_bf16(&plan->tmA, reinterpret_cast<uint64_t>(src), 2, dims, stride, box) != FE2O3_OK) return false;
     plan->p.gather_perm = perm;
-    plan->p.gather_src = src;
     plan->p.gather_tokens = tokens;
     return true;
 }

@@ -48,11 +48,10 @@ struct GemmParams {
     uint32_t bulk_store;     // C is addressable by the copy engine (tensor map tmC is valid)
     uint32_t *status;
     GemmEp ep;
-    // Gathered A (first GEMM of the single-GPU expert FFN): row r of A is row (gather_perm[r] >> 1) of
-    // gather_src ([gather_tokens][K] bf16), or zero when gather_perm[r] names no route; the block is then
+    // Gathered A (first GEMM of the single-GPU expert FFN): row r of A is row (gather_perm[r] >> 1) of the
+    // tensor that tmA covers ([gather_tokens][K] bf16), or zero when gather_perm[r] names no route; the block is then
     // launched with four warps more, which have the copy engine gather the rows into the swizzled A stage.
     const uint32_t *gather_perm;
-    const void *gather_src;
     uint32_t gather_tokens;
     // EPI_COMBINE_ADD (second GEMM of the single-GPU expert FFN with the combine folded in): row r is the expert
     // output of route combine_perm[r]; it is multiplied by that route's weight and added to row (route >> 1) of
@@ -80,7 +79,7 @@ struct GemmTcPlan {
     uint32_t smem;
     uint32_t overlap_previous;   // launch with programmatic stream serialization: 1 = may run beside the (small) blocks of the
                                  // kernel before it on the same SMs, 2 = takes over SMs as blocks of the kernel before it exit (these two
-                                 // synchronise through flags); 0 = started early too, but waits for that kernel to complete
+                                 // synchronise through flags); 0 = p.after_previous says
 };
 
 int32_t fe2o3_make_tmap_bf16(CUtensorMap *out, uint64_t base, uint32_t rank, const uint64_t *dims,
@@ -91,7 +90,7 @@ bool gemm_tc_supported(uint64_t a, uint64_t b, uint32_t lda, uint32_t ldb, uint3
 int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, uint64_t c, uint32_t M, uint32_t N,
                      uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta, uint32_t epilogue,
                      const uint32_t *expert_offsets, uint32_t experts, uint32_t expert_mod = 0, uint32_t b_matrices = 0,
-                     const GemmEp *ep = nullptr, uint32_t expected_rows = 0);
+                     const GemmEp *ep = nullptr);
 int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s);
 int32_t gemm_tc_init_device();
 bool gemm_tc_set_gather(GemmTcPlan *plan, const uint32_t *perm, const void *src, uint32_t tokens);

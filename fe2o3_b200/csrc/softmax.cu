@@ -18,8 +18,8 @@
 //   bits stay in registers.
 //   Rows of up to 64 columns share a warp (8 or 16 lanes a row), otherwise most
 //   lanes of the warp would idle.
-// 65536 x 1024: 91.8 us -> 81.8 us (6.56 TB/s) against the earlier form that kept
-// activity bits per element; 5000 x 3001 masked: 79.9 -> 31.5 us against one block
+// 65536 x 1024: 91.6 us -> 79.5 us (6.75 TB/s) against the earlier form that kept
+// activity bits per element; 5000 x 3001 masked: 79.9 -> 29.7 us against one block
 // per row with scalar accesses, four block barriers and a division per element.
 // Input, output and mask that are not aligned to one another (views at different
 // offsets) take one block per row with scalar accesses.
@@ -31,7 +31,7 @@ __device__ __forceinline__ bool finite4(float4 v) {
     return isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w);
 }
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256, kMaxCols = 4096;
 
 // Combines over the LANES threads of a row; every one receives the result.  Up to 32 lanes: a shuffle
 // tree.  More: each warp leaves its value in shared memory (`slots`, one per warp of the row) and the row's
@@ -182,8 +182,8 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// One 256-thread block per row, up to 4096 columns, scalar accesses: any alignment.
-constexpr int kBlockRowItems = 16;
+// One 256-thread block per row, scalar accesses: any alignment.
+constexpr int kBlockRowItems = kMaxCols / kThreads;
 
 __global__ void __launch_bounds__(kThreads)
 row_softmax_block_kernel(const float *__restrict__ in, float *__restrict__ out, const uint8_t *__restrict__ mask,
@@ -251,8 +251,9 @@ cudaError_t launch_row(const fe2o3_row_softmax_v1_args *a, bool shifted, cudaStr
     const float *in = reinterpret_cast<const float *>(a->input.ptr);
     float *out = reinterpret_cast<float *>(a->output.ptr);
     const uint8_t *mask = reinterpret_cast<const uint8_t *>(a->mask.ptr);
-    auto kernel = shifted ? (mask ? row_softmax_kernel<LANES, NV, true, true> : row_softmax_kernel<LANES, NV, false, true>)
-                          : (mask ? row_softmax_kernel<LANES, NV, true, false> : row_softmax_kernel<LANES, NV, false, false>);
+    auto kernel = mask ? row_softmax_kernel<LANES, NV, true, true> : row_softmax_kernel<LANES, NV, false, true>;
+    if constexpr (LANES * NV <= kMaxCols / 4)   // more vectors than that only rows have that start inside one
+        if (!shifted) kernel = mask ? row_softmax_kernel<LANES, NV, true, false> : row_softmax_kernel<LANES, NV, false, false>;
     return fe2o3_launch_early(kernel, grid, kThreads, 0, s, 1, in, out, mask, a->rows, a->cols, status);
 }
 
