@@ -569,8 +569,10 @@ def wl_moe(h, steps, warmup, cpu=True, exchange="auto", **shape):
                         "peer_mapping": getattr(layer, "peer_mapping", None),
                         "cuda_graph": bool(graphed), "kernels_per_pass": per_pass,
                         "algorithmic_flops_per_step": flops,
-                        "ffn_tiles": {"rows_this_rank": ffn_rows, "tile": "128x256", "sms": sms,
-                                      "waves_gemm1": m_tiles * (-(-f // 256)) / sms, "waves_gemm2": m_tiles * (-(-d // 256)) / sms},
+                        # the expert-parallel GEMMs keep this tile; on one GPU the shape is chosen at prepare
+                        "ffn_tiles": {"rows_this_rank": ffn_rows, "sms": sms, **(
+                            {"tile": "128x256", "waves_gemm1": m_tiles * (-(-f // 256)) / sms,
+                             "waves_gemm2": m_tiles * (-(-d // 256)) / sms} if layer.exchange == "peer" else {})},
                         "share_outside_ffn": max(0.0, 1.0 - ffn_ms / float(np.mean(ms))),
                         "l2": "weights (256 MiB) + activations larger than L2"}}
     # end to end through the C ABI with host buffers: pinned H2D of this rank's tokens into the layer's
