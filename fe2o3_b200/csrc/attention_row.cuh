@@ -13,11 +13,13 @@ template <>
 __device__ __forceinline__ float attention_ld<uint16_t>(const uint16_t *p, uint64_t i) { return bf16_bits_to_f32(p[i]); }
 
 // Row `qr` of the head at element `base` over its first `keys` keys, written to `out` unless a value that the row reads
-// or its sum is not finite; false then.  PER_LANE * 32 >= dim.  STOP_EARLY ends at the first such value.
-template <typename T, int PER_LANE, bool STOP_EARLY>
+// or its sum is not finite; false then.  PER_LANE * 32 >= dim.  AHEAD keys are fetched together and their scores summed up
+// side by side, with the same result for any AHEAD.  CHECK: the keys may hold non-finite values.  A row may take long:
+// `tick` is called every AHEAD keys.
+template <typename T, int PER_LANE, int AHEAD, bool CHECK, typename Tick>
 __device__ __forceinline__ bool attention_row(const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v,
                                               float *__restrict__ out, uint64_t base, uint32_t qr, uint32_t keys,
-                                              uint32_t dim, float scale, uint32_t lane) {
+                                              uint32_t dim, float scale, uint32_t lane, Tick tick) {
     float qv[PER_LANE], acc[PER_LANE];
     bool finite = true;
 #pragma unroll
@@ -27,39 +29,52 @@ __device__ __forceinline__ bool attention_row(const T *__restrict__ q, const T *
         acc[i] = 0.0f;
         finite = finite && isfinite(qv[i]);
     }
+    if (!__all_sync(0xffffffffu, finite)) return false;
     float m = 0.0f, l = 0.0f;
-    for (uint32_t kr = 0; kr < keys; ++kr) {
-        float part = 0.0f;
-        float vv[PER_LANE];
+    for (uint32_t k0 = 0; k0 < keys; k0 += AHEAD) {
+        tick(k0);
+        float part[AHEAD], vv[AHEAD][PER_LANE];
 #pragma unroll
-        for (int i = 0; i < PER_LANE; ++i) {
-            const uint32_t f = lane + 32 * i;
-            float kv = 0.0f;
-            vv[i] = 0.0f;
-            if (f < dim) {
-                kv = attention_ld<T>(k, base + (uint64_t)kr * dim + f);
-                vv[i] = attention_ld<T>(v, base + (uint64_t)kr * dim + f);
+        for (int a = 0; a < AHEAD; ++a) {
+            const uint32_t kr = k0 + a;
+            part[a] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < PER_LANE; ++i) {
+                const uint32_t f = lane + 32 * i;
+                float kv = 0.0f;
+                vv[a][i] = 0.0f;
+                if (f < dim && (AHEAD == 1 || kr < keys)) {
+                    kv = attention_ld<T>(k, base + (uint64_t)kr * dim + f);
+                    vv[a][i] = attention_ld<T>(v, base + (uint64_t)kr * dim + f);
+                }
+                if (CHECK) finite = finite && isfinite(kv) && isfinite(vv[a][i]);
+                part[a] = fmaf(qv[i], kv, part[a]);
             }
-            finite = finite && isfinite(kv) && isfinite(vv[i]);
-            part = fmaf(qv[i], kv, part);
         }
-        if (STOP_EARLY && !__all_sync(0xffffffffu, finite)) return false;
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-        const float s = part * scale;
-        if (kr == 0) {
-            m = s;
-            l = 1.0f;
+        for (int off = 16; off >= 1; off >>= 1) {
 #pragma unroll
-            for (int i = 0; i < PER_LANE; ++i) acc[i] = vv[i];
-            continue;
+            for (int a = 0; a < AHEAD; ++a) part[a] += __shfl_xor_sync(0xffffffffu, part[a], off);
         }
-        const float nm = fmaxf(m, s);
-        const float pw = expf(m - nm), cw = expf(s - nm);
-        l = l * pw + cw;
 #pragma unroll
-        for (int i = 0; i < PER_LANE; ++i) acc[i] = acc[i] * pw + vv[i] * cw;
-        m = nm;
+        for (int a = 0; a < AHEAD; ++a) {
+            const uint32_t kr = k0 + a;
+            if (AHEAD > 1 && kr >= keys) break;
+            const float s = part[a] * scale;
+            if (kr == 0) {
+                m = s;
+                l = 1.0f;
+#pragma unroll
+                for (int i = 0; i < PER_LANE; ++i) acc[i] = vv[a][i];
+                continue;
+            }
+            const float nm = fmaxf(m, s);
+            const float pw = expf(m - nm), cw = expf(s - nm);
+            l = l * pw + cw;
+#pragma unroll
+            for (int i = 0; i < PER_LANE; ++i) acc[i] = acc[i] * pw + vv[a][i] * cw;
+            m = nm;
+        }
     }
     if (!__all_sync(0xffffffffu, finite && isfinite(l) && l > 0.0f)) return false;
 #pragma unroll

@@ -18,8 +18,8 @@ attention_simt_kernel(const T *__restrict__ q, const T *__restrict__ k, const T 
     if (row >= (uint64_t)bh * seq) return;
     const uint32_t head = (uint32_t)(row / seq), qr = (uint32_t)(row % seq);
     // finite-input policy: a row that reads a non-finite value is left unwritten, and a status word recorded
-    if (!attention_row<T, kMaxPerLane, false>(q, k, v, out, (uint64_t)head * seq * dim, qr, causal ? qr + 1 : seq, dim, scale, lane) &&
-        lane == 0)
+    if (!attention_row<T, kMaxPerLane, 1, true>(q, k, v, out, (uint64_t)head * seq * dim, qr, causal ? qr + 1 : seq, dim, scale, lane,
+                                            [](uint32_t) {}) && lane == 0)
         kstatus_set(status, FE2O3_KSTATUS_NONFINITE);
 }
 

@@ -24,10 +24,11 @@
 //   direction (round 0 forwards, round 1 backwards); a tile stops at its own last block.
 //   Head sizes below 64 or between 64 and 128 are zero-filled by the copy engine on the
 //   way in and clipped on the way out; Q*K^T takes only the k steps in use.
-//   A row that met a non-finite score or value is settled one by one by the CUDA-core
-//   recurrence (attention_row.cuh), which reads the row's own keys only: the tensor core
+//   A row that met a non-finite score or value is settled one by one: the tensor core
 //   also multiplies the values of keys that a causal row does not admit, by probabilities
-//   of 0, and 0 x Inf is NaN.  What that finds non-finite too is left unwritten and reported.
+//   of 0, and 0 x Inf is NaN.  The first key of the head with a non-finite K or V is
+//   searched once; a row that admits it is left unwritten and reported, the others are
+//   computed by the CUDA-core recurrence (attention_row.cuh).
 //   The other warps may wait long meanwhile, so waits that run out start over as long as
 //   rows are being settled (Waits).
 // B2 H12 S1900 D128 causal: 8017 us on the CUDA cores, 65 us here (340 TFLOP/s of the
@@ -123,7 +124,7 @@ __device__ __forceinline__ uint32_t cut_bf16x2(uint64_t v, uint64_t &rest) {
     return __byte_perm(l, h, 0x7632);
 }
 
-// Waits on another role of the block.  `settled` counts rows settled one by one.
+// Waits on another role of the block.  `settled` moves on as long as rows are being settled one by one.
 struct Waits {
     const volatile uint32_t *settled;
     __device__ __forceinline__ bool operator()(uint64_t *bar, uint32_t parity) const {
@@ -136,6 +137,39 @@ struct Waits {
         return true;
     }
 };
+
+// The first of a head's first `keys` keys whose K or V row holds a non-finite value, or `keys`: no row that admits it has
+// a result.  Rows are whole 16-byte pieces.
+template <typename Tick>
+__device__ __forceinline__ uint32_t first_nonfinite_key(const uint16_t *k, const uint16_t *v, uint32_t keys, uint32_t dim, uint32_t lane, Tick tick) {
+    constexpr int kAhead = 4;
+    const uint32_t pieces = dim / 8;
+    const uint64_t end = (uint64_t)keys * pieces;
+    auto holds = [](uint4 w) {
+        auto one = [](uint32_t x) { return (x & 0x7f80u) == 0x7f80u || (x & 0x7f800000u) == 0x7f800000u; };
+        return one(w.x) || one(w.y) || one(w.z) || one(w.w);
+    };
+    for (uint64_t i0 = 0; i0 < end; i0 += 32 * kAhead) {
+        tick(0u);
+        uint4 w[kAhead][2];
+#pragma unroll
+        for (int a = 0; a < kAhead; ++a) {
+            const uint64_t i = i0 + a * 32 + lane;
+            w[a][0] = w[a][1] = make_uint4(0u, 0u, 0u, 0u);
+            if (i < end) {
+                w[a][0] = __ldg(reinterpret_cast<const uint4 *>(k) + i);
+                w[a][1] = __ldg(reinterpret_cast<const uint4 *>(v) + i);
+            }
+        }
+        uint32_t first = keys;
+#pragma unroll
+        for (int a = kAhead - 1; a >= 0; --a)
+            if (holds(w[a][0]) || holds(w[a][1])) first = (uint32_t)((i0 + a * 32 + lane) / pieces);
+        first = __reduce_min_sync(0xffffffffu, first);
+        if (first < keys) return first;
+    }
+    return keys;
+}
 
 template <int NG>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -505,12 +539,17 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     for (int q = 0; q < 32; ++q)
                         if (h * 32 + q < p.dim) dst[h * 32 + q] = __uint_as_float(o[h][q]);
             }
-            for (uint32_t rows = unsettled; rows != 0; rows &= rows - 1) {
-                const uint32_t row = row0 + __ffs(rows) - 1;
-                if (!attention_row<uint16_t, NG * 2, true>(p.q, p.k, p.v, p.out, (uint64_t)u.head * p.seq * p.dim, row,
-                                                           p.causal ? row + 1 : p.seq, p.dim, p.scale, lane) && lane == 0)
-                    kstatus_set(p.status, FE2O3_KSTATUS_NONFINITE);
-                if (lane == 0) atomicAdd(settled, 1u);
+            if (unsettled != 0) {
+                auto tick = [settled, lane](uint32_t) { if (lane == 0) atomicAdd(settled, 1u); };
+                const uint64_t head = (uint64_t)u.head * p.seq * p.dim;
+                const uint32_t last = row0 + 31 - __clz(unsettled);
+                const uint32_t bad_key = first_nonfinite_key(p.k + head, p.v + head, p.causal ? last + 1 : p.seq, p.dim, lane, tick);
+                for (uint32_t rows = unsettled; rows != 0; rows &= rows - 1) {
+                    const uint32_t row = row0 + __ffs(rows) - 1, keys = p.causal ? row + 1 : p.seq;
+                    if ((bad_key < keys || !attention_row<uint16_t, NG * 2, 4, false>(p.q, p.k, p.v, p.out, head, row, keys, p.dim, p.scale, lane, tick)) &&
+                        lane == 0)
+                        kstatus_set(p.status, FE2O3_KSTATUS_NONFINITE);
+                }
             }
             __syncwarp();
             // the next unit's first P*V overwrites O: order this thread's reads of O before its p_ready arrival
