@@ -9,7 +9,21 @@
 // truncation into three bf16 terms, hi + mid + lo, which hold the 24 bits exactly
 // (each term takes the top eight significant bits of what is left), and P*V is three
 // products accumulated into the same O: every product is exact, only the f32
-// accumulation rounds.  Per 128 x 64 block at head size 128 the tensor pipe then
+// accumulation rounds.
+//   That accumulation truncates, twelve times a block and always towards zero, which
+// over a whole row is up to ten times the error of the CUDA-core kernel (4096 keys of
+// head size 128: 1.4e-5 against 1.5e-6 of the result, 2-norm, against f64).  So a sum
+// in tensor memory covers a group of one, two or four blocks (starts_group: short rows
+// have the least error to hide it behind) and the groups are added in registers, where
+// additions round to nearest: 7.7e-7 at 4096 keys, and not above the CUDA cores from 50
+// to 4096 keys.  The price is a read of O per group between one P*V and the next, and
+// the registers of a row of O: beyond 64 columns half of the scores is fetched twice,
+// and the probabilities wait as f32 in the scores' registers and are cut after the wait
+// for the previous P*V (cut before it, 96 words do not fit beside the row; both looks
+// after it: 110 us for the 82.6 below; one half's exponentials after it: 87).
+// B2 H12 S1900 D128 causal: 65 us with one sum per row, 82.6 so; not causal 127, 158;
+// 64 heads of 1024 x 32, causal: 41, 52.5.
+//   Per 128 x 64 block at head size 128 the tensor pipe then
 // works 256 (Q*K^T) + 3 x 256 cycles, against 512 of the exponential unit.
 //
 // Structure, as in attention_tc.cu: persistent CTAs, one per SM, over units of 256
@@ -31,8 +45,8 @@
 //   computed by the CUDA-core recurrence (attention_row.cuh).
 //   The other warps may wait long meanwhile, so waits that run out start over as long as
 //   rows are being settled (Waits).
-// B2 H12 S1900 D128 causal: 8017 us on the CUDA cores, 65 us here (340 TFLOP/s of the
-// 22.2 GFLOP the function needs; longest unit 30 of an average 19.5 block pairs).
+// B2 H12 S1900 D128 causal: 8017 us on the CUDA cores, 82.6 us here (longest unit 30 of
+// an average 19.5 block pairs).
 // The rule in front (attention_split_supported) is what the copy engine can address:
 // rows of whole 16 bytes and 16-byte aligned bases; the rest, f32 inputs and head sizes
 // above 128 stay on the CUDA cores.  All waits are bounded.
@@ -47,8 +61,10 @@ constexpr int BQ = 128;          // query rows per tile
 constexpr int BKV = 64;          // keys per block
 constexpr int QT = 2;            // query tiles per unit
 constexpr int KV_STAGES = 4;
-constexpr int kRegsControl = 48, kRegsSoftmax = 224;   // as in attention_tc.cu: 128 * 48 + 256 * 224 <= 65536
 constexpr int kThreads = 32 * (4 + 4 * QT);
+// (56 and 224: 84.8 us for 82.6, in spite of fewer bytes spilled, 168 against 256 at two column groups, 20 against 84 at one)
+constexpr int kRegsControl = 40, kRegsSoftmax = 232;
+static_assert(128 * kRegsControl + QT * 128 * kRegsSoftmax <= kThreads * 168, "the warpgroups share what the block is launched with");
 constexpr float kRescaleThreshold = 8.0f;              // log2 units
 
 // NG: groups of 64 head columns (128 bytes) per row
@@ -103,6 +119,9 @@ __device__ __forceinline__ bool unit_at(const SplitParams &p, uint32_t i, Unit &
     }
     return true;
 }
+
+// Key blocks whose P*V starts a new sum in tensor memory; the sum before is added to the row's registers.
+__device__ __forceinline__ bool starts_group(uint32_t j) { return (j & (j < 4 ? 0u : j < 16 ? 1u : 3u)) == 0; }
 
 template <int N>
 __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -354,7 +373,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
                 __syncwarp();
                 if (pending) issue_pv();
-                pv_st = st; pv_ph = ph; pv_gt = gt; pv_acc = j != 0u;
+                pv_st = st; pv_ph = ph; pv_gt = gt; pv_acc = starts_group(j) ? 0u : 1u;
                 pending = true;
                 ++gt;
             }
@@ -375,6 +394,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const uint32_t tP = tmem_base + kColP + t * BKV + lane_addr;
         uint8_t *slice = smem + L::kOffP + t * L::kPTile + quad * 4096;   // this warp's 32 rows of the lo term
         const float c = p.scale_log2;
+        constexpr int kHalves = NG == 1 ? 2 : 1;   // halves of a block's scores that stay in registers after the first look
         bool ok = true;
         uint32_t gt = 0;
         Unit u;
@@ -385,51 +405,72 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             float m_ref = -INFINITY;   // exponent offset, in raw score units
             float l = 0.0f;
             bool bad = false;          // a non-finite score of an admitted key
+            uint64_t o2[NG * 32];      // the row's output so far, two columns a word
+#pragma unroll
+            for (int q = 0; q < NG * 32; ++q) o2[q] = 0ull;
+            auto add_group = [&]() {   // the group of blocks that tensor memory holds, once it is complete
+#pragma unroll
+                for (int h = 0; h < NG * 4; ++h) {
+                    uint32_t v[16];
+                    tmem_ld_32x32b_x16(tO + h * 16, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        o2[h * 8 + q] = add_f32x2(o2[h * 8 + q], pack_f32x2(__uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1])));
+                }
+            };
 
             for (uint32_t j = 0; j < mine; ++j, ++gt) {
                 if (!wait(&s_full[t], gt & 1)) { ok = false; break; }
                 tc_fence_after();
-                uint32_t s[2][32];
-                tmem_ld_32x32b_x32(tS, s[0]);
-                tmem_ld_32x32b_x32(tS + 32, s[1]);
-                tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_empty[t]);
-
                 const uint32_t key0 = j * BKV;
-                if (key0 + BKV > p.seq || (p.causal && key0 + BKV - 1 > first_row)) {
+                const bool edge = key0 + BKV > p.seq || (p.causal && key0 + BKV - 1 > first_row);
+                auto admitted = [&](uint32_t key) { return key < p.seq && (!p.causal || key <= qrow); };
+                // A first look at the scores, 32 keys at a time, for their maximum.  What fits beside the row's output stays in
+                // registers: both halves at head sizes up to 64, else the second.
+                uint32_t s[kHalves][32];
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+                auto release_scores = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&s_empty[t]);
+                };
+                auto mask = [&](uint32_t (&x)[32], uint32_t first_key) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                    for (int q = 0; q < 32; ++q)
+                        if (!admitted(first_key + q)) x[q] = 0xff800000u;  // -inf
+                };
 #pragma unroll
-                        for (int q = 0; q < 32; ++q) {
-                            const uint32_t key = key0 + h * 32 + q;
-                            if (key < p.seq && (!p.causal || key <= qrow))
-                                bad = bad || !isfinite(__uint_as_float(s[h][q]));
-                            else
-                                s[h][q] = 0xff800000u;  // -inf
-                        }
-                } else {
-                    // a score of -inf would pass unseen as p = 0; the other non-finite ones reach the sums
-                    float mn[2] = {INFINITY, INFINITY};
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t (&x)[32] = s[h % kHalves];
+                    if (kHalves == 1 || h == 0) {
+                        tmem_ld_32x32b_x32(tS + h * 32, x);
+                        if (kHalves == 2) tmem_ld_32x32b_x32(tS + 32, s[kHalves - 1]);
+                        tmem_ld_wait();
+                        if (kHalves == 2) release_scores();
+                    }
+                    if (edge) {
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                        for (int q = 0; q < 32; ++q)
+                            if (admitted(key0 + h * 32 + q)) bad = bad || !isfinite(__uint_as_float(x[q]));
+                        mask(x, key0 + h * 32);
+                    } else {
+                        // a score of -inf would pass unseen as p = 0; the other non-finite ones reach the sums
 #pragma unroll
                         for (int q = 0; q < 32; q += 2) {
                             float d;
-                            asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(mn[h]), "f"(__uint_as_float(s[h][q])), "f"(__uint_as_float(s[h][q + 1])));
-                            mn[h] = d;
+                            asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(mn[q / 2 % 4]), "f"(__uint_as_float(x[q])), "f"(__uint_as_float(x[q + 1])));
+                            mn[q / 2 % 4] = d;
                         }
-                    bad = bad || fminf(mn[0], mn[1]) == -INFINITY;
-                }
-                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
+                    }
 #pragma unroll
                     for (int q = 0; q < 32; q += 8)
 #pragma unroll
                         for (int w = 0; w < 4; ++w)
-                            mx[w] = max3(mx[w], __uint_as_float(s[h][q + 2 * w]), __uint_as_float(s[h][q + 2 * w + 1]));
+                            mx[w] = max3(mx[w], __uint_as_float(x[q + 2 * w]), __uint_as_float(x[q + 2 * w + 1]));
+                }
+                bad = bad || fminf(fminf(mn[0], mn[1]), fminf(mn[2], mn[3])) == -INFINITY;
                 const float rowmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
                 // move the reference only when the block maximum outgrows it by more than the threshold
                 const bool move = (rowmax - m_ref) * c > kRescaleThreshold;  // true for the first admitted key (m_ref = -inf)
@@ -438,23 +479,68 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 const float mc = (m_ref == -INFINITY ? 0.0f : m_ref) * c;
                 const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
                 uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
-                uint32_t hi[32], mid[32], lo[32];   // 64 probabilities, two per word
+                auto probability = [&](uint32_t s0, uint32_t s1, int q) {
+                    const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(s0), __uint_as_float(s1)), c2, nmc2);
+                    float x0, x1;
+                    unpack_f32x2(x2, x0, x1);
+                    const uint64_t e = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
+                    sum2[q & 3] = add_f32x2(sum2[q & 3], e);
+                    return e;
+                };
+                uint64_t e2[32];   // the probabilities, in the registers of their scores
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int q = 0; q < kHalves * 16; ++q) e2[32 - kHalves * 16 + q] = probability(s[q / 16][2 * (q % 16)], s[q / 16][2 * (q % 16) + 1], q);
+                if constexpr (kHalves == 1) {   // the scores of the first half are fetched again
+                    tmem_ld_32x32b_x32(tS, s[0]);
+                    tmem_ld_wait();
+                    release_scores();
+                    if (edge) mask(s[0], key0);
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(s[h][2 * q]), __uint_as_float(s[h][2 * q + 1])), c2, nmc2);
-                        float x0, x1;
-                        unpack_f32x2(x2, x0, x1);
-                        const uint64_t e2 = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
-                        sum2[q & 3] = add_f32x2(sum2[q & 3], e2);
+                    for (int q = 0; q < 16; ++q) e2[q] = probability(s[0][2 * q], s[0][2 * q + 1], q);
+                }
+                // P of the previous block must have been consumed and O must be quiescent
+                if (j > 0) {
+                    if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    const bool first = starts_group(j);
+                    if (first) add_group();
+                    if (__any_sync(0xffffffffu, move)) {
+                        const uint64_t f2 = pack_f32x2(factor, factor);
+#pragma unroll
+                        for (int q = 0; q < NG * 32; ++q) o2[q] = mul_f32x2(o2[q], f2);
+                        if (!first) {
+#pragma unroll 1
+                            for (uint32_t gcol = 0; gcol < p.dim; gcol += 8) {
+                                uint32_t ov[8];
+                                tmem_ld_32x32b_x8(tO + gcol, ov);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int q = 0; q < 8; ++q) ov[q] = __float_as_uint(__uint_as_float(ov[q]) * factor);
+                                tmem_st_32x32b_x8(tO + gcol, ov);
+                            }
+                        }
+                    }
+                }
+                auto store_p = [&](int h, const uint64_t *e) {   // 16 keys
+                    uint32_t hi[8], mid[8], lo[8];   // two probabilities a word
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
                         uint64_t rest;
-                        hi[h * 16 + q] = cut_bf16x2(e2, rest);
-                        mid[h * 16 + q] = cut_bf16x2(rest, rest);
+                        hi[q] = cut_bf16x2(e[q], rest);
+                        mid[q] = cut_bf16x2(rest, rest);
                         float r0, r1;
                         unpack_f32x2(rest, r0, r1);   // at most eight bits are left
-                        lo[h * 16 + q] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+                        lo[q] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
                     }
+                    tmem_st_32x32b_x8(tP + h * 8, hi);
+                    tmem_st_32x32b_x8(tP + 32 + h * 8, mid);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        *reinterpret_cast<uint4 *>(slice + lane * 128 + (((2 * h + k) ^ (lane & 7)) * 16)) =
+                            make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
+                };
+#pragma unroll
+                for (int h = 0; h < 4; ++h) store_p(h, e2 + h * 8);
                 float sum[4];
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
@@ -462,29 +548,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     unpack_f32x2(sum2[w], a, b);
                     sum[w] = a + b;
                 }
-                // P of the previous block must have been consumed and O must be quiescent
-                if (j > 0) {
-                    if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
-                    tc_fence_after();
-                    if (__any_sync(0xffffffffu, move)) {
-#pragma unroll 1
-                        for (uint32_t gcol = 0; gcol < p.dim; gcol += 8) {
-                            uint32_t ov[8];
-                            tmem_ld_32x32b_x8(tO + gcol, ov);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) ov[q] = __float_as_uint(__uint_as_float(ov[q]) * factor);
-                            tmem_st_32x32b_x8(tO + gcol, ov);
-                        }
-                    }
-                }
                 l = fmaf(l, factor, (sum[0] + sum[1]) + (sum[2] + sum[3]));
-                tmem_st_32x32b_x32(tP, hi);
-                tmem_st_32x32b_x32(tP + 32, mid);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
-                        make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
                 tmem_st_wait();
                 fence_proxy_async_smem();   // the lo term is read by the tensor core
                 tc_fence_before();
@@ -494,20 +558,17 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             if (!ok) break;
             if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
             tc_fence_after();
+            add_group();
             const float inv = 1.0f / l;
             bool good = !bad && isfinite(l) && l > 0.0f;
             const uint32_t row0 = first_row + quad * 32;   // first query row of this warp
-            uint32_t o[NG * 2][32];
+            const uint64_t inv2 = pack_f32x2(inv, inv);
 #pragma unroll
-            for (int h = 0; h < NG * 2; ++h) {
-                tmem_ld_32x32b_x32(tO + h * 32, o[h]);
-                tmem_ld_wait();
-#pragma unroll
-                for (int q = 0; q < 32; ++q) {
-                    const float v = __uint_as_float(o[h][q]) * inv;
-                    if (h * 32 + q < p.dim) good = good && isfinite(v);
-                    o[h][q] = __float_as_uint(v);
-                }
+            for (int q = 0; q < NG * 32; ++q) {
+                o2[q] = mul_f32x2(o2[q], inv2);
+                float v0, v1;
+                unpack_f32x2(o2[q], v0, v1);
+                if (2 * q < p.dim) good = good && isfinite(v0) && isfinite(v1);   // (the head size is even)
             }
             const uint32_t unsettled = __ballot_sync(0xffffffffu, !good && qrow < p.seq);
             if (unsettled == 0) {
@@ -522,7 +583,8 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
-                            make_uint4(o[h][4 * k], o[h][4 * k + 1], o[h][4 * k + 2], o[h][4 * k + 3]);
+                            make_uint4((uint32_t)o2[h * 16 + 2 * k], (uint32_t)(o2[h * 16 + 2 * k] >> 32), (uint32_t)o2[h * 16 + 2 * k + 1],
+                                       (uint32_t)(o2[h * 16 + 2 * k + 1] >> 32));
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0 && row0 < p.seq) {   // rows beyond seq and columns beyond the head size are clipped
@@ -534,10 +596,12 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             } else if (good && qrow < p.seq) {
                 float *dst = p.out + ((uint64_t)u.head * p.seq + qrow) * p.dim;
 #pragma unroll
-                for (int h = 0; h < NG * 2; ++h)
-#pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        if (h * 32 + q < p.dim) dst[h * 32 + q] = __uint_as_float(o[h][q]);
+                for (int q = 0; q < NG * 32; ++q)
+                    if (2 * q < p.dim) {
+                        float2 v;
+                        unpack_f32x2(o2[q], v.x, v.y);
+                        reinterpret_cast<float2 *>(dst)[q] = v;
+                    }
             }
             if (unsettled != 0) {
                 auto tick = [settled, lane](uint32_t) { if (lane == 0) atomicAdd(settled, 1u); };
