@@ -15,8 +15,8 @@
 // head size 128: 1.4e-5 against 1.5e-6 of the result, 2-norm, against f64).  So a sum
 // in tensor memory covers a group of one, two or four blocks (starts_group: short rows
 // have the least error to hide it behind) and the groups are added in registers, where
-// additions round to nearest: 7.7e-7 at 4096 keys, and not above the CUDA cores from 50
-// to 4096 keys.  The price is a read of O per group between one P*V and the next, and
+// additions round to nearest: 7.7e-7 at 4096 keys, and not above the CUDA cores from 333
+// to 4096 keys; at 50, one block, either may be the nearer by a fifth.  The price is a read of O per group between one P*V and the next, and
 // the registers of a row of O: beyond 64 columns half of the scores is fetched twice,
 // and the probabilities wait as f32 in the scores' registers and are cut after the wait
 // for the previous P*V (cut before it, 96 words do not fit beside the row; both looks
