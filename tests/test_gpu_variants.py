@@ -331,6 +331,46 @@ def test_attention_split_probabilities(gpu, orc, B, H, S, D, causal):
     assert np.abs(got - want).max() <= 2.5e-5 * np.abs(v32).max()
 
 
+def attention_f64(q, k, v, scale, causal):
+    scores = q.astype(np.float64) @ k.astype(np.float64).transpose(0, 2, 1) * np.float64(np.float32(scale))
+    if causal:
+        scores[:, np.triu(np.ones(scores.shape[1:], bool), 1)] = -np.inf
+    top = scores.max(-1, keepdims=True)
+    w = np.exp(scores - top)
+    return w @ v.astype(np.float64) / w.sum(-1, keepdims=True), np.abs(scores[np.isfinite(scores)]).max()
+
+
+@pytest.mark.parametrize("S,D,causal", [(333, 128, True), (1025, 72, False), (1900, 128, True), (1900, 48, False), (4096, 128, False)])
+def test_attention_split_error_is_not_above_the_cuda_cores(gpu, S, D, causal):
+    """The tensor core truncates its running sum at every accumulation; the kernel may not let that build up over a row.
+    The same values given as f32 take the CUDA-core kernel, which serves as the measure."""
+    from fe2o3_b200 import synth
+    from test_gpu_parity import attn_run
+    fe = gpu[0]
+    q, k, v = (synth.normal_bf16(3, d, 2 * S * D, 1.0).reshape(1, 2, S, D) for d in (1, 2, 3))
+    wide = [synth.bf16_to_f32(x) for x in (q, k, v)]
+    want, _ = attention_f64(*(x[0] for x in wide), 1.0 / np.sqrt(D), causal)
+    err = [np.linalg.norm(attn_run(gpu, *x, 1.0 / np.sqrt(D), causal, dtype)[0][0] - want)
+           for x, dtype in (((q, k, v), fe.DTYPE_BF16), (wide, fe.DTYPE_F32))]
+    assert err[0] <= err[1]
+
+
+@pytest.mark.parametrize("S,D,causal", [(1900, 48, False), (1900, 128, True), (2100, 72, False)])
+def test_attention_split_rising_scores(gpu, S, D, causal):
+    """Scores that grow along the keys: the reference exponent moves in the first block of a group and inside one."""
+    from fe2o3_b200 import synth
+    from test_gpu_parity import attn_run
+    fe = gpu[0]
+    q, k, v = (synth.normal_bf16(3, d, 2 * S * D, 1.0).reshape(1, 2, S, D) for d in (1, 2, 3))
+    ramp = synth.bf16_to_f32(k) * np.linspace(0.0, 20.0, S, dtype=np.float32)[:, None]
+    k = (ramp.view(np.uint32) >> 16).astype(np.uint16)
+    q32, k32, v32 = (synth.bf16_to_f32(x)[0] for x in (q, k, v))
+    want, top = attention_f64(q32, k32, v32, 1.0 / np.sqrt(D), causal)
+    got, _ = attn_run(gpu, q, k, v, 1.0 / np.sqrt(D), causal, fe.DTYPE_BF16)
+    # a score is wrong by up to D / 16 + 2 roundings of its size, a weight by as much relatively, and a result by twice that
+    assert np.abs(got[0] - want).max() <= 2 * top * (D / 16 + 2) * 2.0 ** -23 * np.abs(v32).max() + 2.5e-5
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_attention_split_leaves_bad_rows_unwritten(gpu, orc, causal):
     from fe2o3_b200 import synth
@@ -377,3 +417,58 @@ def test_attention_split_bad_value_spares_rows_that_do_not_admit_it(gpu, orc, S,
     lost[0, 1, key if causal else 0:] = True
     assert (got[lost] == -7).all()
     assert np.abs(got - want)[~lost].max() <= 2.5e-5 * 6   # as above: largest |v| below 6
+
+
+# ---- launches that start early: inside a graph behind copies and clears, and where two streams join
+def test_early_launches_in_a_captured_graph(gpu):
+    import torch
+    fe, ctx, _ = gpu
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    src = torch.rand(512 * 512, generator=gen, device="cuda")
+    x, y, z, c, total = (torch.zeros_like(src) for _ in range(5))
+    a, b = (torch.rand(256 * 256, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    g32 = torch.zeros(256 * 256, device="cuda")
+    soft = fe.prepare(ctx, "row_softmax_v1", input=x, output=y, rows=512, cols=512)
+    scan = fe.prepare(ctx, "device_scan_f32", values=y, output=z, exclusive=0)
+    exact = fe.prepare(ctx, "scalar_gemm_v1", a=y, b=y, c=c, m=512, n=512, k=512)
+    gemm = fe.prepare(ctx, "tiled_gemm_v1", a=a, b=b, c=g32, m=256, n=256, k=256)
+    last = fe.prepare(ctx, "device_scan_f32", values=total, output=x, exclusive=0)
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    s, o = ctx.wrap_stream(side.cuda_stream), ctx.wrap_stream(other.cuda_stream)
+
+    def work():
+        x.copy_(src)
+        soft.launch(s)
+        other.wait_stream(side)
+        with torch.cuda.stream(other):
+            exact.launch(o)
+            gemm.launch(o)
+            c.mul_(2.0)
+            gemm.launch(o)
+        scan.launch(s)
+        total.zero_()
+        side.wait_stream(other)
+        soft.launch(s)   # behind a clear and a kernel of the other stream
+        exact.launch(s)
+        torch.add(c, z, out=total)
+        last.launch(s)
+
+    with torch.cuda.stream(side):
+        work()
+        side.synchronize()
+        outs = (x, y, z, c, g32, total)
+        want = [t.clone() for t in outs]
+        side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        work()
+    for _ in range(3):
+        for t in outs:
+            t.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert ctx.take_kernel_status(s) == 0
+        for t, w in zip(outs, want):
+            assert (t.view(torch.int32) == w.view(torch.int32)).all()
