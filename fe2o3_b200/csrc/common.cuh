@@ -266,6 +266,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, c
     }
     return __all_sync(0xffffffffu, done) != 0;
 }
+// How many of the next `limit` stages of a ring of S, from `stage` on, have completed the phase awaited: one look of the
+// whole warp, a lane to a stage.  A role that waits, issues and steps on stage by stage is held up by the latency of each
+// look, vote and election (some 200 to 400 cycles a stage together); one look lets it issue for all stages that are ready.
+template <int S>
+__device__ __forceinline__ uint32_t ready_stages(uint64_t *bars, uint32_t stage, uint32_t parity, uint32_t limit, uint32_t lane) {
+    static_assert(S < 32, "one lane a stage");
+    uint32_t at = stage + lane;
+    if (at >= S) { at -= S; parity ^= 1; }
+    const bool ready = lane < min(limit, (uint32_t)S) && mbar_test(&bars[at], parity);
+    return __ffs(~__ballot_sync(0xffffffffu, ready)) - 1;
+}
 // Arrival with a count: stands in for `n` parties at once.
 __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");

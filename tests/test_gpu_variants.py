@@ -87,6 +87,23 @@ def test_gemm_tile_shapes_exact(gpu, orc, m, n, k, ldc, beta):
         assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
 
 
+# ring lengths: fewer k blocks than stages, as many, and a ring that ends inside a tile, two rounds of tiles
+@pytest.mark.parametrize("k", [8, 64, 448, 520, 576, 1088])
+@pytest.mark.parametrize("m,n", [(100, 100), (2600, 2600), (1300, 5000)])
+def test_gemm_ring_lengths_exact(gpu, m, n, k):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    a, b = synth.gemm_inputs_v1(m * k, 1, 1, 5)[0], synth.gemm_inputs_v1(1, k * ((n + 7) // 8 * 8), 1, 6)[1]
+    ldb = (n + 7) // 8 * 8
+    A, B = Guarded(fe, stream, a), Guarded(fe, stream, b[:(k - 1) * ldb + n])
+    Cb = Guarded(fe, stream, np.zeros(m * n, np.float32))
+    run(fe, ctx, stream, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_TCGEN05, a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k,
+        lda=k, ldb=ldb, ldc=n, alpha=1.0, beta=0.0)
+    wide = lambda v: (v.astype(np.uint32) << 16).view(np.float32)
+    want = wide(a).reshape(m, k) @ wide(b).reshape(k, ldb)[:, :n]   # dyadic alphabet: every summation order is exact
+    assert (Cb.read().reshape(m, n) == want).all()
+
+
 @pytest.mark.parametrize("T,d,f,E,cap", [(1000, 1088, 1152, 4, 2000), (1040, 1152, 1088, 4, 500),
                                          # few rows a group: copies of 32 and 64 rows, groups without rows
                                          (1, 128, 256, 8, 2), (40, 128, 256, 4, 3), (90, 192, 320, 4, 180),
