@@ -115,6 +115,30 @@ def test_moe_tile_shapes(gpu, orc, T, d, f, E, cap):
     assert_close(compact[: accepted * d], want_compact[: accepted * d], 2e-2, 2e-3, "compact expert output")
 
 
+@pytest.mark.parametrize("d,f,rows", [(64, 64, 128), (64, 64, 77), (128, 200, 300), (64, 384, 33)])
+def test_expert_ffn_gelu_values(gpu, d, f, rows):
+    """Hidden activations of chosen arguments (W1 copies column c of the row to columns c, c + d, ...): half a bf16 step, and
+    1e-6 for the tail's polynomial (8.3e-8), its evaluation and the exponential (a few f32 roundings of at most 1.2)."""
+    import math
+    fe, ctx, stream = gpu
+    B = lambda a: fe.DeviceBuffer.from_host(stream, a)
+    rng = np.random.default_rng(7)
+    x = np.concatenate([rng.normal(0, 2, rows * d - 12), [0.0, -0.0, 10, -10, 10.5, -10.5, 64, -64, 3e38, -3e38, 1e-39, -5.5]]).astype(np.float32)
+    xb = (x.view(np.uint32) >> 16).astype(np.uint16)
+    x = (xb.astype(np.uint32) << 16).view(np.float32).astype(np.float64).reshape(rows, d)
+    w1 = np.zeros((d, f), np.uint16)
+    w1[np.arange(f) % d, np.arange(f)] = 0x3f80
+    HID = Guarded(fe, stream, np.zeros(rows * f, np.uint16))
+    run(fe, ctx, stream, "moe_expert_ffn_v1", x=B(xb), w1=B(w1.ravel()), w2=B(np.zeros(f * d, np.uint16)),
+        permutation=B(np.arange(0, 2 * rows, 2, dtype=np.uint32)), expert_offsets=B(np.array([0, rows], np.uint32)),
+        compact_x=B(np.zeros(rows * d, np.uint16)), hidden=HID.slice, compact_output=B(np.zeros(rows * d, np.float32)),
+        tokens=rows, d_model=d, d_ff=f, experts=1)
+    got = (HID.read().astype(np.uint32) << 16).view(np.float32).astype(np.float64).reshape(rows, f)
+    arg = x[:, np.arange(f) % d]
+    want = 0.5 * arg * np.vectorize(math.erfc)(-arg / math.sqrt(2))
+    assert (np.abs(got - want) <= np.abs(want) * 2.0 ** -8 + 1e-6).all()
+
+
 def test_expert_ffn_without_tokens(gpu):
     """No token to gather, and a table that claims rows all the same: rows of zeros, and no launch for an empty output."""
     fe, ctx, stream = gpu
