@@ -15,27 +15,32 @@
 // head size 128: 1.4e-5 against 1.5e-6 of the result, 2-norm, against f64).  So a sum
 // in tensor memory covers a group of one, two or four blocks (starts_group: short rows
 // have the least error to hide it behind) and the groups are added in registers, where
-// additions round to nearest: 7.7e-7 at 4096 keys, and not above the CUDA cores from 333
-// to 4096 keys; at 50, one block, either may be the nearer by a fifth.  The price is a read of O per group between one P*V and the next, and
-// the registers of a row of O: beyond 64 columns half of the scores is fetched twice,
-// and the probabilities wait as f32 in the scores' registers and are cut after the wait
-// for the previous P*V (cut before it, 96 words do not fit beside the row; both looks
-// after it: 110 us for the 82.6 below; one half's exponentials after it: 87).
-// B2 H12 S1900 D128 causal: 65 us with one sum per row, 82.6 so; not causal 127, 158;
-// 64 heads of 1024 x 32, causal: 41, 52.5.
-//   Per 128 x 64 block at head size 128 the tensor pipe then
-// works 256 (Q*K^T) + 3 x 256 cycles, against 512 of the exponential unit.
+// additions round to nearest: 7.5e-7 at 4096 keys, and not above the CUDA cores from 333
+// to 4096 keys; at 50, one block, either may be the nearer by a fifth.  The price is a read of O per group between one
+// P*V and the next, and the registers of a row of O: beyond 64 columns half of the scores is fetched twice, and the
+// probabilities wait as f32 in the scores' registers and are cut after the wait for the previous P*V (before it, 96
+// words do not fit beside the row).
 //
-// Structure, as in attention_tc.cu: persistent CTAs, one per SM, over units of 256
-// query rows handled as two 128-row tiles that share every K/V block; warp 0 loads
-// (TMA), warps 1 and 2 issue the MMAs of tile 0 and tile 1, warps 4-7 and 8-11 are
-// the softmax warps of the tiles, one thread per row, with most of the registers.
-//   64-key blocks and P's lo term in shared memory instead of tensor memory are what
-//   fits two tiles at head size 128: S 2 x 64, O 2 x 128 and hi, mid 2 x 2 x 32 make
-//   the 512 columns.  So S has columns of its own and the next Q*K^T overlaps the
-//   exponentials.  The lo buffer doubles as the staging buffer of the output.
+// Structure: persistent CTAs, one per SM, over units of 128 query rows.  The key blocks of a unit go to two streams in
+// turn, each with S, P, O, reference and sum of its own, so that one stream's exponentials overlap the other's products;
+// the streams meet in shared memory at the end of the unit, where each finishes half of the columns.  Two 128-row tiles
+// that shared their key blocks (until then) made units twice as long for the same work a block: B2 H12 S1900 D128 causal
+// came to 30 steps on the longest SM of 23 on average, 20 of 19.5 so, and a call with few rows leaves no stream idle.
+//   Warp 0 loads (TMA), warp 1 issues Q*K^T of both streams, warps 2 and 3 P*V of a stream each, warps 4-7 and
+// 8-11 are the softmax warps of the streams, one thread per row, with most of the registers.  With one issuer a
+// tile, Q*K^T of a block waited behind P*V of the block before and that for its softmax: 3500 of a block's 3800 cycles
+// were the issuer's.  Its loops are rolled and its waits short because code is what they cost: eight warps run through
+// some 900 instructions a block, and what runs once in between is fetched anew each time (some 6 cycles an instruction).
+//   What bounds it: of some 3700 cycles for a block of each stream the softmax warps, two a scheduler, work 2800 (a look for
+// the maximum, 64 exponentials, the cut: 18 cycles of the ALU, 16 of the exponential unit and 8 of the f32 pipe a pair of keys
+// and warp), the tensor pipe 2300.  Tried: four warps a tile of 16 rows each (20 instructions a score for 14: no faster), the
+// cut in a rolled loop that fetches scores as it goes (5400), exponentials of half a block ahead of its maximum (4400).
+//   A reference is a whole number of log2 units, so rescaling and the meeting of the streams are exact.
+//   64-key blocks and P's lo term in shared memory instead of tensor memory are what fits two streams at head size 128:
+//   S 2 x 64, O 2 x 128 and hi, mid 2 x 2 x 32 make the 512 columns.  So S has columns of its own and the next Q*K^T overlaps
+//   the exponentials.
 //   Causal units are ordered by length, longest first, and dealt out in alternating
-//   direction (round 0 forwards, round 1 backwards); a tile stops at its own last block.
+//   direction (round 0 forwards, round 1 backwards).
 //   Head sizes below 64 or between 64 and 128 are zero-filled by the copy engine on the
 //   way in and clipped on the way out; Q*K^T takes only the k steps in use.
 //   A row that met a non-finite score or value is settled one by one: the tensor core
@@ -45,8 +50,8 @@
 //   computed by the CUDA-core recurrence (attention_row.cuh).
 //   The other warps may wait long meanwhile, so waits that run out start over as long as
 //   rows are being settled (Waits).
-// B2 H12 S1900 D128 causal: 8017 us on the CUDA cores, 82.6 us here (longest unit 30 of
-// an average 19.5 block pairs).
+// Two tiles a unit / so, us: B2 H12 S1900 D128 causal 80.5 / 56.7, not causal 156 / 98; B1 H1 S4096 113 / 66; B8 H8 S256 16.3 / 11.8;
+// B4 H16 S2048 D32 262 / 228.  On the CUDA cores the first takes 8017.
 // The rule in front (attention_split_supported) is what the copy engine can address:
 // rows of whole 16 bytes and 16-byte aligned bases; the rest, f32 inputs and head sizes
 // above 128 stay on the CUDA cores.  All waits are bounded.
@@ -57,14 +62,13 @@
 
 namespace {
 
-constexpr int BQ = 128;          // query rows per tile
+constexpr int BQ = 128;          // query rows per unit
 constexpr int BKV = 64;          // keys per block
-constexpr int QT = 2;            // query tiles per unit
-constexpr int KV_STAGES = 4;
-constexpr int kThreads = 32 * (4 + 4 * QT);
-// (56 and 224: 84.8 us for 82.6, in spite of fewer bytes spilled, 168 against 256 at two column groups, 20 against 84 at one)
+constexpr int STREAMS = 2;       // key blocks of a unit go to them in turn
+constexpr int KV_STAGES = 3;
+constexpr int kThreads = 32 * (4 + 4 * STREAMS);
 constexpr int kRegsControl = 40, kRegsSoftmax = 232;
-static_assert(128 * kRegsControl + QT * 128 * kRegsSoftmax <= kThreads * 168, "the warpgroups share what the block is launched with");
+static_assert(128 * kRegsControl + STREAMS * 128 * kRegsSoftmax <= kThreads * 168, "the warpgroups share what the block is launched with");
 constexpr float kRescaleThreshold = 8.0f;              // log2 units
 
 // NG: groups of 64 head columns (128 bytes) per row
@@ -73,14 +77,17 @@ struct Layout {
     static constexpr uint32_t kQTile = NG * BQ * 128;      // [group][128 rows][128 bytes]
     static constexpr uint32_t kKvTile = NG * BKV * 128;    // [group][64 keys][128 bytes]
     static constexpr uint32_t kPTile = BQ * 128;           // lo term: [128 rows][64 keys]
-    static constexpr uint32_t kOffK = QT * kQTile;
+    static constexpr uint32_t kOffK = kQTile;
     static constexpr uint32_t kOffV = kOffK + KV_STAGES * kKvTile;
     static constexpr uint32_t kOffP = kOffV + KV_STAGES * kKvTile;
-    static constexpr uint32_t kOffBar = kOffP + QT * kPTile;
-    static constexpr uint32_t kTotal = kOffBar + 512 + 1024;   // + alignment slack
+    static constexpr uint32_t kOffMerge = kOffP + STREAMS * kPTile;        // a unit's output: [stream][32 rows][32 columns][32 rows][128 bytes]
+    static constexpr uint32_t kOffRow = kOffMerge + NG * 64 * BQ * 4;      // reference and sum of each row, a stream
+    static constexpr uint32_t kOffBar = kOffRow + STREAMS * 2 * BQ * 4;
+    static constexpr uint32_t kTotal = kOffBar + 256;
+    static_assert(kTotal <= 227 * 1024, "shared memory of a block");
 };
 
-// TMEM columns: S tile t at t*64, O tile t at 128 + t*128, P tile t at 384 + t*64 (hi 32, mid 32)
+// TMEM columns: S of stream t at t*64, O at 128 + t*128, P at 384 + t*64 (hi 32, mid 32)
 constexpr uint32_t kTmemCols = 512, kColO = 128, kColP = 384;
 
 struct SplitParams {
@@ -89,39 +96,29 @@ struct SplitParams {
     uint32_t bh, seq, dim;
     float scale, scale_log2;   // scale_log2 = scale * log2(e)
     uint32_t causal;
-    uint32_t q_blocks;  // 256-row blocks per head
-    uint32_t units;     // work units; `half`: of one tile each, two per block
-    uint32_t half;
+    uint32_t q_blocks;  // 128-row blocks per head
+    uint32_t units;     // work units: heads * q_blocks
+    float whole;        // 1: references are whole numbers; 0: the maxima themselves (rows of one block, never rescaled)
     uint32_t *status;
 };
 
 struct Unit {
-    uint32_t head, q0, nkv;
-    uint32_t n[QT];     // key blocks of each tile, 0 = no such tile here; nkv = the larger
+    uint32_t head, q0, n;   // n: key blocks
 };
 
 // The i-th unit of this CTA; false when there is none.  Every role walks the same sequence.
 __device__ __forceinline__ bool unit_at(const SplitParams &p, uint32_t i, Unit &u) {
     const uint32_t idx = i * gridDim.x + ((i & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     if (idx >= p.units) return false;
-    const uint32_t block = p.half ? idx >> 1 : idx;
-    const uint32_t qb = p.causal ? p.q_blocks - 1 - block / p.bh : block % p.q_blocks;
-    u.head = p.causal ? block % p.bh : block / p.q_blocks;
-    u.q0 = qb * (QT * BQ) + (p.half ? (idx & 1) * BQ : 0);
-    u.nkv = 0;
-#pragma unroll
-    for (uint32_t t = 0; t < QT; ++t) {
-        const uint32_t first = u.q0 + t * BQ;
-        u.n[t] = 0;
-        if (first < p.seq && !(p.half && t > 0))
-            u.n[t] = ((p.causal ? min(p.seq, first + BQ) : p.seq) + BKV - 1) / BKV;
-        u.nkv = max(u.nkv, u.n[t]);
-    }
+    const uint32_t qb = p.causal ? p.q_blocks - 1 - idx / p.bh : idx % p.q_blocks;
+    u.head = p.causal ? idx % p.bh : idx / p.q_blocks;
+    u.q0 = qb * BQ;
+    u.n = ((p.causal ? min(p.seq, u.q0 + BQ) : p.seq) + BKV - 1) / BKV;
     return true;
 }
 
 // Key blocks whose P*V starts a new sum in tensor memory; the sum before is added to the row's registers.
-__device__ __forceinline__ bool starts_group(uint32_t j) { return (j & (j < 4 ? 0u : j < 16 ? 1u : 3u)) == 0; }
+__device__ __forceinline__ bool starts_group(uint32_t j) { return (j & (j < 2 ? 0u : j < 8 ? 1u : 3u)) == 0; }
 
 template <int N>
 __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -143,15 +140,18 @@ __device__ __forceinline__ uint32_t cut_bf16x2(uint64_t v, uint64_t &rest) {
     return __byte_perm(l, h, 0x7632);
 }
 
-// Waits on another role of the block.  `settled` moves on as long as rows are being settled one by one.
+// Waits on another role of the block.  `settled` moves on as long as rows are being settled one by one.  Few instructions:
+// the roles' loops share the instruction caches with the softmax warps' long ones.
 struct Waits {
     const volatile uint32_t *settled;
     __device__ __forceinline__ bool operator()(uint64_t *bar, uint32_t parity) const {
-        uint32_t seen = 0;
-        while (!mbar_wait_warp(bar, parity)) {
+        uint32_t polls = 0, seen = 0;
+        while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+            if (++polls < FE2O3_SPIN_LIMIT) continue;
             const uint32_t now = __shfl_sync(0xffffffffu, *settled, 0);
             if (now == seen) return false;
             seen = now;
+            polls = 0;
         }
         return true;
     }
@@ -195,8 +195,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, SplitParams p) {
     using L = Layout<NG>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];   // (swizzle atoms are 1 KiB; there is no room to round up)
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::kOffBar);
     uint64_t *q_full = bars;
     uint64_t *q_empty = q_full + 1;
@@ -204,29 +203,33 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     uint64_t *k_empty = k_full + KV_STAGES;
     uint64_t *v_full = k_empty + KV_STAGES;
     uint64_t *v_empty = v_full + KV_STAGES;
-    uint64_t *s_full = v_empty + KV_STAGES;        // QT each
-    uint64_t *s_empty = s_full + QT;
-    uint64_t *p_ready = s_empty + QT;
-    uint64_t *pv_done = p_ready + QT;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pv_done + QT);
+    uint64_t *s_full = v_empty + KV_STAGES;        // STREAMS each
+    uint64_t *s_empty = s_full + STREAMS;
+    uint64_t *p_ready = s_empty + STREAMS;
+    uint64_t *pv_done = p_ready + STREAMS;
+    uint64_t *merge_full = pv_done + STREAMS;
+    uint64_t *merge_empty = merge_full + STREAMS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(merge_empty + STREAMS);
     uint32_t *settled = tmem_slot + 1;
     const Waits wait{settled};
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        mbar_init(q_empty, QT);
+        mbar_init(q_empty, 1);
         for (int i = 0; i < KV_STAGES; ++i) {
             mbar_init(&k_full[i], 1);
-            mbar_init(&k_empty[i], QT);
+            mbar_init(&k_empty[i], 1);
             mbar_init(&v_full[i], 1);
-            mbar_init(&v_empty[i], QT);
+            mbar_init(&v_empty[i], 1);
         }
-        for (int t = 0; t < QT; ++t) {
+        for (int t = 0; t < STREAMS; ++t) {
             mbar_init(&s_full[t], 1);
             mbar_init(&s_empty[t], 4);
             mbar_init(&p_ready[t], 4);
             mbar_init(&pv_done[t], 1);
+            mbar_init(&merge_full[t], 4);
+            mbar_init(&merge_empty[t], 4);
         }
         *settled = 0;
         mbar_fence_init();
@@ -256,20 +259,15 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         uint32_t n_units = 0;
         Unit u;
         for (uint32_t i = 0; ok && unit_at(p, i, u); ++i) {
-            if (u.nkv == 0) continue;   // every role skips a unit whose rows all lie beyond seq
             if (!wait(q_empty, (n_units & 1) ^ 1)) { ok = false; break; }
             ++n_units;
             if (elect_one()) {
-                mbar_arrive_expect_tx(q_full, ((u.n[0] ? 1u : 0u) + (u.n[1] ? 1u : 0u)) * L::kQTile);
-                for (uint32_t t = 0; t < QT; ++t) {
-                    if (u.n[t] == 0) continue;
+                mbar_arrive_expect_tx(q_full, L::kQTile);
 #pragma unroll
-                    for (int h = 0; h < NG; ++h)
-                        tma_load_3d(smem + t * L::kQTile + h * BQ * 128, &tmQ, q_full, h * 64, (int32_t)(u.q0 + t * BQ), (int32_t)u.head);
-                }
+                for (int h = 0; h < NG; ++h) tma_load_3d(smem + h * BQ * 128, &tmQ, q_full, h * 64, (int32_t)u.q0, (int32_t)u.head);
             }
             __syncwarp();
-            for (uint32_t j = 0; j < u.nkv; ++j, ++g) {
+            for (uint32_t j = 0; j < u.n; ++j, ++g) {
                 const uint32_t st = g % KV_STAGES, ph = (g / KV_STAGES) & 1;
                 if (!wait(&k_empty[st], ph ^ 1)) { ok = false; break; }
                 if (elect_one()) {
@@ -303,91 +301,80 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             mbar_wait_warp(&v_full[st], ph);
         }
         if (n_units) mbar_wait_warp(q_full, (n_units - 1) & 1);
-    } else if (warp == 1 || warp == 2) {
-        // ---------------------------------------------------------- MMA issuers, one warp per query tile
-        // Per tile: Q*K^T of block b+1 (its S columns are free once the softmax has read block b), then P*V of
-        // block b; block b+1 may already belong to the next unit.
-        const uint32_t t = warp - 1;
-        const uint32_t k_steps = (p.dim + 15) / 16;
+    } else if (warp == 1) {
+        // ---------------------------------------------------------- Q*K^T of both streams, in the order of the key blocks
         constexpr uint32_t idesc_qk = umma_idesc(1u, BQ, BKV, 0u, 0u);
-        constexpr uint32_t idesc_pv = umma_idesc(1u, BQ, NG * 64, 0u, 1u);   // whole column groups: zeros past the head size
-        const uint64_t dQ = umma_smem_desc(smem_u32(smem) + t * L::kQTile, 16, 1024),
-                       dK = umma_smem_desc(smem_u32(smem) + L::kOffK, 16, 1024),
-                       dV = umma_smem_desc(smem_u32(smem) + L::kOffV, BKV * 128, 1024),
-                       dP = umma_smem_desc(smem_u32(smem) + L::kOffP + t * L::kPTile, 16, 1024);
-        const uint32_t tS = tmem_base + t * BKV, tO = tmem_base + kColO + t * 128, tP = tmem_base + kColP + t * BKV;
+        const uint32_t k_steps = (p.dim + 15) / 16;
+        const uint64_t dQ = umma_smem_desc(smem_u32(smem), 16, 1024), dK = umma_smem_desc(smem_u32(smem) + L::kOffK, 16, 1024);
         bool ok = true;
-        uint32_t g = 0;    // key blocks over all units: ring position of K/V
-        uint32_t gt = 0;   // key blocks this tile has processed: parity of s_* / p_ready / pv_done
-        uint32_t n = 0;    // units with keys seen so far
-        bool pending = false;
-        uint32_t pv_st = 0, pv_ph = 0, pv_gt = 0, pv_acc = 0;
-        auto issue_pv = [&]() {
-            pending = false;
-            if (!wait(&p_ready[t], pv_gt & 1) || !wait(&v_full[pv_st], pv_ph)) { ok = false; return; }
-            tc_fence_after();
-            if (elect_one()) {
-                const uint64_t dVs = dV + ((pv_st * L::kKvTile) >> 4);
-#pragma unroll
-                for (int kk = 0; kk < BKV / 16; ++kk)   // lo term: P from shared memory
-                    umma_f16(tO, dP + ((kk * 32) >> 4), dVs + ((kk * 2048) >> 4), idesc_pv, kk == 0 ? pv_acc : 1u);
-#pragma unroll
-                for (int term = 1; term >= 0; --term)   // mid, then hi: P from tensor memory
-#pragma unroll
-                    for (int kk = 0; kk < BKV / 16; ++kk)
-                        umma_f16_ts(tO, tP + term * (BKV / 2) + kk * 8, dVs + ((kk * 2048) >> 4), idesc_pv, 1u);
-                umma_commit(&pv_done[t]);
-                umma_commit(&v_empty[pv_st]);
-            }
-            __syncwarp();
-        };
+        uint32_t st = 0, ph = 0;          // ring position
+        uint32_t given = 0;               // blocks: even bits of a count a stream (parity of s_full / s_empty)
+        uint32_t n = 0;                   // units seen so far
         Unit u;
-        for (uint32_t i = 0; ok && unit_at(p, i, u); ++i) {
-            if (u.nkv == 0) continue;
-            const uint32_t qph = n & 1, mine = t == 0 ? u.n[0] : u.n[1];
-            ++n;
-            if (!wait(q_full, qph)) { ok = false; break; }
-            if (mine == 0 && lane == 0) mbar_arrive(q_empty);   // no such tile here: nothing of Q is read
-            for (uint32_t j = 0; ok && j < u.nkv; ++j, ++g) {
-                const uint32_t st = g % KV_STAGES, ph = (g / KV_STAGES) & 1;
-                if (j >= mine) {   // past this tile's last block: only hand the other tile's K/V blocks on
-                    if (pending) issue_pv();
-                    if (!ok || !wait(&k_full[st], ph)) { ok = false; break; }
-                    if (lane == 0) mbar_arrive(&k_empty[st]);
-                    if (!wait(&v_full[st], ph)) { ok = false; break; }
-                    if (lane == 0) mbar_arrive(&v_empty[st]);
-                    continue;
-                }
-                if (!wait(&s_empty[t], (gt & 1) ^ 1) || !wait(&k_full[st], ph)) { ok = false; break; }
+        for (uint32_t i = 0; ok && unit_at(p, i, u); ++i, ++n) {
+            if (!wait(q_full, n & 1)) { ok = false; break; }
+            for (uint32_t j = 0; j < u.n; ++j) {
+                const uint32_t t = j % STREAMS;
+                if (!wait(&k_full[st], ph) || !wait(&s_empty[t], (given >> t & 1) ^ 1)) { ok = false; break; }
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint64_t dKs = dK + ((st * L::kKvTile) >> 4);
-#pragma unroll
-                    for (uint32_t kk = 0; kk < NG * 4; ++kk)
-                        if (kk < k_steps)
-                            umma_f16(tS, dQ + (((kk >> 2) * BQ * 128 + (kk & 3) * 32) >> 4),
-                                     dKs + (((kk >> 2) * BKV * 128 + (kk & 3) * 32) >> 4), idesc_qk, kk != 0);
+                    uint64_t q = dQ, k = dK + ((st * L::kKvTile) >> 4);
+#pragma unroll 1
+                    for (uint32_t kk = 0; kk < k_steps; ++kk) {
+                        umma_f16(tmem_base + t * BKV, q, k, idesc_qk, kk != 0);
+                        q += kk == 3 ? (BQ * 128 - 96) >> 4 : 2;   // 16 columns on; the second 64 columns are a group of their own
+                        k += kk == 3 ? (BKV * 128 - 96) >> 4 : 2;
+                    }
                     umma_commit(&s_full[t]);
                     umma_commit(&k_empty[st]);
-                    if (j + 1 == mine) umma_commit(q_empty);
+                    if (j + 1 == u.n) umma_commit(q_empty);
                 }
                 __syncwarp();
-                if (pending) issue_pv();
-                pv_st = st; pv_ph = ph; pv_gt = gt; pv_acc = starts_group(j) ? 0u : 1u;
-                pending = true;
-                ++gt;
+                given ^= 1u << t;
+                if (++st == KV_STAGES) { st = 0; ph ^= 1; }
             }
         }
-        if (ok && pending) issue_pv();
+        if (!ok && lane == 0) kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
+    } else if (warp < 4) {
+        // ---------------------------------------------------------- P*V, one warp per stream
+        constexpr uint32_t idesc_pv = umma_idesc(1u, BQ, NG * 64, 0u, 1u);   // whole column groups: zeros past the head size
+        const uint32_t t = warp - 2;
+        const uint64_t dV = umma_smem_desc(smem_u32(smem) + L::kOffV, BKV * 128, 1024),
+                       dP = umma_smem_desc(smem_u32(smem) + L::kOffP + t * L::kPTile, 16, 1024);
+        const uint32_t tO = tmem_base + kColO + t * 128, tP = tmem_base + kColP + t * BKV;
+        bool ok = true;
+        uint32_t g0 = 0;   // key blocks of the units before: ring position of V
+        uint32_t gt = 0;   // blocks of this stream: parity of p_ready / pv_done
+        Unit u;
+        for (uint32_t i = 0; ok && unit_at(p, i, u); ++i) {
+            for (uint32_t j = t; j < u.n; j += STREAMS, ++gt) {
+                const uint32_t g = g0 + j, st = g % KV_STAGES;
+                if (!wait(&v_full[st], (g / KV_STAGES) & 1) || !wait(&p_ready[t], gt & 1)) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t v = dV + ((st * L::kKvTile) >> 4);
+                    const uint32_t first = starts_group(j / STREAMS) ? 0u : 1u;
+#pragma unroll 1
+                    for (uint32_t kk = 0; kk < BKV / 16; ++kk)   // lo term: P from shared memory
+                        umma_f16(tO, dP + kk * 2, v + kk * 128, idesc_pv, kk == 0 ? first : 1u);
+#pragma unroll 1
+                    for (uint32_t kk = 0; kk < BKV / 8; ++kk)    // mid, then hi: P from tensor memory
+                        umma_f16_ts(tO, tP + ((kk ^ 4u) * 8), v + (kk & 3) * 128, idesc_pv, 1u);
+                    umma_commit(&pv_done[t]);
+                    umma_commit(&v_empty[st]);
+                }
+                __syncwarp();
+            }
+            g0 += u.n;
+        }
         if (!ok && lane == 0) kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
     }
-    // warp 3 idles: it keeps the softmax warps at four per scheduler and their TMEM quadrant equal to warp % 4
     } else {
         regs_take<kRegsSoftmax>();
-        // ---------------------------------------------------------- softmax warps, one thread per query row
+        // ---------------------------------------------------------- softmax warps, one thread per query row and stream
         const uint32_t t = (warp - 4) / 4;
         const uint32_t quad = warp & 3;
-        const uint32_t r = quad * 32 + lane;                // row inside the tile
+        const uint32_t r = quad * 32 + lane;                // row inside the unit
         const uint32_t lane_addr = (quad * 32u) << 16;
         const uint32_t tS = tmem_base + t * BKV + lane_addr;
         const uint32_t tO = tmem_base + kColO + t * 128 + lane_addr;
@@ -397,22 +384,35 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         constexpr int kHalves = NG == 1 ? 2 : 1;   // halves of a block's scores that stay in registers after the first look
         bool ok = true;
         uint32_t gt = 0;
+        uint32_t n = 0;        // units so far
+        // Each stream finishes half of the columns: this warp's 32 rows of them, a 4 KiB piece of 32 columns after the
+        // other, swizzled as the copy engine stores them.  The other stream writes its part there.
+        constexpr uint32_t kHalfCols = NG * 32;
+        uint8_t *const rows_out = smem + L::kOffMerge + (t * 4 + quad) * (NG * 4096);
+        uint8_t *const rows_given = smem + L::kOffMerge + ((t ^ 1) * 4 + quad) * (NG * 4096);
+        auto piece = [&](uint8_t *rows, int q) { return reinterpret_cast<float4 *>(rows + (q >> 3) * 4096 + lane * 128 + (((q & 7) ^ (lane & 7)) * 16)); };
+        const uint32_t tMine = tO + t * kHalfCols, tGiven = tO + (t ^ 1) * kHalfCols;
+        bool storing = false;  // the copy engine may still be reading rows_out
+        auto release_rows = [&]() {
+            if (lane == 0) tma_store_wait_read();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&merge_empty[t]);
+            storing = false;
+        };
         Unit u;
         for (uint32_t i = 0; ok && unit_at(p, i, u); ++i) {
-            const uint32_t mine = t == 0 ? u.n[0] : u.n[1];
-            if (mine == 0) continue;
-            const uint32_t first_row = u.q0 + t * BQ, qrow = first_row + r;
-            float m_ref = -INFINITY;   // exponent offset, in raw score units
+            const uint32_t qrow = u.q0 + r;
+            float m_ref = -INFINITY;   // exponent offset: a whole number of log2 units, so that every rescaling is exact
             float l = 0.0f;
             bool bad = false;          // a non-finite score of an admitted key
-            uint64_t o2[NG * 32];      // the row's output so far, two columns a word
+            uint64_t o2[NG * 32];      // the row's output so far, two columns a word; the columns that this stream finishes come first
 #pragma unroll
             for (int q = 0; q < NG * 32; ++q) o2[q] = 0ull;
             auto add_group = [&]() {   // the group of blocks that tensor memory holds, once it is complete
 #pragma unroll
                 for (int h = 0; h < NG * 4; ++h) {
                     uint32_t v[16];
-                    tmem_ld_32x32b_x16(tO + h * 16, v);
+                    tmem_ld_32x32b_x16((h < NG * 2 ? tMine : tGiven) + h % (NG * 2) * 16, v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
@@ -420,89 +420,93 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
             };
 
-            for (uint32_t j = 0; j < mine; ++j, ++gt) {
+            for (uint32_t j = t; j < u.n; j += STREAMS, ++gt) {
                 if (!wait(&s_full[t], gt & 1)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t key0 = j * BKV;
-                const bool edge = key0 + BKV > p.seq || (p.causal && key0 + BKV - 1 > first_row);
-                auto admitted = [&](uint32_t key) { return key < p.seq && (!p.causal || key <= qrow); };
-                // A first look at the scores, 32 keys at a time, for their maximum.  What fits beside the row's output stays in
-                // registers: both halves at head sizes up to 64, else the second.
-                uint32_t s[kHalves][32];
+                const bool edge = key0 + BKV > p.seq || (p.causal && key0 + BKV - 1 > u.q0);
+                // Keys of this block that the row admits.  A score of -inf would pass unseen as p = 0, so the least score is
+                // looked at too; the other non-finite ones reach the sums.  That of a key that is not admitted makes
+                // the row suspect as well, no more: suspects are settled one by one.
+                const uint32_t end = p.causal ? min(p.seq, qrow + 1) : p.seq, limit = end > key0 ? end - key0 : 0u;
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-                auto release_scores = [&]() {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&s_empty[t]);
-                };
-                auto mask = [&](uint32_t (&x)[32], uint32_t first_key) {
+                auto look = [&](uint32_t (&x)[32], uint32_t first) {
 #pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        if (!admitted(first_key + q)) x[q] = 0xff800000u;  // -inf
-                };
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t (&x)[32] = s[h % kHalves];
-                    if (kHalves == 1 || h == 0) {
-                        tmem_ld_32x32b_x32(tS + h * 32, x);
-                        if (kHalves == 2) tmem_ld_32x32b_x32(tS + 32, s[kHalves - 1]);
-                        tmem_ld_wait();
-                        if (kHalves == 2) release_scores();
+                    for (int q = 0; q < 32; q += 2) {
+                        float d;
+                        asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(mn[q / 2 % 4]), "f"(__uint_as_float(x[q])), "f"(__uint_as_float(x[q + 1])));
+                        mn[q / 2 % 4] = d;
                     }
                     if (edge) {
 #pragma unroll
                         for (int q = 0; q < 32; ++q)
-                            if (admitted(key0 + h * 32 + q)) bad = bad || !isfinite(__uint_as_float(x[q]));
-                        mask(x, key0 + h * 32);
-                    } else {
-                        // a score of -inf would pass unseen as p = 0; the other non-finite ones reach the sums
-#pragma unroll
-                        for (int q = 0; q < 32; q += 2) {
-                            float d;
-                            asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(mn[q / 2 % 4]), "f"(__uint_as_float(x[q])), "f"(__uint_as_float(x[q + 1])));
-                            mn[q / 2 % 4] = d;
-                        }
+                            if (first + q >= limit) x[q] = 0xff800000u;  // -inf
                     }
 #pragma unroll
                     for (int q = 0; q < 32; q += 8)
 #pragma unroll
                         for (int w = 0; w < 4; ++w)
                             mx[w] = max3(mx[w], __uint_as_float(x[q + 2 * w]), __uint_as_float(x[q + 2 * w + 1]));
+                };
+                auto release_scores = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&s_empty[t]);
+                };
+                const uint64_t c2 = pack_f32x2(c, c);
+                uint64_t e2[32];   // the probabilities, two keys a word
+                uint64_t sum2[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+                auto exponentials = [&](const uint32_t (&x)[32], int half, uint64_t nmc2) {
+                    sum2[half][0] = sum2[half][1] = 0ull;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) {
+                        float x0, x1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(x[2 * q]), __uint_as_float(x[2 * q + 1])), c2, nmc2), x0, x1);
+                        e2[half * 16 + q] = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
+                        sum2[half][q & 1] = add_f32x2(sum2[half][q & 1], e2[half * 16 + q]);
+                    }
+                };
+                // What fits beside the row's output stays in registers after this look: both halves at head sizes up to 64, else
+                // the second; the first is fetched again.
+                uint32_t x[kHalves][32];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (kHalves == 1 || h == 0) {
+                        tmem_ld_32x32b_x32(tS + h * 32, x[0]);
+                        if (kHalves == 2) tmem_ld_32x32b_x32(tS + 32, x[kHalves - 1]);
+                        tmem_ld_wait();
+                        if (kHalves == 2) release_scores();
+                    }
+                    look(x[h % kHalves], h * 32);
                 }
                 bad = bad || fminf(fminf(mn[0], mn[1]), fminf(mn[2], mn[3])) == -INFINITY;
                 const float rowmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
                 // move the reference only when the block maximum outgrows it by more than the threshold
-                const bool move = (rowmax - m_ref) * c > kRescaleThreshold;  // true for the first admitted key (m_ref = -inf)
-                const float factor = move ? ex2_approx((m_ref - rowmax) * c) : 1.0f;
-                if (move) m_ref = rowmax;
-                const float mc = (m_ref == -INFINITY ? 0.0f : m_ref) * c;
-                const uint64_t c2 = pack_f32x2(c, c), nmc2 = pack_f32x2(-mc, -mc);
-                uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
-                auto probability = [&](uint32_t s0, uint32_t s1, int q) {
-                    const uint64_t x2 = fma_f32x2(pack_f32x2(__uint_as_float(s0), __uint_as_float(s1)), c2, nmc2);
-                    float x0, x1;
-                    unpack_f32x2(x2, x0, x1);
-                    const uint64_t e = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
-                    sum2[q & 3] = add_f32x2(sum2[q & 3], e);
-                    return e;
-                };
-                uint64_t e2[32];   // the probabilities, in the registers of their scores
-#pragma unroll
-                for (int q = 0; q < kHalves * 16; ++q) e2[32 - kHalves * 16 + q] = probability(s[q / 16][2 * (q % 16)], s[q / 16][2 * (q % 16) + 1], q);
-                if constexpr (kHalves == 1) {   // the scores of the first half are fetched again
-                    tmem_ld_32x32b_x32(tS, s[0]);
+                const float top = rowmax * c;
+                const bool move = top - m_ref > kRescaleThreshold;  // true for the first admitted key (m_ref = -inf)
+                const float moved = fmaf(rintf(top) - top, p.whole, top);
+                const float factor = move ? ex2_approx(m_ref - moved) : 1.0f;
+                if (move) m_ref = moved;
+                const float mc = m_ref == -INFINITY ? 0.0f : m_ref;
+                const uint64_t nmc2 = pack_f32x2(-mc, -mc);
+                exponentials(x[kHalves - 1], 1, nmc2);
+                if constexpr (kHalves == 1) {
+                    tmem_ld_32x32b_x32(tS, x[0]);
                     tmem_ld_wait();
                     release_scores();
-                    if (edge) mask(s[0], key0);
+                    if (edge) {
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) e2[q] = probability(s[0][2 * q], s[0][2 * q + 1], q);
+                        for (int q = 0; q < 32; ++q)
+                            if (q >= limit) x[0][q] = 0xff800000u;  // -inf
+                    }
                 }
+                exponentials(x[0], 0, nmc2);
                 // P of the previous block must have been consumed and O must be quiescent
-                if (j > 0) {
+                if (j >= STREAMS) {
                     if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
                     tc_fence_after();
-                    const bool first = starts_group(j);
+                    const bool first = starts_group(j / STREAMS);
                     if (first) add_group();
                     if (__any_sync(0xffffffffu, move)) {
                         const uint64_t f2 = pack_f32x2(factor, factor);
@@ -545,7 +549,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {
                     float a, b;
-                    unpack_f32x2(sum2[w], a, b);
+                    unpack_f32x2(sum2[w >> 1][w & 1], a, b);
                     sum[w] = a + b;
                 }
                 l = fmaf(l, factor, (sum[0] + sum[1]) + (sum[2] + sum[3]));
@@ -554,56 +558,80 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_ready[t]);
+                if (storing) release_rows();   // the unit before's: by now they have been read
             }
             if (!ok) break;
-            if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
-            tc_fence_after();
-            add_group();
-            const float inv = 1.0f / l;
-            bool good = !bad && isfinite(l) && l > 0.0f;
-            const uint32_t row0 = first_row + quad * 32;   // first query row of this warp
-            const uint64_t inv2 = pack_f32x2(inv, inv);
+            if (t < u.n) {
+                if (!wait(&pv_done[t], (gt - 1) & 1)) { ok = false; break; }
+                tc_fence_after();
+                add_group();
+                // the next unit's first P*V overwrites O: order this thread's reads of O before its p_ready arrival
+                tc_fence_before();
+            }
+            if (storing) release_rows();
+            // The streams' parts of the row meet in shared memory.  A part that is not finite makes the sum NaN for both.
+            float *const ref = reinterpret_cast<float *>(smem + L::kOffRow) + r;
+            uint64_t check2[2] = {0ull, 0ull};        // 0, or NaN once a value was not finite
 #pragma unroll
-            for (int q = 0; q < NG * 32; ++q) {
-                o2[q] = mul_f32x2(o2[q], inv2);
-                float v0, v1;
-                unpack_f32x2(o2[q], v0, v1);
-                if (2 * q < p.dim) good = good && isfinite(v0) && isfinite(v1);   // (the head size is even)
+            for (int q = 0; q < NG * 32; ++q) check2[q & 1] = fma_f32x2(o2[q], 0ull, check2[q & 1]);   // (columns past the head size are zeros)
+            float4 check;
+            unpack_f32x2(check2[0], check.x, check.y);
+            unpack_f32x2(check2[1], check.z, check.w);
+            if (bad) l = NAN;
+            l += (check.x + check.y) + (check.z + check.w);
+            if (!wait(&merge_empty[t ^ 1], (n & 1) ^ 1)) { ok = false; break; }
+#pragma unroll
+            for (int q = 0; q < NG * 8; ++q) {
+                float4 v;
+                unpack_f32x2(o2[NG * 16 + 2 * q], v.x, v.y);
+                unpack_f32x2(o2[NG * 16 + 2 * q + 1], v.z, v.w);
+                *piece(rows_given, q) = v;
+            }
+            ref[t * 2 * BQ] = m_ref;
+            ref[t * 2 * BQ + BQ] = l;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&merge_full[t ^ 1]);
+            if (!wait(&merge_full[t], n & 1)) { ok = false; break; }
+            ++n;
+            const float m1 = ref[(t ^ 1) * 2 * BQ], l1 = ref[(t ^ 1) * 2 * BQ + BQ];
+            const float m = fmaxf(m_ref, m1), mc = m == -INFINITY ? 0.0f : m;
+            const float f0 = ex2_approx(m_ref - mc), f1 = ex2_approx(m1 - mc);   // powers of two
+            const float sum = l * f0 + l1 * f1;   // one rounding: the streams agree on it
+            const float inv = 1.0f / sum;
+            const bool good = isfinite(sum) && sum > 0.0f;
+            const uint32_t row0 = u.q0 + quad * 32;   // first query row of this warp
+            const uint64_t f02 = pack_f32x2(f0, f0), f12 = pack_f32x2(f1, f1), inv2 = pack_f32x2(inv, inv);
+#pragma unroll
+            for (int q = 0; q < NG * 8; ++q) {
+                const float4 v = *piece(rows_out, q);
+                float4 w;
+                unpack_f32x2(mul_f32x2(fma_f32x2(o2[2 * q], f02, mul_f32x2(pack_f32x2(v.x, v.y), f12)), inv2), w.x, w.y);
+                unpack_f32x2(mul_f32x2(fma_f32x2(o2[2 * q + 1], f02, mul_f32x2(pack_f32x2(v.z, v.w), f12)), inv2), w.z, w.w);
+                *piece(rows_out, q) = w;
             }
             const uint32_t unsettled = __ballot_sync(0xffffffffu, !good && qrow < p.seq);
-            if (unsettled == 0) {
-                // through shared memory and the copy engine: full-line writes that do not hold the warp
+            if (unsettled == 0) {   // full-line writes that do not hold the warp
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {   // rows beyond seq and columns beyond the head size are clipped
 #pragma unroll
-                for (int h = 0; h < NG * 2; ++h) {
-                    if (h * 32 >= p.dim) break;
-                    if (h > 0) {
-                        if (lane == 0) tma_store_wait_read();   // the slice is still being read by the previous copy
-                        __syncwarp();
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
-                            make_uint4((uint32_t)o2[h * 16 + 2 * k], (uint32_t)(o2[h * 16 + 2 * k] >> 32), (uint32_t)o2[h * 16 + 2 * k + 1],
-                                       (uint32_t)(o2[h * 16 + 2 * k + 1] >> 32));
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && row0 < p.seq) {   // rows beyond seq and columns beyond the head size are clipped
-                        tma_store_3d(&tmO, slice, h * 32, (int32_t)row0, (int32_t)u.head);
-                        tma_store_commit();
-                    }
+                    for (uint32_t h = 0; h < NG; ++h)
+                        if (t * kHalfCols + h * 32 < p.dim && row0 < p.seq)
+                            tma_store_3d(&tmO, rows_out + h * 4096, (int32_t)(t * kHalfCols + h * 32), (int32_t)row0, (int32_t)u.head);
+                    tma_store_commit();
                 }
-                if (lane == 0) tma_store_wait_read();   // before the next unit's lo term overwrites the slice
-            } else if (good && qrow < p.seq) {
-                float *dst = p.out + ((uint64_t)u.head * p.seq + qrow) * p.dim;
-#pragma unroll
-                for (int q = 0; q < NG * 32; ++q)
-                    if (2 * q < p.dim) {
-                        float2 v;
-                        unpack_f32x2(o2[q], v.x, v.y);
-                        reinterpret_cast<float2 *>(dst)[q] = v;
-                    }
+                storing = true;
+            } else {
+                if (good && qrow < p.seq) {
+                    float *dst = p.out + ((uint64_t)u.head * p.seq + qrow) * p.dim + t * kHalfCols;
+#pragma unroll 1
+                    for (uint32_t q = 0; q < NG * 8; ++q)
+                        if (t * kHalfCols + 4 * q < p.dim) reinterpret_cast<float4 *>(dst)[q] = *piece(rows_out, q);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&merge_empty[t]);
             }
-            if (unsettled != 0) {
+            if (unsettled != 0 && t == 0) {
                 auto tick = [settled, lane](uint32_t) { if (lane == 0) atomicAdd(settled, 1u); };
                 const uint64_t head = (uint64_t)u.head * p.seq * p.dim;
                 const uint32_t last = row0 + 31 - __clz(unsettled);
@@ -616,10 +644,8 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
             }
             __syncwarp();
-            // the next unit's first P*V overwrites O: order this thread's reads of O before its p_ready arrival
-            tc_fence_before();
-            __syncwarp();
         }
+        if (storing && lane == 0) tma_store_wait_read();   // the rows must stay until the copies have read them
         if (!ok && lane == 0) kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
     }
     tc_fence_before();
@@ -660,17 +686,14 @@ int32_t attention_split_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args
         st = fe2o3_make_tmap_f32(&plan->tmO, a->output.ptr, 3, dims, ostrides, obox);
     }
     if (st != FE2O3_OK) { delete plan; return st; }
-    // Two-tile units share their K/V loads and overlap one tile's exponentials with the other's MMAs; where they
-    // would leave half of the SMs without work, single tiles.
-    const uint32_t q_blocks = (uint32_t)(((uint64_t)a->seq + QT * BQ - 1) / (QT * BQ));
+    const uint32_t q_blocks = (uint32_t)(((uint64_t)a->seq + BQ - 1) / BQ);
     const uint64_t units = (uint64_t)bh * q_blocks;
     const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
     if (units > 0x7fffffffull) { delete plan; fe2o3_set_error("UnsupportedShape: too many rows"); return FE2O3_ERR_UNSUPPORTED_SHAPE; }
-    const bool half = 2 * units <= sms;
     plan->p = SplitParams{reinterpret_cast<const uint16_t *>(a->q.ptr), reinterpret_cast<const uint16_t *>(a->k.ptr),
                           reinterpret_cast<const uint16_t *>(a->v.ptr), reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->dim,
                           a->scale, a->scale * 1.4426950408889634f, a->causal,
-                          q_blocks, (uint32_t)(half ? 2 * units : units), half ? 1u : 0u, ctx->status_word};
+                          q_blocks, (uint32_t)units, a->seq <= BKV ? 0.0f : 1.0f, ctx->status_word};
     plan->grid = plan->p.units < sms ? plan->p.units : sms;
     plan->groups = a->dim <= 64 ? 1 : 2;
     *out = plan;

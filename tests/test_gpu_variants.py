@@ -354,7 +354,7 @@ def test_row_softmax_views_and_bad_rows(gpu, orc, cols, in_at, out_at):
 # ---- attention with f32-precision probabilities (head sizes other than 64): 128-row tiles, 64-key blocks
 @pytest.mark.parametrize("B,H,S,D,causal", [(1, 1, 1, 128, False), (1, 3, 63, 128, True), (2, 1, 65, 96, True), (1, 2, 129, 72, False),
                                             (1, 1, 257, 32, True), (1, 5, 300, 128, True), (1, 1, 600, 8, False), (2, 13, 500, 56, True),
-                                            # more two-tile units than SMs: several rounds, dealt in both directions
+                                            # more units than SMs: several rounds, dealt in both directions
                                             (4, 50, 200, 128, False), (4, 45, 400, 40, True)])
 def test_attention_split_probabilities(gpu, orc, B, H, S, D, causal):
     from fe2o3_b200 import synth
@@ -410,6 +410,30 @@ def test_attention_split_rising_scores(gpu, S, D, causal):
     got, _ = attn_run(gpu, q, k, v, 1.0 / np.sqrt(D), causal, fe.DTYPE_BF16)
     # a score is wrong by up to D / 16 + 2 roundings of its size, a weight by as much relatively, and a result by twice that
     assert np.abs(got[0] - want).max() <= 2 * top * (D / 16 + 2) * 2.0 ** -23 * np.abs(v32).max() + 2.5e-5
+
+
+@pytest.mark.parametrize("S,D,causal", [(200, 128, False), (300, 40, True)])
+def test_attention_split_goes_on_after_rows_that_are_settled(gpu, S, D, causal):
+    """A head with a non-finite key among several rounds of units: its blocks settle rows and then take further units."""
+    from fe2o3_b200 import synth
+    fe, ctx, stream = gpu
+    B, H = 1, 160
+    q, k, v = (synth.normal_bf16(3, d, H * S * D, 1.0).reshape(H, S, D) for d in (1, 2, 3))
+    for h in (0, 77, 159):
+        k[h, S - 3, 5] = 0xff80   # -Inf
+    Q, K, V = (Guarded(fe, stream, x) for x in (q, k, v))
+    O = Guarded(fe, stream, np.full(H * S * D, 7.0, np.float32))
+    p = fe.prepare(ctx, "flash_attention_v1", q=Q.slice, k=K.slice, v=V.slice, output=O.slice, batch=B, heads=H, seq=S, dim=D,
+                   scale=1.0 / np.sqrt(D), causal=int(causal), input_dtype=fe.DTYPE_BF16)
+    with pytest.raises(fe.Fe2o3Error):
+        p.launch_and_wait(stream)
+    got = O.read().reshape(H, S, D)
+    want, _ = attention_f64(*(synth.bf16_to_f32(np.where(x == 0xff80, 0, x).astype(np.uint16)) for x in (q, k, v)), 1.0 / np.sqrt(D), causal)
+    spared = S - 3 if causal else 0   # rows that do not admit the bad key
+    for h in range(H):
+        rows = spared if h in (0, 77, 159) else S
+        assert np.abs(got[h, :rows] - want[h, :rows]).max(initial=0.0) <= 2.5e-5 * 6, h   # |v| below 6
+        assert (got[h, rows:] == 7.0).all(), h
 
 
 @pytest.mark.parametrize("causal", [False, True])
