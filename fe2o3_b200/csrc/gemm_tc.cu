@@ -44,7 +44,8 @@ constexpr int kGroupM = 16;     // m-tiles per rasterisation band (keeps a wave'
 // own 128 rows of A and its half of B's columns, so a k block costs 32 KiB of staging per SM instead of 48.
 template <int BN, int CG>
 struct SmemLayout {
-    static constexpr int kStages = BN == 64 ? 8 : BN == 128 || CG == 2 ? 6 : 4;   // 192 KiB in flight whatever the tile
+    static constexpr int kStages = BN == 64 ? 8 : BN == 128 || CG == 2 ? 6 : 4;   // 192 KiB in flight, 160 at 192 columns
+    static constexpr uint32_t kTmemCols = BN == 192 ? 512 : 2 * BN;            // (a power of two)
     static constexpr uint32_t kABytes = BM * BK * 2;
     static constexpr uint32_t kBBytes = BN / CG * BK * 2;
     static constexpr uint32_t kStageBytes = kABytes + kBBytes;
@@ -221,52 +222,50 @@ __device__ __forceinline__ void gelu_pairs(const uint32_t *x, uint32_t *out) {  
 // One 32 x 32 chunk of f32 output out of a warp's swizzled slice into C, VEC elements per access: 32 / VEC lanes
 // cover a row's 128 bytes, so an instruction touches VEC whole row segments.  With one lane per row (each lane
 // walking its own row) the alpha/beta form cost 32 sectors per 4-byte access: 1000 x 3001 x 1111 took 98.8 us, 22.5 so.
-// For alpha/beta the old values of a whole batch of rows are fetched before the first is used.
+// `old` holds the chunk's old values for alpha/beta, from fetch_chunk with the same lane layout.
 template <int VEC>
-__device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, const uint8_t *slice,
-                                            uint32_t lane, const GemmParams &p) {
+__device__ __forceinline__ void fetch_chunk(float (&old)[32], const float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, uint32_t lane) {
     constexpr uint32_t kLanes = 32 / VEC;        // lanes per row
-    constexpr uint32_t kBatch = VEC == 4 ? 8 : 16;
     const uint32_t sub = lane / kLanes, c = (lane % kLanes) * VEC;
-    const bool update = p.epilogue == EPI_ALPHA_BETA;
-#pragma unroll 1
-    for (uint32_t b = 0; b < 32; b += kBatch * VEC) {
-        float old[kBatch][VEC];
-        if (update) {
 #pragma unroll
-            for (uint32_t i = 0; i < kBatch; ++i) {
-                const uint32_t rr = b + i * VEC + sub;
-                const float *src = chunk + (uint64_t)rr * ldc + c;
-                if (rr < rows && c < cols) {
-                    if constexpr (VEC == 4) {
-                        const float4 v = *reinterpret_cast<const float4 *>(src);
-                        old[i][0] = v.x; old[i][1] = v.y; old[i][2] = v.z; old[i][3] = v.w;
-                    } else {
-                        old[i][0] = *src;
-                    }
-                }
+    for (uint32_t i = 0; i < 32 / VEC; ++i) {
+        const uint32_t rr = i * VEC + sub;
+        const float *src = chunk + (uint64_t)rr * ldc + c;
+        if (rr < rows && c < cols) {
+            if constexpr (VEC == 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(src);
+                old[4 * i] = v.x; old[4 * i + 1] = v.y; old[4 * i + 2] = v.z; old[4 * i + 3] = v.w;
+            } else {
+                old[i] = *src;
             }
         }
+    }
+}
+template <int VEC>
+__device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, const uint8_t *slice,
+                                            uint32_t lane, const GemmParams &p, const float (&old)[32]) {
+    constexpr uint32_t kLanes = 32 / VEC;
+    const uint32_t sub = lane / kLanes, c = (lane % kLanes) * VEC;
+    const bool update = p.epilogue == EPI_ALPHA_BETA;
 #pragma unroll
-        for (uint32_t i = 0; i < kBatch; ++i) {
-            const uint32_t rr = b + i * VEC + sub;
-            if (rr < rows && c < cols) {
-                const uint8_t *at = slice + rr * 128 + (((c >> 2) ^ (rr & 7)) * 16) + (c & 3) * 4;
-                float v[VEC];
-                if constexpr (VEC == 4) {
-                    const float4 x = *reinterpret_cast<const float4 *>(at);
-                    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-                } else {
-                    v[0] = *reinterpret_cast<const float *>(at);
-                }
-                if (update) {
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) v[q] = __fadd_rn(__fmul_rn(p.alpha, v[q]), __fmul_rn(p.beta, old[i][q]));
-                }
-                float *dst = chunk + (uint64_t)rr * ldc + c;
-                if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-                else *dst = v[0];
+    for (uint32_t i = 0; i < 32 / VEC; ++i) {
+        const uint32_t rr = i * VEC + sub;
+        if (rr < rows && c < cols) {
+            const uint8_t *at = slice + rr * 128 + (((c >> 2) ^ (rr & 7)) * 16) + (c & 3) * 4;
+            float v[VEC];
+            if constexpr (VEC == 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(at);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            } else {
+                v[0] = *reinterpret_cast<const float *>(at);
             }
+            if (update) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) v[q] = __fadd_rn(__fmul_rn(p.alpha, v[q]), __fmul_rn(p.beta, old[VEC * i + q]));
+            }
+            float *dst = chunk + (uint64_t)rr * ldc + c;
+            if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            else *dst = v[0];
         }
     }
 }
@@ -385,10 +384,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #endif
     if (warp == 1) {
         if constexpr (CG == 2) {
-            tmem_alloc_pair(tmem_slot, 2 * BN);
+            tmem_alloc_pair(tmem_slot, L::kTmemCols);
             tmem_relinquish_pair();
         } else {
-            tmem_alloc(tmem_slot, 2 * BN);
+            tmem_alloc(tmem_slot, L::kTmemCols);
             tmem_relinquish();
         }
     }
@@ -647,13 +646,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
-            if (!mbar_wait_warp(&tmem_full[buf], acc_phase, &s_abort)) { ok = false; break; }
-            tc_fence_after();
             const uint32_t row0 = t.m0 + quad * 32;
             const uint32_t row = row0 + lane;
             const bool row_ok = row < t.m_end;
             const bool bulk = p.bulk_store && row0 + 32 <= t.m_end;   // warp-uniform
             const uint32_t col_base = t.n0 * BN + col_half * (BN / 2);
+            // alpha/beta: the old values of C, a chunk of 32 columns ahead; the first while the tile is being multiplied
+            const uint32_t rows_here = min(32u, t.m_end > row0 ? t.m_end - row0 : 0u);
+            float *const c0 = reinterpret_cast<float *>(p.c) + (uint64_t)row0 * p.ldc;
+            const bool vec = p.ldc % 4u == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15u) == 0;
+            auto fetch = [&](float (&to)[32], uint32_t col) {
+                if (col >= p.N) return;
+                if (vec && col + 32 <= p.N) fetch_chunk<4>(to, c0 + col, p.ldc, rows_here, 32, lane);
+                else fetch_chunk<1>(to, c0 + col, p.ldc, rows_here, min(32u, p.N - col), lane);
+            };
+            float old[32];
+            if (REGS > 128 && p.epilogue == EPI_ALPHA_BETA) {
+                fetch(old, col_base);
+#pragma unroll
+                for (uint32_t g = 1; g < kChunks; ++g)
+                    if (row_ok && col_base + g * 32 < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + (uint64_t)lane * p.ldc + col_base + g * 32));
+            }
+            if (!mbar_wait_warp(&tmem_full[buf], acc_phase, &s_abort)) { ok = false; break; }
+            tc_fence_after();
             const uint32_t taddr = tmem_base + buf * BN + col_half * (BN / 2) + ((quad * 32u) << 16);
             // scatter epilogue: where this lane's row goes (0 = nowhere)
             unsigned long long dst_row = 0;
@@ -738,6 +753,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
+            } else if (REGS > 128 && p.epilogue == EPI_ALPHA_BETA) {
+                // ---- alpha/beta
+                float next[32];
+#pragma unroll 1
+                for (int g = 0; g < kChunks; ++g) {
+                    const uint32_t col = col_base + g * 32;
+                    if (g + 1 < kChunks) fetch(next, col + 32);
+                    uint32_t r[32];
+                    tmem_ld_32x32b_x32(taddr + g * 32, r);
+                    tmem_ld_wait();
+                    if (g == kChunks - 1) {   // the accumulator has been read completely
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) release_accumulator(buf);
+                    }
+                    if (col >= p.N) continue;
+                    __syncwarp();   // the previous chunk has been read out of the slice
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
+                            make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+                    __syncwarp();
+                    if (vec && col + 32 <= p.N) write_chunk<4>(c0 + col, p.ldc, rows_here, 32, slice, lane, p, old);
+                    else write_chunk<1>(c0 + col, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, old);
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) old[k] = next[k];
+                }
             } else if constexpr (REGS > 128) {
                 // ---- f32 output: one chunk (32 columns) per 128-byte group (the 128-register build has bf16 output only)
 #pragma unroll 1
@@ -811,12 +853,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
                                 make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
                         __syncwarp();
-                        const uint32_t rows_here = min(32u, t.m_end > row0 ? t.m_end - row0 : 0u);
-                        float *chunk = reinterpret_cast<float *>(p.c) + (uint64_t)row0 * p.ldc + col;
-                        if (col + 32 <= p.N && p.ldc % 4u == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15u) == 0)
-                            write_chunk<4>(chunk, p.ldc, rows_here, 32, slice, lane, p);
+                        float *chunk = c0 + col;
+                        const float none[32] = {};
+                        if (vec && col + 32 <= p.N)
+                            write_chunk<4>(chunk, p.ldc, rows_here, 32, slice, lane, p, none);
                         else
-                            write_chunk<1>(chunk, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p);
+                            write_chunk<1>(chunk, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, none);
                     }
                 }
             }
@@ -845,8 +887,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if constexpr (CG == 2) cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, 2 * BN);
-        else tmem_dealloc(tmem_base, 2 * BN);
+        if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, L::kTmemCols);
+        else tmem_dealloc(tmem_base, L::kTmemCols);
     }
 #ifdef FE2O3_EP_TRACE
     if (p.ep.trace_flags && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
@@ -968,6 +1010,7 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
         consider(128, 0, 68 * rounds(BM, 128, sms));
         // (bf16 output leaves in pieces of 64 columns a warp, half a tile's columns)
         if (epilogue != EPI_GELU_BF16) consider(64, 0, 55 * rounds(BM, 64, sms));
+        if (!experts) consider(192, 0, 84 * rounds(BM, 192, sms));
         // A group's tile takes only the copies of A that hold its rows: of 32 rows up to 24 rows a group on average
         // (16 rows, d 2048: 96.5 -> 93.6 us a layer pass), of 64 up to 48; with more, one copy of the whole tile is
         // cheaper than several (64 rows a group: 98.2 against 96.3 us)
@@ -1008,7 +1051,7 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
     const uint32_t group = plan->pair ? 2 : 1;   // blocks per tile
     const uint64_t tiles = m_tiles * n_tiles, slots = ctx->sm_count / group;
     plan->grid = group * (uint32_t)(tiles < slots ? (tiles ? tiles : 1) : slots);
-    plan->smem = plan->pair ? SmemLayout<256, 2>::kTotal : plan->bn == 256 ? SmemLayout<256, 1>::kTotal : plan->bn == 128 ? SmemLayout<128, 1>::kTotal : SmemLayout<64, 1>::kTotal;
+    plan->smem = plan->pair ? SmemLayout<256, 2>::kTotal : plan->bn == 256 ? SmemLayout<256, 1>::kTotal : plan->bn == 192 ? SmemLayout<192, 1>::kTotal : plan->bn == 128 ? SmemLayout<128, 1>::kTotal : SmemLayout<64, 1>::kTotal;
     plan->overlap_previous = 0;
     return FE2O3_OK;
 }
@@ -1017,6 +1060,7 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
 int32_t gemm_tc_init_device() {
     auto set = [](auto kernel, uint32_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
     FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 1>, SmemLayout<256, 1>::kTotal));
+    FE2O3_CUDA(set(gemm_tc_kernel<192, 168, 1>, SmemLayout<192, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<128, 168, 1>, SmemLayout<128, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<64, 168, 1>, SmemLayout<64, 1>::kTotal));
     FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 1>, SmemLayout<256, 1>::kTotal));
@@ -1056,6 +1100,7 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
     else
         e = plan->pair ? launch(gemm_tc_kernel<256, 168, 2>)
                        : plan->bn == 256 ? launch(gemm_tc_kernel<256, 168, 1>)
+                       : plan->bn == 192 ? launch(gemm_tc_kernel<192, 168, 1>)
                        : plan->bn == 128 ? launch(gemm_tc_kernel<128, 168, 1>) : launch(gemm_tc_kernel<64, 168, 1>);
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "gemm_tc");

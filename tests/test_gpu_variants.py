@@ -69,7 +69,9 @@ def test_gemm_tcgen05_direct_output_exact(gpu, orc, m, n, k, ldc, offset):
 # no rows or no columns
 @pytest.mark.parametrize("m,n,k,ldc,beta", [(1, 130, 1025, 131, -1.0), (129, 72, 520, 72, 0.0), (1000, 1000, 96, 1003, 0.5),
                                             (1100, 2050, 64, 2052, 0.0), (1281, 1912, 1032, 1912, 0.0), (1281, 2000, 1100, 2003, -1.0),
-                                            (700, 3400, 1040, 3400, 0.0), (700, 3400, 72, 3400, 0.0)])
+                                            (700, 3400, 1040, 3400, 0.0), (700, 3400, 72, 3400, 0.0),
+                                            # 192 columns: C in vectors and by elements, tiles that end inside
+                                            (1000, 3001, 1100, 3004, -0.25), (1000, 2900, 200, 2903, 1.0)])
 def test_gemm_tile_shapes_exact(gpu, orc, m, n, k, ldc, beta):
     fe, ctx, stream = gpu
     from fe2o3_b200 import synth
@@ -85,6 +87,20 @@ def test_gemm_tile_shapes_exact(gpu, orc, m, n, k, ldc, beta):
     for r in range(m):
         assert (bits(got[r * ldc:r * ldc + n]) == bits(want[r * n:(r + 1) * n])).all(), r
         assert (bits(got[r * ldc + n:(r + 1) * ldc]) == bits(c[r * ldc + n:(r + 1) * ldc])).all(), r
+
+
+# packed operands, one size for each tile shape: 64, 128, 192, 256 columns and pairs
+@pytest.mark.parametrize("m,n,k", [(512, 512, 512), (1536, 1536, 512), (1008, 3008, 1104), (2048, 2048, 512), (2304, 2304, 1104)])
+def test_tiled_gemm_v1_tile_shapes_exact(gpu, m, n, k):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    a, b = synth.gemm_inputs_v1(m * k, 1, 1, 5)[0], synth.gemm_inputs_v1(1, k * n, 1, 6)[1]
+    A, B = Guarded(fe, stream, a), Guarded(fe, stream, b)
+    Cb = Guarded(fe, stream, np.zeros(m * n, np.float32))
+    run(fe, ctx, stream, "tiled_gemm_v1", a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k)
+    wide = lambda v: (v.astype(np.uint32) << 16).view(np.float32)
+    want = wide(a).reshape(m, k) @ wide(b).reshape(k, n)   # dyadic alphabet: every summation order is exact
+    assert (Cb.read().reshape(m, n) == want).all()
 
 
 # ring lengths: fewer k blocks than stages, as many, and a ring that ends inside a tile, two rounds of tiles
