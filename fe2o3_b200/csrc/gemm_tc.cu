@@ -10,7 +10,7 @@
 // Layout.  A is row-major [M][K] (K contiguous, "K-major"); B is row-major
 // [K][N] (N contiguous, "MN-major") exactly as the reference stores them, so no
 // transpose pass is needed: the instruction descriptor marks B as MN-major.
-// A CTA owns a 128 x BN output tile; one K block is 64 bf16 = 128 bytes.
+// A CTA owns a 128 x BN output tile (BN 64, 128, 192 or 256); one K block is 64 bf16 = 128 bytes.
 //   A stage: one TMA box {64 k, 128 rows}  -> 128 rows x 128 B, 8-row groups 1 KiB apart
 //   B stage: BN/64 TMA boxes {64 n, 64 k}   -> per box 64 k-rows x 128 B (8 KiB)
 // What bounds the large products is power (at 1000 W the clock falls to 1.1 GHz, and the tensor pipe is 90 % busy
@@ -60,20 +60,28 @@ struct TileCoord {
     bool valid;
 };
 
+// What a build of the kernel is for.  One for all of them was 0.5 us slower a launch, whatever it was launched for: code that
+// a launch steps over still has to come past the instruction caches.
+enum GemmKind : int { kPlain, kUpdate /* alpha/beta */, kGrouped /* f32 rows, or added to token rows */, kGroupedGelu,
+                      kPeer /* expert-parallel: rows scattered to their home ranks */, kPeerGelu };
+__host__ __device__ constexpr bool is_grouped(int kind) { return kind >= kGrouped; }
+__host__ __device__ constexpr bool is_gelu(int kind) { return kind == kGroupedGelu || kind == kPeerGelu; }
+__host__ __device__ constexpr bool is_peer(int kind) { return kind >= kPeer; }
+
 // Static tile order.  Plain: bands of kGroupM m-tiles, m fastest inside a band.
 // Grouped: expert-major; inside an expert m fastest.  Grouped with per-source waiting (first GEMM of
 // the expert-parallel FFN): by the source rank of the tile's first row, this rank's own rows first
 // (they never cross NVLink), then ranks +1, +2, ... which is the order in which the other ranks send
 // to this one; inside a source by local expert, then m, n fastest.
 // TM: rows of a tile (128, or 256 for a pair of blocks).
-template <int TM>
+template <int TM, int KIND>
 __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &p, uint32_t n_tiles,
                                                  const uint32_t *s_off, const uint32_t *s_pair) {
     TileCoord t;
     t.valid = false;
     t.expert = 0;
     t.m0 = t.n0 = t.m_end = t.mt_index = 0;
-    if (p.experts == 0) {
+    if constexpr (!is_grouped(KIND)) {
         constexpr uint32_t kBand = kGroupM * BM / TM;
         const uint32_t m_tiles = (p.M + TM - 1) / TM;
         if (id >= m_tiles * n_tiles) return t;
@@ -87,7 +95,7 @@ __device__ __forceinline__ TileCoord decode_tile(uint32_t id, const GemmParams &
         t.valid = true;
         return t;
     }
-    if (TM == BM && (p.ep.rows_flags || p.ep.progress_mode)) {
+    if (is_peer(KIND) && TM == BM && (p.ep.rows_flags || p.ep.progress_mode)) {
         // groups = (run j, local expert le): the tiles whose first row belongs to source (rank + j) mod W; inside
         // an expert's segment the runs lie in exactly that order (the owner's own rows first)
         const uint32_t W = p.ep.world;
@@ -241,12 +249,11 @@ __device__ __forceinline__ void fetch_chunk(float (&old)[32], const float *chunk
         }
     }
 }
-template <int VEC>
+template <int VEC, bool UPDATE>
 __device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, const uint8_t *slice,
                                             uint32_t lane, const GemmParams &p, const float (&old)[32]) {
     constexpr uint32_t kLanes = 32 / VEC;
     const uint32_t sub = lane / kLanes, c = (lane % kLanes) * VEC;
-    const bool update = p.epilogue == EPI_ALPHA_BETA;
 #pragma unroll
     for (uint32_t i = 0; i < 32 / VEC; ++i) {
         const uint32_t rr = i * VEC + sub;
@@ -259,7 +266,7 @@ __device__ __forceinline__ void write_chunk(float *chunk, uint32_t ldc, uint32_t
             } else {
                 v[0] = *reinterpret_cast<const float *>(at);
             }
-            if (update) {
+            if constexpr (UPDATE) {
 #pragma unroll
                 for (int q = 0; q < VEC; ++q) v[q] = __fadd_rn(__fmul_rn(p.alpha, v[q]), __fmul_rn(p.beta, old[VEC * i + q]));
             }
@@ -302,15 +309,20 @@ __device__ __forceinline__ uint32_t walk_ring(uint64_t *bars, uint32_t &stage, u
     return n;
 }
 
-// REGS = 168 is what the block's 320 threads can have; REGS = 128 (still no spills) is for the GEMM that runs
+// REGS = 168 is what the block's 320 threads can have; REGS = 128 (no spills) is for the GEMM that runs
 // beside the expert-parallel dispatch kernel: registers are handed out to four warps at a time, so the ten
 // warps count as twelve, and 12 x 32 x 128 leaves room for one block of that kernel on the same SM.  It and the
 // build with loader warps (a gathered A) run the first GEMM of an expert FFN only, so REGS = 128 has no f32 output.
-template <int BN, int REGS, int CG>
+template <int BN, int REGS, int CG, int KIND>
 __global__ void __maxnreg__(REGS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, GemmParams p) {
     using L = SmemLayout<BN, CG>;
+    // what this kind of launch does not have is known here
+    const GemmEp ep = is_peer(KIND) ? p.ep : GemmEp{};
+    const uint32_t experts = is_grouped(KIND) ? p.experts : 0u;
+    const uint32_t epilogue = KIND == kPlain ? EPI_STORE : KIND == kUpdate ? EPI_ALPHA_BETA : is_gelu(KIND) ? EPI_GELU_BF16 : KIND == kPeer ? EPI_SCATTER_PEER : p.epilogue;
+    const uint32_t *const gather_perm = KIND == kGroupedGelu ? p.gather_perm : nullptr;
     constexpr int kStages = L::kStages;
     constexpr bool kAhead = BN < 256;   // roles issue for every stage that is ready (walk_ring)
     extern __shared__ uint8_t smem_raw[];
@@ -333,13 +345,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t crank = CG == 2 ? cluster_rank() : 0u;
     const uint32_t first_tile = blockIdx.x / CG, tile_step = gridDim.x / CG;
     // the second GEMM of the expert FFN may take over each SM as this kernel's CTA leaves it
-    if (p.ep.progress_mode == 1) launch_dependents();
+    if (ep.progress_mode == 1) launch_dependents();
 
     if (threadIdx.x == 0) {
         // Expert-parallel passes chain kernels through flags on other ranks: once a kernel of the pass has
         // reported a fault (a wait that ran out, a bad table), the later ones must not publish anything.
         // They find the status word set and do nothing but their arrival counting.
-        s_abort = (p.ep.pair_offsets && p.status && __ldcg(p.status) != 0u) ? 1 : 0;
+        s_abort = (ep.pair_offsets && p.status && __ldcg(p.status) != 0u) ? 1 : 0;
         for (int i = 0; i < kStages; ++i) {
             mbar_init(&full[i], 1);   // the producer's expect-tx arrival; in a pair rank 0's barrier counts both blocks' bytes
             mbar_init(&empty[i], 1);
@@ -351,36 +363,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         mbar_fence_init();
     }
     __shared__ int s_table_bad;
-    const uint32_t ep_epoch = p.ep.epoch_counter ? __ldcg(p.ep.epoch_counter) + 1u : p.ep.epoch;
+    const uint32_t ep_epoch = ep.epoch_counter ? __ldcg(ep.epoch_counter) + 1u : ep.epoch;
     // hand-over counters: two sets used by alternate passes; this pass's set was cleared during the previous one
-    uint32_t *const progress = p.ep.progress ? p.ep.progress + (ep_epoch & 1u) * p.ep.progress_len : nullptr;
+    uint32_t *const progress = ep.progress ? ep.progress + (ep_epoch & 1u) * ep.progress_len : nullptr;
     // A launch that starts early (programmatic stream serialization) touches nothing of the kernels before it until
     // they have completed; only then may the next one start early, so that what lies two launches back is complete.
     // The second GEMM of a pair launched together (kEarlyWeights) does read its weights and the segment table ahead:
     // the GEMM just before it writes neither, and everything before that one is complete.
-    const bool early = p.after_previous == kEarlyWeights;
-    if (p.experts && warp == 2) {
+    const bool early = is_grouped(KIND) && p.after_previous == kEarlyWeights;
+    if (experts && warp == 2) {
         // The dispatch kernel that writes the table may still be running beside this kernel: wait for its
         // "table written" flag before reading (bounded like every wait).
         if (p.after_previous && !early) grid_dependency_wait();
-        const bool here = !p.ep.table_flag || flag_wait(p.ep.table_flag, ep_epoch, p.ep.spin_limit);
+        const bool here = !ep.table_flag || flag_wait(ep.table_flag, ep_epoch, ep.spin_limit);
         if (!__all_sync(0xffffffffu, here) && lane == 0) kstatus_set(p.status, FE2O3_KSTATUS_WAIT_EXPIRED);
         if (lane == 0) s_table_bad = !here;
 #ifdef FE2O3_EP_TRACE
-        if (lane == 0 && p.ep.trace_flags && p.ep.table_flag && p.ep.progress_mode != 2 && blockIdx.x == 0) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_TABLE_HERE);
+        if (lane == 0 && ep.trace_flags && ep.table_flag && ep.progress_mode != 2 && blockIdx.x == 0) ep_trace(ep.trace_flags, FE2O3_EP_T_FFN1_TABLE_HERE);
 #endif
         // The segment table is device data (in the expert-parallel layer it derives from other ranks'
         // counts): it is made monotone and cut off at M here, so that no row index derived from it can
         // leave A or C, and the fault is reported instead.
-        if (load_table(s_off, p.expert_offsets, p.ep.pair_offsets ? p.ep.world : 1u, p.experts, p.M, lane) && lane == 0)
+        if (load_table(s_off, p.expert_offsets, ep.pair_offsets ? ep.world : 1u, experts, p.M, lane) && lane == 0)
             kstatus_set(p.status, FE2O3_KSTATUS_SLOT_RANGE);
-        if (p.ep.pair_offsets) load_table(s_pair, p.ep.pair_offsets, 1u, p.experts * p.ep.world, p.M, lane);   // at most 32 pairs
+        if (ep.pair_offsets) load_table(s_pair, ep.pair_offsets, 1u, experts * ep.world, p.M, lane);   // at most 32 pairs
     }
-    if (p.ep.peer_ret)
-        for (uint32_t i = threadIdx.x; i < p.ep.world; i += blockDim.x) s_peer[i] = p.ep.peer_ret[i];
+    if (ep.peer_ret)
+        for (uint32_t i = threadIdx.x; i < ep.world; i += blockDim.x) s_peer[i] = ep.peer_ret[i];
 #ifdef FE2O3_EP_TRACE
-    if (p.ep.trace_flags && blockIdx.x == 0 && threadIdx.x == 0)
-        ep_trace(p.ep.trace_flags, p.ep.rows_flags ? FE2O3_EP_T_FFN1_BEGIN : FE2O3_EP_T_FFN2_BEGIN);
+    if (ep.trace_flags && blockIdx.x == 0 && threadIdx.x == 0)
+        ep_trace(ep.trace_flags, ep.rows_flags ? FE2O3_EP_T_FFN1_BEGIN : FE2O3_EP_T_FFN2_BEGIN);
 #endif
     if (warp == 1) {
         if constexpr (CG == 2) {
@@ -406,7 +418,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         atomicExch(&s_abort, 1);
         if constexpr (CG == 2) st_shared_cluster(cluster_addr(&s_abort, crank ^ 1u), 1u);
     };
-    const bool dead = s_abort != 0 || (p.experts && s_table_bad);   // uniform over the CTA: read after the barrier, before any role can set it
+    const bool dead = s_abort != 0 || (experts && s_table_bad);   // uniform over the CTA: read after the barrier, before any role can set it
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer (warp converged, one elected lane issues)
@@ -420,40 +432,40 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t seen = 0;   // sources whose "rows complete" flag this CTA has already acquired
         bool ok = !dead;
         for (uint32_t id = first_tile; ok; id += tile_step) {
-            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
+            TileCoord t = decode_tile<BM * CG, KIND>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
-            if (p.ep.rows_flags) {
+            if (ep.rows_flags) {
                 // Sources with rows in this tile.  Their rows were written by the source ranks' SMs
                 // (generic proxy, then a system-scope release of the flag); this warp acquires the flag
                 // and orders that observation before its bulk tensor loads (asynchronous proxy) with a
                 // proxy fence.
                 const uint32_t hi = min(t.m0 + BM, t.m_end);
                 uint32_t need = 0;
-                if (lane < p.experts * p.ep.world && s_pair[lane] < hi && s_pair[lane + 1] > t.m0)
-                    need = 1u << (lane % p.ep.world);
+                if (lane < experts * ep.world && s_pair[lane] < hi && s_pair[lane + 1] > t.m0)
+                    need = 1u << (lane % ep.world);
                 need = __reduce_or_sync(0xffffffffu, need) & ~seen;
                 seen |= need;
                 while (need) {   // bit k = run k of a segment = source (rank + k) mod W
-                    const uint32_t src = (p.ep.rank + __ffs(need) - 1) % p.ep.world;
+                    const uint32_t src = (ep.rank + __ffs(need) - 1) % ep.world;
                     need &= need - 1;
-                    if (!__all_sync(0xffffffffu, flag_wait(p.ep.rows_flags + src, ep_epoch, p.ep.spin_limit))) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, flag_wait(ep.rows_flags + src, ep_epoch, ep.spin_limit))) { ok = false; break; }
                 }
                 if (!ok) break;
                 fence_proxy_async_global();
 #ifdef FE2O3_EP_TRACE
-                if (blockIdx.x == 0 && lane == 0 && p.ep.trace_flags) {
-                    if (id == first_tile) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_FIRST_WAIT_DONE);
-                    if (seen == (1u << p.ep.world) - 1u) ep_trace(p.ep.trace_flags, FE2O3_EP_T_FFN1_LAST_WAIT_DONE);
+                if (blockIdx.x == 0 && lane == 0 && ep.trace_flags) {
+                    if (id == first_tile) ep_trace(ep.trace_flags, FE2O3_EP_T_FFN1_FIRST_WAIT_DONE);
+                    if (seen == (1u << ep.world) - 1u) ep_trace(ep.trace_flags, FE2O3_EP_T_FFN1_LAST_WAIT_DONE);
                 }
 #endif
             }
-            if (p.ep.progress_mode == 2) {
+            if (ep.progress_mode == 2) {
                 // The rows of this tile are the first GEMM's output, stored by the copy engine (asynchronous
                 // proxy) and announced through a counter: acquire the count, then order it before the bulk
                 // tensor loads below.
-                if (t.mt_index >= p.ep.progress_len ||
-                    !__all_sync(0xffffffffu, flag_wait(progress + t.mt_index, p.ep.progress_target, p.ep.spin_limit))) {
+                if (t.mt_index >= ep.progress_len ||
+                    !__all_sync(0xffffffffu, flag_wait(progress + t.mt_index, ep.progress_target, ep.spin_limit))) {
                     ok = false;
                     break;
                 }
@@ -461,7 +473,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             // bytes of a k block that rank 0's (or the only) barrier counts: of A only what holds rows of the group
             uint32_t bytes = CG * L::kStageBytes;
-            if (p.gather_perm) {
+            if (gather_perm) {
                 bytes = CG * L::kBBytes + fetched_quads(t.m0, t.m_end) * 512u;
                 if (CG == 2) bytes += fetched_quads(t.m0 + BM, t.m_end) * 512u;   // (rank 1's rows; only rank 0 uses this)
             } else if (CG == 1 && p.a_box_rows < (uint32_t)BM) {
@@ -488,7 +500,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                     for (int j = 0; j < BN / CG / 64; ++j) {
                         const int32_t col = (int32_t)(t.n0 * BN + crank * (BN / CG) + j * 64);
-                        if (p.experts) tma_load_3d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK), (int32_t)t.expert);
+                        if (experts) tma_load_3d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK), (int32_t)t.expert);
                         else tma_load_2d_pair(sb + j * 8192, &tmB, bar, col, (int32_t)(kb * BK));
                     }
                 } else {
@@ -496,7 +508,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                     for (int j = 0; j < BN / 64; ++j) {
                         const int32_t col = (int32_t)(t.n0 * BN + j * 64);
-                        if (p.experts) tma_load_3d(sb + j * 8192, &tmB, &full[st], col, (int32_t)(kb * BK), (int32_t)t.expert);
+                        if (experts) tma_load_3d(sb + j * 8192, &tmB, &full[st], col, (int32_t)(kb * BK), (int32_t)t.expert);
                         else tma_load_2d(sb + j * 8192, &tmB, &full[st], col, (int32_t)(kb * BK));
                     }
                 }
@@ -510,7 +522,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             auto load = [&](uint32_t i, uint32_t kb, uint32_t st) {
                 if (loaded + i >= primed) load_b(kb, st);
-                if (!p.gather_perm) load_a(kb, st);
+                if (!gather_perm) load_a(kb, st);
             };
             for (uint32_t kb = 0; kb < num_kb;) {
                 const uint32_t n = walk_ring<kStages, kAhead>(empty, stage, phase, 1, kb, num_kb, lane, &s_abort, load);
@@ -535,7 +547,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint64_t desc_a0 = umma_smem_desc(smem_u32(smem), 16, 1024);
         const uint64_t desc_b0 = umma_smem_desc(smem_u32(smem) + L::kABytes, 8192, 1024);
         for (uint32_t id = first_tile; ok; id += tile_step, ++it) {
-            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
+            TileCoord t = decode_tile<BM * CG, KIND>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
@@ -583,12 +595,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t stage = 0, phase = 0;
         bool ok = !dead;
         for (uint32_t id = first_tile; ok; id += tile_step) {
-            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
+            TileCoord t = decode_tile<BM * CG, KIND>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;
             const uint32_t quads = (fetched_quads(t.m0, t.m_end) + 3 - gw) / 4;   // this warp's: 1 to 8
             const uint32_t row = t.m0 + ((lane >> 2) * 4 + gw) * 4 + (lane & 3);
-            const uint32_t route = row < t.m_end ? __ldg(p.gather_perm + row) : 0xffffffffu;
+            const uint32_t route = row < t.m_end ? __ldg(gather_perm + row) : 0xffffffffu;
             const uint32_t mine = route == 0xffffffffu ? p.gather_tokens : min(route >> 1, p.gather_tokens);
             int32_t tok[32];
 #pragma unroll
@@ -628,7 +640,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t col_half = ew >> 2;
         constexpr int kChunks = BN / 32 / 2;   // 32-column chunks per warp
         uint8_t *slice = smem + L::kStagingOffset + ew * 4096;
-        const bool out_bf16 = p.epilogue == EPI_GELU_BF16;
         uint32_t it = 0;
         bool ok = !dead;
         bool store_pending = false;
@@ -636,13 +647,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if constexpr (CG == 2) mbar_arrive_cluster(cluster_addr(&tmem_empty[buf], 0));
             else mbar_arrive(&tmem_empty[buf]);
         };
-        if (p.zero_ptr && !dead) {
+        if (KIND == kGroupedGelu && p.zero_ptr && !dead) {
             const uint64_t stride = (uint64_t)gridDim.x * (kEpilogueWarps * 32);
             for (uint64_t i = (uint64_t)blockIdx.x * (kEpilogueWarps * 32) + ew * 32 + lane; i < p.zero_vecs; i += stride)
                 p.zero_ptr[i] = make_uint4(0u, 0u, 0u, 0u);
         }
         for (uint32_t id = first_tile; ok; id += tile_step, ++it) {
-            TileCoord t = decode_tile<BM * CG>(id, p, n_tiles, s_off, s_pair);
+            TileCoord t = decode_tile<BM * CG, KIND>(id, p, n_tiles, s_off, s_pair);
             if (!t.valid) break;
             if constexpr (CG == 2) t.m0 += crank * BM;   // this block's rows of the pair's tile
             const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
@@ -661,7 +672,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 else fetch_chunk<1>(to, c0 + col, p.ldc, rows_here, min(32u, p.N - col), lane);
             };
             float old[32];
-            if (REGS > 128 && p.epilogue == EPI_ALPHA_BETA) {
+            if constexpr (KIND == kUpdate) {
                 fetch(old, col_base);
 #pragma unroll
                 for (uint32_t g = 1; g < kChunks; ++g)
@@ -672,15 +683,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t taddr = tmem_base + buf * BN + col_half * (BN / 2) + ((quad * 32u) << 16);
             // scatter epilogue: where this lane's row goes (0 = nowhere)
             unsigned long long dst_row = 0;
-            if (p.epilogue == EPI_SCATTER_PEER && row_ok) {
-                const uint2 meta = __ldcg(p.ep.row_meta + row);   // (route id, home rank), written by the source rank
-                if (meta.y < p.ep.world && meta.x < p.ep.ret_rows)
+            if (epilogue == EPI_SCATTER_PEER && row_ok) {
+                const uint2 meta = __ldcg(ep.row_meta + row);   // (route id, home rank), written by the source rank
+                if (meta.y < ep.world && meta.x < ep.ret_rows)
                     dst_row = s_peer[meta.y] + (unsigned long long)meta.x * p.N * sizeof(float);
                 else
                     kstatus_set(p.status, FE2O3_KSTATUS_SLOT_RANGE);
             }
             float row_weight = 0.0f;
-            if (p.epilogue == EPI_COMBINE_ADD && row_ok) {
+            if (epilogue == EPI_COMBINE_ADD && row_ok) {
                 // where this lane's row is added and with which weight: route id of the slot, the token's two
                 // weights checked like the separate combine does (finite, non-negative, summing to exactly 1)
                 const uint32_t route = __ldg(p.combine_perm + row);
@@ -694,11 +705,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                 }
             }
-            if (row0 >= t.m_end) {   // none of this warp's rows belong to the group
+            if (is_grouped(KIND) && row0 >= t.m_end) {   // none of this warp's rows belong to the group
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) release_accumulator(buf);
-            } else if (out_bf16) {
+            } else if constexpr (is_gelu(KIND)) {
                 // ---- GELU, bf16 output: 64 columns to a 128-byte group, 16 at a time.  The loops stay rolled: a block of a
                 // small batch runs this code once, and waits for its instructions (unrolled: 2 us more a pass of 64 tokens).
                 uint32_t r[16];
@@ -753,7 +764,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-            } else if (REGS > 128 && p.epilogue == EPI_ALPHA_BETA) {
+            } else if constexpr (KIND == kUpdate) {
                 // ---- alpha/beta
                 float next[32];
 #pragma unroll 1
@@ -775,13 +786,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         *reinterpret_cast<uint4 *>(slice + lane * 128 + ((k ^ (lane & 7)) * 16)) =
                             make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
                     __syncwarp();
-                    if (vec && col + 32 <= p.N) write_chunk<4>(c0 + col, p.ldc, rows_here, 32, slice, lane, p, old);
-                    else write_chunk<1>(c0 + col, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, old);
+                    if (vec && col + 32 <= p.N) write_chunk<4, true>(c0 + col, p.ldc, rows_here, 32, slice, lane, p, old);
+                    else write_chunk<1, true>(c0 + col, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, old);
 #pragma unroll
                     for (int k = 0; k < 32; ++k) old[k] = next[k];
                 }
-            } else if constexpr (REGS > 128) {
-                // ---- f32 output: one chunk (32 columns) per 128-byte group (the 128-register build has bf16 output only)
+            } else {
+                // ---- f32 output: one chunk (32 columns) per 128-byte group
 #pragma unroll 1
                 for (int g = 0; g < kChunks; ++g) {
                     uint32_t r[32];
@@ -794,7 +805,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     const uint32_t col = col_base + g * 32;
                     if (col >= p.N) continue;
-                    if (p.epilogue == EPI_SCATTER_PEER || p.epilogue == EPI_COMBINE_ADD) {
+                    if (epilogue == EPI_SCATTER_PEER || epilogue == EPI_COMBINE_ADD) {
                         // Every row of the tile has its own destination (the return buffer of its home
                         // rank, at its route id).  The chunk is transposed through the warp's slice of
                         // shared memory so that each store instruction writes four whole 128-byte
@@ -814,7 +825,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             const float wgt = __shfl_sync(0xffffffffu, row_weight, rr);
                             if (dst != 0 && col + piece * 4 < p.N) {
                                 const unsigned long long at = dst + (unsigned long long)(col + piece * 4) * sizeof(float);
-                                if (p.epilogue == EPI_COMBINE_ADD)   // weight * row (one rounding), then one addition per element
+                                if (epilogue == EPI_COMBINE_ADD)   // weight * row (one rounding), then one addition per element
                                     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(at),
                                                  "f"(__fmul_rn(wgt, __uint_as_float(v.x))), "f"(__fmul_rn(wgt, __uint_as_float(v.y))),
                                                  "f"(__fmul_rn(wgt, __uint_as_float(v.z))), "f"(__fmul_rn(wgt, __uint_as_float(v.w)))
@@ -823,7 +834,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                     *reinterpret_cast<uint4 *>(at) = v;
                             }
                         }
-                    } else if (bulk && p.epilogue == EPI_STORE) {
+                    } else if (bulk && epilogue == EPI_STORE) {
                         if (store_pending) {
                             if (lane == 0) tma_store_wait_read();
                             __syncwarp();
@@ -856,13 +867,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         float *chunk = c0 + col;
                         const float none[32] = {};
                         if (vec && col + 32 <= p.N)
-                            write_chunk<4>(chunk, p.ldc, rows_here, 32, slice, lane, p, none);
+                            write_chunk<4, false>(chunk, p.ldc, rows_here, 32, slice, lane, p, none);
                         else
-                            write_chunk<1>(chunk, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, none);
+                            write_chunk<1, false>(chunk, p.ldc, rows_here, min(32u, p.N - col), slice, lane, p, none);
                     }
                 }
             }
-            if (p.ep.progress_mode == 1) {
+            if (ep.progress_mode == 1) {
                 // this warp's part of the hidden rows of the tile is in memory: bulk stores complete (not merely
                 // read out of shared memory), direct stores fenced; then one count per warp
                 if (store_pending) {
@@ -872,13 +883,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 __threadfence();
                 __syncwarp();
                 fence_proxy_async_global();
-                if (lane == 0 && t.mt_index < p.ep.progress_len) atomicAdd(progress + t.mt_index, 1u);
+                if (lane == 0 && t.mt_index < ep.progress_len) atomicAdd(progress + t.mt_index, 1u);
             }
         }
         // the staging slice must stay intact until the last copy has read it
         if (store_pending && lane == 0) tma_store_wait_read();
         // rows stored into other ranks' memory must be visible there before "outputs ready" is raised
-        if (p.epilogue == EPI_SCATTER_PEER) __threadfence_system();
+        if (epilogue == EPI_SCATTER_PEER) __threadfence_system();
         if (!ok && lane == 0) give_up();
     }
     tc_fence_before();
@@ -891,22 +902,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         else tmem_dealloc(tmem_base, L::kTmemCols);
     }
 #ifdef FE2O3_EP_TRACE
-    if (p.ep.trace_flags && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-        ep_trace(p.ep.trace_flags, p.ep.rows_flags ? FE2O3_EP_T_FFN1_END : FE2O3_EP_T_FFN2_END);
+    if (ep.trace_flags && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        ep_trace(ep.trace_flags, ep.rows_flags ? FE2O3_EP_T_FFN1_END : FE2O3_EP_T_FFN2_END);
 #endif
-    if (p.ep.done_counter && threadIdx.x == 0) {
+    if (ep.done_counter && threadIdx.x == 0) {
         // The last CTA of the grid to finish raises "outputs ready" on every rank, unless some CTA gave
         // up on a wait (the pass is void then).  A failed CTA still arrives, so the counter is re-armed.
         const bool failed = s_abort != 0;
-        const uint32_t old = atomicAdd(p.ep.done_counter, failed ? 0x10001u : 1u);
+        const uint32_t old = atomicAdd(ep.done_counter, failed ? 0x10001u : 1u);
         if ((old & 0xffffu) == gridDim.x - 1) {
-            atomicExch(p.ep.done_counter, 0u);
-            if (p.ep.progress_mode == 2)   // the other set of hand-over counters, for the next pass (nobody uses it during this one)
-                for (uint32_t i = 0; i < p.ep.progress_len; ++i) p.ep.progress[((ep_epoch & 1u) ^ 1u) * p.ep.progress_len + i] = 0u;
+            atomicExch(ep.done_counter, 0u);
+            if (ep.progress_mode == 2)   // the other set of hand-over counters, for the next pass (nobody uses it during this one)
+                for (uint32_t i = 0; i < ep.progress_len; ++i) ep.progress[((ep_epoch & 1u) ^ 1u) * ep.progress_len + i] = 0u;
             if (!failed && (old >> 16) == 0) {
                 __threadfence_system();
-                for (uint32_t w = 0; w < p.ep.world; ++w)
-                    st_release_sys(reinterpret_cast<uint32_t *>(p.ep.peer_flags[w]) + FE2O3_EP_FLAG_OUTPUTS(p.ep.world) + p.ep.rank,
+                for (uint32_t w = 0; w < ep.world; ++w)
+                    st_release_sys(reinterpret_cast<uint32_t *>(ep.peer_flags[w]) + FE2O3_EP_FLAG_OUTPUTS(ep.world) + ep.rank,
                                    ep_epoch);
             }
         }
@@ -980,25 +991,37 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
                      uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta, uint32_t epilogue,
                      const uint32_t *expert_offsets, uint32_t experts, uint32_t expert_mod, uint32_t b_matrices,
                      const GemmEp *ep) {
-    // Tile shape.  A launch costs its rounds of tiles times what a round takes, which beyond the fixed ~4 us of a
-    // launch goes as 0.55 : 0.68 : 1 for 64, 128 and 256 columns (measured, us: 1024^3 8.3 : 9.4 : 11.3 in one round
-    // each, 2048x2048x512 14.4 : 11.1 : 9.3 in four, two and one), so a small result takes the narrowest tile that
-    // still needs one round: 512^3 8.4 -> 6.1, 1536^3 14.1 -> 11.8.
-    // 256-row tiles on pairs of SMs stage a third less per multiply-add, which shortens a round by about a tenth
-    // where the k loop sets its length: 8192^3 907 against 832 us, 2048x2048x4096 36.9 against 34.8.  A pair's two
-    // epilogues run in step, so where the output does (K = 128 of 8192x8192: 54 against 61 us, K = 1024: 13.9
-    // against 14.3) single blocks stay, as they do where coarser tiles make more rounds (512 rows an expert, d 2048:
-    // 194 against 209 us a layer pass).  Groups end in a partly filled tile, half of one on average.
-    // The expert-parallel GEMMs count finished 256-wide tiles and keep them: half-width ones re-read A twice as
-    // often and were slower there on 4096 and 8192 rows (530 against 481 us and 686 against 590 us a pass).
     plan->bn = N > 128 ? 256 : 128;
     plan->pair = 0;
     uint32_t a_box = BM;
-    if (!ep) {
-        const uint64_t sms = ctx->sm_count;
+    const uint64_t sms = ctx->sm_count, k_blocks = (K + BK - 1) / BK;
+    if (!ep && !experts) {
+        // Tile shape: the cheapest of what a launch costs by itself, its k blocks in every round of tiles, and what of
+        // the output of a round the next one does not hide (alpha/beta reads C too).  Fitted to 90 products of up to
+        // 8192 x 8192 x 8192, all five shapes each: the choice is within 0.1 % of the best on average, 1.5 % at worst.  A narrow
+        // tile has the shortest launch and the dearest multiply-add, a pair of SMs the opposite: it stages a third less.
+        // us: 512^3 64 columns 5.2, 128 6.4, 192 7.5, 256 7.9, pair 9.2; 1000 x 3001 x 1111 alpha/beta 19.8, 19.1, 13.8, 16.5, 16.9;
+        // 3072 x 3072 x 1024 32.3, 24.8, 25.6, 21.3, 19.5.
+        static const struct { uint32_t bn, pair, launch, k_block, output; } shapes[] = {   // ns
+            {64, 0, 4380, 195, 1080}, {128, 0, 4800, 258, 1650}, {192, 0, 5440, 320, 2500}, {256, 0, 5200, 380, 3460}, {256, 1, 6900, 277, 3630}};
+        uint64_t best = ~0ull;
+        for (const auto &shape : shapes) {
+            const uint64_t rows = shape.pair ? 2 * BM : BM, slots = shape.pair ? sms / 2 : sms;
+            if (slots == 0) continue;
+            const uint64_t tiles = ((M + rows - 1) / rows) * ((N + shape.bn - 1) / shape.bn), rounds = (tiles + slots - 1) / slots;
+            const uint64_t product = k_blocks * shape.k_block, output = epilogue == EPI_ALPHA_BETA ? shape.output * 9 / 5 : shape.output;
+            const uint64_t cost = shape.launch + rounds * product + (output > product && rounds > 1 ? (rounds - 1) * (output - product) : 0);
+            if (cost < best) { best = cost; plan->bn = shape.bn; plan->pair = shape.pair; }
+        }
+    } else if (!ep) {
+        // Groups: rounds of tiles times what a round takes, as 0.55 : 0.68 : 1 for 64, 128 and 256 columns; a group ends in
+        // a partly filled tile, half of one on average.  256-row tiles on pairs of SMs shorten a round by about a tenth where
+        // the k loop sets its length, but not where coarser tiles make more rounds (512 rows an expert, d 2048: 194
+        // against 209 us a layer pass).
+        // The expert-parallel GEMMs count finished 256-wide tiles and keep them: half-width ones re-read A twice as
+        // often and were slower there on 4096 and 8192 rows (530 against 481 us and 686 against 590 us a pass).
         auto rounds = [&](uint64_t tile_rows, uint64_t tile_cols, uint64_t slots) {
-            uint64_t m_tiles = (M + tile_rows - 1) / tile_rows;
-            if (experts) m_tiles = M <= experts * tile_rows / 2 ? experts : (2 * (uint64_t)M + experts * tile_rows) / (2 * tile_rows);
+            const uint64_t m_tiles = M <= experts * tile_rows / 2 ? experts : (2 * (uint64_t)M + experts * tile_rows) / (2 * tile_rows);
             return (m_tiles * ((N + tile_cols - 1) / tile_cols) + slots - 1) / slots;
         };
         uint64_t best = 100 * rounds(BM, 256, sms);
@@ -1010,11 +1033,10 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
         consider(128, 0, 68 * rounds(BM, 128, sms));
         // (bf16 output leaves in pieces of 64 columns a warp, half a tile's columns)
         if (epilogue != EPI_GELU_BF16) consider(64, 0, 55 * rounds(BM, 64, sms));
-        if (!experts) consider(192, 0, 84 * rounds(BM, 192, sms));
         // A group's tile takes only the copies of A that hold its rows: of 32 rows up to 24 rows a group on average
         // (16 rows, d 2048: 96.5 -> 93.6 us a layer pass), of 64 up to 48; with more, one copy of the whole tile is
         // cheaper than several (64 rows a group: 98.2 against 96.3 us)
-        if (experts && !plan->pair) a_box = M <= 24 * experts ? 32 : M <= 48 * experts ? 64 : BM;
+        if (!plan->pair) a_box = M <= 24 * experts ? 32 : M <= 48 * experts ? 64 : BM;
     }
     uint64_t dA[2] = {K, M}, sA[1] = {(uint64_t)lda * 2};
     uint32_t bA[2] = {BK, a_box};
@@ -1056,18 +1078,67 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
     return FE2O3_OK;
 }
 
+// The builds in use: every tile shape of a plain or alpha/beta product (192 columns there only), of the others what
+// their plans choose.  REGS = 128: see the kernel.
+template <typename F>
+static void with_kernel(const GemmTcPlan *plan, F f) {
+    const GemmParams &p = plan->p;
+    if (p.experts == 0) {
+#define FE2O3_SHAPES(KIND)                                                                                       \
+        if (plan->pair) f(gemm_tc_kernel<256, 168, 2, KIND>);                                                     \
+        else if (plan->bn == 256) f(gemm_tc_kernel<256, 168, 1, KIND>);                                           \
+        else if (plan->bn == 192) f(gemm_tc_kernel<192, 168, 1, KIND>);                                           \
+        else if (plan->bn == 128) f(gemm_tc_kernel<128, 168, 1, KIND>);                                           \
+        else f(gemm_tc_kernel<64, 168, 1, KIND>)
+        if (p.epilogue == EPI_ALPHA_BETA) { FE2O3_SHAPES(kUpdate); }
+        else { FE2O3_SHAPES(kPlain); }
+#undef FE2O3_SHAPES
+    } else if (p.ep.pair_offsets) {
+        // the first GEMM may share its SM with the small blocks of the dispatch kernel before it
+        if (p.epilogue == EPI_GELU_BF16) {
+            if (plan->bn == 256) f(gemm_tc_kernel<256, 128, 1, kPeerGelu>);
+            else f(gemm_tc_kernel<128, 128, 1, kPeerGelu>);
+        } else {
+            if (plan->bn == 256) f(gemm_tc_kernel<256, 168, 1, kPeer>);
+            else f(gemm_tc_kernel<128, 168, 1, kPeer>);
+        }
+    } else if (p.epilogue == EPI_GELU_BF16) {   // (with or without the warps that gather A)
+        if (plan->pair) f(gemm_tc_kernel<256, 128, 2, kGroupedGelu>);
+        else if (plan->bn == 256) f(gemm_tc_kernel<256, 128, 1, kGroupedGelu>);
+        else f(gemm_tc_kernel<128, 128, 1, kGroupedGelu>);
+    } else {
+        if (plan->pair) f(gemm_tc_kernel<256, 168, 2, kGrouped>);
+        else if (plan->bn == 256) f(gemm_tc_kernel<256, 168, 1, kGrouped>);
+        else if (plan->bn == 128) f(gemm_tc_kernel<128, 168, 1, kGrouped>);
+        else f(gemm_tc_kernel<64, 168, 1, kGrouped>);
+    }
+}
+
 // Function attributes are per device: called by fe2o3_ctx_create with the context's device current.
 int32_t gemm_tc_init_device() {
-    auto set = [](auto kernel, uint32_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
-    FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 1>, SmemLayout<256, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<192, 168, 1>, SmemLayout<192, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<128, 168, 1>, SmemLayout<128, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<64, 168, 1>, SmemLayout<64, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 1>, SmemLayout<256, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<128, 128, 1>, SmemLayout<128, 1>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<256, 168, 2>, SmemLayout<256, 2>::kTotal));
-    FE2O3_CUDA(set(gemm_tc_kernel<256, 128, 2>, SmemLayout<256, 2>::kTotal));
-    return FE2O3_OK;
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto kernel, uint32_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+#define FE2O3_SHAPES(KIND)                                                     \
+    set(gemm_tc_kernel<256, 168, 2, KIND>, SmemLayout<256, 2>::kTotal);        \
+    set(gemm_tc_kernel<256, 168, 1, KIND>, SmemLayout<256, 1>::kTotal);        \
+    set(gemm_tc_kernel<128, 168, 1, KIND>, SmemLayout<128, 1>::kTotal);        \
+    set(gemm_tc_kernel<64, 168, 1, KIND>, SmemLayout<64, 1>::kTotal)
+    FE2O3_SHAPES(kPlain);
+    FE2O3_SHAPES(kUpdate);
+    FE2O3_SHAPES(kGrouped);
+#undef FE2O3_SHAPES
+    set(gemm_tc_kernel<192, 168, 1, kPlain>, SmemLayout<192, 1>::kTotal);
+    set(gemm_tc_kernel<192, 168, 1, kUpdate>, SmemLayout<192, 1>::kTotal);
+    set(gemm_tc_kernel<256, 128, 2, kGroupedGelu>, SmemLayout<256, 2>::kTotal);
+    set(gemm_tc_kernel<256, 128, 1, kGroupedGelu>, SmemLayout<256, 1>::kTotal);
+    set(gemm_tc_kernel<128, 128, 1, kGroupedGelu>, SmemLayout<128, 1>::kTotal);
+    set(gemm_tc_kernel<256, 168, 1, kPeer>, SmemLayout<256, 1>::kTotal);
+    set(gemm_tc_kernel<128, 168, 1, kPeer>, SmemLayout<128, 1>::kTotal);
+    set(gemm_tc_kernel<256, 128, 1, kPeerGelu>, SmemLayout<256, 1>::kTotal);
+    set(gemm_tc_kernel<128, 128, 1, kPeerGelu>, SmemLayout<128, 1>::kTotal);
+    return fe2o3_cuda_status(e, "cudaFuncSetAttribute(gemm_tc)");
 }
 
 int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
@@ -1090,18 +1161,8 @@ int32_t gemm_tc_launch(const GemmTcPlan *plan, cudaStream_t s) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    cudaError_t e;
-    // the 128-register build: for a block that shares its SM with the small blocks of the kernel before it, and for
-    // one that carries the loader warps of a gathered A
-    auto launch = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, plan->tmA, plan->tmB, plan->tmC, plan->p); };
-    if (plan->overlap_previous == 1 || plan->p.gather_perm)
-        e = plan->pair ? launch(gemm_tc_kernel<256, 128, 2>)
-                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 128, 1>) : launch(gemm_tc_kernel<128, 128, 1>);
-    else
-        e = plan->pair ? launch(gemm_tc_kernel<256, 168, 2>)
-                       : plan->bn == 256 ? launch(gemm_tc_kernel<256, 168, 1>)
-                       : plan->bn == 192 ? launch(gemm_tc_kernel<192, 168, 1>)
-                       : plan->bn == 128 ? launch(gemm_tc_kernel<128, 168, 1>) : launch(gemm_tc_kernel<64, 168, 1>);
+    cudaError_t e = cudaSuccess;
+    with_kernel(plan, [&](auto kernel) { e = cudaLaunchKernelEx(&cfg, kernel, plan->tmA, plan->tmB, plan->tmC, plan->p); });
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "gemm_tc");
 }
@@ -1137,9 +1198,9 @@ void gemm_tc_geometry(const GemmTcPlan *plan, fe2o3_geometry *geo) {
 }
 
 // kernel symbols of the runtime adapter carried by this source (the schedule a large launch resolves to)
-static Fe2o3KernelRegistration reg_tiled("tiled_gemm_lds_slice1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
-static Fe2o3KernelRegistration reg_general("tiled_gemm_general_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
-static Fe2o3KernelRegistration reg_ffn("moe_expert_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
-static Fe2o3KernelRegistration reg_gffn("moe_grouped_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
-static Fe2o3KernelRegistration reg_ffnc("moe_expert_ffn_combine_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1>));
-static Fe2o3KernelRegistration reg_epffn("moe_ep_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1>));
+static Fe2o3KernelRegistration reg_tiled("tiled_gemm_lds_slice1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1, kPlain>));
+static Fe2o3KernelRegistration reg_general("tiled_gemm_general_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 168, 1, kUpdate>));
+static Fe2o3KernelRegistration reg_ffn("moe_expert_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1, kGroupedGelu>));
+static Fe2o3KernelRegistration reg_gffn("moe_grouped_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1, kGroupedGelu>));
+static Fe2o3KernelRegistration reg_ffnc("moe_expert_ffn_combine_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1, kGroupedGelu>));
+static Fe2o3KernelRegistration reg_epffn("moe_ep_ffn_v1", reinterpret_cast<const void *>(gemm_tc_kernel<256, 128, 1, kPeerGelu>));
