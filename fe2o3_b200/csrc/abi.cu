@@ -36,7 +36,7 @@ int32_t launch_moe_combine(fe2o3_ctx *, cudaStream_t, const void *, fe2o3_geomet
 int32_t launch_moe_ep_exchange(fe2o3_ctx *, cudaStream_t, const void *, fe2o3_geometry *, bool);
 int32_t launch_moe_compact(cudaStream_t, uint64_t x, uint64_t perm, uint64_t compact_x, uint32_t rows,
                            uint32_t d_model, uint32_t tokens);
-int32_t launch_gemm_exact(cudaStream_t, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c, uint32_t M,
+int32_t launch_gemm_exact(fe2o3_ctx *, cudaStream_t, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c, uint32_t M,
                           uint32_t N, uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta,
                           fe2o3_geometry *, bool);
 int32_t launch_attention_simt(fe2o3_ctx *, cudaStream_t, const fe2o3_flash_attention_v1_args *, fe2o3_geometry *, bool);
@@ -653,7 +653,7 @@ int32_t resolve_gemm(fe2o3_prepared *p, uint32_t schedule, uint32_t dtype, uint6
         // each operand into bf16 terms (gemm_split.cu) and is specified by a bound, not bit-exact
         if (schedule != FE2O3_GEMM_SCHEDULE_TCGEN05) {
             p->schedule = FE2O3_GEMM_SCHEDULE_EXACT_ORDER;
-            return launch_gemm_exact(nullptr, dtype, epilogue, a, b, c, M, N, K, lda, ldb, ldc, alpha, beta, &p->geo, true);
+            return launch_gemm_exact(p->ctx, nullptr, dtype, epilogue, a, b, c, M, N, K, lda, ldb, ldc, alpha, beta, &p->geo, true);
         }
         if (epilogue || lda != K || ldb != N || !gemm_split_supported(a, b, N, K))
             return unsupported("tcgen05 schedule for f32 operands needs packed A and B, 16-byte aligned, K and N multiples of 8");
@@ -681,7 +681,7 @@ int32_t resolve_gemm(fe2o3_prepared *p, uint32_t schedule, uint32_t dtype, uint6
         gemm_tc_geometry(&p->gemm[0], &p->geo);
         return FE2O3_OK;
     }
-    return launch_gemm_exact(nullptr, dtype, epilogue, a, b, c, M, N, K, lda, ldb, ldc, alpha, beta, &p->geo, true);
+    return launch_gemm_exact(p->ctx, nullptr, dtype, epilogue, a, b, c, M, N, K, lda, ldb, ldc, alpha, beta, &p->geo, true);
 }
 
 int32_t prepare_common(fe2o3_ctx *ctx, uint32_t op, const void *args, fe2o3_prepared **out) {
@@ -726,13 +726,13 @@ int32_t launch_prepared(fe2o3_prepared *p, cudaStream_t s) {
                 return gemm_tc_launch(&p->gemm[0], s);
             }
             if (p->schedule == FE2O3_GEMM_SCHEDULE_TCGEN05) return gemm_tc_launch(&p->gemm[0], s);
-            return launch_gemm_exact(s, p->op == OP_SCALAR_GEMM ? FE2O3_DTYPE_F32 : FE2O3_DTYPE_BF16, false, a->a.ptr,
+            return launch_gemm_exact(ctx, s, p->op == OP_SCALAR_GEMM ? FE2O3_DTYPE_F32 : FE2O3_DTYPE_BF16, false, a->a.ptr,
                                      a->b.ptr, a->c.ptr, a->m, a->n, a->k, a->k, a->n, a->n, 1.f, 0.f, nullptr, false);
         }
         case OP_TILED_GEMM_GENERAL: {
             const fe2o3_tiled_gemm_general_v1_args *a = reinterpret_cast<const fe2o3_tiled_gemm_general_v1_args *>(p->kernarg);
             if (p->schedule == FE2O3_GEMM_SCHEDULE_TCGEN05) return gemm_tc_launch(&p->gemm[0], s);
-            return launch_gemm_exact(s, FE2O3_DTYPE_BF16, true, a->a.ptr, a->b.ptr, a->c.ptr, a->m, a->n, a->k, a->lda,
+            return launch_gemm_exact(ctx, s, FE2O3_DTYPE_BF16, true, a->a.ptr, a->b.ptr, a->c.ptr, a->m, a->n, a->k, a->lda,
                                      a->ldb, a->ldc, a->alpha, a->beta, nullptr, false);
         }
         case OP_FLASH_ATTENTION: {

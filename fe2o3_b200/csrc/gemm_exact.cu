@@ -10,173 +10,367 @@
 // bit-identical to the CPU oracle for every finite or non-finite input, any
 // strides and any tails.
 //
-// Bound: the f32 pipe, two operations per multiply-add that may not be fused
-// (512^3: 7.5 us on 148 SMs).  The sizes that come here are small, so the tile is
-// 32x64 outputs per 128-thread block, which makes 128 blocks of a 512x512 result
-// (64x64 tiles made 64 blocks for 148 SMs): one warp per scheduler, each thread
-// with 4x4 outputs.  The 16 chains advance by 16 products and eight packed f32x2
-// sums per k (each half rounded exactly like the scalar instruction; the products
-// stay scalar because a packed product feeding a packed sum came out fused, with
-// one rounding), enough independent work for one warp to cover the latency of the
-// additions; operands
-// come as one 16-byte shared-memory read each per k, and the next 32-deep k block
-// is on its way from global memory in registers while the current one is
-// multiplied (two shared-memory buffers, one barrier per block).  512^3: 51.2 us a
-// launch with 64x64 tiles and a single buffer, 19.0 us so.
+// Bound: the f32 pipe, two operations per multiply-add that may not be fused (512^3: 7.5 us on 148 SMs).  A block of 128
+// threads owns 8 RM x 16 RN outputs, RM x RN a thread.
+//   f32: tiles of 32 k go to shared memory by asynchronous copies, a ring of three, one barrier a tile; pieces of four
+// bytes where rows do not start on 16.  Both operands lie as they do in memory: a thread reads four k of each of its
+// rows and four rows of B, 16 bytes each, for RM x RN x 4 products.  Products are scalar, sums packed f32x2 (each half
+// rounded like the scalar instruction; a packed product feeding a packed sum came out fused, with one rounding).
+// us, with operands passed through registers and A transposed on the way (until then) / so: 512^3 18.2 / 15.8, 1024^3 134 / 91,
+// 256^3 9.8 / 5.8, 900 x 40 x 800 31 / 15; at 1024^3 the f32 pipe is three quarters busy.
+//   bf16: operands are widened on the way, through registers.  Products of bf16 values are exact in f32 unless they leave its
+// range, so a fused multiply-add rounds just as a product and a sum do: where every value of a tile is zero or between
+// 2^-62 and 2^63 the fused form is used, which halves the work of the pipe; other tiles take the two-step form.
+// us, alpha/beta, always two steps / so: 2999^3 at odd addresses 2299 / 1445, 300 x 1001 x 501 55 / 33, 100^3 13.0 / 5.3.
 #include "common.cuh"
 
 namespace {
 
-constexpr int TM = 32, TN = 64, TK = 32, kThreads = 128;
+constexpr int TK = 32, kThreads = 128;
 
-template <typename T>
-__device__ __forceinline__ float widen(T v);
-template <>
-__device__ __forceinline__ float widen<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float widen<uint16_t>(uint16_t v) { return bf16_bits_to_f32(v); }
+template <int RM, int RN, int STAGES>
+struct __align__(16) ExactTiles {
+    float a[STAGES][8 * RM][TK + 4];   // rows of 144 bytes: a warp's two rows fall on different banks
+    float b[STAGES][TK][16 * RN];
+};
 
-// Four consecutive elements of a row, widened; `vec` when all four exist and their address is aligned to their size.
-__device__ __forceinline__ float4 load4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
-__device__ __forceinline__ float4 load4(const uint16_t *p) {
-    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(p));
-    return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
-                       __uint_as_float(w.y & 0xffff0000u));
-}
-template <typename T>
-__device__ __forceinline__ float4 load4_guarded(const T *row, uint32_t first, uint32_t end, bool row_ok, bool vec) {
-    if (row_ok && vec && first + 4 <= end) return load4(row + first);
-    float v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = row_ok && first + i < end ? widen<T>(row[first + i]) : 0.0f;
-    return make_float4(v[0], v[1], v[2], v[3]);
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void *dst, const void *src, uint32_t valid) {
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid) : "memory");
 }
 
-template <typename T, bool EPILOGUE>
-__global__ void __launch_bounds__(kThreads)
-gemm_exact_kernel(const T *__restrict__ A, const T *__restrict__ B, float *C, uint32_t M, uint32_t N, uint32_t K,
-                  uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha, float beta) {
-    __shared__ __align__(16) float As[2][TK][TM + 4];   // k-major, so that a thread's four rows are one 16-byte read
-    __shared__ __align__(16) float Bs[2][TK][TN];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const uint32_t row_tiles = (M - 1) / TM + 1;
-    const uint32_t row0 = blockIdx.x % row_tiles * TM, col0 = blockIdx.x / row_tiles * TN;
-    const bool vec_a = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % (4 * sizeof(T)) == 0;
-    const bool vec_b = ldb % 4 == 0 && reinterpret_cast<uintptr_t>(B) % (4 * sizeof(T)) == 0;
-
-    // A: row = thread / 4, eight k values in two groups of four, 16 apart; B: 16 groups of four columns, 8 k rows a pass
-    const uint32_t ar = threadIdx.x >> 2, ak = (threadIdx.x & 3) * 4;
-    const uint32_t bc = tx * 4, bk = ty;
-    const bool a_ok = row0 + ar < M;
-    const T *a_row = A + (uint64_t)(a_ok ? row0 + ar : 0) * lda;
-    float4 a_next[2], b_next[4];
-    auto fetch = [&](uint32_t k0) {
+// The operands of a thread for four k, and its RM x RN sums over them.
+template <int RM, int RN>
+struct Operands {
+    float4 a[RM];
+    float b[4][RN];
+    __device__ __forceinline__ void load(const float (*as)[TK + 4], const float (*bs)[16 * RN], int row, int col, int kk) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) a_next[i] = load4_guarded<T>(a_row, k0 + ak + i * 16, K, a_ok, vec_a);
+        for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4 *>(&as[row + i][kk]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t k = k0 + bk + i * 8;
-            b_next[i] = load4_guarded<T>(B + (uint64_t)(k < K ? k : 0) * ldb, col0 + bc, N, k < K, vec_b);
-        }
-    };
-    auto stage = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            As[buf][ak + i * 16 + 0][ar] = a_next[i].x;
-            As[buf][ak + i * 16 + 1][ar] = a_next[i].y;
-            As[buf][ak + i * 16 + 2][ar] = a_next[i].z;
-            As[buf][ak + i * 16 + 3][ar] = a_next[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(&Bs[buf][bk + i * 8][bc]) = b_next[i];
-    };
-
-    uint64_t acc[4][2];   // rows ty*4 + i, columns tx*4 + {0,1} and {2,3}
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0ull;   // pairs of +0.0f
-    auto step = [&](int buf, int kk) {
-        const float4 a = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-        const float4 b = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            acc[i][0] = add_f32x2(acc[i][0], pack_f32x2(__fmul_rn(av[i], b.x), __fmul_rn(av[i], b.y)));
-            acc[i][1] = add_f32x2(acc[i][1], pack_f32x2(__fmul_rn(av[i], b.z), __fmul_rn(av[i], b.w)));
-        }
-    };
-
-    begin_after_previous();
-    if (K > 0) {
-        fetch(0);
-        stage(0);
-        __syncthreads();
-    }
-    int buf = 0;
-    for (uint32_t k0 = 0; k0 < K; k0 += TK, buf ^= 1) {
-        const bool more = k0 + TK < K;
-        if (more) fetch(k0 + TK);
-        if (K - k0 >= (uint32_t)TK) {
-#pragma unroll
-            for (int kk = 0; kk < TK; ++kk) step(buf, kk);
-        } else {
-            // the recurrence stops at K: the zero padding of the last block is never multiplied
-            const int kmax = (int)(K - k0);
-            for (int kk = 0; kk < kmax; ++kk) step(buf, kk);
-        }
-        if (more) stage(buf ^ 1);   // nobody reads that buffer: the barrier below ended its last use
-        __syncthreads();
-    }
-    const bool vec_c = ldc % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t r = row0 + ty * 4 + i, c0 = col0 + tx * 4;
-        if (r >= M) continue;
-        float v[4];
-        unpack_f32x2(acc[i][0], v[0], v[1]);
-        unpack_f32x2(acc[i][1], v[2], v[3]);
-        float *dst = C + (uint64_t)r * ldc + c0;
-        if (vec_c && c0 + 4 <= N) {
-            if (EPILOGUE) {
-                const float4 old = *reinterpret_cast<const float4 *>(dst);
-                const float o[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, o[j]));
+        for (int q = 0; q < 4; ++q) {
+            if constexpr (RN == 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(&bs[kk + q][col]);
+                b[q][0] = v.x; b[q][1] = v.y; b[q][2] = v.z; b[q][3] = v.w;
+            } else {
+                const float2 v = *reinterpret_cast<const float2 *>(&bs[kk + q][col]);
+                b[q][0] = v.x; b[q][1] = v.y;
             }
-            *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+};
+
+template <int RM, int RN, bool FUSED>
+__device__ __forceinline__ void one_step(uint64_t (&acc)[RM][RN / 2], const float (&a)[RM], const float (&b)[RN]) {
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) {
+            if constexpr (FUSED) acc[i][j] = fma_f32x2(pack_f32x2(a[i], a[i]), pack_f32x2(b[2 * j], b[2 * j + 1]), acc[i][j]);
+            else acc[i][j] = add_f32x2(acc[i][j], pack_f32x2(__fmul_rn(a[i], b[2 * j]), __fmul_rn(a[i], b[2 * j + 1])));
+        }
+}
+
+template <int RM, int RN, bool FUSED>
+__device__ __forceinline__ void four_steps(uint64_t (&acc)[RM][RN / 2], const Operands<RM, RN> &o) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float a[RM];
+#pragma unroll
+        for (int i = 0; i < RM; ++i) a[i] = q == 0 ? o.a[i].x : q == 1 ? o.a[i].y : q == 2 ? o.a[i].z : o.a[i].w;
+        one_step<RM, RN, FUSED>(acc, a, o.b[q]);
+    }
+}
+
+// The first `steps` k of a tile.
+template <int RM, int RN, bool FUSED>
+__device__ __forceinline__ void multiply_tile(uint64_t (&acc)[RM][RN / 2], const float (*as)[TK + 4], const float (*bs)[16 * RN], int row, int col,
+                                              uint32_t steps) {
+    if (steps == TK && RM == 2 && RN == 2) {
+        // few blocks, and a scheduler has one warp at most: operands come four k ahead
+        Operands<RM, RN> even, odd;
+        even.load(as, bs, row, col, 0);
+#pragma unroll 1
+        for (int kk = 0; kk < TK; kk += 8) {
+            odd.load(as, bs, row, col, kk + 4);
+            four_steps<RM, RN, FUSED>(acc, even);
+            even.load(as, bs, row, col, (kk + 8) % TK);   // (the last of a tile are not used)
+            four_steps<RM, RN, FUSED>(acc, odd);
+        }
+    } else if (steps == TK) {
+#pragma unroll
+        for (int kk = 0; kk < TK; kk += 4) {
+            Operands<RM, RN> o;
+            o.load(as, bs, row, col, kk);
+            four_steps<RM, RN, FUSED>(acc, o);
+        }
+    } else {   // the recurrence stops at K: the padding of the last tile is never multiplied
+#pragma unroll 1
+        for (uint32_t kk = 0; kk < steps; ++kk) {
+            float a[RM], b[RN];
+#pragma unroll
+            for (int i = 0; i < RM; ++i) a[i] = as[row + i][kk];
+#pragma unroll
+            for (int j = 0; j < RN; ++j) b[j] = bs[kk][col + j];
+            one_step<RM, RN, FUSED>(acc, a, b);
+        }
+    }
+}
+
+template <int RM, int RN, bool EPILOGUE>
+__device__ __forceinline__ void write_sums(const uint64_t (&acc)[RM][RN / 2], float *C, uint32_t row0, uint32_t c0, uint32_t M, uint32_t N,
+                                           uint32_t ldc, float alpha, float beta) {
+    const bool vec = ldc % RN == 0 && reinterpret_cast<uintptr_t>(C) % (4 * RN) == 0 && c0 + RN <= N;
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        const uint32_t r = row0 + i;
+        if (r >= M) continue;
+        float v[RN];
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) unpack_f32x2(acc[i][j], v[2 * j], v[2 * j + 1]);
+        float *dst = C + (uint64_t)r * ldc + c0;
+        if (vec) {
+            if constexpr (EPILOGUE) {
+                float o[RN];
+                if constexpr (RN == 4) {
+                    const float4 old = *reinterpret_cast<const float4 *>(dst);
+                    o[0] = old.x; o[1] = old.y; o[2] = old.z; o[3] = old.w;
+                } else {
+                    const float2 old = *reinterpret_cast<const float2 *>(dst);
+                    o[0] = old.x; o[1] = old.y;
+                }
+#pragma unroll
+                for (int j = 0; j < RN; ++j) v[j] = __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, o[j]));
+            }
+            if constexpr (RN == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            else *reinterpret_cast<float2 *>(dst) = make_float2(v[0], v[1]);
             continue;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < RN; ++j) {
             if (c0 + j >= N) continue;
             dst[j] = EPILOGUE ? __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, dst[j])) : v[j];
         }
     }
 }
 
+// ---- f32 operands: asynchronous copies
+template <int RM, int RN>
+__global__ void __launch_bounds__(kThreads)
+gemm_exact_f32_kernel(const float *__restrict__ A, const float *__restrict__ B, float *C, uint32_t M, uint32_t N, uint32_t K, uint32_t lda,
+                      uint32_t ldb, uint32_t ldc, float, float) {
+    constexpr int TM = 8 * RM, TN = 16 * RN, STAGES = 3;
+    __shared__ ExactTiles<RM, RN, STAGES> tiles;
+    const uint32_t tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const uint32_t row_tiles = (M - 1) / TM + 1;
+    const uint32_t row0 = blockIdx.x % row_tiles * TM, col0 = blockIdx.x / row_tiles * TN;
+    const bool vec_a = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
+    const bool vec_b = ldb % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+    // what lies past M, N or K arrives as zeros; nothing past a row's end is read
+    auto copy = [&](uint32_t k0, uint32_t st) {
+        if (vec_a) {
+#pragma unroll
+            for (int i = 0; i < TM * TK / 4 / kThreads; ++i) {
+                const uint32_t g = i * kThreads + tid, r = g / (TK / 4), k = g % (TK / 4) * 4;
+                const bool in = row0 + r < M && k0 + k < K;
+                copy_async<16>(&tiles.a[st][r][k], in ? A + (uint64_t)(row0 + r) * lda + k0 + k : A, in ? min(K - k0 - k, 4u) * 4 : 0u);
+            }
+        } else {
+            const uint32_t k = tid % TK, r0 = tid / TK;   // every thread keeps its k
+            const float *src = A + min(k0 + k, K - 1);
+#pragma unroll 8
+            for (int i = 0; i < TM * TK / kThreads; ++i) {
+                const uint32_t r = r0 + i * (kThreads / TK);
+                copy_async<4>(&tiles.a[st][r][k], src + (uint64_t)min(row0 + r, M - 1) * lda, row0 + r < M && k0 + k < K ? 4u : 0u);
+            }
+        }
+        if (vec_b) {
+#pragma unroll
+            for (int i = 0; i < TK * TN / 4 / kThreads; ++i) {
+                const uint32_t g = i * kThreads + tid, k = g / (TN / 4), c = g % (TN / 4) * 4;
+                const bool in = k0 + k < K && col0 + c < N;
+                copy_async<16>(&tiles.b[st][k][c], in ? B + (uint64_t)(k0 + k) * ldb + col0 + c : B, in ? min(N - col0 - c, 4u) * 4 : 0u);
+            }
+        } else {
+            const uint32_t c = tid % TN, q0 = tid / TN;   // every thread keeps its column
+            const float *src = B + min(col0 + c, N - 1);
+#pragma unroll 8
+            for (int i = 0; i < TK * TN / kThreads; ++i) {
+                const uint32_t k = q0 + i * (kThreads / TN);
+                copy_async<4>(&tiles.b[st][k][c], src + (uint64_t)min(k0 + k, K - 1) * ldb, col0 + c < N && k0 + k < K ? 4u : 0u);
+            }
+        }
+    };
+    uint64_t acc[RM][RN / 2];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) acc[i][j] = 0ull;   // pairs of +0.0f
+    begin_after_previous();
+#pragma unroll 1
+    for (uint32_t s = 0; s + 1 < STAGES; ++s) {
+        if (s * TK < K) copy(s * TK, s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    uint32_t st = 0, next = STAGES - 1;
+    for (uint32_t k0 = 0; k0 < K; k0 += TK) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();   // the tile is there, and everybody is done with the one before, whose place the next copy takes
+        if (K - k0 > (STAGES - 1) * TK) copy(k0 + (STAGES - 1) * TK, next);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        multiply_tile<RM, RN, false>(acc, tiles.a[st], tiles.b[st], ty * RM, tx * RN, min(K - k0, (uint32_t)TK));
+        st = st + 1 == STAGES ? 0 : st + 1;
+        next = next + 1 == STAGES ? 0 : next + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    write_sums<RM, RN, false>(acc, C, row0 + ty * RM, col0 + tx * RN, M, N, ldc, 1.0f, 0.0f);
+}
+
+// ---- bf16 operands: widened on the way through registers
+// Four consecutive elements of a row as the aligned words that hold at least one of them each: two, or three from the middle
+// of the first (true then).  They are put together only when they are stored: until then nothing waits for them.
+__device__ __forceinline__ bool load4(uint32_t (&w)[3], const uint16_t *row, uint32_t first, uint32_t end, bool row_ok, bool vec) {
+    if (row_ok && first + 4 <= end) {
+        if (vec) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(row + first));
+            w[0] = v.x; w[1] = v.y;
+            return false;
+        }
+        const uintptr_t at = reinterpret_cast<uintptr_t>(row + first);
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3));
+        w[0] = __ldg(words);
+        w[1] = __ldg(words + 1);
+        if ((at & 2u) == 0) return false;
+        w[2] = __ldg(words + 2);
+        return true;
+    }
+    uint32_t v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = row_ok && first + i < end ? row[first + i] : 0u;
+    w[0] = v[0] | v[1] << 16;
+    w[1] = v[2] | v[3] << 16;
+    return false;
+}
+
+template <int RM, int RN, bool EPILOGUE>
+__global__ void __launch_bounds__(kThreads)
+gemm_exact_bf16_kernel(const uint16_t *__restrict__ A, const uint16_t *__restrict__ B, float *C, uint32_t M, uint32_t N, uint32_t K, uint32_t lda,
+                       uint32_t ldb, uint32_t ldc, float alpha, float beta) {
+    constexpr int TM = 8 * RM, TN = 16 * RN, GA = TM * TK / 4 / kThreads, GB = TK * TN / 4 / kThreads;
+    __shared__ ExactTiles<RM, RN, 2> tiles;
+    const uint32_t tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const uint32_t row_tiles = (M - 1) / TM + 1;
+    const uint32_t row0 = blockIdx.x % row_tiles * TM, col0 = blockIdx.x / row_tiles * TN;
+    const bool vec_a = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 8 == 0;
+    const bool vec_b = ldb % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 8 == 0;
+    uint32_t a_next[GA][3], b_next[GB][3], halves = 0;   // halves: a bit for each piece that starts in the middle of a word
+    auto fetch = [&](uint32_t k0) {
+        halves = 0;
+#pragma unroll
+        for (int i = 0; i < GA; ++i) {
+            const uint32_t g = i * kThreads + tid, r = g / (TK / 4), k = g % (TK / 4) * 4;
+            const bool in = row0 + r < M;
+            halves |= (uint32_t)load4(a_next[i], A + (uint64_t)(in ? row0 + r : 0) * lda, k0 + k, K, in, vec_a) << i;
+        }
+#pragma unroll
+        for (int i = 0; i < GB; ++i) {
+            const uint32_t g = i * kThreads + tid, k = k0 + g / (TN / 4), c = g % (TN / 4) * 4;
+            halves |= (uint32_t)load4(b_next[i], B + (uint64_t)(k < K ? k : 0) * ldb, col0 + c, N, k < K, vec_b) << (GA + i);
+        }
+    };
+    // Returns whether a product with one of the values may not be exact: exponents other than that of zero and those
+    // between 65 and 189 (2^-62 to below 2^63).
+    auto stage = [&](uint32_t st) {
+        uint32_t least = 0xffffffffu, most = 0u;
+        auto put = [&](float *dst, const uint32_t (&w)[3], bool half) {
+            const uint32_t x = half ? __byte_perm(w[0], w[1], 0x5432) : w[0], y = half ? __byte_perm(w[1], w[2], 0x5432) : w[1];
+            const uint32_t v[4] = {x << 16, x & 0xffff0000u, y << 16, y & 0xffff0000u};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t size = v[q] << 1;   // without its sign
+                least = min(least, size - 1u);      // (zero is the largest then)
+                most = max(most, size);
+            }
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+        };
+#pragma unroll
+        for (int i = 0; i < GA; ++i) {
+            const uint32_t g = i * kThreads + tid;
+            put(&tiles.a[st][g / (TK / 4)][g % (TK / 4) * 4], a_next[i], halves >> i & 1u);
+        }
+#pragma unroll
+        for (int i = 0; i < GB; ++i) {
+            const uint32_t g = i * kThreads + tid;
+            put(&tiles.b[st][g / (TN / 4)][g % (TN / 4) * 4], b_next[i], halves >> (GA + i) & 1u);
+        }
+        return least < (65u << 24) - 1u || most >= (190u << 24);
+    };
+    uint64_t acc[RM][RN / 2];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN / 2; ++j) acc[i][j] = 0ull;   // pairs of +0.0f
+    begin_after_previous();
+    int wide = 0;
+    if (K > 0) {
+        fetch(0);
+        wide = __syncthreads_or(stage(0));
+    }
+    uint32_t st = 0;
+    for (uint32_t k0 = 0; k0 < K; k0 += TK, st ^= 1) {
+        const bool more = K - k0 > (uint32_t)TK;
+        if (more) fetch(k0 + TK);
+        const uint32_t steps = min(K - k0, (uint32_t)TK);
+        if (wide) multiply_tile<RM, RN, false>(acc, tiles.a[st], tiles.b[st], ty * RM, tx * RN, steps);
+        else multiply_tile<RM, RN, true>(acc, tiles.a[st], tiles.b[st], ty * RM, tx * RN, steps);
+        if (more) wide = __syncthreads_or(stage(st ^ 1));   // nobody reads that buffer: the barrier before ended its last use
+    }
+    write_sums<RM, RN, EPILOGUE>(acc, C, row0 + ty * RM, col0 + tx * RN, M, N, ldc, alpha, beta);
+}
+
 }  // namespace
 
-// dtype: FE2O3_DTYPE_F32 or FE2O3_DTYPE_BF16 inputs.
-int32_t launch_gemm_exact(cudaStream_t s, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c,
+// dtype: FE2O3_DTYPE_F32 (without epilogue only) or FE2O3_DTYPE_BF16 inputs.
+int32_t launch_gemm_exact(fe2o3_ctx *ctx, cudaStream_t s, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c,
                           uint32_t M, uint32_t N, uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha,
                           float beta, fe2o3_geometry *geo, bool plan_only) {
+    // Tiles.  f32: 16 x 64, two warps a scheduler at 512^3 (32 x 64, one warp: 16.8 us for 15.8; 64 x 64 at 1024^3: 96 for 91),
+    // and 16 x 32 where that leaves every other SM without a block (64 x 64 x 1024: 18.4 for 21.2); copies of four bytes,
+    // where rows do not start on 16, want more work a copy (32 x 64: 700 x 700 x 333 19.3 for 20.5).  bf16, whose staging
+    // costs more: 64 x 64 from four blocks an SM on (2999^3 1445 us for 1672), 32 x 64 from two (500 x 2001 x 77 13.4 for 16.2),
+    // else 16 x 32 (300 x 1001 x 501 33 for 40).
+    const uint64_t sms = ctx->sm_count > 0 ? ctx->sm_count : 1;
+    auto count = [&](uint32_t rows, uint32_t cols) { return (uint64_t)ceil_div_u32(M, rows) * ceil_div_u32(N, cols); };
+    const bool f32 = dtype == FE2O3_DTYPE_F32;
+    const bool pieces = ((a | b) & 15u) != 0 || lda % 4 != 0 || ldb % 4 != 0;
+    const uint32_t rows = f32 ? (pieces && count(32, 64) >= sms ? 32 : 16) : count(64, 64) >= 4 * sms ? 64 : count(32, 64) >= 2 * sms ? 32 : 16;
+    const uint32_t cols = (f32 ? rows == 16 && 2 * count(16, 64) <= sms : rows == 16) ? 32 : 64;
     // one flat index, rows first: the second and third grid dimensions end at 65535 tiles, which either a tall or a
     // wide result can have
-    const uint64_t tiles = (uint64_t)ceil_div_u32(M, TM) * ceil_div_u32(N, TN);
+    const uint64_t tiles = count(rows, cols);
     if (tiles > 0x7fffffffull) { fe2o3_set_error("UnsupportedShape: too many output tiles"); return FE2O3_ERR_UNSUPPORTED_SHAPE; }
     const uint32_t grid = (uint32_t)tiles;
     if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kThreads, 1, 1}, 0, 1};
     if (plan_only || M == 0 || N == 0) return FE2O3_OK;
     float *C = reinterpret_cast<float *>(c);
     cudaError_t e;
-    if (dtype == FE2O3_DTYPE_F32) {
+    if (f32) {
         const float *A = reinterpret_cast<const float *>(a), *B = reinterpret_cast<const float *>(b);
-        e = fe2o3_launch_early(epilogue ? gemm_exact_kernel<float, true> : gemm_exact_kernel<float, false>, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
+        auto kernel = cols == 32 ? gemm_exact_f32_kernel<2, 2> : rows == 16 ? gemm_exact_f32_kernel<2, 4> : gemm_exact_f32_kernel<4, 4>;
+        e = fe2o3_launch_early(kernel, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
     } else {
         const uint16_t *A = reinterpret_cast<const uint16_t *>(a), *B = reinterpret_cast<const uint16_t *>(b);
-        e = fe2o3_launch_early(epilogue ? gemm_exact_kernel<uint16_t, true> : gemm_exact_kernel<uint16_t, false>, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
+        auto kernel = epilogue ? (rows == 64   ? gemm_exact_bf16_kernel<8, 4, true>
+                                  : rows == 32 ? gemm_exact_bf16_kernel<4, 4, true>
+                                               : gemm_exact_bf16_kernel<2, 2, true>)
+                               : (rows == 64   ? gemm_exact_bf16_kernel<8, 4, false>
+                                  : rows == 32 ? gemm_exact_bf16_kernel<4, 4, false>
+                                               : gemm_exact_bf16_kernel<2, 2, false>);
+        e = fe2o3_launch_early(kernel, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
     }
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "gemm_exact");
 }
 
-static Fe2o3KernelRegistration reg_scalar("scalar_gemm_v1", reinterpret_cast<const void *>(gemm_exact_kernel<float, false>));
+static Fe2o3KernelRegistration reg_scalar("scalar_gemm_v1", reinterpret_cast<const void *>(gemm_exact_f32_kernel<2, 4>));

@@ -17,7 +17,9 @@ def gpu():
 
 
 # ---- exact-order GEMM: 32 x 64 tiles, k in blocks of 32
-@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (32, 64, 32), (33, 65, 33), (31, 63, 31), (65, 1, 64), (1, 130, 97), (100, 68, 64)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (32, 64, 32), (33, 65, 33), (31, 63, 31), (65, 1, 64), (1, 130, 97), (100, 68, 64),
+                                   # 16 x 64 and 32 x 64 tiles, rows on 16 bytes and not; three tiles of k in flight
+                                   (1600, 1532, 70), (1601, 1533, 31), (520, 516, 100), (500, 700, 97)])
 def test_scalar_gemm_tile_edges_bit_exact(gpu, orc, m, n, k):
     fe, ctx, stream = gpu
     from fe2o3_b200 import synth
@@ -27,6 +29,30 @@ def test_scalar_gemm_tile_edges_bit_exact(gpu, orc, m, n, k):
     run(fe, ctx, stream, "scalar_gemm_v1", a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k)
     assert (bits(Cb.read()) == bits(orc.gemm_f32(m, n, k, a, b))).all()
     A.unchanged(); B.unchanged()
+
+
+# bf16 operands: products that are exact in f32 are fused with their sum, tiles with values that may leave its range are not
+@pytest.mark.parametrize("low,high", [(65, 189), (60, 189), (65, 192), (1, 254), (0, 255)])
+@pytest.mark.parametrize("m,n,k,pad", [(33, 65, 100, 0), (70, 200, 64, 3), (1700, 1500, 40, 1)])
+def test_exact_bf16_gemm_any_exponent_bit_exact(gpu, orc, m, n, k, pad, low, high):
+    fe, ctx, stream = gpu
+    rng = np.random.default_rng(low * 1000 + high)
+    lda, ldb = k + pad, n + pad
+
+    def values(count):
+        v = (rng.integers(0, 2, count) << 15 | rng.integers(low, high + 1, count) << 7 | rng.integers(0, 128, count)).astype(np.uint16)
+        v[rng.random(count) < 0.05] = 0
+        return v
+    a, b = values((m - 1) * lda + k), values((k - 1) * ldb + n)
+    c = values(2 * m * n).view(np.float32)
+    c[~np.isfinite(c)] = 1.0
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, c)
+    run(fe, ctx, stream, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_EXACT_ORDER, a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k,
+        lda=lda, ldb=ldb, ldc=n, alpha=0.5, beta=-0.25)
+    want = orc.gemm_bf16(m, n, k, a, b, lda=lda, ldb=ldb, ldc=n, alpha=0.5, beta=-0.25, c=c)
+    got = Cb.read()
+    assert (np.isnan(got) == np.isnan(want)).all()
+    assert (bits(got) == bits(want))[~np.isnan(want)].all()
 
 
 # more tiles in one direction than a second grid dimension holds (65535)
