@@ -16,6 +16,9 @@
 // last round would leave more than half of the SMs idle its units are split
 // into single 128-row tiles, one per CTA.
 //
+// Calls with a causal limit, and those of fewer units than SMs, go to
+// attention_tc_streams.cu (the rule and its figures are in attention_tc_plan).
+//
 // Twelve warps: 0 = TMA producer, 1 and 2 = MMA issuers of tile 0 and tile 1
 // (warp 1 owns the TMEM allocation), 3 idle, 4-7 = softmax for tile 0, 8-11 =
 // softmax for tile 1.  A softmax thread owns one query row (one TMEM lane): it
@@ -80,7 +83,6 @@ struct AttnParams {
     float *out;
     uint32_t bh, seq;
     float scale_log2;   // scale * log2(e)
-    uint32_t causal;
     uint32_t q_blocks;  // 256-row blocks per head
     uint32_t n_full;    // units of two tiles: indices [0, n_full)
     uint32_t n_half;    // single-tile units: indices [n_full, n_full + n_half), two per 256-row block
@@ -103,11 +105,8 @@ __device__ __forceinline__ bool unit_at(const AttnParams &p, uint32_t i, Unit &u
         return false;
     }
     u.head = block / p.q_blocks;
-    uint32_t qb = block % p.q_blocks;
-    if (p.causal) qb = p.q_blocks - 1 - qb;   // the longest key ranges first
-    u.q0 = qb * (QT * BQ) + sub * BQ;
-    const uint32_t kv_limit = p.causal ? min(p.seq, u.q0 + u.nt * BQ) : p.seq;
-    u.nkv = u.q0 < p.seq ? (kv_limit + BKV - 1) / BKV : 0;
+    u.q0 = block % p.q_blocks * (QT * BQ) + sub * BQ;
+    u.nkv = u.q0 < p.seq ? (p.seq + BKV - 1) / BKV : 0;
     return true;
 }
 
@@ -392,15 +391,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 ATTN_STAMP(tr, tslot + 2);
 
                 const uint32_t key0 = j * BKV;
-                const bool need_mask = (j * BKV + BKV > p.seq) || (p.causal && j * BKV + BKV - 1 > u.q0 + t * BQ);
+                const bool need_mask = j * BKV + BKV > p.seq;
                 if (need_mask) {
 #pragma unroll
                     for (int ch = 0; ch < NCH; ++ch) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const uint32_t key = key0 + ch * 32 + i;
-                            const bool valid = key < p.seq && (!p.causal || key <= qrow);
-                            if (!valid) s[ch][i] = 0xff800000u;  // -inf
+                            if (key0 + ch * 32 + i >= p.seq) s[ch][i] = 0xff800000u;  // -inf
                         }
                     }
                 }
@@ -563,10 +560,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 }  // namespace
 
+int32_t attention_streams_init_device();
+cudaError_t attention_streams_launch(cudaStream_t s, uint32_t grid, const CUtensorMap &tmQ, const CUtensorMap &tmK, const CUtensorMap &tmV,
+                                     const CUtensorMap &tmO, float *out, uint32_t bh, uint32_t seq, float scale_log2, uint32_t causal,
+                                     uint32_t *status);
+uint32_t attention_streams_smem();
+
 struct AttnTcPlan {
     CUtensorMap tmQ, tmK, tmV, tmO;
     AttnParams p;
     uint32_t grid;
+    uint32_t streams, causal;   // attention_tc_streams.cu takes the call
 };
 
 bool attention_tc_supported(const fe2o3_flash_attention_v1_args *a) {
@@ -593,25 +597,24 @@ int32_t attention_tc_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args *a
     if (st != FE2O3_OK) { delete plan; return st; }
     // Schedule: one CTA per SM; full rounds of two-tile units, and a last partial round that is split
     // into single tiles when that keeps every tile on its own CTA.
-    const uint32_t q_blocks = (a->seq + QT * BQ - 1) / (QT * BQ);
-    const uint32_t units = bh * q_blocks;
+    const uint32_t q_blocks = (uint32_t)(((uint64_t)a->seq + QT * BQ - 1) / (QT * BQ)), tiles = (uint32_t)(((uint64_t)a->seq + BQ - 1) / BQ);
+    const uint64_t units = (uint64_t)bh * q_blocks;
     const uint32_t sms = ctx->sm_count > 0 ? (uint32_t)ctx->sm_count : 1u;
-    uint32_t grid, n_full = units, n_half = 0;
-    if (2 * units <= sms) {
-        grid = 2 * units;
-        n_full = 0;
-        n_half = 2 * units;
-    } else {
-        grid = units < sms ? units : sms;
-        const uint32_t rem = units % grid;
-        if (rem != 0 && 2 * rem <= grid) {
-            n_full = units - rem;
-            n_half = 2 * rem;
-        }
-    }
-    plan->p = AttnParams{reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->scale * 1.4426950408889634f, a->causal,
-                         q_blocks, n_full, n_half, ctx->status_word};
+    const uint32_t grid = (uint32_t)(units < sms ? units : sms), rem = (uint32_t)(units % grid);
+    const bool split = rem != 0 && 2 * rem <= grid;
+    plan->p = AttnParams{reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->scale * 1.4426950408889634f,
+                         q_blocks, (uint32_t)(split ? units - rem : units), split ? 2 * rem : 0u, ctx->status_word};
     plan->grid = grid;
+    // Tiles or streams: what the longest SM does, in quarters of a step of two blocks (a block of a single tile takes three).
+    // A step of a stream unit takes 8 % more, which also stands for a unit being half as long (us, tiles / streams: B4 H16 S2048
+    // 105.6 / 110.5 with 240 / 224 quarters, B1 H16 S4096 104.5 / 118.7 with 256 / 256, B2 H12 S1900 49.2 / 47.5 with 105 / 96).
+    // Causal tiles are not dealt out by length, and few units leave SMs idle.
+    const uint64_t blocks = tiles;   // key blocks of 128
+    const uint64_t tile_cost = 4 * blocks * ((units - (split ? rem : 0)) / grid + (!split && rem != 0)) + (split ? 3 * blocks : 0);
+    const uint64_t stream_cost = 4 * (((uint64_t)bh * tiles + sms - 1) / sms) * ((blocks + 1) / 2);
+    plan->causal = a->causal;
+    plan->streams = a->causal || units < sms || 25 * tile_cost > 27 * stream_cost;
+    if (plan->streams) plan->grid = (uint64_t)bh * tiles < sms ? bh * tiles : sms;
     *out = plan;
     return FE2O3_OK;
 }
@@ -619,19 +622,22 @@ int32_t attention_tc_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args *a
 // Function attributes are per device: called by fe2o3_ctx_create with the context's device current.
 int32_t attention_tc_init_device() {
     FE2O3_CUDA(cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal));
-    return FE2O3_OK;
+    return attention_streams_init_device();
 }
 
 int32_t attention_tc_launch(const AttnTcPlan *plan, cudaStream_t s) {
     if (plan->grid == 0) return FE2O3_OK;
-    const cudaError_t e = fe2o3_launch_early(attention_tc_kernel, plan->grid, kThreads, kSmemTotal, s, 1, plan->tmQ, plan->tmK, plan->tmV,
-                                             plan->tmO, plan->p);
+    const cudaError_t e =
+        plan->streams ? attention_streams_launch(s, plan->grid, plan->tmQ, plan->tmK, plan->tmV, plan->tmO, plan->p.out, plan->p.bh, plan->p.seq,
+                                                 plan->p.scale_log2, plan->causal, plan->p.status)
+                      : fe2o3_launch_early(attention_tc_kernel, plan->grid, kThreads, kSmemTotal, s, 1, plan->tmQ, plan->tmK, plan->tmV,
+                                           plan->tmO, plan->p);
     fe2o3_count_launch(1);
     return fe2o3_cuda_status(e, "flash_attention_v1(tcgen05)");
 }
 
 void attention_tc_geometry(const AttnTcPlan *plan, fe2o3_geometry *geo) {
-    *geo = fe2o3_geometry{{plan->grid, 1, 1}, {kThreads, 1, 1}, kSmemTotal, 1};
+    *geo = fe2o3_geometry{{plan->grid, 1, 1}, {kThreads, 1, 1}, plan->streams ? attention_streams_smem() : kSmemTotal, 1};
 }
 
 void attention_tc_free(AttnTcPlan *plan) { delete plan; }

@@ -423,6 +423,24 @@ def attention_f64(q, k, v, scale, causal):
     return w @ v.astype(np.float64) / w.sum(-1, keepdims=True), np.abs(scores[np.isfinite(scores)]).max()
 
 
+# ---- attention at head size 64: units of two tiles, or of two streams, by the number of units, the length and the limit
+@pytest.mark.parametrize("B,H,S,causal", [(1, 1, 1, False), (1, 2, 128, True), (1, 3, 129, False), (1, 2, 257, True), (1, 1, 640, False),
+                                          (1, 147, 200, False), (1, 148, 200, False), (4, 40, 300, False), (4, 40, 300, True),
+                                          (1, 100, 600, False), (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False)])
+def test_attention_bf16_tiles_and_streams(gpu, B, H, S, causal):
+    from fe2o3_b200 import synth
+    from test_gpu_parity import attn_run
+    fe = gpu[0]
+    D = 64
+    q, k, v = (synth.normal_bf16(5, d, B * H * S * D, 1.0).reshape(B, H, S, D) for d in (1, 2, 3))
+    got, _ = attn_run(gpu, q, k, v, 1.0 / np.sqrt(D), causal, fe.DTYPE_BF16)
+    q32, k32, v32 = (synth.bf16_to_f32(x).reshape(B * H, S, D) for x in (q, k, v))
+    want, _ = attention_f64(q32, k32, v32, 1.0 / np.sqrt(D), causal)
+    size, _ = attention_f64(q32, k32, np.abs(v32), 1.0 / np.sqrt(D), causal)
+    # a probability is cut to eight bits, by less than 2^-7 of itself, and the centring gives back 2^-9
+    assert (np.abs(got.reshape(want.shape) - want) <= 2.0 ** -7 * size).all()
+
+
 @pytest.mark.parametrize("S,D,causal", [(333, 128, True), (1025, 72, False), (1900, 128, True), (1900, 48, False), (4096, 128, False)])
 def test_attention_split_error_is_not_above_the_cuda_cores(gpu, S, D, causal):
     """The tensor core truncates its running sum at every accumulation; the kernel may not let that build up over a row.
