@@ -18,9 +18,16 @@
 //   bits stay in registers.
 //   Rows of up to 64 columns share a warp (8 or 16 lanes a row), otherwise most
 //   lanes of the warp would idle.
+//   There is a build for every number of vectors a thread: what a row does not need
+//   costs instructions (5000 rows of 3001 columns are as much issue time as traffic) and
+//   registers, hence blocks an SM.
 // 65536 x 1024: 91.6 us -> 79.5 us (6.75 TB/s) against the earlier form that kept
-// activity bits per element; 5000 x 3001 masked: 79.9 -> 29.7 us against one block
-// per row with scalar accesses, four block barriers and a division per element.
+// activity bits per element; 5000 x 3001 masked: 79.9 -> 29.3 us against one block
+// per row with scalar accesses, four block barriers and a division per element, and
+// -> 24.9 (5.4 TB/s) with six vectors a thread instead of eight (25.5) and the tests for
+// the row's ends and for finite inputs only where they are needed; 8000 x 2560 28.3 -> 25.5,
+// 20000 x 701 22.6 -> 19.4.  Two warps a row of 3001 with twelve vectors a thread take 26.9,
+// one with 24 takes 39.
 // Input, output and mask that are not aligned to one another (views at different
 // offsets) take one block per row with scalar accesses.
 #include "common.cuh"
@@ -77,13 +84,18 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
     const uint8_t *msk = MASKED ? mask + base - shift : nullptr;
     const uint32_t end = shift + cols;
 
+    // No thread has vectors to spare (launch_row_softmax), so only the first and the last ones can straddle an end of the row or
+    // lie outside it; shifted rows may end one vector earlier.  (Aligned rows under a mask keep the test at every vector:
+    // without it the compiler takes other registers, and 16384 x 2000 goes from 45.5 to 47.5 us.)
+    auto inside = [](int i) { return SHIFTED ? i > 0 && i < NV - 2 : !MASKED && i < NV - 1; };
     float4 v[NV];
+    float poison = 0.f;   // NaN once an input was not finite
     bool ok = true;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const uint32_t e = (i * LANES + lane) * 4;
-        v[i] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-        const bool whole = SHIFTED ? e >= shift && e + 4 <= end : e < end;
+        v[i] = SHIFTED ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        const bool whole = inside(i) || (SHIFTED ? e >= shift && e + 4 <= end : e < end);
         if (whole) {
             v[i] = __ldcs(reinterpret_cast<const float4 *>(src + e));
         } else if (SHIFTED && e < end) {   // straddles an end of the row (e + 4 > shift always: shift < 4)
@@ -99,7 +111,7 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
         for (int i = 0; i < NV; ++i) {
             const uint32_t e = (i * LANES + lane) * 4;
             m4[i] = 0;
-            const bool whole = SHIFTED ? e >= shift && e + 4 <= end : e < end;
+            const bool whole = inside(i) || (SHIFTED ? e >= shift && e + 4 <= end : e < end);
             if (whole) {
                 m4[i] = *reinterpret_cast<const uint32_t *>(msk + e);
             } else if (SHIFTED && e < end) {
@@ -113,11 +125,17 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const uint32_t e = (i * LANES + lane) * 4;
-        if (!SHIFTED) {
-            ok = ok && (e >= end || finite4(v[i]));
-        } else {   // the filler outside the row is not an input
-            ok = ok && (e + 0 < shift || e + 0 >= end || isfinite(v[i].x)) && (e + 1 < shift || e + 1 >= end || isfinite(v[i].y)) &&
-                 (e + 2 < shift || e + 2 >= end || isfinite(v[i].z)) && (e + 3 >= end || isfinite(v[i].w));
+        if (SHIFTED) {   // what lies outside the row was filled with zeros
+            poison = fmaf(v[i].x, 0.f, fmaf(v[i].y, 0.f, fmaf(v[i].z, 0.f, fmaf(v[i].w, 0.f, poison))));
+            const bool whole = inside(i) || (e >= shift && e + 4 <= end);
+            if (!MASKED && !whole) {   // (the mask's words hold zeros there)
+                if (e + 0 < shift || e + 0 >= end) v[i].x = -INFINITY;
+                if (e + 1 < shift || e + 1 >= end) v[i].y = -INFINITY;
+                if (e + 2 < shift || e + 2 >= end) v[i].z = -INFINITY;
+                if (e + 3 < shift || e + 3 >= end) v[i].w = -INFINITY;
+            }
+        } else {
+            ok = ok && (inside(i) || e < end ? finite4(v[i]) : true);
         }
         if (MASKED) {
             if ((m4[i] & 0xffu) == 0) v[i].x = -INFINITY;
@@ -130,7 +148,7 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
     const uint32_t barrier = 1 + local;
     float *slots = &s_red[0][0] + local * (LANES / 32);
     // a non-finite input anywhere in the row travels with the maximum, as +inf, which no row of finite inputs has
-    mx = row_combine<LANES>(ok ? mx : INFINITY, [](float a, float b) { return fmaxf(a, b); }, slots, barrier);
+    mx = row_combine<LANES>(ok && poison == 0.f ? mx : INFINITY, [](float a, float b) { return fmaxf(a, b); }, slots, barrier);
     const bool good = mx != INFINITY && mx != -INFINITY;   // -inf: no active element
     float sum = 0.f;
     if (good) {
@@ -158,7 +176,7 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const uint32_t e = (i * LANES + lane) * 4;
-        const bool whole = SHIFTED ? e >= shift && e + 4 <= end : e < end;
+        const bool whole = inside(i) || (SHIFTED ? e >= shift && e + 4 <= end : e < end);
         const float4 r = make_float4(quotient(v[i].x), quotient(v[i].y), quotient(v[i].z), quotient(v[i].w));
         if (whole) {
             __stcs(reinterpret_cast<float4 *>(dst + e), r);
@@ -282,7 +300,23 @@ int32_t launch_row_softmax(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2
                 else e = launch_row<32, 1>(a, shifted, s, grid, st);
                 break;
             case 2: e = launch_row<32, 2>(a, shifted, s, grid, st); break;
-            case 3: case 4: e = launch_row<32, 4>(a, shifted, s, grid, st); break;
+            case 3: e = launch_row<32, 3>(a, shifted, s, grid, st); break;
+            case 4: e = launch_row<32, 4>(a, shifted, s, grid, st); break;
+            case 5:
+                if (lanes == 32) e = launch_row<32, 5>(a, shifted, s, grid, st);
+                else if (lanes == 64) e = launch_row<64, 5>(a, shifted, s, grid, st);
+                else e = launch_row<128, 5>(a, shifted, s, grid, st);
+                break;
+            case 6:
+                if (lanes == 32) e = launch_row<32, 6>(a, shifted, s, grid, st);
+                else if (lanes == 64) e = launch_row<64, 6>(a, shifted, s, grid, st);
+                else e = launch_row<128, 6>(a, shifted, s, grid, st);
+                break;
+            case 7:
+                if (lanes == 32) e = launch_row<32, 7>(a, shifted, s, grid, st);
+                else if (lanes == 64) e = launch_row<64, 7>(a, shifted, s, grid, st);
+                else e = launch_row<128, 7>(a, shifted, s, grid, st);
+                break;
             case 9: e = launch_row<128, 9>(a, shifted, s, grid, st); break;   // up to 1025 vectors: 4095 columns at phase 3
             default:
                 if (lanes == 32) e = launch_row<32, 8>(a, shifted, s, grid, st);

@@ -365,6 +365,28 @@ def test_row_softmax_widths(gpu, orc, cols):
     assert (bits(got[~mask]) == 0).all()
 
 
+# every number of vectors a thread, at its fewest and most columns, aligned and not; a bad row's neighbours share its vectors
+@pytest.mark.parametrize("cols", [c for lanes, nvs in ((32, range(2, 9)), (64, range(5, 9)), (128, range(5, 9))) for nv in nvs
+                                  for c in (4 * lanes * (nv - 1) + 4, 4 * lanes * nv - 3, 4 * lanes * nv)])
+def test_row_softmax_vectors_a_thread(gpu, orc, cols):
+    from fe2o3_b200 import synth
+    fe, ctx, stream = gpu
+    rows = 9
+    x = synth.normal_f32(2, 70 + cols, rows * cols, 2.0).reshape(rows, cols)
+    x[4, 0] = x[4, cols - 1] = np.inf
+    good = [r for r in range(rows) if r != 4]
+    for mask in (None, (synth.u32_below(2, 6000 + cols, rows * cols, 4) != 0).reshape(rows, cols)):
+        i, o = Guarded(fe, stream, x), Guarded(fe, stream, np.full(x.size, -1, np.float32))
+        m = Guarded(fe, stream, mask.astype(np.uint8)) if mask is not None else None
+        p = fe.prepare(ctx, "row_softmax_v1", input=i.slice, output=o.slice, mask=m.slice if m else None, rows=rows, cols=cols)
+        with pytest.raises(fe.Fe2o3Error):
+            p.launch_and_wait(stream)
+        got = o.read().reshape(rows, cols)
+        _, want = orc.row_softmax(x[good], None if mask is None else mask[good])
+        assert (np.abs(got[good] - want) <= 1e-5 * np.abs(want)).all()
+        assert (got[4] == -1).all()
+
+
 @pytest.mark.parametrize("cols", [20, 64, 1000, 1023, 4095])
 @pytest.mark.parametrize("in_at,out_at", [(1, 1), (2, 3)])   # the same phase in a vector, and different ones
 def test_row_softmax_views_and_bad_rows(gpu, orc, cols, in_at, out_at):
