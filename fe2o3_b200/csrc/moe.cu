@@ -615,9 +615,97 @@ moe_gate_chain_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict
     if (tok0 + tt < tokens) logits[(uint64_t)(tok0 + tt) * E + e] = acc;
 }
 
-// Shared memory that a launch of the chain kernel may ask for beside its own (see launch_moe_gate).  The limit without
+// ---- gate logits of a small batch: one chain per lane, fed by four warps of products ------------
+// The same arithmetic and order.  While no SM has more than one block, the kernel above takes 8.6 cycles a k where the
+// additions take 4.2, because one warp also widens, reads both operands and multiplies.  Here the warp that adds does
+// nothing else: a 16-byte read for four additions, asked for sixteen k ahead.  Four warps beside it stream a quarter of a
+// chunk each of the block's tokens and of Wg into a ring with asynchronous copies, a lane a k, multiply all 32 pairs of
+// that k and leave them in shared memory, a chunk ahead of the sums.  Chunks are long (128 k) because each begins with a
+// barrier and the latency of a read.  Warp 4 has nothing to do: it would share a scheduler and its instruction cache with the
+// chain.  us a launch, d_model 2048, 64 tokens of 8 experts: 7.1 (5.5 cycles a k); 7.6 with warp 4 for warp 5, 7.8 with the
+// operands widened instead of multiplied, 8.4 with one product a read and two warps, 10.3 in the kernel above.
+template <int E>
+__global__ void __launch_bounds__(192)
+moe_gate_fed_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ wg, float *__restrict__ logits,
+                    uint32_t tokens, uint32_t d_model) {
+    constexpr int KC = 128, PART = KC / 4, STAGES = E == 16 ? 3 : 4, TPW = 32 / E;
+    constexpr int kXG = TPW * PART / 8, kWG = PART * E / 8;   // 16-byte pieces of a quarter of a chunk of x and of Wg
+    __shared__ __align__(16) uint4 ring[4][STAGES][kXG + kWG];
+    __shared__ __align__(16) float products[2][32][KC + 4];   // rows are padded for the 16-byte reads
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tok0 = blockIdx.x * TPW;
+    const uint32_t nchunks = (d_model + KC - 1) / KC;   // the last one may be a half
+    // named barriers of the whole block: 1, 2 = a buffer of products is written; 3, 4 = it has been added up
+    auto meet = [](uint32_t id) { asm volatile("bar.sync %0, 160;" ::"r"(id) : "memory"); };
+    begin_after_previous();
+    if (warp == 0) {
+        float acc = 0.0f;
+        auto add_up = [&](const float4 *p) {
+            constexpr int A = 4;   // reads ahead of the sums
+            float4 v[A + 1];
+#pragma unroll
+            for (int k = 0; k < A; ++k) v[k] = p[k];
+#pragma unroll
+            for (int k = 0; k < KC / 8; ++k) {
+                if (k + A < KC / 8) v[(k + A) % (A + 1)] = p[k + A];
+                const float4 &q = v[k % (A + 1)];
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, q.x), q.y), q.z), q.w);
+            }
+        };
+        for (uint32_t c = 0; c < nchunks; ++c) {
+            meet(1 + (c & 1));
+            const float4 *p = reinterpret_cast<const float4 *>(products[c & 1][lane]);
+            add_up(p);
+            if (c * KC + KC / 2 < d_model) add_up(p + KC / 8);
+            if (c + 2 < nchunks) asm volatile("bar.arrive %1, 160;" : "+f"(acc) : "r"(3 + (c & 1)) : "memory");
+        }
+        if (tok0 + lane / E < tokens) logits[(uint64_t)(tok0 + lane / E) * E + lane % E] = acc;
+        return;
+    }
+    if (warp == 4) return;   // would share the scheduler and its instruction cache with the chain
+    const uint32_t part = warp < 4 ? warp - 1 : 3;
+    auto copy = [&](uint32_t c) {
+        const uint32_t k0 = c * KC + part * PART;
+        if (k0 < d_model) {
+            uint4 *stage = ring[part][c % STAGES];
+#pragma unroll
+            for (int i = 0; i < (kXG + kWG + 31) / 32; ++i) {
+                const uint32_t g = i * 32 + lane, gx = g - kWG;
+                if (g < (uint32_t)kWG) cp_async_16(stage + g, wg + (uint64_t)k0 * E + g * 8);
+                else if (gx < (uint32_t)kXG)   // rows beyond the batch re-read the last row
+                    cp_async_16(stage + g, x + (uint64_t)min(tok0 + gx / (PART / 8), tokens - 1) * d_model + k0 + gx % (PART / 8) * 8);
+            }
+        }
+        cp_async_commit();   // an empty group keeps the group count uniform at the tail
+    };
+#pragma unroll
+    for (int c = 0; c < STAGES - 1; ++c) copy(c);
+    for (uint32_t c = 0; c < nchunks; ++c) {
+        cp_async_wait<STAGES - 2>();    // this lane's pieces of chunk c have landed
+        __syncwarp();                   // everybody's have, and everybody has read chunk c - 1
+        copy(c + STAGES - 1);           // into the stage of chunk c - 1
+        const uint4 *stage = ring[part][c % STAGES];
+        const uint32_t *wr = reinterpret_cast<const uint32_t *>(stage) + lane * (E / 2);
+        const uint16_t *xr = reinterpret_cast<const uint16_t *>(stage + kWG) + lane;
+        float w[E], xv[TPW];
+#pragma unroll
+        for (int e = 0; e < E / 2; ++e) {
+            w[2 * e] = __uint_as_float(wr[e] << 16);
+            w[2 * e + 1] = __uint_as_float(wr[e] & 0xffff0000u);
+        }
+#pragma unroll
+        for (int t = 0; t < TPW; ++t) xv[t] = __uint_as_float((uint32_t)xr[t * PART] << 16);
+        if (c >= 2) meet(3 + (c & 1));
+        float *column = &products[c & 1][0][part * PART + lane];
+#pragma unroll
+        for (int o = 0; o < 32; ++o) column[o * (KC + 4)] = __fmul_rn(xv[o / E], w[o % E]);   // (past d_model: not read)
+        asm volatile("bar.arrive %0, 160;" ::"r"(1 + (c & 1)) : "memory");
+    }
+    cp_async_wait<0>();
+}
+
+// Shared memory that a launch of the two kernels above may ask for beside its own (see launch_moe_gate).  The limit without
 // opt-in, 48 KiB, is for both together, so the opt-in is made for every size: 35 KiB beside 18 of its own are refused too.
-constexpr uint32_t kGateSpreadMax = 192u * 1024u;
+constexpr uint32_t kGateSpreadMax = 192u * 1024u, kGateFedSpreadMax = 176u * 1024u;
 
 // ---- top-2 routing over many blocks --------------------------------------------
 // Same result as moe_top2_kernel.  Block b owns tokens [256 b, 256 b + 256).
@@ -1048,8 +1136,11 @@ moe_combine_kernel(const float *__restrict__ compact, const uint32_t *__restrict
 // Function attributes are per device: called by fe2o3_ctx_create with the context's device current.
 int32_t moe_gate_init_device() {
     FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_fed_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateFedSpreadMax));
     FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_fed_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateFedSpreadMax));
     FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_chain_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(moe_gate_fed_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGateFedSpreadMax));
     return FE2O3_OK;
 }
 
@@ -1075,19 +1166,25 @@ int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_
             const bool wide = (uint64_t)a->tokens * E > 65536u;
             auto one_chain = E == 4 ? moe_gate_chain_kernel<4> : E == 8 ? moe_gate_chain_kernel<8> : moe_gate_chain_kernel<16>;
             const uint32_t chain_grid = ceil_div_u32(a->tokens, 32 / E);
+            // Up to one block an SM the products come from warps of their own; beyond, the blocks of an SM share its shared memory
+            // and the issue slots (d 2048, 8 experts, one warp / products, us: 64 tokens 10.3 / 7.1, 590 tokens 10.5 / 7.2; an earlier
+            // form of it at 1024 10.6 / 10.5, at 4096 20.8 / 28.4)
+            const bool fed = chain_grid <= (uint32_t)ctx->sm_count;
+            if (fed) one_chain = E == 4 ? moe_gate_fed_kernel<4> : E == 8 ? moe_gate_fed_kernel<8> : moe_gate_fed_kernel<16>;
+            const uint32_t threads = fed ? 192u : 32u;
 #define FE2O3_GATE_LANES(EE, g) launch_gate_lanes<EE, 4, 8, 6>(s, x, wg, lg, a->tokens, a->d_model, g)
             // Launched early, the blocks would pile up on the first SMs that the kernel before leaves (twelve to an SM:
             // 107 against 94 us a pass of 512 tokens): they ask for so much shared memory that they spread evenly.
             const uint32_t per_sm = ceil_div_u32(chain_grid, (uint32_t)ctx->sm_count);
-            const uint32_t own = E == 16 ? 29u : 20u;   // KiB of its own, with what each block reserves
-            const uint32_t spread = 220u / per_sm > own ? min((220u / per_sm - own) * 1024u, kGateSpreadMax) : 0u;
-            fe2o3_geometry g{{chain_grid, 1, 1}, {32, 1, 1}, wide ? 0u : spread, 1};
+            const uint32_t own = fed ? 48u : E == 16 ? 29u : 20u;   // KiB of its own, with what each block reserves
+            const uint32_t spread = 220u / per_sm > own ? min((220u / per_sm - own) * 1024u, fed ? kGateFedSpreadMax : kGateSpreadMax) : 0u;
+            fe2o3_geometry g{{chain_grid, 1, 1}, {wide ? 32u : threads, 1, 1}, wide ? 0u : spread, 1};
             cudaError_t e = cudaSuccess;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, &g) : E == 8 ? FE2O3_GATE_LANES(8, &g) : FE2O3_GATE_LANES(16, &g);
             if (geo) *geo = g;
             if (plan_only) return FE2O3_OK;
             if (wide) e = E == 4 ? FE2O3_GATE_LANES(4, nullptr) : E == 8 ? FE2O3_GATE_LANES(8, nullptr) : FE2O3_GATE_LANES(16, nullptr);
-            else e = fe2o3_launch_early(one_chain, chain_grid, 32, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
+            else e = fe2o3_launch_early(one_chain, chain_grid, threads, spread, s, 1, x, wg, lg, a->tokens, a->d_model);
 #undef FE2O3_GATE_LANES
             if (e != cudaSuccess) return fe2o3_cuda_status(e, "moe_gate_v1");
             fe2o3_count_launch(1);

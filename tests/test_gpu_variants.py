@@ -222,6 +222,20 @@ print("ok")
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
 
 
+# ---- gate fed by warps of products: half chunks, one block to one per SM (148) and the first count beyond
+@pytest.mark.parametrize("d", [64, 128, 192, 448, 2048])
+@pytest.mark.parametrize("T,E", [(1, 4), (9, 4), (1, 8), (5, 8), (592, 8), (593, 8), (3, 16), (296, 16), (297, 16)])
+def test_moe_gate_small_batches_bit_exact(gpu, orc, T, E, d):
+    from fe2o3_b200 import synth
+    fe, ctx, stream = gpu
+    if d * E * 4 > 96 * 1024:
+        d = 1472
+    x, wg = synth.normal_bf16(4, d, T * d, 1.0), synth.normal_bf16(4, d + 1, d * E, 0.1)
+    X, W, L = Guarded(fe, stream, x), Guarded(fe, stream, wg), Guarded(fe, stream, np.full(T * E, np.nan, np.float32))
+    run(fe, ctx, stream, "moe_gate_v1", x=X.slice, wg=W.slice, logits=L.slice, tokens=T, d_model=d, experts=E)
+    assert (bits(L.read()) == bits(orc.moe_gate_logits(x, wg, T, d, E))).all()
+
+
 # ---- routing in one launch: one warp to eight blocks of two passes, and the sizes around each step
 @pytest.mark.parametrize("T,E,cap,bad", [(1, 2, 1, 0), (33, 8, 100, 0), (1000, 5, 300, 0), (1024, 16, 2048, 0), (1025, 8, 200, 0),
                                          (2049, 32, 4098, 0), (4097, 8, 900, 0), (8192, 8, 2100, 0), (8193, 16, 16386, 0),
