@@ -22,6 +22,7 @@
 // range, so a fused multiply-add rounds just as a product and a sum do: where every value of a tile is zero or between
 // 2^-62 and 2^63 the fused form is used, which halves the work of the pipe; other tiles take the two-step form.
 // us, alpha/beta, always two steps / so: 2999^3 at odd addresses 2299 / 1445, 300 x 1001 x 501 55 / 33, 100^3 13.0 / 5.3.
+#include "bf16_piece.h"
 #include "common.cuh"
 
 namespace {
@@ -228,30 +229,14 @@ gemm_exact_f32_kernel(const float *__restrict__ A, const float *__restrict__ B, 
 }
 
 // ---- bf16 operands: widened on the way through registers
-// Four consecutive elements of a row as the aligned words that hold at least one of them each: two, or three from the middle
-// of the first (true then).  They are put together only when they are stored: until then nothing waits for them.
-__device__ __forceinline__ bool load4(uint32_t (&w)[3], const uint16_t *row, uint32_t first, uint32_t end, bool row_ok, bool vec) {
-    if (row_ok && first + 4 <= end) {
-        if (vec) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(row + first));
-            w[0] = v.x; w[1] = v.y;
-            return false;
-        }
-        const uintptr_t at = reinterpret_cast<uintptr_t>(row + first);
-        const uint32_t *words = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3));
-        w[0] = __ldg(words);
-        w[1] = __ldg(words + 1);
-        if ((at & 2u) == 0) return false;
-        w[2] = __ldg(words + 2);
-        return true;
+struct GlobalPieces {
+    static __device__ __forceinline__ uint32_t half(const uint16_t *p) { return __ldg(p); }
+    static __device__ __forceinline__ uint32_t word(const uint16_t *p) { return __ldg(reinterpret_cast<const uint32_t *>(p)); }
+    static __device__ __forceinline__ void two_words(const uint16_t *p, uint32_t &a, uint32_t &b) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+        a = v.x; b = v.y;
     }
-    uint32_t v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = row_ok && first + i < end ? row[first + i] : 0u;
-    w[0] = v[0] | v[1] << 16;
-    w[1] = v[2] | v[3] << 16;
-    return false;
-}
+};
 
 template <int RM, int RN, bool EPILOGUE>
 __global__ void __launch_bounds__(kThreads)
@@ -271,12 +256,12 @@ gemm_exact_bf16_kernel(const uint16_t *__restrict__ A, const uint16_t *__restric
         for (int i = 0; i < GA; ++i) {
             const uint32_t g = i * kThreads + tid, r = g / (TK / 4), k = g % (TK / 4) * 4;
             const bool in = row0 + r < M;
-            halves |= (uint32_t)load4(a_next[i], A + (uint64_t)(in ? row0 + r : 0) * lda, k0 + k, K, in, vec_a) << i;
+            halves |= (uint32_t)load_piece<GlobalPieces>(a_next[i], A + (uint64_t)(in ? row0 + r : 0) * lda, k0 + k, K, in, vec_a) << i;
         }
 #pragma unroll
         for (int i = 0; i < GB; ++i) {
             const uint32_t g = i * kThreads + tid, k = k0 + g / (TN / 4), c = g % (TN / 4) * 4;
-            halves |= (uint32_t)load4(b_next[i], B + (uint64_t)(k < K ? k : 0) * ldb, col0 + c, N, k < K, vec_b) << (GA + i);
+            halves |= (uint32_t)load_piece<GlobalPieces>(b_next[i], B + (uint64_t)(k < K ? k : 0) * ldb, col0 + c, N, k < K, vec_b) << (GA + i);
         }
     };
     // Returns whether a product with one of the values may not be exact: exponents other than that of zero and those
@@ -284,7 +269,8 @@ gemm_exact_bf16_kernel(const uint16_t *__restrict__ A, const uint16_t *__restric
     auto stage = [&](uint32_t st) {
         uint32_t least = 0xffffffffu, most = 0u;
         auto put = [&](float *dst, const uint32_t (&w)[3], bool half) {
-            const uint32_t x = half ? __byte_perm(w[0], w[1], 0x5432) : w[0], y = half ? __byte_perm(w[1], w[2], 0x5432) : w[1];
+            uint32_t x, y;
+            join_piece(w, half, x, y);
             const uint32_t v[4] = {x << 16, x & 0xffff0000u, y << 16, y & 0xffff0000u};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
