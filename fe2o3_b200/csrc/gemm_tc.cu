@@ -712,17 +712,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             } else if constexpr (is_gelu(KIND)) {
                 // ---- GELU, bf16 output: 64 columns to a 128-byte group, 16 at a time.  The loops stay rolled: a block of a
                 // small batch runs this code once, and waits for its instructions (unrolled: 2 us more a pass of 64 tokens).
-                uint32_t r[16];
-                tmem_ld_32x32b_x16(taddr, r);
+                // The next 16 columns are on their way meanwhile, and are there before the loop goes back: registers that a
+                // load has yet to fill may not be copied from.
+                uint32_t x[16];
+                tmem_ld_32x32b_x16(taddr, x);
+                tmem_ld_wait_for(x);
 #pragma unroll 1
                 for (int q = 0; q < BN / 32; ++q) {
                     const uint32_t at = (q & 3) * 2;   // 16-byte pieces of the group
-                    uint32_t x[16], w[8];
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) x[i] = r[i];
-                    if (q + 1 < BN / 32) {
-                        tmem_ld_32x32b_x16(taddr + (q + 1) * 16, r);
+                    const bool more = q + 1 < BN / 32;
+                    uint32_t next[16], w[8];
+                    if (more) {
+                        tmem_ld_32x32b_x16(taddr + (q + 1) * 16, next);
                     } else {   // the accumulator has been read completely
                         tc_fence_before();
                         __syncwarp();
@@ -730,6 +731,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     gelu_pairs<4>(x, w);
                     gelu_pairs<4>(x + 8, w + 4);
+                    if (more) {
+                        tmem_ld_wait_for(next);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) x[i] = next[i];
+                    }
                     if (at == 0) {   // the slice has been read out
                         if (store_pending && lane == 0) tma_store_wait_read();
                         __syncwarp();
