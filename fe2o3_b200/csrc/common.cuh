@@ -275,7 +275,9 @@ __device__ __forceinline__ uint32_t ready_stages(uint64_t *bars, uint32_t stage,
     uint32_t at = stage + lane;
     if (at >= S) { at -= S; parity ^= 1; }
     const bool ready = lane < min(limit, (uint32_t)S) && mbar_test(&bars[at], parity);
-    return __ffs(~__ballot_sync(0xffffffffu, ready)) - 1;
+    const uint32_t n = __ffs(~__ballot_sync(0xffffffffu, ready)) - 1;
+    __syncwarp();   // what a lane saw complete is complete for the one that issues: a ballot orders no memory
+    return n;
 }
 // Arrival with a count: stands in for `n` parties at once.
 __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
