@@ -16,8 +16,8 @@
 // last round would leave more than half of the SMs idle its units are split
 // into single 128-row tiles, one per CTA.
 //
-// Calls with a causal limit, and those of fewer units than SMs, go to
-// attention_tc_streams.cu (the rule and its figures are in attention_tc_plan).
+// Calls with a causal limit, and those whose two-tile units would leave SMs
+// idle, go to attention_tc_streams.cu (the rule and its figures are in attention_tc_plan).
 //
 // Twelve warps: 0 = TMA producer, 1 and 2 = MMA issuers of tile 0 and tile 1
 // (warp 1 owns the TMEM allocation), 3 idle, 4-7 = softmax for tile 0, 8-11 =
@@ -605,15 +605,22 @@ int32_t attention_tc_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args *a
     plan->p = AttnParams{reinterpret_cast<float *>(a->output.ptr), bh, a->seq, a->scale * 1.4426950408889634f,
                          q_blocks, (uint32_t)(split ? units - rem : units), split ? 2 * rem : 0u, ctx->status_word};
     plan->grid = grid;
-    // Tiles or streams: what the longest SM does, in quarters of a step of two blocks (a block of a single tile takes three).
-    // A step of a stream unit takes 8 % more, which also stands for a unit being half as long (us, tiles / streams: B4 H16 S2048
-    // 105.6 / 110.5 with 240 / 224 quarters, B1 H16 S4096 104.5 / 118.7 with 256 / 256, B2 H12 S1900 49.2 / 47.5 with 105 / 96).
-    // Causal tiles are not dealt out by length, and few units leave SMs idle.
+    // Tiles or streams: with a causal limit always streams, for tiles are not dealt out by length; without one the cheaper by a
+    // cost of the launch and, on the SM that has most, of each unit and its key blocks.  Fitted in ns to 139 calls of 64 to
+    // 4096 keys, both kernels each: the choice is within 0.1 % of the better one on average, 3 % at worst.
+    // A stream unit is half of a two-tile unit and takes more than half of its time, so tiles win where the rounds come out
+    // even and streams where tiles would leave SMs idle.  One whole key block a head is all beginning and end, of which a
+    // tile has less (masked keys cost it more, below 128 keys streams are ahead again).
+    // us, tiles / streams: B1 H16 S2048 29.8 / 33.7, B4 H16 S2048 105.6 / 110.5, 118 heads of 256 keys 8.5 / 10.5,
+    // 18 heads of 1900 28.6 / 32.4, 24 of them 48.2 / 47.0, 5 of them 27.2 / 17.7, 162 heads of 300 23.0 / 20.5,
+    // 2 heads of 128 5.4 / 5.9, of 127 6.6 / 6.1.
     const uint64_t blocks = tiles;   // key blocks of 128
-    const uint64_t tile_cost = 4 * blocks * ((units - (split ? rem : 0)) / grid + (!split && rem != 0)) + (split ? 3 * blocks : 0);
-    const uint64_t stream_cost = 4 * (((uint64_t)bh * tiles + sms - 1) / sms) * ((blocks + 1) / 2);
+    const uint64_t full = (units - (split ? rem : 0)) / grid + (!split && rem != 0), rounds = ((uint64_t)bh * tiles + sms - 1) / sms;
+    const uint64_t tile_cost = 2000 + full * (2900 + 1560 * blocks) + (split ? 1300 + 1200 * blocks : 0);
+    const uint64_t stream_cost = 3500 + rounds * (2000 + 830 * blocks);
+    const bool one_whole_block = a->seq == BKV && units <= sms;
     plan->causal = a->causal;
-    plan->streams = a->causal || units < sms || 25 * tile_cost > 27 * stream_cost;
+    plan->streams = a->causal || (stream_cost < tile_cost && !one_whole_block);
     if (plan->streams) plan->grid = (uint64_t)bh * tiles < sms ? bh * tiles : sms;
     *out = plan;
     return FE2O3_OK;

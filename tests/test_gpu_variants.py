@@ -462,7 +462,11 @@ def attention_f64(q, k, v, scale, causal):
 # ---- attention at head size 64: units of two tiles, or of two streams, by the number of units, the length and the limit
 @pytest.mark.parametrize("B,H,S,causal", [(1, 1, 1, False), (1, 2, 128, True), (1, 3, 129, False), (1, 2, 257, True), (1, 1, 640, False),
                                           (1, 147, 200, False), (1, 148, 200, False), (4, 40, 300, False), (4, 40, 300, True),
-                                          (1, 100, 600, False), (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False)])
+                                          (1, 100, 600, False), (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False),
+                                          # two-tile units of which the last few are split into single tiles
+                                          (1, 150, 200, False), (3, 50, 512, False),
+                                          # one whole key block
+                                          (1, 2, 128, False), (1, 100, 128, False)])
 def test_attention_bf16_tiles_and_streams(gpu, B, H, S, causal):
     from fe2o3_b200 import synth
     from test_gpu_parity import attn_run
@@ -475,6 +479,31 @@ def test_attention_bf16_tiles_and_streams(gpu, B, H, S, causal):
     size, _ = attention_f64(q32, k32, np.abs(v32), 1.0 / np.sqrt(D), causal)
     # a probability is cut to eight bits, by less than 2^-7 of itself, and the centring gives back 2^-9
     assert (np.abs(got.reshape(want.shape) - want) <= 2.0 ** -7 * size).all()
+    # ... which leaves 2^-9 - 2^-7 U / m of it, U uniform in [0, 1) and m log-uniform in [1, 2): 1.95e-3 root mean square, 3.3e-3
+    # without the centring.  Independent from key to key, these add up in squares.
+    scores = q32.astype(np.float64) @ k32.astype(np.float64).transpose(0, 2, 1) / np.sqrt(D)
+    if causal:
+        scores[:, np.triu(np.ones((S, S), bool), 1)] = -np.inf
+    weights = np.exp(scores - scores.max(-1, keepdims=True))
+    weights /= weights.sum(-1, keepdims=True)
+    expected = 1.95e-3 * np.sqrt((weights ** 2 @ v32.astype(np.float64) ** 2).sum())
+    assert np.linalg.norm(got.reshape(want.shape) - want) <= expected   # (less for a row's largest probability, which is exact)
+
+
+# The kernel that a call without a causal limit takes is the faster one (figures in attention_tc_plan): shared memory tells which.
+@pytest.mark.parametrize("H,S,streams", [(5, 1900, True), (12, 1900, False), (18, 1900, False), (16, 2048, False), (64, 2048, False),
+                                         (9, 4096, False), (4, 4096, True), (36, 1024, False), (118, 256, False), (74, 256, True),
+                                         (81, 129, False), (150, 200, False), (150, 512, False), (74, 512, False), (40, 300, True),
+                                         (162, 300, True), (49, 640, False), (108, 640, True), (57, 2048, False), (458, 100, True),
+                                         (2, 128, False), (148, 128, False), (281, 128, True), (2, 127, True)])
+def test_attention_bf16_takes_the_faster_kernel(gpu, H, S, streams):
+    fe, ctx, stream = gpu
+    n = H * S * 64
+    q, k, v = (fe.DeviceBuffer.zeroed(stream, n, np.uint16) for _ in range(3))
+    o = fe.DeviceBuffer.zeroed(stream, n, np.float32)
+    used = [fe.prepare(ctx, "flash_attention_v1", q=q, k=k, v=v, output=o, batch=1, heads=H, seq=S, dim=64, scale=0.125, causal=causal,
+                       input_dtype=fe.DTYPE_BF16).geometry.dynamic_shared_bytes for causal in (0, 1)]
+    assert (used[0] == used[1]) == streams   # with a limit it is always streams
 
 
 @pytest.mark.parametrize("S,D,causal", [(333, 128, True), (1025, 72, False), (1900, 128, True), (1900, 48, False), (4096, 128, False)])
