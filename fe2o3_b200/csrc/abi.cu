@@ -753,9 +753,7 @@ int32_t launch_prepared(fe2o3_prepared *p, cudaStream_t s) {
             return gemm_tc_launch(&p->gemm[1], s);
         }
         case OP_MOE_FFN_COMBINE: {
-            const fe2o3_moe_expert_ffn_combine_v1_args *a = reinterpret_cast<const fe2o3_moe_expert_ffn_combine_v1_args *>(p->kernarg);
-            (void)a;   // (the first GEMM clears the output the second one adds into)
-            int32_t st = gemm_tc_launch(&p->gemm[0], s);
+            int32_t st = gemm_tc_launch(&p->gemm[0], s);   // (it clears the output that the second one adds into)
             if (st != FE2O3_OK) return st;
             return gemm_tc_launch(&p->gemm[1], s);
         }

@@ -62,6 +62,7 @@ __device__ __forceinline__ float row_combine(float v, F op, float *slots, uint32
 
 // SHIFTED: rows may start anywhere in a 16-byte vector (same phase for input and output, the mask's
 // 4-byte phase alike); otherwise every row starts on a vector and cols is a multiple of 4.
+#pragma nv_diag_suppress 186   // rows that start on a vector compare with a shift of 0
 template <int LANES, int NV, bool MASKED, bool SHIFTED>
 __global__ void __launch_bounds__(kThreads)
 row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const uint8_t *__restrict__ mask, uint32_t rows,
@@ -188,6 +189,8 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
         }
     }
 }
+
+#pragma nv_diag_default 186
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
