@@ -55,6 +55,32 @@ def test_exact_bf16_gemm_any_exponent_bit_exact(gpu, orc, m, n, k, pad, low, hig
     assert (bits(got) == bits(want))[~np.isnan(want)].all()
 
 
+# bf16 operands, a case for each tile: 16 x 32, 32 x 64 and 64 x 64, with and without old values; rows at odd addresses too
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("rows,cols,m,n,k", [(16, 32, 304, 1008, 112), (32, 64, 512, 2000, 80), (64, 64, 1712, 1504, 48)])
+def test_exact_bf16_gemm_every_tile_bit_exact(gpu, orc, rows, cols, m, n, k, offset):
+    fe, ctx, stream = gpu
+    rng = np.random.default_rng(m + offset)
+    values = lambda count: (rng.normal(0, 1, count).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    a, b, c = values(m * k), values(k * n), rng.normal(0, 1, m * n).astype(np.float32)
+    A, B = (Guarded(fe, stream, np.concatenate([np.zeros(offset, np.uint16), v])) for v in (a, b))
+    for update in (False, True):
+        # an odd size where the shape allows one
+        mm, nn, kk = (m - 1, n - 3, k - 1) if update and offset else (m, n, k)
+        Cb = Guarded(fe, stream, c[:mm * nn])
+        args = dict(schedule=fe.SCHEDULE_EXACT_ORDER, a=A.buf.view(GUARD + offset, mm * kk), b=B.buf.view(GUARD + offset, kk * nn), c=Cb.slice,
+                    m=mm, n=nn, k=kk)
+        if update:
+            prepared = fe.prepare(ctx, "tiled_gemm_general_v1", lda=kk, ldb=nn, ldc=nn, alpha=0.5, beta=-0.25, **args)
+            want = orc.gemm_bf16(mm, nn, kk, a[:mm * kk], b[:kk * nn], lda=kk, ldb=nn, ldc=nn, alpha=0.5, beta=-0.25, c=c[:mm * nn])
+        else:
+            prepared = fe.prepare(ctx, "tiled_gemm_v1", **args)
+            want = orc.gemm_bf16_rows(mm, nn, kk, a, b).ravel()
+        assert prepared.geometry.grid[0] == -(-mm // rows) * -(-nn // cols)
+        prepared.launch_and_wait(stream)
+        assert (bits(Cb.read()) == bits(want.ravel())).all()
+
+
 # more tiles in one direction than a second grid dimension holds (65535)
 @pytest.mark.parametrize("m,n", [(1, 5_000_000), (5_000_000, 1), (2, 65535 * 64 + 1)])
 def test_scalar_gemm_long_results_bit_exact(gpu, m, n):
@@ -144,6 +170,62 @@ def test_gemm_ring_lengths_exact(gpu, m, n, k):
     wide = lambda v: (v.astype(np.uint32) << 16).view(np.float32)
     want = wide(a).reshape(m, k) @ wide(b).reshape(k, ldb)[:, :n]   # dyadic alphabet: every summation order is exact
     assert (Cb.read().reshape(m, n) == want).all()
+
+
+# Every tile shape with an edge inside its last tiles, by the count of its blocks: rows x columns of a tile, and blocks a tile.
+# Pairs of SMs: the last pair's second block has no rows or 42 of them, and no columns or two.
+SHAPES = {64: (128, 64, 1), 128: (128, 128, 1), 192: (128, 192, 1), 256: (128, 256, 1), "pair": (256, 256, 2)}
+
+
+def shape_is(geometry, shape, m, n):
+    rows, cols, blocks = SHAPES[shape]
+    tiles = -(-m // rows) * -(-n // cols)
+    return geometry.grid[0] == blocks * min(tiles, 148 // blocks)
+
+
+def exact_product(a, b, m, n, k, lda, ldb):   # dyadic alphabet: every summation order is exact
+    wide = lambda v: (v.astype(np.uint32) << 16).view(np.float32)
+    full = lambda v, rows, ld: np.concatenate([wide(v), np.zeros(rows * ld - v.size, np.float32)]).reshape(rows, ld)
+    return full(a, m, lda)[:, :k] @ full(b, k, ldb)[:, :n]
+
+
+@pytest.mark.parametrize("pad,offset", [(4, 0), (3, 1)])   # C in vectors, and by elements
+@pytest.mark.parametrize("shape,m,n,k", [(64, 300, 3001, 700), (128, 1281, 1400, 300), (192, 1281, 2300, 300), (256, 1281, 2700, 300),
+                                         ("pair", 1281, 2900, 1500), ("pair", 1281, 2946, 1500), ("pair", 1450, 2946, 1500),
+                                         ("pair", 2200, 2400, 1500)])   # (two rounds)
+def test_gemm_update_every_tile_shape_exact(gpu, shape, m, n, k, pad, offset):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    lda, ldb, ldc = (k + 7) // 8 * 8, (n + 7) // 8 * 8, (n + 3) // 4 * 4 + pad
+    a = synth.gemm_inputs_v1((m - 1) * lda + k, 1, 1, 5)[0]
+    b = synth.gemm_inputs_v1(1, (k - 1) * ldb + n, 1, 6)[1]
+    size = (m - 1) * ldc + n
+    c = synth.uniform_f32(0, 9, size)
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, np.concatenate([np.zeros(offset, np.float32), c]))
+    prepared = fe.prepare(ctx, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_TCGEN05, a=A.slice, b=B.slice, c=Cb.buf.view(GUARD + offset, size),
+                          m=m, n=n, k=k, lda=lda, ldb=ldb, ldc=ldc, alpha=0.5, beta=-0.25)
+    assert shape_is(prepared.geometry, shape, m, n)
+    prepared.launch_and_wait(stream)
+    rows = lambda v: np.concatenate([v, np.zeros(ldc - n, np.float32)]).reshape(m, ldc)
+    got, old = rows(Cb.read()[offset:]), rows(c)
+    want = np.float32(0.5) * exact_product(a, b, m, n, k, lda, ldb) + np.float32(-0.25) * old[:, :n]
+    assert (bits(got[:, :n].ravel()) == bits(want.ravel())).all()
+    assert (bits(got[:, n:].ravel()) == bits(old[:, n:].ravel())).all()
+
+
+@pytest.mark.parametrize("offset", [0, 1])   # C by the copy engine, and by elements
+@pytest.mark.parametrize("shape,m,n,k", [("pair", 1296, 2832, 1504), ("pair", 1296, 2960, 1504), (256, 1296, 2704, 304), (192, 1296, 2320, 304),
+                                         (128, 1296, 1424, 304), (64, 304, 3008, 704)])
+def test_tiled_gemm_v1_every_tile_shape_exact(gpu, shape, m, n, k, offset):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    a, b = synth.gemm_inputs_v1(m * k, 1, 1, 5)[0], synth.gemm_inputs_v1(1, k * n, 1, 6)[1]
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, np.zeros(m * n + offset, np.float32))
+    prepared = fe.prepare(ctx, "tiled_gemm_v1", a=A.slice, b=B.slice, c=Cb.buf.view(GUARD + offset, m * n), m=m, n=n, k=k)
+    assert shape_is(prepared.geometry, shape, m, n)
+    prepared.launch_and_wait(stream)
+    got = Cb.read()
+    assert (got[:offset] == 0).all() and (got[offset:].reshape(m, n) == exact_product(a, b, m, n, k, k, n)).all()
 
 
 @pytest.mark.parametrize("T,d,f,E,cap", [(1000, 1088, 1152, 4, 2000), (1040, 1152, 1088, 4, 500),
@@ -462,11 +544,7 @@ def attention_f64(q, k, v, scale, causal):
 # ---- attention at head size 64: units of two tiles, or of two streams, by the number of units, the length and the limit
 @pytest.mark.parametrize("B,H,S,causal", [(1, 1, 1, False), (1, 2, 128, True), (1, 3, 129, False), (1, 2, 257, True), (1, 1, 640, False),
                                           (1, 147, 200, False), (1, 148, 200, False), (4, 40, 300, False), (4, 40, 300, True),
-                                          (1, 100, 600, False), (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False),
-                                          # two-tile units of which the last few are split into single tiles
-                                          (1, 150, 200, False), (3, 50, 512, False),
-                                          # one whole key block
-                                          (1, 2, 128, False), (1, 100, 128, False)])
+                                          (1, 100, 600, False), (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False)])
 def test_attention_bf16_tiles_and_streams(gpu, B, H, S, causal):
     from fe2o3_b200 import synth
     from test_gpu_parity import attn_run
@@ -479,15 +557,32 @@ def test_attention_bf16_tiles_and_streams(gpu, B, H, S, causal):
     size, _ = attention_f64(q32, k32, np.abs(v32), 1.0 / np.sqrt(D), causal)
     # a probability is cut to eight bits, by less than 2^-7 of itself, and the centring gives back 2^-9
     assert (np.abs(got.reshape(want.shape) - want) <= 2.0 ** -7 * size).all()
-    # ... which leaves 2^-9 - 2^-7 U / m of it, U uniform in [0, 1) and m log-uniform in [1, 2): 1.95e-3 root mean square, 3.3e-3
-    # without the centring.  Independent from key to key, these add up in squares.
-    scores = q32.astype(np.float64) @ k32.astype(np.float64).transpose(0, 2, 1) / np.sqrt(D)
+
+
+# ... and in the 2-norm, where a lost centring would show: the cut leaves 2^-9 - 2^-7 U / m of a probability, U uniform in [0, 1)
+# and m log-uniform in [1, 2): 1.95e-3 root mean square, 3.3e-3 without the centring.  Independent from key to key, these add up
+# in squares.
+@pytest.mark.parametrize("B,H,S,causal", [(1, 1, 1, False), (1, 2, 128, True), (1, 3, 129, False), (1, 2, 257, True), (1, 1, 640, False),
+                                          (1, 148, 200, False), (4, 40, 300, False), (4, 40, 300, True), (1, 100, 600, False),
+                                          (2, 90, 520, True), (1, 320, 100, True), (1, 330, 64, False),
+                                          # two-tile units of which the last few are split into single tiles
+                                          (1, 150, 200, False), (3, 50, 512, False),
+                                          # one whole key block
+                                          (1, 2, 128, False), (1, 100, 128, False)])
+def test_attention_bf16_error_norm(gpu, B, H, S, causal):
+    from fe2o3_b200 import synth
+    from test_gpu_parity import attn_run
+    D = 64
+    q, k, v = (synth.normal_bf16(5, d, B * H * S * D, 1.0).reshape(B, H, S, D) for d in (1, 2, 3))
+    got, _ = attn_run(gpu, q, k, v, 1.0 / np.sqrt(D), causal, gpu[0].DTYPE_BF16)
+    q64, k64, v64 = (synth.bf16_to_f32(x).reshape(B * H, S, D).astype(np.float64) for x in (q, k, v))
+    scores = q64 @ k64.transpose(0, 2, 1) / np.sqrt(D)
     if causal:
         scores[:, np.triu(np.ones((S, S), bool), 1)] = -np.inf
     weights = np.exp(scores - scores.max(-1, keepdims=True))
     weights /= weights.sum(-1, keepdims=True)
-    expected = 1.95e-3 * np.sqrt((weights ** 2 @ v32.astype(np.float64) ** 2).sum())
-    assert np.linalg.norm(got.reshape(want.shape) - want) <= expected   # (less for a row's largest probability, which is exact)
+    expected = 1.95e-3 * np.sqrt((weights ** 2 @ v64 ** 2).sum())
+    assert np.linalg.norm(got.reshape(B * H, S, D) - weights @ v64) <= expected   # (less for a row's largest probability, which is exact)
 
 
 # The kernel that a call without a causal limit takes is the faster one (figures in attention_tc_plan): shared memory tells which.
