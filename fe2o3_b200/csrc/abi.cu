@@ -60,6 +60,7 @@ void attention_split_geometry(const AttnSplitPlan *, fe2o3_geometry *);
 void attention_split_free(AttnSplitPlan *);
 int32_t attention_split_init_device();
 int32_t moe_gate_init_device();
+int32_t gemm_exact_init_device();
 int32_t device_scan_init_device();
 
 // ---- error bookkeeping ---------------------------------------------------------
@@ -849,6 +850,7 @@ int32_t fe2o3_ctx_create(int32_t device, fe2o3_ctx **out) {
     if (init == FE2O3_OK) init = attention_tc_init_device();
     if (init == FE2O3_OK) init = attention_split_init_device();
     if (init == FE2O3_OK) init = moe_gate_init_device();
+    if (init == FE2O3_OK) init = gemm_exact_init_device();
     if (init == FE2O3_OK) init = device_scan_init_device();
     if (init != FE2O3_OK) return init;
     fe2o3_ctx *ctx = new (std::nothrow) fe2o3_ctx();

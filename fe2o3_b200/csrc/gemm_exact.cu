@@ -12,7 +12,7 @@
 //
 // Bound: the f32 pipe, two operations per multiply-add that may not be fused (512^3: 7.5 us on 148 SMs).  A block of 128
 // threads owns 8 RM x 16 RN outputs, RM x RN a thread.
-//   f32: tiles of 32 k go to shared memory by asynchronous copies, a ring of three, one barrier a tile; pieces of four
+//   f32: tiles of 32 k go to shared memory by asynchronous copies, a ring of three (two for 64 rows), one barrier a tile; pieces of four
 // bytes where rows do not start on 16.  Both operands lie as they do in memory: a thread reads four k of each of its
 // rows and four rows of B, 16 bytes each, for RM x RN x 4 products.  Products are scalar, sums packed f32x2 (each half
 // rounded like the scalar instruction; a packed product feeding a packed sum came out fused, with one rounding).
@@ -24,6 +24,8 @@
 // us, alpha/beta, always two steps / so: 2999^3 at odd addresses 2299 / 1445, 300 x 1001 x 501 55 / 33, 100^3 13.0 / 5.3.
 #include "bf16_piece.h"
 #include "common.cuh"
+
+#include <math.h>
 
 namespace {
 
@@ -157,11 +159,13 @@ __device__ __forceinline__ void write_sums(const uint64_t (&acc)[RM][RN / 2], fl
 }
 
 // ---- f32 operands: asynchronous copies
+template <int RM>
+constexpr int kF32Stages = RM == 8 ? 2 : 3;   // (a block's 48 KiB)
 template <int RM, int RN>
 __global__ void __launch_bounds__(kThreads)
 gemm_exact_f32_kernel(const float *__restrict__ A, const float *__restrict__ B, float *C, uint32_t M, uint32_t N, uint32_t K, uint32_t lda,
                       uint32_t ldb, uint32_t ldc, float, float) {
-    constexpr int TM = 8 * RM, TN = 16 * RN, STAGES = 3;
+    constexpr int TM = 8 * RM, TN = 16 * RN, STAGES = kF32Stages<RM>;
     __shared__ ExactTiles<RM, RN, STAGES> tiles;
     const uint32_t tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const uint32_t row_tiles = (M - 1) / TM + 1;
@@ -317,34 +321,66 @@ gemm_exact_bf16_kernel(const uint16_t *__restrict__ A, const uint16_t *__restric
 
 }  // namespace
 
+// Function attributes are per device: called by fe2o3_ctx_create with the context's device current.  What a launch may ask for
+// beside its own shared memory (see launch_gemm_exact): the limit without opt-in, 48 KiB, is for both together.
+int32_t gemm_exact_init_device() {
+    constexpr int kSpreadMax = 64 * 1024;
+    FE2O3_CUDA(cudaFuncSetAttribute(gemm_exact_f32_kernel<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(gemm_exact_f32_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadMax));
+    FE2O3_CUDA(cudaFuncSetAttribute(gemm_exact_f32_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpreadMax));
+    return FE2O3_OK;
+}
+
 // dtype: FE2O3_DTYPE_F32 (without epilogue only) or FE2O3_DTYPE_BF16 inputs.
 int32_t launch_gemm_exact(fe2o3_ctx *ctx, cudaStream_t s, uint32_t dtype, bool epilogue, uint64_t a, uint64_t b, uint64_t c,
                           uint32_t M, uint32_t N, uint32_t K, uint32_t lda, uint32_t ldb, uint32_t ldc, float alpha,
                           float beta, fe2o3_geometry *geo, bool plan_only) {
-    // Tiles.  f32: 16 x 64, two warps a scheduler at 512^3 (32 x 64, one warp: 16.8 us for 15.8; 64 x 64 at 1024^3: 96 for 91),
-    // and 16 x 32 where that leaves every other SM without a block (64 x 64 x 1024: 18.4 for 21.2); copies of four bytes,
-    // where rows do not start on 16, want more work a copy (32 x 64: 700 x 700 x 333 19.3 for 20.5).  bf16, whose staging
-    // costs more: 64 x 64 from four blocks an SM on (2999^3 1445 us for 1672), 32 x 64 from two (500 x 2001 x 77 13.4 for 16.2),
-    // else 16 x 32 (300 x 1001 x 501 33 for 40).
+    // Tiles of f32: 16, 32 or 64 rows by 64 columns, the cheapest by a cost of the launch and, for each k, of the tiles on the SM
+    // that has most, fitted in ns to 56 products of up to 4096 x 4096: the choice is within 5 % of the best.  Larger tiles read
+    // less shared memory a product, smaller ones share the SMs more evenly; a tile alone on an SM waits for itself, and beyond
+    // what the SMs hold at once 16 rows never win.  us, 16 / 32 / 64 rows: 512^3 15.6 / 16.6 / 32, 900 x 900 x 300 25.3 / 23.2 / 30,
+    // 1024^3 90 / 94 / 96, 1200 x 1200 x 512 64 / 58 / 70, 2048 x 2048 x 256 88 / 78 / 77.
+    // Where 16 x 64 leaves every other SM without a block, 16 x 32 (64 x 64 x 1024: 18.4 for 21.2).
+    // bf16, whose staging costs more: 64 x 64 from four blocks an SM on (2999^3 1445 us for 1672), 32 x 64 from two
+    // (500 x 2001 x 77 13.4 for 16.2), else 16 x 32 (300 x 1001 x 501 33 for 40).
     const uint64_t sms = ctx->sm_count > 0 ? ctx->sm_count : 1;
     auto count = [&](uint32_t rows, uint32_t cols) { return (uint64_t)ceil_div_u32(M, rows) * ceil_div_u32(N, cols); };
     const bool f32 = dtype == FE2O3_DTYPE_F32;
-    const bool pieces = ((a | b) & 15u) != 0 || lda % 4 != 0 || ldb % 4 != 0;
-    const uint32_t rows = f32 ? (pieces && count(32, 64) >= sms ? 32 : 16) : count(64, 64) >= 4 * sms ? 64 : count(32, 64) >= 2 * sms ? 32 : 16;
+    uint32_t rows = count(64, 64) >= 4 * sms ? 64 : count(32, 64) >= 2 * sms ? 32 : 16, spread = 0;
+    if (f32) {
+        static const struct { uint32_t rows; double launch, tile, alone; uint32_t held, bytes; } shapes[] = {   // held: blocks that an SM holds
+            {16, 2650, 12.2, 20.1, 7, sizeof(ExactTiles<2, 4, kF32Stages<2>>)},
+            {32, 2700, 22.1, 27.5, 5, sizeof(ExactTiles<4, 4, kF32Stages<4>>)},
+            {64, 4400, 43.2, 55.3, 4, sizeof(ExactTiles<8, 4, kF32Stages<8>>)}};
+        double best = HUGE_VAL;
+        for (const auto &shape : shapes) {
+            const uint64_t tiles = count(shape.rows, 64), most = (tiles + sms - 1) / sms;
+            if (shape.rows == 16 && most > shape.held) continue;
+            const double on_sm = most <= shape.held ? (double)most : (double)tiles / (double)sms;
+            const double cost = shape.launch + K * (most > 1 ? on_sm * shape.tile : shape.alone);
+            if (cost >= best) continue;
+            best = cost;
+            rows = shape.rows;
+            // Launched early, the blocks would pile up on the SMs that the kernel before leaves first, up to as many as these hold,
+            // where two launches do not fit side by side (900 x 900 x 300 back to back, 32 rows: 34.7 us for 23.2): they ask
+            // for so much shared memory that they spread evenly.
+            spread = most <= shape.held && 2 * most > shape.held ? (228u * 1024u / (uint32_t)most - 1024u - shape.bytes) / 128u * 128u : 0u;
+        }
+    }
     const uint32_t cols = (f32 ? rows == 16 && 2 * count(16, 64) <= sms : rows == 16) ? 32 : 64;
     // one flat index, rows first: the second and third grid dimensions end at 65535 tiles, which either a tall or a
     // wide result can have
     const uint64_t tiles = count(rows, cols);
     if (tiles > 0x7fffffffull) { fe2o3_set_error("UnsupportedShape: too many output tiles"); return FE2O3_ERR_UNSUPPORTED_SHAPE; }
     const uint32_t grid = (uint32_t)tiles;
-    if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kThreads, 1, 1}, 0, 1};
+    if (geo) *geo = fe2o3_geometry{{grid, 1, 1}, {kThreads, 1, 1}, spread, 1};
     if (plan_only || M == 0 || N == 0) return FE2O3_OK;
     float *C = reinterpret_cast<float *>(c);
     cudaError_t e;
     if (f32) {
         const float *A = reinterpret_cast<const float *>(a), *B = reinterpret_cast<const float *>(b);
-        auto kernel = cols == 32 ? gemm_exact_f32_kernel<2, 2> : rows == 16 ? gemm_exact_f32_kernel<2, 4> : gemm_exact_f32_kernel<4, 4>;
-        e = fe2o3_launch_early(kernel, grid, kThreads, 0, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
+        auto kernel = cols == 32 ? gemm_exact_f32_kernel<2, 2> : rows == 16 ? gemm_exact_f32_kernel<2, 4> : rows == 32 ? gemm_exact_f32_kernel<4, 4> : gemm_exact_f32_kernel<8, 4>;
+        e = fe2o3_launch_early(kernel, grid, kThreads, spread, s, 1, A, B, C, M, N, K, lda, ldb, ldc, alpha, beta);
     } else {
         const uint16_t *A = reinterpret_cast<const uint16_t *>(a), *B = reinterpret_cast<const uint16_t *>(b);
         auto kernel = epilogue ? (rows == 64   ? gemm_exact_bf16_kernel<8, 4, true>

@@ -55,6 +55,23 @@ def test_exact_bf16_gemm_any_exponent_bit_exact(gpu, orc, m, n, k, pad, low, hig
     assert (bits(got) == bits(want))[~np.isnan(want)].all()
 
 
+# f32 operands: the tile is the one that was measured to be the fastest (launch_gemm_exact), with rows on 16 bytes and not
+@pytest.mark.parametrize("rows,m,n,k", [(16, 301, 1036, 100), (16, 801, 804, 100), (16, 1001, 1001, 65), (32, 768, 768, 64), (32, 900, 900, 36),
+                                        (32, 701, 701, 65), (32, 1201, 1201, 33), (64, 2301, 2300, 252), (64, 2301, 2297, 251)])
+def test_scalar_gemm_takes_the_fastest_tile_bit_exact(gpu, orc, rows, m, n, k):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    a, b = synth.uniform_f32(0, 1, m * k), synth.uniform_f32(0, 2, k * n)
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, np.full(m * n, np.nan, np.float32))
+    prepared = fe.prepare(ctx, "scalar_gemm_v1", a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k)
+    assert prepared.geometry.grid[0] == -(-m // rows) * -(-n // 64)
+    for _ in range(3):   # (the later ones start early)
+        prepared.launch(stream)
+    prepared.launch_and_wait(stream)
+    assert (bits(Cb.read()) == bits(orc.gemm_f32(m, n, k, a, b))).all()
+    A.unchanged(); B.unchanged()
+
+
 # bf16 operands, a case for each tile: 16 x 32, 32 x 64 and 64 x 64, with and without old values; rows at odd addresses too
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("rows,cols,m,n,k", [(16, 32, 304, 1008, 112), (32, 64, 512, 2000, 80), (64, 64, 1712, 1504, 48)])
