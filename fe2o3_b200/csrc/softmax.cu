@@ -87,15 +87,19 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
 
     // No thread has vectors to spare (launch_row_softmax), so only the first and the last ones can straddle an end of the row or
     // lie outside it; shifted rows may end one vector earlier.  (Aligned rows under a mask keep the test at every vector:
-    // without it the compiler takes other registers, and 16384 x 2000 goes from 45.5 to 47.5 us.)
-    auto inside = [](int i) { return SHIFTED ? i > 0 && i < NV - 2 : !MASKED && i < NV - 1; };
+    // without it the compiler takes other registers, and 16384 x 2000 goes from 45.5 to 47.5 us.  So do four shifted ones under a
+    // mask: with one vector of them inside, it makes do with 32 registers, and 5000 x 401 takes 5.77 us for 4.91.)
+    auto inside = [](int i) { return SHIFTED ? !(MASKED && NV == 4) && i > 0 && i < NV - 2 : !MASKED && i < NV - 1; };
+    // One vector a thread without a mask has the ends of the row in every thread: tests there are cheaper than fillers put right
+    // (60000 x 101 13.2 / 13.7 us; under a mask 16.2 / 15.2).
+    constexpr bool kZeros = SHIFTED && (MASKED || NV > 1);   // what lies outside the row is filled with zeros, else with -inf
     float4 v[NV];
     float poison = 0.f;   // NaN once an input was not finite
     bool ok = true;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const uint32_t e = (i * LANES + lane) * 4;
-        v[i] = SHIFTED ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        v[i] = kZeros ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
         const bool whole = inside(i) || (SHIFTED ? e >= shift && e + 4 <= end : e < end);
         if (whole) {
             v[i] = __ldcs(reinterpret_cast<const float4 *>(src + e));
@@ -126,7 +130,7 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         const uint32_t e = (i * LANES + lane) * 4;
-        if (SHIFTED) {   // what lies outside the row was filled with zeros
+        if (kZeros) {
             poison = fmaf(v[i].x, 0.f, fmaf(v[i].y, 0.f, fmaf(v[i].z, 0.f, fmaf(v[i].w, 0.f, poison))));
             const bool whole = inside(i) || (e >= shift && e + 4 <= end);
             if (!MASKED && !whole) {   // (the mask's words hold zeros there)
@@ -135,6 +139,9 @@ row_softmax_kernel(const float *__restrict__ in, float *__restrict__ out, const 
                 if (e + 2 < shift || e + 2 >= end) v[i].z = -INFINITY;
                 if (e + 3 < shift || e + 3 >= end) v[i].w = -INFINITY;
             }
+        } else if (SHIFTED) {   // the filler outside the row is not an input
+            ok = ok && (e + 0 < shift || e + 0 >= end || isfinite(v[i].x)) && (e + 1 < shift || e + 1 >= end || isfinite(v[i].y)) &&
+                 (e + 2 < shift || e + 2 >= end || isfinite(v[i].z)) && (e + 3 >= end || isfinite(v[i].w));
         } else {
             ok = ok && (inside(i) || e < end ? finite4(v[i]) : true);
         }
