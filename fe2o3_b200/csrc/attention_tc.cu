@@ -98,14 +98,16 @@ __device__ __forceinline__ bool unit_at(const AttnParams &p, uint32_t i, Unit &u
     const uint32_t idx = blockIdx.x + i * gridDim.x;
     uint32_t block, sub;
     if (idx < p.n_full) {
-        block = idx; sub = 0; u.nt = QT;
+        block = idx; sub = 0;
     } else if (idx - p.n_full < p.n_half) {
-        block = p.n_full + ((idx - p.n_full) >> 1); sub = (idx - p.n_full) & 1; u.nt = 1;
+        block = p.n_full + ((idx - p.n_full) >> 1); sub = (idx - p.n_full) & 1;
     } else {
         return false;
     }
     u.head = block / p.q_blocks;
     u.q0 = block % p.q_blocks * (QT * BQ) + sub * BQ;
+    // a head's last 256-row block may end in its first tile: the second one is left out (heads of 128 rows: 5.9 -> 5.2 us)
+    u.nt = idx < p.n_full && u.q0 + BQ < p.seq ? QT : 1;
     u.nkv = u.q0 < p.seq ? (p.seq + BKV - 1) / BKV : 0;
     return true;
 }
