@@ -1168,8 +1168,8 @@ int32_t launch_moe_gate(fe2o3_ctx *ctx, cudaStream_t s, const void *args, fe2o3_
             const uint32_t chain_grid = ceil_div_u32(a->tokens, 32 / E);
             // Up to one block an SM the products come from warps of their own; beyond, the blocks of an SM share its shared memory
             // and the issue slots (d 2048, 8 experts, one warp / products, us: 64 tokens 10.3 / 7.1, 590 tokens 10.5 / 7.2; an earlier
-            // form of it at 1024 10.6 / 10.5, at 4096 20.8 / 28.4)
-            const bool fed = chain_grid <= (uint32_t)ctx->sm_count;
+            // form of it at 1024 10.6 / 10.5, at 4096 20.8 / 28.4).  At 64 k there is nothing to be ahead of (300 tokens 1.44 / 1.52, one token of 4 experts 1.21 / 1.32).
+            const bool fed = chain_grid <= (uint32_t)ctx->sm_count && a->d_model > 64u;
             if (fed) one_chain = E == 4 ? moe_gate_fed_kernel<4> : E == 8 ? moe_gate_fed_kernel<8> : moe_gate_fed_kernel<16>;
             const uint32_t threads = fed ? 192u : 32u;
 #define FE2O3_GATE_LANES(EE, g) launch_gate_lanes<EE, 4, 8, 6>(s, x, wg, lg, a->tokens, a->d_model, g)
