@@ -50,8 +50,9 @@
 //   computed by the CUDA-core recurrence (attention_row.cuh).
 //   The other warps may wait long meanwhile, so waits that run out start over as long as
 //   rows are being settled (Waits).
-// Two tiles a unit / so, us: B2 H12 S1900 D128 causal 80.5 / 56.7, not causal 156 / 98; B1 H1 S4096 113 / 66; B8 H8 S256 16.3 / 11.8;
-// B4 H16 S2048 D32 262 / 228.  On the CUDA cores the first takes 8017.
+// Two tiles a unit / so, us, the same inputs again and again: B2 H12 S1900 D128 causal 79.8 / 56.0 (with others each time
+// 83.7 / 63.2), not causal 156 / 97; B1 H1 S4096 D128 111 / 63; B8 H8 S256 D128 15.7 / 11.3; B4 H16 S2048 D32 262 / 223.  On the CUDA
+// cores the first takes 8017.
 // The rule in front (attention_split_supported) is what the copy engine can address:
 // rows of whole 16 bytes and 16-byte aligned bases; the rest, f32 inputs and head sizes
 // above 128 stay on the CUDA cores.  All waits are bounded.
@@ -80,7 +81,7 @@ struct Layout {
     static constexpr uint32_t kOffK = kQTile;
     static constexpr uint32_t kOffV = kOffK + KV_STAGES * kKvTile;
     static constexpr uint32_t kOffP = kOffV + KV_STAGES * kKvTile;
-    static constexpr uint32_t kOffMerge = kOffP + STREAMS * kPTile;        // a unit's output: [stream][32 rows][32 columns][32 rows][128 bytes]
+    static constexpr uint32_t kOffMerge = kOffP + STREAMS * kPTile;        // a unit's output: [stream][4 warps][NG x 32 columns][32 rows][128 bytes]
     static constexpr uint32_t kOffRow = kOffMerge + NG * 64 * BQ * 4;      // reference and sum of each row, a stream
     static constexpr uint32_t kOffBar = kOffRow + STREAMS * 2 * BQ * 4;
     static constexpr uint32_t kTotal = kOffBar + 256;

@@ -38,7 +38,7 @@ constexpr uint32_t kTileBytes = 128 * D * 2;     // 16 KiB: a 128 x 64 bf16 tile
 constexpr uint32_t kOffQ = 0;
 constexpr uint32_t kOffK = kOffQ + Q_STAGES * kTileBytes;
 constexpr uint32_t kOffV = kOffK + KV_STAGES * kTileBytes;
-constexpr uint32_t kOffMerge = kOffV + KV_STAGES * kTileBytes;       // a unit's output: [32 rows][32 columns][32 rows][128 bytes]
+constexpr uint32_t kOffMerge = kOffV + KV_STAGES * kTileBytes;       // a unit's output: [4 warps][2 x 32 columns][32 rows][128 bytes]
 constexpr uint32_t kOffRow = kOffMerge + BQ * D * 4;                   // reference and sum of each row in stream 0
 constexpr uint32_t kOffBar = kOffRow + 2 * BQ * 4;
 constexpr uint32_t kSmemTotal = kOffBar + 512 + 1024;   // + alignment slack

@@ -190,10 +190,10 @@ __device__ __forceinline__ uint32_t cvt_bf16x2(float lo, float hi) {
 
 // GELU(x) = x * (1 + erf(x / sqrt 2)) / 2 = max(x, 0) - |x| * Q(|x|), where Q(u) = erfc(u / sqrt 2) / 2 is the upper tail
 // of the normal distribution.  log2 Q is smooth: a polynomial of degree 6 (fitted here by linear programming, the
-// weighted error of u * Q(u) at most 8.3e-8 on [0, 5.5]) and one exp2 give it, so a pair of values costs nine packed f32
+// error of u * Q(u) with these coefficients at most 8.7e-8) and one exp2 give it, so a pair of values costs nine packed f32
 // operations and two of the special function unit, which together bound the epilogue (Abramowitz & Stegun 7.1.26, used
 // before, costs twelve and four; its error is 2.1e-7).  64 tokens of d 2048: the tail of the first GEMM 8 -> 4.7 us, the
-// layer 77.5 -> 73.6.  Beyond |x| = 10 the tail is below 2^-79 either way, and the clamp
+// layer 77.5 -> 73.6.  At |x| = 10 the tail is below 2^-75 either way, and the clamp
 // keeps the polynomial where it falls.
 //   Four pairs go side by side: one after the other, the chain of dependent operations of each would set the pace.
 template <int N>
@@ -229,7 +229,8 @@ __device__ __forceinline__ void gelu_pairs(const uint32_t *x, uint32_t *out) {  
 
 // One 32 x 32 chunk of f32 output out of a warp's swizzled slice into C, VEC elements per access: 32 / VEC lanes
 // cover a row's 128 bytes, so an instruction touches VEC whole row segments.  With one lane per row (each lane
-// walking its own row) the alpha/beta form cost 32 sectors per 4-byte access: 1000 x 3001 x 1111 took 98.8 us, 22.5 so.
+// walking its own row) the alpha/beta form cost 32 sectors per 4-byte access: 1000 x 3001 x 1111 took 98.8 us
+// for 22.5 (with 128 columns a tile; 16.5 now).
 // `old` holds the chunk's old values for alpha/beta, from fetch_chunk with the same lane layout.
 template <int VEC>
 __device__ __forceinline__ void fetch_chunk(float (&old)[32], const float *chunk, uint32_t ldc, uint32_t rows, uint32_t cols, uint32_t lane) {
@@ -633,8 +634,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // Eight warps: two per TMEM lane quadrant, each taking half of the tile's columns.  A warp
         // turns 128 bytes of each of its 32 rows at a time (32 f32 or 64 bf16 columns) into a
         // 128-byte-swizzled 4 KiB slice of shared memory and hands it to the copy engine, so the
-        // global writes are full lines and do not hold the warp; ragged rows, the alpha/beta form and
-        // outputs the copy engine cannot address are written by the threads directly.
+        // global writes are full lines and do not hold the warp; ragged rows and outputs the copy engine cannot
+        // address are written by the threads directly, and so is the alpha/beta form, in a branch of its own.
         const uint32_t ew = warp - 2;
         const uint32_t quad = warp & 3;  // TMEM lane quadrant this warp may read
         const uint32_t col_half = ew >> 2;
@@ -857,9 +858,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                         store_pending = true;
                     } else {
-                        // Rows the copy engine cannot take (a ragged group's last rows, C it cannot address, the
-                        // alpha/beta form): the chunk goes through the warp's slice of shared memory so that every
-                        // access to C is a run of whole row segments.
+                        // Rows the copy engine cannot take (a ragged group's last rows, C it cannot address): the chunk
+                        // goes through the warp's slice of shared memory so that every access to C is a run of whole
+                        // row segments.
                         if (store_pending) {
                             if (lane == 0) tma_store_wait_read();
                             store_pending = false;
@@ -1006,8 +1007,9 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
         // the output of a round the next one does not hide (alpha/beta reads C too).  Fitted to 90 products of up to
         // 8192 x 8192 x 8192, all five shapes each: the choice is within 0.1 % of the best on average, 1.5 % at worst.  A narrow
         // tile has the shortest launch and the dearest multiply-add, a pair of SMs the opposite: it stages a third less.
-        // us: 512^3 64 columns 5.2, 128 6.4, 192 7.5, 256 7.9, pair 9.2; 1000 x 3001 x 1111 alpha/beta 19.8, 19.1, 13.8, 16.5, 16.9;
-        // 3072 x 3072 x 1024 32.3, 24.8, 25.6, 21.3, 19.5.
+        // us, the same operands again and again, 64 / 128 / 192 / 256 columns / pair: 512^3 4.8 / 5.8 / 6.8 / 7.6 / 8.4; 1000 x 3001 x
+        // 1111 alpha/beta, C's pitch 3004, 22.4 / 22.2 / 16.5 / 20.1 / 18.4 (pitch 3001: 22.6 / 23.5 / 18.8 / 22.8 / 20.8);
+        // 3072 x 3072 x 1024 31.0 / 22.9 / 22.9 / 19.0 / 18.5.
         static const struct { uint32_t bn, pair, launch, k_block, output; } shapes[] = {   // ns
             {64, 0, 4380, 195, 1080}, {128, 0, 4800, 258, 1650}, {192, 0, 5440, 320, 2500}, {256, 0, 5200, 380, 3460}, {256, 1, 6900, 277, 3630}};
         uint64_t best = ~0ull;
