@@ -24,7 +24,7 @@
 // 65536 x 1024: 91.6 us -> 79.5 us (6.75 TB/s) against the earlier form that kept
 // activity bits per element; 5000 x 3001 masked: 79.9 -> 29.3 us against one block
 // per row with scalar accesses, four block barriers and a division per element, and
-// -> 25.6 (5.3 TB/s) with six vectors a thread instead of eight (26.1) and the tests for
+// -> 24.9 (5.4 TB/s) with six vectors a thread instead of eight (25.5) and the tests for
 // the row's ends and for finite inputs only where they are needed; 8000 x 2560 28.3 -> 25.5,
 // 20000 x 701 22.6 -> 19.4.  Two warps a row of 3001 with twelve vectors a thread take 26.9,
 // one with 24 takes 39.
