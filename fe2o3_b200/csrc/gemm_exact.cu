@@ -109,8 +109,15 @@ __device__ __forceinline__ void multiply_tile(uint64_t (&acc)[RM][RN / 2], const
             four_steps<RM, RN, FUSED>(acc, o);
         }
     } else {   // the recurrence stops at K: the padding of the last tile is never multiplied
+        uint32_t kk = 0;
 #pragma unroll 1
-        for (uint32_t kk = 0; kk < steps; ++kk) {
+        for (; kk + 4 <= steps; kk += 4) {
+            Operands<RM, RN> o;
+            o.load(as, bs, row, col, kk);
+            four_steps<RM, RN, FUSED>(acc, o);
+        }
+#pragma unroll 1
+        for (; kk < steps; ++kk) {
             float a[RM], b[RN];
 #pragma unroll
             for (int i = 0; i < RM; ++i) a[i] = as[row + i][kk];
@@ -125,35 +132,44 @@ template <int RM, int RN, bool EPILOGUE>
 __device__ __forceinline__ void write_sums(const uint64_t (&acc)[RM][RN / 2], float *C, uint32_t row0, uint32_t c0, uint32_t M, uint32_t N,
                                            uint32_t ldc, float alpha, float beta) {
     const bool vec = ldc % RN == 0 && reinterpret_cast<uintptr_t>(C) % (4 * RN) == 0 && c0 + RN <= N;
+    // all old values are asked for before the first sum is written, for a load may not overtake a store to C
+    float old[RM][RN];
+    if constexpr (EPILOGUE) {
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+            const float *src = C + (uint64_t)(row0 + i) * ldc + c0;
+            if (row0 + i < M && vec) {
+                if constexpr (RN == 4) {
+                    const float4 x = *reinterpret_cast<const float4 *>(src);
+                    old[i][0] = x.x; old[i][1] = x.y; old[i][2] = x.z; old[i][3] = x.w;
+                } else {
+                    const float2 x = *reinterpret_cast<const float2 *>(src);
+                    old[i][0] = x.x; old[i][1] = x.y;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < RN; ++j) old[i][j] = row0 + i < M && c0 + j < N ? src[j] : 0.0f;
+            }
+        }
+    }
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
-        const uint32_t r = row0 + i;
-        if (r >= M) continue;
+        if (row0 + i >= M) continue;
         float v[RN];
 #pragma unroll
         for (int j = 0; j < RN / 2; ++j) unpack_f32x2(acc[i][j], v[2 * j], v[2 * j + 1]);
-        float *dst = C + (uint64_t)r * ldc + c0;
-        if (vec) {
-            if constexpr (EPILOGUE) {
-                float o[RN];
-                if constexpr (RN == 4) {
-                    const float4 old = *reinterpret_cast<const float4 *>(dst);
-                    o[0] = old.x; o[1] = old.y; o[2] = old.z; o[3] = old.w;
-                } else {
-                    const float2 old = *reinterpret_cast<const float2 *>(dst);
-                    o[0] = old.x; o[1] = old.y;
-                }
+        if constexpr (EPILOGUE) {
 #pragma unroll
-                for (int j = 0; j < RN; ++j) v[j] = __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, o[j]));
-            }
+            for (int j = 0; j < RN; ++j) v[j] = __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, old[i][j]));
+        }
+        float *dst = C + (uint64_t)(row0 + i) * ldc + c0;
+        if (vec) {
             if constexpr (RN == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
             else *reinterpret_cast<float2 *>(dst) = make_float2(v[0], v[1]);
-            continue;
-        }
+        } else {
 #pragma unroll
-        for (int j = 0; j < RN; ++j) {
-            if (c0 + j >= N) continue;
-            dst[j] = EPILOGUE ? __fadd_rn(__fmul_rn(alpha, v[j]), __fmul_rn(beta, dst[j])) : v[j];
+            for (int j = 0; j < RN; ++j)
+                if (c0 + j < N) dst[j] = v[j];
         }
     }
 }
