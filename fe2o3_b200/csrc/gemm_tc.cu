@@ -1021,6 +1021,9 @@ int32_t gemm_tc_plan(fe2o3_ctx *ctx, GemmTcPlan *plan, uint64_t a, uint64_t b, u
             const uint64_t cost = shape.launch + rounds * product + (output > product && rounds > 1 ? (rounds - 1) * (output - product) : 0);
             if (cost < best) { best = cost; plan->bn = shape.bn; plan->pair = shape.pair; }
         }
+        // Few rows: copies of A hold 32 or 64.  What a copy fills in beyond the last row delays the blocks that want the same few
+        // rows of A (us, 128 / 32 or 64 rows a copy: 8 x 3707 x 2317 16.2 / 10.1, 16 x 5120 x 2304 17.0 / 9.3, 48 x 3707 x 2317 10.6 / 10.2).
+        if (!plan->pair) a_box = M <= 32 ? 32 : M <= 64 ? 64 : BM;
     } else if (!ep) {
         // Groups: rounds of tiles times what a round takes, as 0.55 : 0.68 : 1 for 64, 128 and 256 columns; a group ends in
         // a partly filled tile, half of one on average.  256-row tiles on pairs of SMs shorten a round by about a tenth where

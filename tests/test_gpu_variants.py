@@ -230,9 +230,30 @@ def test_gemm_update_every_tile_shape_exact(gpu, shape, m, n, k, pad, offset):
     assert (bits(got[:, n:].ravel()) == bits(old[:, n:].ravel())).all()
 
 
+# few rows: copies of A of 32, 64 and 128 rows, most of them past the last one
+@pytest.mark.parametrize("m", [1, 8, 31, 32, 33, 64, 65])
+@pytest.mark.parametrize("n,k,pad", [(130, 40, 3), (1000, 1100, 4), (9473, 200, 0)])
+def test_gemm_few_rows_exact(gpu, m, n, k, pad):
+    fe, ctx, stream = gpu
+    from fe2o3_b200 import synth
+    lda, ldb, ldc = (k + 7) // 8 * 8, (n + 7) // 8 * 8, n + pad
+    a = synth.gemm_inputs_v1((m - 1) * lda + k, 1, 1, 5)[0]
+    b = synth.gemm_inputs_v1(1, (k - 1) * ldb + n, 1, 6)[1]
+    c = synth.uniform_f32(0, 9, (m - 1) * ldc + n)
+    A, B, Cb = Guarded(fe, stream, a), Guarded(fe, stream, b), Guarded(fe, stream, c)
+    run(fe, ctx, stream, "tiled_gemm_general_v1", schedule=fe.SCHEDULE_TCGEN05, a=A.slice, b=B.slice, c=Cb.slice, m=m, n=n, k=k, lda=lda, ldb=ldb,
+        ldc=ldc, alpha=0.5, beta=-0.25)
+    rows = lambda v: np.concatenate([v, np.zeros(pad, np.float32)]).reshape(m, ldc)
+    got, old = rows(Cb.read()), rows(c)
+    want = np.float32(0.5) * exact_product(a, b, m, n, k, lda, ldb) + np.float32(-0.25) * old[:, :n]
+    assert (bits(got[:, :n].ravel()) == bits(want.ravel())).all()
+    assert (bits(got[:, n:].ravel()) == bits(old[:, n:].ravel())).all()
+
+
 @pytest.mark.parametrize("offset", [0, 1])   # C by the copy engine, and by elements
 @pytest.mark.parametrize("shape,m,n,k", [("pair", 1296, 2832, 1504), ("pair", 1296, 2960, 1504), (256, 1296, 2704, 304), (192, 1296, 2320, 304),
-                                         (128, 1296, 1424, 304), (64, 304, 3008, 704)])
+                                         (128, 1296, 1424, 304), (64, 304, 3008, 704), (64, 16, 3008, 704),
+                                         (64, 48, 3008, 704)])
 def test_tiled_gemm_v1_every_tile_shape_exact(gpu, shape, m, n, k, offset):
     fe, ctx, stream = gpu
     from fe2o3_b200 import synth
