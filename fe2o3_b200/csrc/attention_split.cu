@@ -121,11 +121,6 @@ __device__ __forceinline__ bool unit_at(const SplitParams &p, uint32_t i, Unit &
 // Key blocks whose P*V starts a new sum in tensor memory; the sum before is added to the row's registers.
 __device__ __forceinline__ bool starts_group(uint32_t j) { return (j & (j < 2 ? 0u : j < 8 ? 1u : 3u)) == 0; }
 
-template <int N>
-__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 __device__ __forceinline__ uint64_t sub_f32x2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

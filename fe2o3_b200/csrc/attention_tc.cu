@@ -140,12 +140,6 @@ __device__ __forceinline__ void attn_stamp_cta(uint32_t slot) {
 #define ATTN_STAMP_CTA(cond, slot) do { } while (0)
 #endif
 
-// Register re-balance between warpgroups (all four warps of a warpgroup execute it).
-template <int N>
-__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, AttnParams p) {

@@ -83,12 +83,6 @@ __device__ __forceinline__ bool wait(uint64_t *bar, uint32_t parity) {
     return true;
 }
 
-// Register re-balance between warpgroups (all four warps of a warpgroup execute it).
-template <int N>
-__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 __global__ void __launch_bounds__(kThreads, 1)
 attention_streams_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, AttnParams p) {

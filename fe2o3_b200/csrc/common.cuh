@@ -266,6 +266,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, c
     }
     return __all_sync(0xffffffffu, done) != 0;
 }
+// Register re-balance between warpgroups (all four warps of a warpgroup execute it).
+template <int N>
+__device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 // How many of the next `limit` stages of a ring of S, from `stage` on, have completed the phase awaited: one look of the
 // whole warp, a lane to a stage.  A role that waits, issues and steps on stage by stage is held up by the latency of each
 // look, vote and election (some 200 to 400 cycles a stage together); one look lets it issue for all stages that are ready.
