@@ -110,11 +110,13 @@ __device__ __forceinline__ void multiply_tile(uint64_t (&acc)[RM][RN / 2], const
         }
     } else {   // the recurrence stops at K: the padding of the last tile is never multiplied
         uint32_t kk = 0;
+        if constexpr (RM > 2) {   // (two rows a thread lose 2 % of their whole tiles to it: other registers)
 #pragma unroll 1
-        for (; kk + 4 <= steps; kk += 4) {
-            Operands<RM, RN> o;
-            o.load(as, bs, row, col, kk);
-            four_steps<RM, RN, FUSED>(acc, o);
+            for (; kk + 4 <= steps; kk += 4) {
+                Operands<RM, RN> o;
+                o.load(as, bs, row, col, kk);
+                four_steps<RM, RN, FUSED>(acc, o);
+            }
         }
 #pragma unroll 1
         for (; kk < steps; ++kk) {
