@@ -603,20 +603,23 @@ int32_t attention_tc_plan(fe2o3_ctx *ctx, const fe2o3_flash_attention_v1_args *a
     plan->grid = grid;
     // Tiles or streams: with a causal limit always streams, for tiles are not dealt out by length; without one the cheaper by a
     // cost of the launch and, on the SM that has most, of each unit and its key blocks.  Fitted in ns to 308 calls of 1 to
-    // 4096 keys, both kernels each: the choice is within 0.1 % of the better one on average, 6 % at worst.
+    // 4096 keys, both kernels each: the choice is within 0.6 % of the better one on average.
     // A stream unit is half of a two-tile unit and takes more than half of its time, so tiles win where the rounds come out
     // even and streams where tiles would leave SMs idle.  One key block a head is all beginning and end, of which a
     // tile has less; masked keys cost it more, so that streams are ahead again from some hundred heads on.
     // us, tiles / streams: B1 H16 S2048 29.8 / 33.7, B4 H16 S2048 105.6 / 110.5, 118 heads of 256 keys 8.6 / 10.4,
     // 18 heads of 1900 26.7 / 32.5, 5 of them 25.9 / 17.1, 162 heads of 257 23.0 / 20.3, 12 heads of 127 5.7 / 6.2,
     // 118 of them 6.9 / 6.7.
+    // The kernels round P differently (within the same error), so a call that fills the SMs with two-tile units is not moved for less
+    // than 8 % of the steps of its longest SM, in quarters of a step of two blocks.
     const uint64_t blocks = tiles;   // key blocks of 128
     const uint64_t full = (units - (split ? rem : 0)) / grid + (!split && rem != 0), rounds = ((uint64_t)bh * tiles + sms - 1) / sms;
     const uint64_t tile_cost = 2390 + full * (3290 + 1520 * blocks) + (split ? 1190 + 1110 * blocks : 0);
     const uint64_t stream_cost = 3480 + rounds * (2170 + 860 * blocks);
     const bool one_block = blocks == 1 && (a->seq == BKV ? units <= 2 * sms : 3 * units <= 2 * sms);
+    const bool fewer_steps = units < sms || 25 * (4 * full + (split ? 3 : 0)) * blocks > 27 * 4 * rounds * ((blocks + 1) / 2);
     plan->causal = a->causal;
-    plan->streams = a->causal || (stream_cost < tile_cost && !one_block);
+    plan->streams = a->causal || (fewer_steps && stream_cost < tile_cost && !one_block);
     if (plan->streams) plan->grid = (uint64_t)bh * tiles < sms ? bh * tiles : sms;
     *out = plan;
     return FE2O3_OK;

@@ -627,9 +627,9 @@ def test_attention_bf16_error_norm(gpu, B, H, S, causal):
 @pytest.mark.parametrize("H,S,streams", [(5, 1900, True), (12, 1900, False), (18, 1900, False), (16, 2048, False), (64, 2048, False),
                                          (9, 4096, False), (4, 4096, True), (36, 1024, False), (118, 256, False), (74, 256, True),
                                          (81, 129, False), (150, 200, False), (150, 512, False), (74, 512, False), (40, 300, True),
-                                         (162, 300, True), (49, 640, False), (108, 640, True), (57, 2048, False), (458, 100, True),
-                                         (2, 128, False), (148, 128, False), (281, 128, False), (330, 128, True), (2, 127, False), (1, 1, False),
-                                         (148, 100, True)])
+                                         (162, 300, False), (49, 640, False), (108, 640, True), (57, 2048, False), (458, 100, False),
+                                         (2, 128, False), (148, 128, False), (281, 128, False), (330, 128, False), (2, 127, False), (1, 1, False),
+                                         (100, 100, True), (148, 100, False)])
 def test_attention_bf16_takes_the_faster_kernel(gpu, H, S, streams):
     fe, ctx, stream = gpu
     n = H * S * 64
